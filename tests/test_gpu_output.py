@@ -61,6 +61,54 @@ def test_output_moments_and_particles_match_the_oracle(torch_cuda, precision):
     ctx.close()
 
 
+@pytest.mark.parametrize("count", [1, 31, 33, 700, 20000])
+@pytest.mark.parametrize("order", ["sorted", "shuffled"])
+@pytest.mark.parametrize("wanted", ["rho", "rho+j", "j+p"])
+def test_output_moments_over_record_orders_and_counts(torch_cuda, count, order, wanted):
+    """Chunks of 32 records and their remainders, several cells in a chunk and several chunks in a
+    cell, any record order, one-cell axes, each subset of the outputs; invalid and nonfinite records
+    add nothing anywhere and are counted. Sums of m terms of one cell: m eps of the terms' sum."""
+    import torch
+    from gpu_helpers import StageContext
+    from tpic_b200 import _lib
+    from tpic_b200.plasma import GridSpec
+    g = GridSpec(5, 3, 1, 2.0, 1.5, 0.5)
+    rng = np.random.default_rng(count)
+    c = [rng.integers(0, m, count) for m in (g.nx, g.ny, g.nz)]
+    key = g.encode(*c).astype(np.int32)
+    if order == "sorted":
+        key = np.sort(key)
+    d = {k: rng.random(count) for k in ("rx", "ry", "rz")}
+    d.update({k: rng.normal(size=count) for k in ("u", "v", "w")}, q=rng.random(count), cell=key)
+    good = np.ones(count, bool)
+    if count > 40:
+        bad = {3: ("rx", 1.5), 8: ("q", np.nan), 9: ("cell", -1), 34: ("rz", -0.25), 35: ("q", np.inf)}
+        if wanted != "rho":
+            bad[36] = ("u", np.nan)
+        for at, (k, value) in bad.items():
+            d[k][at] = value
+            good[at] = False
+    ctx = StageContext(g)
+    parts = ctx.upload_particles(d)
+    p = ctx.struct(parts, count)
+    sizes = {"rho": 1, "j": 3, "p": 6}
+    unique = g.nx * g.ny * g.nz
+    out = {k: torch.zeros(m * unique, dtype=torch.float64, device="cuda") for k, m in sizes.items()
+           if k in wanted.split("+")}
+    ptr = [out[k].data_ptr() if k in out else 0 for k in sizes]
+    _lib.check(ctx.lib.tpicb200_output_moments(ctx.ctx, 2.0, C.byref(p), *ptr, ctx.stream))
+    invalid = C.c_uint32()
+    _lib.check(ctx.lib.tpicb200_read_invalid(ctx.ctx, C.byref(invalid), 1, ctx.stream))
+    assert invalid.value == np.count_nonzero(~good)
+    kept = {k: v[good] for k, v in d.items()}
+    size = {k: np.abs(v) if k != "cell" else v for k, v in kept.items()}
+    for k, want, terms in zip(sizes, O.output_moments(g, kept, 2.0), O.output_moments(g, size, 2.0)):
+        if k in out:
+            got = out[k].cpu().numpy().reshape(want.shape)
+            assert np.abs(got - want).max() <= 4 * count * 2.0**-53 * terms.max(), k
+    ctx.close()
+
+
 def test_runner_writes_snapshots(torch_cuda, tmp_path):
     """A shrunk two-stream deck for 2 cycles with fields every cycle and
     particles every 2: E, B, rho and J files at cycles 0, 1, 2 and particle

@@ -13,12 +13,14 @@
 //
 // The transpose of a gather at the particle positions is a scatter, so the
 // backward of the mover scatters into E_theta and B, and the backward of the
-// deposition gathers the gradient fields at the particles. Each thread takes
-// one record; a warp's lanes reduce their corner contributions over runs of
-// equal cell keys (the records are sorted by cell) before one lane per run
-// adds them into the unique nodes with FP64 atomics. Adjoint arithmetic is
+// deposition gathers the gradient fields at the particles. Each lane takes
+// one record; the corner contributions of a warp's records are summed per
+// cell on the FP64 tensor cores (corner_sums.cuh; the records are sorted by
+// cell) before they are added into the unique nodes with FP64 atomics.
+// Adjoint arithmetic is
 // FP64 in both precision modes (the forward values are read in their stored
 // types). Particle adjoints are indexed by record id.
+#include "corner_sums.cuh"
 #include "kernels.cuh"
 #include "stencils.cuh"
 
@@ -28,7 +30,8 @@ namespace tpicb200 {
 namespace {
 
 constexpr int kAdjointThreads = 256;
-constexpr unsigned kFull = 0xffffffffu;
+constexpr int kRecordThreads = 128;
+constexpr int kRecordBlocks = 3;  // per SM: 168 registers a thread
 
 struct AdjointConstants {
   double beta, boc, dt, inv[3], inv_volume;
@@ -63,61 +66,58 @@ struct AdjointRecords {
   double* qbar;  // [nid]
 };
 
-// A record's cell and CIC factors. Corner a of the cell has offset
-// (a&1, a>>1&1, a>>2&1); its node in a consistent field (duplicates hold the
-// unique values) and the unique node it scatters into are formed on the fly.
+// A record's cell and CIC factors. The corner nodes are base + {0, 1} +
+// {0, NX} + {0, NX*NY} in a consistent field (duplicates hold the unique values).
 struct Loaded {
   bool ok;
   int32_t key;
   long long pid;
-  int i, j, k;
   long long base;           // node (i, j, k)
   double X[2], Y[2], Z[2];  // per-axis CIC factors (1 - f, f)
   double v[3];
-  __device__ __forceinline__ long long node(const Geom& g, int a) const {
-    return base + (a & 1) + (long long)g.NX * (((a >> 1) & 1) + (long long)g.NY * ((a >> 2) & 1));
-  }
-  __device__ __forceinline__ long long unique(const Geom& g, int a) const {
-    const int ci = i + (a & 1), cj = j + ((a >> 1) & 1), ck = k + ((a >> 2) & 1);
-    return g.node(ci == g.nx ? 0 : ci, cj == g.ny ? 0 : cj, ck == g.nz ? 0 : ck);
-  }
-  // The (wx*wy)*wz grouping of cic_weights.
-  __device__ __forceinline__ double weight(int a) const { return X[a & 1] * Y[(a >> 1) & 1] * Z[(a >> 2) & 1]; }
-  __device__ __forceinline__ void weight_gradient(int a, double d[3]) const {
-    const int bx = a & 1, by = (a >> 1) & 1, bz = (a >> 2) & 1;
-    d[0] = (bx ? 1.0 : -1.0) * Y[by] * Z[bz];
-    d[1] = X[bx] * (by ? 1.0 : -1.0) * Z[bz];
-    d[2] = X[bx] * Y[by] * (bz ? 1.0 : -1.0);
-  }
 };
 
-template <class F>
-__device__ __forceinline__ void gather3(const Geom& g, const F* __restrict__ f, const Loaded& L, double out[3]) {
-  out[0] = out[1] = out[2] = 0;
+// A node field at a record: its value and its gradient in cells.
+struct Sampled {
+  double v[3];
+  double d[3][3];  // [component][axis]
+};
+
+// The trilinear value (and gradient) by axis: x edges, then y, then z. Each
+// corner is read once for both: gathering the value and the position term
+// from the corners by their own weights read 240 values per record of the
+// cycle's pass where this reads 72.
+template <bool kGradient, class F>
+__device__ __forceinline__ void sample(const Geom& g, const F* __restrict__ f, const Loaded& L, Sampled& s) {
+  const long long sy = g.NX, sz = (long long)g.NX * g.NY;
 #pragma unroll
-  for (int a = 0; a < 8; ++a) {
-    const long long n = L.node(g, a);
-    const double w = L.weight(a);
-    out[0] += w * double(f[n]);
-    out[1] += w * double(f[g.nodes + n]);
-    out[2] += w * double(f[2 * g.nodes + n]);
+  for (int c = 0; c < 3; ++c) {
+    const F* p = f + c * g.nodes + L.base;
+    double vz[2], dx[2], dy[2];
+#pragma unroll
+    for (int z = 0; z < 2; ++z) {
+      const F* q = p + z * sz;
+      const double a0 = double(q[0]), a1 = double(q[1]), b0 = double(q[sy]), b1 = double(q[sy + 1]);
+      const double va = L.X[0] * a0 + L.X[1] * a1, vb = L.X[0] * b0 + L.X[1] * b1;
+      vz[z] = L.Y[0] * va + L.Y[1] * vb;
+      if constexpr (kGradient) {
+        dx[z] = L.Y[0] * (a1 - a0) + L.Y[1] * (b1 - b0);
+        dy[z] = vb - va;
+      }
+    }
+    s.v[c] = L.Z[0] * vz[0] + L.Z[1] * vz[1];
+    if constexpr (kGradient) {
+      s.d[c][0] = L.Z[0] * dx[0] + L.Z[1] * dx[1];
+      s.d[c][1] = L.Z[0] * dy[0] + L.Z[1] * dy[1];
+      s.d[c][2] = vz[1] - vz[0];
+    }
   }
 }
 
-// sum_a dW_a/dx_axis (f_a . gv) into out[axis].
-template <class F>
-__device__ __forceinline__ void position_term(const Geom& g, const F* __restrict__ f, const Loaded& L,
-                                              const double gv[3], double out[3]) {
+// out[axis] += d(field . gv)/dx_axis.
+__device__ __forceinline__ void position_term(const Sampled& s, const double gv[3], double out[3]) {
 #pragma unroll
-  for (int a = 0; a < 8; ++a) {
-    const long long n = L.node(g, a);
-    const double d = double(f[n]) * gv[0] + double(f[g.nodes + n]) * gv[1] + double(f[2 * g.nodes + n]) * gv[2];
-    double dw[3];
-    L.weight_gradient(a, dw);
-    out[0] += dw[0] * d;
-    out[1] += dw[1] * d;
-    out[2] += dw[2] * d;
-  }
+  for (int a = 0; a < 3; ++a) out[a] += s.d[0][a] * gv[0] + s.d[1][a] * gv[1] + s.d[2][a] * gv[2];
 }
 
 __device__ __forceinline__ void transpose_apply(const double r[9], const double x[3], double out[3]) {
@@ -143,39 +143,13 @@ __device__ __forceinline__ void response_gradient(const double om[3], const doub
   }
 }
 
-// Adds w_a * val (the 8 corners of this lane's record) into the unique nodes
-// of `field`. A run is a maximal group of consecutive lanes with equal keys
-// (the records are sorted by cell, so a run is usually a cell's records in
-// this warp); per corner, each lane sums the lanes after it within its run
-// and the first lane of the run adds the run's total. Every lane of the warp
-// calls it; inactive lanes pass a key no other lane has.
-__device__ __forceinline__ void warp_scatter(const Geom& g, double* __restrict__ field, const Loaded& L,
-                                             const double val[3]) {
-  const unsigned lane = threadIdx.x & 31u;
-  const int32_t before = __shfl_up_sync(kFull, L.key, 1);
-  const bool head = lane == 0 || before != L.key;
-  const unsigned heads = __ballot_sync(kFull, head);
-  const unsigned later = heads & ~((2u << lane) - 1u);  // run heads after this lane
-  const unsigned end = later ? unsigned(__ffs(later) - 1) : 32u;
-#pragma unroll
-  for (int a = 0; a < 8; ++a) {
-    const double w = L.ok ? L.weight(a) : 0.0;
-    double part[3] = {w * val[0], w * val[1], w * val[2]};
-#pragma unroll
-    for (unsigned off = 1; off < 32; off <<= 1) {
-      const bool add = lane + off < end;
-#pragma unroll
-      for (int comp = 0; comp < 3; ++comp) {
-        const double o = __shfl_down_sync(kFull, part[comp], off);
-        if (add) part[comp] += o;
-      }
-    }
-    if (L.ok && head) {
-      const long long u = L.unique(g, a);
-#pragma unroll
-      for (int comp = 0; comp < 3; ++comp) atomicAdd(field + comp * g.nodes + u, part[comp]);
-    }
-  }
+// Adds a cell's corner total into the unique node of component n of `field`.
+__device__ __forceinline__ void add_corner(const Geom& g, double* __restrict__ field, int32_t key, int a, int n,
+                                           double total) {
+  int i, j, k;
+  g.decode(key, i, j, k);
+  const int ci = i + (a & 1), cj = j + ((a >> 1) & 1), ck = k + ((a >> 2) & 1);
+  atomicAdd(field + n * g.nodes + g.node(ci == g.nx ? 0 : ci, cj == g.ny ? 0 : cj, ck == g.nz ? 0 : ck), total);
 }
 
 template <class P>
@@ -183,9 +157,8 @@ __device__ __forceinline__ void load_record(const Geom& g, const AdjointRecords&
                                             Loaded& L) {
   using Vel = typename P::Vel;
   L.ok = false;
-  L.key = -1 - int32_t(threadIdx.x & 31u);
+  L.key = -1;
   L.pid = 0;
-  L.i = L.j = L.k = 0;
   L.base = 0;
   L.X[0] = L.X[1] = L.Y[0] = L.Y[1] = L.Z[0] = L.Z[1] = 0;
   L.v[0] = L.v[1] = L.v[2] = 0;
@@ -204,7 +177,6 @@ __device__ __forceinline__ void load_record(const Geom& g, const AdjointRecords&
   L.ok = true;
   L.key = key;
   L.pid = (long long)id;
-  L.i = i; L.j = j; L.k = k;
   L.base = g.node(i, j, k);
   L.X[0] = 1 - fx; L.X[1] = fx;
   L.Y[0] = 1 - fy; L.Y[1] = fy;
@@ -220,71 +192,102 @@ __global__ void __launch_bounds__(kAdjointThreads) adjoint_theta_scatter_kernel(
                                                                                double* etheta_bar,
                                                                                uint32_t* invalid) {
   using Fld = typename P::Fld;
+  using Sums = CornerSums<3>;
+  __shared__ typename Sums::Stage stages[kAdjointThreads / 32];
+  typename Sums::Stage& stage = stages[threadIdx.x / 32];
   const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t warp = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-  const uint32_t warps = gridDim.x * (blockDim.x / 32);
-  for (uint32_t base = warp * 32; base < r.count; base += warps * 32) {
+  uint32_t first, last;
+  warp_segment(r.count, first, last);
+  auto sink = [&](int32_t key, int a, int n, double total) { add_corner(g, etheta_bar, key, a, n, total); };
+  Sums sums;
+  sums.begin();
+  for (uint32_t base = first; base < last; base += 32) {
     const uint32_t n = base + lane;
     Loaded L;
-    load_record<P>(g, r, n, n < r.count, L);
-    if (n < r.count && !L.ok) atomicAdd(invalid, 1u);
+    load_record<P>(g, r, n, n < last, L);
+    if (n < last && !L.ok) atomicAdd(invalid, 1u);
     double eb[3] = {0, 0, 0};
     if (L.ok) {
-      double bp[3];
-      gather3(g, (const Fld*)bnode, L, bp);
-      const Response<double> resp(bp[0], bp[1], bp[2], k.boc);
       double gv[3];
 #pragma unroll
       for (int c = 0; c < 3; ++c)
         gv[c] = 2.0 * (r.vbar[c * (long long)r.nid + L.pid] + k.dt * k.inv[c] * r.xbar[c * (long long)r.nid + L.pid]);
+      Sampled b;
+      sample<false>(g, (const Fld*)bnode, L, b);
+      const Response<double> resp(b.v[0], b.v[1], b.v[2], k.boc);
       transpose_apply(resp.a, gv, eb);
 #pragma unroll
       for (int c = 0; c < 3; ++c) eb[c] *= k.beta;
     }
-    warp_scatter(g, etheta_bar, L, eb);
+    const double f[3] = {L.X[1], L.Y[1], L.Z[1]};
+    sums.add(stage, L.ok, L.key, f, eb, sink);
   }
+  sums.flush(sink);
 }
 
-// The record adjoint. kMover: the mover's part (x_bar', v_bar' are the
+// The record adjoint. kAdjointMover: the mover's part (x_bar', v_bar' are the
 // gradients of the moved record; v_bar is replaced, x_bar keeps x_bar' plus
-// its terms). kDeposit: the current and mass part (terms added). The B
-// gradient is scattered into bnode_bar; with kScatterTheta the mover's E_theta
-// gradient into etheta_bar too.
-template <class P, bool kMover, bool kDeposit, bool kScatterTheta>
-__global__ void __launch_bounds__(kAdjointThreads) adjoint_record_kernel(Geom g, AdjointConstants k,
-                                                                        AdjointRecords r, AdjointFields fl,
-                                                                        double* bnode_bar, double* etheta_bar,
-                                                                        uint32_t* invalid) {
+// its terms), the mover's E_theta gradient scattered into etheta_bar.
+// kAdjointDeposit: the current and mass part (terms added). kAdjointCycle:
+// both, for the gradients a cycle has: jbar = mleft (lambda) and mright =
+// theta, so each of the three fields is sampled once. The B gradient is
+// scattered into bnode_bar.
+template <class P, int kMode>
+__global__ void __launch_bounds__(kRecordThreads, kRecordBlocks) adjoint_record_kernel(Geom g, AdjointConstants k,
+                                                                                      AdjointRecords r,
+                                                                                      AdjointFields fl,
+                                                                                      double* bnode_bar,
+                                                                                      double* etheta_bar,
+                                                                                      uint32_t* invalid) {
   using Fld = typename P::Fld;
+  constexpr bool kMover = kMode != kAdjointDeposit, kDeposit = kMode != kAdjointMover;
+  constexpr bool kCycle = kMode == kAdjointCycle, kScatterTheta = kMode == kAdjointMover;
+  using Sums = CornerSums<kScatterTheta ? 6 : 3>;
+  __shared__ typename Sums::Stage stages[kRecordThreads / 32];
+  typename Sums::Stage& stage = stages[threadIdx.x / 32];
   const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t warp = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-  const uint32_t warps = gridDim.x * (blockDim.x / 32);
+  uint32_t first, last;
+  warp_segment(r.count, first, last);
   const long long nid = r.nid;
-  for (uint32_t base = warp * 32; base < r.count; base += warps * 32) {
+  auto sink = [&](int32_t key, int a, int n, double total) {
+    if (kScatterTheta && n >= 3) add_corner(g, etheta_bar, key, a, n - 3, total);
+    else add_corner(g, bnode_bar, key, a, n, total);
+  };
+  Sums sums;
+  sums.begin();
+  for (uint32_t base = first; base < last; base += 32) {
     const uint32_t n = base + lane;
     Loaded L;
-    load_record<P>(g, r, n, n < r.count, L);
-    if (n < r.count && !L.ok) atomicAdd(invalid, 1u);
-    double bb[3] = {0, 0, 0}, eb[3] = {0, 0, 0};
+    load_record<P>(g, r, n, n < last, L);
+    if (n < last && !L.ok) atomicAdd(invalid, 1u);
+    double scatter[kScatterTheta ? 6 : 3];
+#pragma unroll
+    for (int c = 0; c < (kScatterTheta ? 6 : 3); ++c) scatter[c] = 0.0;
     if (L.ok) {
       const long long pid = L.pid;
-      double bp[3];
-      gather3(g, (const Fld*)fl.bnode, L, bp);
-      const Response<double> resp(bp[0], bp[1], bp[2], k.boc);
-      const double om[3] = {k.boc * bp[0], k.boc * bp[1], k.boc * bp[2]};
-      double ab[9];
-#pragma unroll
-      for (int e = 0; e < 9; ++e) ab[e] = 0;
       double xb[3], vn[3], t[3];
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         xb[c] = r.xbar[c * nid + pid];
         vn[c] = r.vbar[c * nid + pid];
       }
+      double q = 0.0, qbar = 0.0;
+      if constexpr (kDeposit) {
+        q = r.q[n];
+        qbar = r.qbar[pid];
+      }
+      Sampled b;
+      sample<true>(g, (const Fld*)fl.bnode, L, b);
+      const Response<double> resp(b.v[0], b.v[1], b.v[2], k.boc);
+      double ab[9];
+#pragma unroll
+      for (int e = 0; e < 9; ++e) ab[e] = 0;
+      Sampled th;
+      double eb[3] = {0, 0, 0};
       if constexpr (kMover) {
         // v' = 2 R (v + beta E_theta) - v, x' = x + dt v' / dx.
-        double ep[3], gv[3];
-        gather3(g, fl.theta, L, ep);
+        double gv[3];
+        sample<true>(g, fl.theta, L, th);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
           const double vt = vn[c] + k.dt * k.inv[c] * xb[c];
@@ -297,22 +300,21 @@ __global__ void __launch_bounds__(kAdjointThreads) adjoint_record_kernel(Geom g,
           vn[c] += t[c];
           eb[c] = k.beta * t[c];
         }
-        const double uu[3] = {L.v[0] + k.beta * ep[0], L.v[1] + k.beta * ep[1], L.v[2] + k.beta * ep[2]};
+        const double uu[3] = {L.v[0] + k.beta * th.v[0], L.v[1] + k.beta * th.v[1], L.v[2] + k.beta * th.v[2]};
 #pragma unroll
         for (int a = 0; a < 3; ++a)
 #pragma unroll
-          for (int b = 0; b < 3; ++b) ab[3 * a + b] += gv[a] * uu[b];
-        position_term(g, fl.theta, L, eb, xb);
+          for (int e = 0; e < 3; ++e) ab[3 * a + e] += gv[a] * uu[e];
+        if constexpr (!kCycle) position_term(th, eb, xb);
       }
       if constexpr (kDeposit) {
-        double qb = 0;
-        const double q = r.q[n];
-        if (fl.jbar) {
+        double gl[3] = {0, 0, 0};  // the gradient at jbar (kCycle: jbar and mleft)
+        Sampled left;
+        if (kCycle || fl.jbar) {
           // J = sum (q/V) W R v: gradient jscale * jbar gathered.
-          double jp[3], h[3];
-          gather3(g, fl.jbar, L, jp);
-#pragma unroll
-          for (int c = 0; c < 3; ++c) jp[c] *= fl.jscale;
+          sample<true>(g, fl.jbar, L, left);
+          const double jp[3] = {fl.jscale * left.v[0], fl.jscale * left.v[1], fl.jscale * left.v[2]};
+          double h[3];
           resp.apply(L.v[0], L.v[1], L.v[2], h[0], h[1], h[2]);
           const double qv = q * k.inv_volume;
           transpose_apply(resp.a, jp, t);
@@ -321,46 +323,60 @@ __global__ void __launch_bounds__(kAdjointThreads) adjoint_record_kernel(Geom g,
 #pragma unroll
           for (int a = 0; a < 3; ++a)
 #pragma unroll
-            for (int b = 0; b < 3; ++b) ab[3 * a + b] += qv * jp[a] * L.v[b];
-          qb += k.inv_volume * (jp[0] * h[0] + jp[1] * h[1] + jp[2] * h[2]);
-          const double gj[3] = {fl.jscale * qv * h[0], fl.jscale * qv * h[1], fl.jscale * qv * h[2]};
-          position_term(g, fl.jbar, L, gj, xb);
+            for (int e = 0; e < 3; ++e) ab[3 * a + e] += qv * jp[a] * L.v[e];
+          qbar += k.inv_volume * (jp[0] * h[0] + jp[1] * h[1] + jp[2] * h[2]);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) gl[c] = fl.jscale * qv * h[c];
+          if constexpr (!kCycle) position_term(left, gl, xb);
         }
-        if (fl.mleft) {
+        if (kCycle || fl.mleft) {
           // mscale * sum_p s lambda_p^T R u_p, s = (beta/c) q.
-          double lp[3], up[3], ru[3], rl[3];
-          gather3(g, fl.mleft, L, lp);
-          gather3(g, fl.mright, L, up);
+          if constexpr (!kCycle) {
+            sample<true>(g, fl.mleft, L, left);
+            sample<true>(g, fl.mright, L, th);
+          }
+          const double* lp = left.v;
+          const double* up = th.v;
+          double ru[3], rl[3];
           resp.apply(up[0], up[1], up[2], ru[0], ru[1], ru[2]);
           transpose_apply(resp.a, lp, rl);
           const double cs = fl.mscale * k.boc * q;
-          qb += fl.mscale * k.boc * (lp[0] * ru[0] + lp[1] * ru[1] + lp[2] * ru[2]);
+          qbar += fl.mscale * k.boc * (lp[0] * ru[0] + lp[1] * ru[1] + lp[2] * ru[2]);
 #pragma unroll
           for (int a = 0; a < 3; ++a)
 #pragma unroll
-            for (int b = 0; b < 3; ++b) ab[3 * a + b] += cs * lp[a] * up[b];
-          const double g1[3] = {cs * ru[0], cs * ru[1], cs * ru[2]};
-          const double g2[3] = {cs * rl[0], cs * rl[1], cs * rl[2]};
-          position_term(g, fl.mleft, L, g1, xb);
-          position_term(g, fl.mright, L, g2, xb);
+            for (int e = 0; e < 3; ++e) ab[3 * a + e] += cs * lp[a] * up[e];
+          double g1[3], g2[3];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            g1[c] = cs * ru[c] + (kCycle ? gl[c] : 0.0);
+            g2[c] = cs * rl[c] + (kCycle ? eb[c] : 0.0);
+          }
+          position_term(left, g1, xb);
+          position_term(th, g2, xb);
         }
-        r.qbar[pid] += qb;
+        r.qbar[pid] = qbar;
       }
       // The response's dependence on B at the record.
+      const double om[3] = {k.boc * b.v[0], k.boc * b.v[1], k.boc * b.v[2]};
       double ob[3];
       response_gradient(om, resp.a, ab, ob);
 #pragma unroll
-      for (int c = 0; c < 3; ++c) bb[c] = k.boc * ob[c];
-      position_term(g, (const Fld*)fl.bnode, L, bb, xb);
+      for (int c = 0; c < 3; ++c) {
+        scatter[c] = k.boc * ob[c];
+        if constexpr (kScatterTheta) scatter[3 + c] = eb[c];
+      }
+      position_term(b, scatter, xb);
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         r.xbar[c * nid + pid] = xb[c];
         r.vbar[c * nid + pid] = vn[c];
       }
     }
-    warp_scatter(g, bnode_bar, L, bb);
-    if constexpr (kScatterTheta) warp_scatter(g, etheta_bar, L, eb);
+    const double f[3] = {L.X[1], L.Y[1], L.Z[1]};
+    sums.add(stage, L.ok, L.key, f, scatter, sink);
   }
+  sums.flush(sink);
 }
 
 // Advance adjoint over the interior nodes 0..n: etheta_bar = a ebar' + far
@@ -466,8 +482,9 @@ AdjointRecords records(const tpicb200_particles* p, uint32_t nid, double* xbar, 
                         p->cell, p->id, p->count, nid, xbar, vbar, qbar};
 }
 
-unsigned record_blocks(uint32_t count) {
-  return grid_for((long long)(count + 31) / 32 * 32, kAdjointThreads, 148u * 8u);
+// One wave of resident blocks; a warp then walks consecutive records.
+unsigned record_blocks(uint32_t count, int threads, unsigned per_sm) {
+  return grid_for((long long)(count + 31) / 32 * 32, threads, 148u * per_sm);
 }
 
 }  // namespace
@@ -480,10 +497,10 @@ cudaError_t launch_adjoint_theta_scatter(int precision, const Geom& g, double qo
   const AdjointConstants k = constants(g, qom, dt, c);
   const AdjointRecords r = records(p, nid, const_cast<double*>(xbar), const_cast<double*>(vbar), nullptr);
   if (precision == TPICB200_PRECISION_DOUBLE)
-    adjoint_theta_scatter_kernel<PDouble><<<record_blocks(p->count), kAdjointThreads, 0, s>>>(g, k, r, bnode,
+    adjoint_theta_scatter_kernel<PDouble><<<record_blocks(p->count, kAdjointThreads, 4), kAdjointThreads, 0, s>>>(g, k, r, bnode,
                                                                                             etheta_bar, invalid);
   else
-    adjoint_theta_scatter_kernel<PMixed><<<record_blocks(p->count), kAdjointThreads, 0, s>>>(g, k, r, bnode,
+    adjoint_theta_scatter_kernel<PMixed><<<record_blocks(p->count, kAdjointThreads, 4), kAdjointThreads, 0, s>>>(g, k, r, bnode,
                                                                                            etheta_bar, invalid);
   count_launches(1);
   return cudaGetLastError();
@@ -498,23 +515,24 @@ cudaError_t launch_adjoint_records(int precision, int mode, const Geom& g, doubl
   const AdjointConstants k = constants(g, qom, dt, c);
   const AdjointRecords r = records(p, nid, xbar, vbar, qbar);
   const AdjointFields fl{theta, bnode, jbar, jscale, mleft, mright, mscale};
-  const unsigned blocks = record_blocks(p->count);
+  const unsigned blocks = record_blocks(p->count, kRecordThreads, kRecordBlocks);
   auto go = [&](auto kernel) {
-    kernel<<<blocks, kAdjointThreads, 0, s>>>(g, k, r, fl, bnode_bar, etheta_bar, invalid);
+    kernel<<<blocks, kRecordThreads, 0, s>>>(g, k, r, fl, bnode_bar, etheta_bar, invalid);
   };
   const bool dbl = precision == TPICB200_PRECISION_DOUBLE;
   switch (mode) {
     case kAdjointMover:
-      if (dbl) go(adjoint_record_kernel<PDouble, true, false, true>);
-      else go(adjoint_record_kernel<PMixed, true, false, true>);
+      if (dbl) go(adjoint_record_kernel<PDouble, kAdjointMover>);
+      else go(adjoint_record_kernel<PMixed, kAdjointMover>);
       break;
     case kAdjointDeposit:
-      if (dbl) go(adjoint_record_kernel<PDouble, false, true, false>);
-      else go(adjoint_record_kernel<PMixed, false, true, false>);
+      if (dbl) go(adjoint_record_kernel<PDouble, kAdjointDeposit>);
+      else go(adjoint_record_kernel<PMixed, kAdjointDeposit>);
       break;
     case kAdjointCycle:
-      if (dbl) go(adjoint_record_kernel<PDouble, true, true, false>);
-      else go(adjoint_record_kernel<PMixed, true, true, false>);
+      if (jbar != mleft || mright != theta || !jbar) return cudaErrorInvalidValue;
+      if (dbl) go(adjoint_record_kernel<PDouble, kAdjointCycle>);
+      else go(adjoint_record_kernel<PMixed, kAdjointCycle>);
       break;
     default:
       return cudaErrorInvalidValue;

@@ -1,0 +1,116 @@
+// Sums over the records of a cell of W_a(record) * value_n(record), the 8
+// CIC corners a by N values, on the FP64 tensor cores: what a per-record
+// deposition onto the corner nodes adds, one total per cell, corner and value.
+//
+// A warp stages 32 records (fractions and values) in shared memory; with
+// m8n8k4 the 8 corners are the rows of A (each lane forms the weight of its
+// corner and record from the staged fractions), the values the columns of B
+// and 4 records one step, so a chunk takes 8 steps per 8 values and the totals
+// stay in two registers per lane and tile. Records are taken in groups of
+// equal cell keys; the totals are kept while consecutive groups have the same
+// key, over chunks too, and handed out when it changes, so sorted records cost
+// one addition per cell, corner and value, and unsorted ones no more than a
+// per-record deposition.
+#pragma once
+
+#include "common.cuh"
+
+namespace tpicb200 {
+
+// D += A B for A 8x4 (row-major), B 4x8: a = A[lane/4][lane%4],
+// b = B[lane%4][lane/4], c = D[lane/4][2*(lane%4) + {0, 1}].
+__device__ __forceinline__ void corner_mma(double& c0, double& c1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(c0), "+d"(c1)
+      : "d"(a), "d"(b));
+}
+
+template <int N>
+struct CornerSums {
+  static constexpr int kTiles = (N + 7) / 8;
+  // 36 records a row: the 16 lanes of a shared-memory phase (4 rows x 4
+  // records) then touch 16 different 8-byte banks.
+  static constexpr int kPitch = 36;
+  struct Stage {  // one per warp
+    double fraction[3][kPitch];
+    double value[N][kPitch];
+  };
+
+  double c[kTiles][2];
+  int32_t key;  // the cell of the totals held; -1: none
+
+  __device__ __forceinline__ void begin() {
+    key = -1;
+#pragma unroll
+    for (int t = 0; t < kTiles; ++t) c[t][0] = c[t][1] = 0.0;
+  }
+
+  // Hands the totals held to sink(key, corner, n, total), this lane's share.
+  template <class Sink>
+  __device__ __forceinline__ void flush(Sink&& sink) {
+    if (key < 0) return;
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int t = 0; t < kTiles; ++t)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int n = 8 * t + 2 * (lane & 3) + h;
+        if (n < N) sink(key, lane >> 2, n, c[t][h]);
+      }
+    begin();
+  }
+
+  // One chunk: this lane's record (ok: it counts; its key, fractions and
+  // values, all finite where their totals are used). Every lane calls it.
+  template <class Sink>
+  __device__ __forceinline__ void add(Stage& s, bool ok, int32_t k, const double f[3], const double v[N],
+                                      Sink&& sink) {
+    const int lane = threadIdx.x & 31, row = lane >> 2, col = lane & 3;
+    __syncwarp();
+#pragma unroll
+    for (int a = 0; a < 3; ++a) s.fraction[a][lane] = ok ? f[a] : 0.0;
+#pragma unroll
+    for (int n = 0; n < N; ++n) s.value[n][lane] = ok ? v[n] : 0.0;
+    __syncwarp();
+    unsigned left = __ballot_sync(0xffffffffu, ok);
+    while (left) {
+      const int32_t group = __shfl_sync(0xffffffffu, k, __ffs(left) - 1);
+      const unsigned members = __ballot_sync(0xffffffffu, k == group) & left;
+      left &= ~members;
+      if (group != key) {
+        flush(sink);
+        key = group;
+      }
+#pragma unroll
+      for (int step = 0; step < 8; ++step) {
+        const unsigned four = (members >> (4 * step)) & 15u;
+        if (four == 0) continue;
+        const int r = 4 * step + col;
+        const double x = s.fraction[0][r], y = s.fraction[1][r], z = s.fraction[2][r];
+        const double w = ((row & 1) ? x : 1.0 - x) * ((row & 2) ? y : 1.0 - y) * ((row & 4) ? z : 1.0 - z);
+        // Both factors of a record outside the group are zero, so a nonfinite
+        // value stays in its own cell's totals.
+        const bool member = (four >> col) & 1u;
+        const double a = member ? w : 0.0;
+#pragma unroll
+        for (int t = 0; t < kTiles; ++t) {
+          const int n = 8 * t + row;
+          corner_mma(c[t][0], c[t][1], a, member && n < N ? s.value[n < N ? n : 0][r] : 0.0);
+        }
+      }
+    }
+  }
+};
+
+// Records [first, last) of this warp: consecutive runs of whole chunks, as
+// equal as the chunks allow, so that a warp's records are neighbours.
+__device__ __forceinline__ void warp_segment(uint32_t count, uint32_t& first, uint32_t& last) {
+  const uint32_t warps = gridDim.x * (blockDim.x / 32), warp = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+  const uint32_t chunks = count / 32 + (count % 32 ? 1 : 0);
+  const uint32_t each = chunks / warps, more = chunks % warps;
+  const uint32_t c0 = warp * each + min(warp, more), c1 = c0 + each + (warp < more ? 1 : 0);
+  first = c0 * 32;
+  last = uint32_t(min((unsigned long long)c1 * 32, (unsigned long long)count));
+}
+
+}  // namespace tpicb200
