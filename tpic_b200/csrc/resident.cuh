@@ -1,0 +1,612 @@
+// The GMRES restart cycle of a small grid as one resident kernel.
+//
+// On grids of up to some ten thousand nodes an Arnoldi step is short work
+// behind nine launches: 36 us a step on a 1024 x 1 x 1 grid, 55 us on 256 x
+// 128 x 1, where the mass matrix and the vectors stay in L2. Here every CTA
+// owns the unique nodes of one tile for the whole cycle, keeps its rows of the
+// Krylov basis in shared memory where they fit, and the CTAs meet at two grid
+// barriers a step:
+//   A  the operator on the last vector (neighbours' rows read from one global
+//      vector), and the dots of its image with the owned basis rows;
+//      -- barrier: the dots of all CTAs --
+//   B  Gram-Schmidt of the owned rows, the squared norm; the unnormalized
+//      vector goes to the global vector;
+//      -- barrier: the norm of all CTAs; each CTA scales what it reads --
+// The Hessenberg column is rotated by one more warp while the others
+// orthogonalize; every CTA does so from the same sums in the same order, so
+// all take the same stopping decision. Vectors hold the unique nodes only; a
+// row of node 0 on an axis stands for its duplicate at node n too, so it
+// counts twice per such axis in the dots and norms, which are then those over
+// the interior nodes. All sums run in a fixed order.
+//
+// A tile of TN (32..256, a power of two) nodes has 256 / TN threads a node
+// that share the 27 mass blocks: small grids take small tiles, so that every
+// SM has one.
+//
+// Launched cooperatively (all CTAs resident). A barrier that does not
+// complete within its polls makes its CTA set ctl->failed and leave; the
+// others then run out at theirs, and the solve fails.
+#pragma once
+
+#include "common.cuh"
+#include "stencils.cuh"
+
+namespace tpicb200 {
+namespace {
+
+// Device-side state of one restart cycle's Arnoldi steps.
+struct ArnoldiControl {
+  int col;        // the step the step kernels take (0-based)
+  int completed;  // steps completed in this cycle
+  int columns;    // step limit of this cycle
+  int stop;       // 0 running; 1 stopped (tolerance, breakdown or limit); 2 nonfinite estimate
+  int breakdown;  // the last step's subdiagonal was zero
+  int failed;     // a grid barrier of the resident kernel ran out of polls
+  double tolerance;
+};
+
+constexpr int kResidentNodeThreads = 256;
+constexpr int kResidentThreads = kResidentNodeThreads + 32;  // and the warp that rotates the Hessenberg column
+constexpr int kResidentRestart = 32;                         // longest restart cycle
+constexpr uint32_t kResidentPolls = 1u << 22;
+
+struct ResidentPlan {
+  Geom g;
+  int tx, ty, tz;          // tile, powers of two; tx*ty*tz = nodes
+  int nodes, parts, shift; // nodes of a tile, threads per node, log2 nodes
+  int tiles_x, tiles_y, tiles;
+  bool shared_basis;       // basis rows in shared memory, else in `basis`
+  double delta, kfac, inv_volume;
+  const void* mass;
+  void* vector;            // [3][unique] S: the last unnormalized vector
+  void* basis;             // owner-private rows, 3 * nodes of each CTA per column
+  double* x;               // [3][unique]
+  double* b;
+  double* r;
+  double* values;          // |r|^2 and (start) |b|^2
+  double* partials;        // kResidentRestart + 2 rows of gridDim.x
+  ArnoldiControl* ctl;
+  unsigned* barrier;       // arrivals, departures (zero between launches)
+  int restart, columns;
+  double tolerance;        // of this cycle's residual estimate
+  double accept;           // start: the relative tolerance; cycle: the absolute one
+  const void* e;           // start: E, B and J, or the right-hand side itself with a zero guess
+  const void* bcell;
+  const void* j;
+  const double* rhs;
+  double* etheta;          // the solution with its ghosts, written when the residual is accepted
+};
+
+// Shared memory of a plan with arithmetic up to double: bytes per array.
+struct ResidentShared {
+  int halo, cells;                 // nodes and cells a tile stages
+  size_t vs, cs, part, h, hcol, rot, sums, basis, image, unode, mult, table, ctable, total;
+};
+inline __host__ __device__ ResidentShared resident_shared(const ResidentPlan& p, size_t scalar) {
+  ResidentShared s;
+  s.halo = (p.tx + 2) * (p.ty + 2) * (p.tz + 2);
+  s.cells = (p.tx + 1) * (p.ty + 1) * (p.tz + 1);
+  const int m = kResidentRestart;
+  size_t at = 0;
+  auto take = [&](size_t bytes) {
+    const size_t here = at;
+    at += (bytes + 15) / 16 * 16;
+    return here;
+  };
+  s.vs = take(size_t(3) * s.halo * 8);
+  s.cs = take(size_t(3) * s.cells * 8);
+  s.part = take(size_t(3) * kResidentNodeThreads * 8);
+  s.h = take(size_t(m) * (m + 1) * 8);
+  s.hcol = take(size_t(m + 1) * 8);
+  s.rot = take(size_t(4) * (m + 1) * 8);  // cosines, sines, right-hand side, coefficients
+  s.sums = take(size_t(kResidentThreads / 32 + 2) * 2 * 8);  // per warp, then the step's diagonal and decision
+  s.basis = take(p.shared_basis ? size_t(p.restart + 1) * 3 * p.nodes * scalar : 0);
+  s.image = take(size_t(3) * p.nodes * scalar);
+  s.unode = take(size_t(p.nodes) * 4);
+  s.mult = take(size_t(p.nodes) * 4);
+  s.table = take(size_t(s.halo) * 4);
+  s.ctable = take(size_t(s.cells) * 4);
+  s.total = at;
+  return s;
+}
+
+// stencil_offset, indexed at run time.
+__constant__ int8_t kResidentOffsets[14][3] = {{0, 0, 0},  {1, 0, 0},  {0, 1, 0},  {0, 0, 1},  {1, 1, 0},
+                                               {1, -1, 0}, {1, 0, 1},  {1, 0, -1}, {0, 1, 1},  {0, 1, -1},
+                                               {1, -1, 1}, {1, 1, -1}, {-1, 1, 1}, {1, 1, 1}};
+
+__device__ __forceinline__ uint32_t load_acquire(const unsigned* p) {
+  uint32_t v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+template <class S, class Mass, class Fld, bool kTranspose>
+struct Resident {
+  const ResidentPlan& p;
+  uint8_t* smem;
+  const ResidentShared L;
+  uint32_t arrivals = 0;
+  bool failed = false;
+
+  __device__ Resident(const ResidentPlan& plan, uint8_t* s) : p(plan), smem(s), L(resident_shared(plan, sizeof(S))) {}
+
+  template <class T> __device__ __forceinline__ T* at(size_t offset) const { return reinterpret_cast<T*>(smem + offset); }
+  __device__ __forceinline__ long long unique() const { return (long long)p.g.nx * p.g.ny * p.g.nz; }
+  __device__ __forceinline__ S* basis(int col) const {
+    const int rows = 3 * p.nodes;
+    return p.shared_basis ? at<S>(L.basis) + col * rows
+                          : static_cast<S*>(p.basis) + ((long long)col * gridDim.x + blockIdx.x) * rows;
+  }
+  __device__ __forceinline__ void origin(int& i0, int& j0, int& k0) const {
+    const int tile = blockIdx.x, row = tile / p.tiles_x;
+    i0 = (tile - row * p.tiles_x) * p.tx;
+    k0 = row / p.tiles_y;
+    j0 = (row - k0 * p.tiles_y) * p.ty;
+    k0 *= p.tz;
+  }
+
+  // All CTAs of the grid. False when it gave up (for every thread of the CTA).
+  __device__ bool grid_barrier() {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      arrivals += gridDim.x;
+      // The CTA's writes are ordered before the arrival (the barrier above and
+      // the release), the others' before what follows the acquire.
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p.barrier) : "memory");
+      uint32_t poll = 0;
+      while (load_acquire(p.barrier) < arrivals && poll < kResidentPolls) ++poll;
+      if (poll == kResidentPolls) {
+        failed = true;
+        p.ctl->failed = 1;
+      }
+    }
+    return !__syncthreads_or(failed);
+  }
+  // The last CTA to leave zeroes the barrier for the next launch.
+  __device__ void leave() {
+    if (threadIdx.x == 0 && !failed && atomicAdd(p.barrier + 1, 1u) == gridDim.x - 1) {
+      p.barrier[0] = 0;
+      p.barrier[1] = 0;
+    }
+  }
+
+  // Tables of the tile: the unique index of every staged node (-1 beyond the
+  // grid's halo) and the staged base node of every cell.
+  __device__ void tables() {
+    const int vx = p.tx + 2, vy = p.ty + 2, cx = p.tx + 1, cy = p.ty + 1;
+    int i0, j0, k0;
+    origin(i0, j0, k0);
+    const Geom& g = p.g;
+    int* table = at<int>(L.table);
+    int* ctable = at<int>(L.ctable);
+    for (int n = threadIdx.x; n < L.halo; n += kResidentThreads) {
+      const int row = n / vx, i = i0 - 1 + n - row * vx, j = j0 - 1 + row % vy, k = k0 - 1 + row / vy;
+      int u = -1;
+      if (i <= g.nx && j <= g.ny && k <= g.nz) {
+        const int wi = i < 0 ? i + g.nx : (i >= g.nx ? i - g.nx : i), wj = j < 0 ? j + g.ny : (j >= g.ny ? j - g.ny : j),
+                  wk = k < 0 ? k + g.nz : (k >= g.nz ? k - g.nz : k);
+        u = wi + g.nx * (wj + g.ny * wk);
+      }
+      table[n] = u;
+    }
+    for (int n = threadIdx.x; n < L.cells; n += kResidentThreads) {
+      const int row = n / cx;
+      ctable[n] = (n - row * cx) + vx * (row % cy + vy * (row / cy));
+    }
+  }
+
+  // Node n of the tile: coordinates, and whether it is in the grid.
+  __device__ __forceinline__ bool node_of(int n, int& i, int& j, int& k) const {
+    origin(i, j, k);
+    i += n & (p.tx - 1);
+    const int row = n / p.tx;
+    j += row & (p.ty - 1);
+    k += row / p.ty;
+    return i < p.g.nx && j < p.g.ny && k < p.g.nz;
+  }
+
+  // The operator on the tile's nodes in arithmetic C: stage() reads the vector
+  // load(component, unique index) over the tile and its halo (the node
+  // threads; a CTA barrier follows), image() calls store(node in tile, its
+  // coordinates, the three values) from the first thread of each node in the
+  // grid. The products and their order are those of maxwell_apply_kernel where
+  // a node has one thread; with more, their partial sums are added in order.
+  template <class C, class Load>
+  __device__ __forceinline__ void stage(Load&& load) {
+    if (threadIdx.x >= kResidentNodeThreads) return;
+    C* vs = at<C>(L.vs);
+    const int* table = at<int>(L.table);
+    const int VN = L.halo;
+    for (int n = threadIdx.x; n < VN; n += kResidentNodeThreads) {
+      const int u = table[n];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) vs[c * VN + n] = u >= 0 ? C(load(c, u)) : C(0);
+    }
+  }
+  template <class C, class Store>
+  __device__ __forceinline__ void image(Store&& store) {
+    const Geom& g = p.g;
+    C* vs = at<C>(L.vs);
+    C* cs = at<C>(L.cs);
+    const int* ctable = at<int>(L.ctable);
+    const int vx = p.tx + 2, vxy = vx * (p.ty + 2), cx = p.tx + 1, cxy = cx * (p.ty + 1);
+    const int VN = L.halo, CN = L.cells;
+    const C inv[3] = {C(g.inv[0]), C(g.inv[1]), C(g.inv[2])};
+    for (int n = threadIdx.x; n < CN; n += kResidentThreads) {
+      const C* v = vs + ctable[n];
+      C q[3][8];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const C* f = v + c * VN;
+        q[c][0] = f[0];       q[c][1] = f[1];       q[c][2] = f[vx];       q[c][3] = f[vxy];
+        q[c][4] = f[vx + 1];  q[c][5] = f[vxy + 1]; q[c][6] = f[vxy + vx]; q[c][7] = f[vxy + vx + 1];
+      }
+      auto dx = [&](const C* w) { return C(0.25) * inv[0] * (w[1] - w[0] + (w[5] - w[3]) + (w[4] - w[2]) + (w[7] - w[6])); };
+      auto dy = [&](const C* w) { return C(0.25) * inv[1] * (w[2] - w[0] + (w[6] - w[3]) + (w[4] - w[1]) + (w[7] - w[5])); };
+      auto dz = [&](const C* w) { return C(0.25) * inv[2] * (w[3] - w[0] + (w[5] - w[1]) + (w[6] - w[2]) + (w[7] - w[4])); };
+      cs[n] = dy(q[2]) - dz(q[1]);
+      cs[CN + n] = dz(q[0]) - dx(q[2]);
+      cs[2 * CN + n] = dx(q[1]) - dy(q[0]);
+    }
+    const int n = threadIdx.x & (p.nodes - 1), part = threadIdx.x >> p.shift;
+    int i = 0, j = 0, k = 0;
+    const bool live = threadIdx.x < kResidentNodeThreads && node_of(n, i, j, k);
+    const int lx = n & (p.tx - 1), ly = (n / p.tx) & (p.ty - 1), lz = n / (p.tx * p.ty);
+    const int vi = (lx + 1) + vx * (ly + 1) + vxy * (lz + 1);
+    C x = C(0), y = C(0), z = C(0);
+    if (live) {
+      // Blocks in stencil order: part r of P takes stencils [14 r / P, 14 (r + 1) / P).
+      const Mass* mass = static_cast<const Mass*>(p.mass);
+      const long long mat = g.mass_vertex(i, j, k);
+      const int s1 = 14 * (part + 1) / p.parts;
+      for (int s = 14 * part / p.parts; s < s1; ++s) {
+        const int ox = kResidentOffsets[s][0], oy = kResidentOffsets[s][1], oz = kResidentOffsets[s][2];
+        const int vo = ox + vx * oy + vxy * oz;
+        product(mass + g.mass_index(mat, 9 * s), vs + vi + vo, VN, x, y, z);
+        if (s > 0) product(mass + g.mass_index(mat - g.mass_offset(ox, oy, oz), 9 * s), vs + vi - vo, VN, x, y, z);
+      }
+      if (part > 0) {
+        C* sum = at<C>(L.part);
+        sum[threadIdx.x] = x;
+        sum[kResidentNodeThreads + threadIdx.x] = y;
+        sum[2 * kResidentNodeThreads + threadIdx.x] = z;
+      }
+    }
+    __syncthreads();
+    if (live && part == 0) {
+      const C* sum = at<C>(L.part);
+      for (int r = 1; r < p.parts; ++r) {
+        const int t = r * p.nodes + n;
+        x += sum[t];
+        y += sum[kResidentNodeThreads + t];
+        z += sum[2 * kResidentNodeThreads + t];
+      }
+      C w[3][8];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const C* f = cs + c * CN + (lx + 1) + cx * (ly + 1) + cxy * (lz + 1);
+        w[c][0] = f[0];        w[c][1] = f[-1];       w[c][2] = f[-cx];       w[c][3] = f[-cxy];
+        w[c][4] = f[-cx - 1];  w[c][5] = f[-cxy - 1]; w[c][6] = f[-cxy - cx]; w[c][7] = f[-cxy - cx - 1];
+      }
+      auto dx = [&](const C* q) { return C(0.25) * inv[0] * (q[0] - q[1] + (q[3] - q[5]) + (q[2] - q[4]) + (q[6] - q[7])); };
+      auto dy = [&](const C* q) { return C(0.25) * inv[1] * (q[0] - q[2] + (q[3] - q[6]) + (q[1] - q[4]) + (q[5] - q[7])); };
+      auto dz = [&](const C* q) { return C(0.25) * inv[2] * (q[0] - q[3] + (q[1] - q[5]) + (q[2] - q[6]) + (q[4] - q[7])); };
+      const C curl[3] = {dy(w[2]) - dz(w[1]), dz(w[0]) - dx(w[2]), dx(w[1]) - dy(w[0])};
+      const C d2 = C(p.delta * p.delta), kf = C(p.kfac), iv = C(p.inv_volume);
+      const C mv[3] = {x * iv, y * iv, z * iv};
+      C value[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) value[c] = (vs[c * VN + vi] + d2 * curl[c]) + kf * mv[c];
+      store(n, i, j, k, value);
+    }
+  }
+
+  template <class C>
+  __device__ __forceinline__ void product(const Mass* __restrict__ b, const C* v, int VN, C& x, C& y, C& z) {
+    const long long es = p.g.mes;
+    C m[9];
+#pragma unroll
+    for (int e = 0; e < 9; ++e) m[e] = C(__ldg(b + e * es));
+    const C v0 = v[0], v1 = v[VN], v2 = v[2 * VN];
+    if constexpr (kTranspose) {
+      x += v0 * m[0] + v1 * m[3] + v2 * m[6];
+      y += v0 * m[1] + v1 * m[4] + v2 * m[7];
+      z += v0 * m[2] + v1 * m[5] + v2 * m[8];
+    } else {
+      x += v0 * m[0] + v1 * m[1] + v2 * m[2];
+      y += v0 * m[3] + v1 * m[4] + v2 * m[5];
+      z += v0 * m[6] + v1 * m[7] + v2 * m[8];
+    }
+  }
+
+  // Block totals of one or two sums, to rows `row` and `row + 1` of the partials.
+  __device__ void publish(double a, double b, int row, bool two) {
+    double* sums = at<double>(L.sums);
+    const int warp = threadIdx.x >> 5;
+    a = warp_sum(a);
+    if (two) b = warp_sum(b);
+    if ((threadIdx.x & 31) == 0) {
+      sums[2 * warp] = a;
+      sums[2 * warp + 1] = b;
+    }
+    __syncthreads();
+    if (threadIdx.x < (two ? 2 : 1)) {
+      double total = 0;
+      for (int w = 0; w < kResidentThreads / 32; ++w) total += sums[2 * w + threadIdx.x];
+      p.partials[(long long)(row + threadIdx.x) * gridDim.x + blockIdx.x] = total;
+    }
+  }
+  // A row of the partials summed over the CTAs (every lane of a warp; fixed order).
+  __device__ __forceinline__ double gathered(int row) const {
+    const double* from = p.partials + (long long)row * gridDim.x;
+    double total = 0;
+    for (unsigned t = threadIdx.x & 31; t < gridDim.x; t += 32) total += __ldcg(from + t);
+    return warp_sum(total);
+  }
+
+  // What the nodes keep: unique indexes, multiplicities and the tables.
+  __device__ void prepare() {
+    int* unode = at<int>(L.unode);
+    float* mult = at<float>(L.mult);
+    for (int t = threadIdx.x; t < p.nodes; t += kResidentThreads) {
+      int i, j, k;
+      const bool live = node_of(t, i, j, k);
+      unode[t] = live ? i + p.g.nx * (j + p.g.ny * k) : -1;
+      mult[t] = live ? float((i == 0 ? 2 : 1) * (j == 0 ? 2 : 1) * (k == 0 ? 2 : 1)) : 0.0f;
+    }
+    S* last = at<S>(L.image);
+    for (int t = threadIdx.x; t < 3 * p.nodes; t += kResidentThreads) last[t] = S(0);
+    tables();
+    __syncthreads();
+  }
+
+  // r = b - A x over the owned nodes (x read through `load`), the sums of r^2
+  // (and of b^2) published.
+  template <class Load>
+  __device__ void residual(Load&& load, bool with_rhs) {
+    double s0 = 0, s1 = 0;
+    const long long U = unique();
+    stage<double>(load);
+    __syncthreads();
+    image<double>([&](int, int i, int j, int k, const double value[3]) {
+      const int u = i + p.g.nx * (j + p.g.ny * k);
+      const double m = (i == 0 ? 2.0 : 1.0) * (j == 0 ? 2.0 : 1.0) * (k == 0 ? 2.0 : 1.0);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const double b = p.b[c * U + u], r = b - value[c];
+        p.r[c * U + u] = r;
+        s0 += m * (r * r);
+        s1 += m * (b * b);
+      }
+    });
+    __syncthreads();
+    publish(s0, s1, 0, with_rhs);
+  }
+
+  // The solution x with its ghosts into etheta (node field).
+  __device__ void write_solution() {
+    const Geom& g = p.g;
+    const long long U = unique();
+    const uint32_t total = uint32_t(g.nodes), NX = uint32_t(g.NX), NY = uint32_t(g.NY);
+    for (uint32_t t = blockIdx.x * kResidentThreads + threadIdx.x; t < total; t += gridDim.x * kResidentThreads) {
+      const uint32_t row = t / NX;
+      const int i = int(t - row * NX) - 1, j = int(row % NY) - 1, k = int(row / NY) - 1;
+      const int u = wrap_index(i, g.nx) + g.nx * (wrap_index(j, g.ny) + g.ny * wrap_index(k, g.nz));
+#pragma unroll
+      for (int c = 0; c < 3; ++c) p.etheta[c * g.nodes + t] = __ldcg(p.x + c * U + u);
+    }
+  }
+};
+
+// The right-hand side, the guess and its residual (values[0] = |r|^2,
+// values[1] = |b|^2).
+template <class S, class Mass, class Fld, bool kTranspose>
+__global__ void __launch_bounds__(kResidentThreads, 2) resident_start_kernel(const __grid_constant__ ResidentPlan p) {
+  extern __shared__ __align__(16) uint8_t resident_smem[];
+  using R = Resident<S, Mass, Fld, kTranspose>;
+  R r(p, resident_smem);
+  r.prepare();
+  const Geom& g = p.g;
+  const long long U = r.unique();
+  const Fld* e = static_cast<const Fld*>(p.e);
+  const Fld inv[3] = {Fld(g.inv[0]), Fld(g.inv[1]), Fld(g.inv[2])};
+  int i, j, k;
+  if (int(threadIdx.x) < p.nodes && r.node_of(threadIdx.x, i, j, k)) {
+    const int u = i + g.nx * (j + g.ny * k);
+    const long long at = g.node(i, j, k);
+    if (p.rhs) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        p.x[c * U + u] = 0.0;
+        p.b[c * U + u] = p.rhs[c * g.nodes + at];
+      }
+    } else {
+      Fld cb[3];
+      curl_c2n_at<Fld>(g, static_cast<const Fld*>(p.bcell), i, j, k, inv, cb);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const Fld ev = e[c * g.nodes + at], jv = static_cast<const Fld*>(p.j)[c * g.nodes + at];
+        p.x[c * U + u] = double(ev);
+        p.b[c * U + u] = double((ev + Fld(p.delta) * cb[c]) + (-Fld(p.kfac)) * jv);
+      }
+    }
+  }
+  __syncthreads();
+  r.residual([&](int c, int u) -> double {
+    if (p.rhs) return 0.0;
+    const int row = u / g.nx, k = row / g.ny;
+    return double(e[c * g.nodes + g.node(u - row * g.nx, row - k * g.ny, k)]);
+  }, true);
+  if (!r.grid_barrier()) return;
+  const double r2 = r.gathered(0), b2 = r.gathered(1);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    p.values[0] = r2;
+    p.values[1] = b2;
+  }
+  const double norm = sqrt(b2);
+  if (sqrt(r2) <= (norm == 0.0 ? 1.0 : norm) * p.accept) r.write_solution();
+  r.leave();
+}
+
+// One restart cycle from the residual r (values[0] = |r|^2): at most
+// `columns` Arnoldi steps, the update of x, its residual (values[0]).
+template <class S, class Mass, class Fld, bool kTranspose>
+__global__ void __launch_bounds__(kResidentThreads, 2) resident_cycle_kernel(const __grid_constant__ ResidentPlan p) {
+  extern __shared__ __align__(16) uint8_t resident_smem[];
+  using R = Resident<S, Mass, Fld, kTranspose>;
+  R r(p, resident_smem);
+  constexpr int m = kResidentRestart, kWarps = kResidentThreads / 32;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long long U = r.unique();
+  const int rows = 3 * p.nodes;
+  double* H = r.template at<double>(r.L.h);      // column c at c * (m + 1)
+  double* hcol = r.template at<double>(r.L.hcol);
+  double* cosine = r.template at<double>(r.L.rot);
+  double* sine = cosine + m + 1;
+  double* rhs = sine + m + 1;
+  double* coefficient = rhs + m + 1;
+  double* shared = r.template at<double>(r.L.sums) + 2 * kWarps;  // diagonal, decision, breakdown
+  S* image = r.template at<S>(r.L.image);
+  const int* unode = r.template at<int>(r.L.unode);
+  const float* mult = r.template at<float>(r.L.mult);
+  S* vector = static_cast<S*>(p.vector);
+  r.prepare();
+  // Row t of the owned rows: its node and its place in a [3][unique] vector.
+  auto place = [&](int t, int& n) -> long long {
+    n = t & (p.nodes - 1);
+    return (t >> p.shift) * U + unode[n];
+  };
+  const double first = p.values[0];
+  double scale = first > 0.0 ? 1.0 / sqrt(first) : 0.0;
+  {
+    S* v = r.basis(0);
+    for (int t = threadIdx.x; t < rows; t += kResidentThreads) {
+      int n;
+      const long long at = place(t, n);
+      v[t] = unode[n] >= 0 ? S(p.r[at] * scale) : S(0);
+    }
+  }
+  if (threadIdx.x == kResidentNodeThreads) {
+    rhs[0] = sqrt(first);
+    shared[1] = 0.0;
+  }
+  int col = 0, stop = 0;
+  while (true) {
+    // A: image = A v_col; its dots with columns 0..col. The decision on the
+    // last step is formed by the other warp while the vector is staged.
+    if (col == 0) r.template stage<S>([&](int c, int u) { return S(__ldcg(p.r + c * U + u) * scale); });
+    else r.template stage<S>([&](int c, int u) { return S(double(__ldcg(vector + c * U + u)) * scale); });
+    __syncthreads();
+    stop = int(shared[1]);
+    if (stop) break;
+    r.template image<S>([&](int n, int, int, int, const S value[3]) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) image[c * p.nodes + n] = value[c];
+    });
+    __syncthreads();
+    for (int c = warp; c <= col; c += kWarps) {
+      const S* v = r.basis(c);
+      double sum = 0;
+      for (int t = lane; t < rows; t += 32)
+        sum += double(v[t]) * (double(image[t]) * double(mult[t & (p.nodes - 1)]));
+      sum = warp_sum(sum);
+      if (lane == 0) p.partials[(long long)c * gridDim.x + blockIdx.x] = sum;
+    }
+    if (!r.grid_barrier()) return;
+    // B: Gram-Schmidt of the owned rows.
+    for (int c = warp; c <= col; c += kWarps) {
+      const double sum = r.gathered(c);
+      if (lane == 0) hcol[c] = sum;
+    }
+    __syncthreads();
+    double norm2 = 0;
+    if (threadIdx.x < kResidentNodeThreads) {
+      for (int t = threadIdx.x; t < rows; t += kResidentNodeThreads) {
+        int n;
+        const long long at = place(t, n);
+        if (unode[n] < 0) continue;
+        double value = double(image[t]);
+        const S* v = r.basis(0) + t;
+        const long long next = r.basis(1) - r.basis(0);
+#pragma unroll 4
+        for (int c = 0; c <= col; ++c) value -= hcol[c] * double(v[c * next]);
+        const S stored = S(value);
+        image[t] = stored;
+        vector[at] = stored;
+        norm2 += double(mult[n]) * (double(stored) * double(stored));
+      }
+    } else if (lane == 0) {
+      // The column through the rotations so far.
+      double* column = H + col * (m + 1);
+      double upper = hcol[0];
+      for (int row = 0; row < col; ++row) {
+        const double lower = hcol[row + 1];
+        column[row] = cosine[row] * upper + sine[row] * lower;
+        upper = -sine[row] * upper + cosine[row] * lower;
+      }
+      shared[0] = upper;
+    }
+    r.publish(norm2, 0.0, m + 1, false);
+    if (!r.grid_barrier()) return;
+    const double n2 = r.gathered(m + 1);
+    scale = n2 > 0.0 ? 1.0 / sqrt(n2) : 0.0;
+    if (threadIdx.x == kResidentNodeThreads) {
+      // ArnoldiLeastSquaresUpdate (gmres_device.hpp:62-98) and the stopping rule (:420-436).
+      const double sub = sqrt(n2), diagonal = shared[0], den = hypot(diagonal, sub);
+      const double c = den != 0.0 ? diagonal / den : 1.0, s = den != 0.0 ? sub / den : 0.0;
+      cosine[col] = c;
+      sine[col] = s;
+      H[col * (m + 1) + col] = c * diagonal + s * sub;
+      const double upper = rhs[col];
+      rhs[col] = c * upper;
+      rhs[col + 1] = -s * upper;
+      const double estimate = fabs(rhs[col + 1]);
+      const bool last = estimate <= p.tolerance || sub == 0.0 || col + 1 >= p.columns;
+      shared[1] = !isfinite(estimate) ? 2.0 : last ? 1.0 : 0.0;
+      shared[2] = sub == 0.0 ? 1.0 : 0.0;
+    } else if (threadIdx.x < kResidentNodeThreads) {
+      S* v = r.basis(col + 1);
+      for (int t = threadIdx.x; t < rows; t += kResidentNodeThreads) v[t] = S(double(image[t]) * scale);
+    }
+    ++col;
+  }
+  const bool breakdown = shared[2] != 0.0;
+  // Back substitution by columns (one warp), then x += V y.
+  __syncthreads();
+  if (warp == 0) {
+    double s = lane < col ? rhs[lane] : 0.0;
+    for (int row = col - 1; row >= 0; --row) {
+      const double diagonal = H[row * (m + 1) + row];
+      const double y = diagonal != 0.0 ? __shfl_sync(0xffffffffu, s, row) / diagonal : 0.0;
+      if (lane < row) s -= H[row * (m + 1) + lane] * y;
+      if (lane == 0) coefficient[row] = y;
+    }
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < rows; t += kResidentThreads) {
+    int n;
+    const long long at = place(t, n);
+    if (unode[n] < 0) continue;
+    double value = p.x[at];
+    const S* v = r.basis(0) + t;
+    const long long next = r.basis(1) - r.basis(0);
+    for (int c = 0; c < col; ++c) value += coefficient[c] * double(v[c * next]);
+    p.x[at] = value;
+  }
+  if (!r.grid_barrier()) return;
+  r.residual([&](int c, int u) { return __ldcg(p.x + c * U + u); }, false);
+  if (!r.grid_barrier()) return;
+  const double r2 = r.gathered(0);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    p.values[0] = r2;
+    p.ctl->completed = col;
+    p.ctl->stop = stop;
+    p.ctl->breakdown = breakdown ? 1 : 0;
+  }
+  if (sqrt(r2) <= p.accept) r.write_solution();
+  r.leave();
+}
+
+}  // namespace
+}  // namespace tpicb200

@@ -19,6 +19,7 @@
 // order, and stores the image straight into the compact Krylov vector: the
 // M records (504 B/node FP32, 1008 B/node FP64) are the only HBM stream.
 #include "kernels.cuh"
+#include "resident.cuh"
 #include "tcgen05.cuh"
 
 #include <cuda.h>
@@ -41,17 +42,6 @@ constexpr int kDotTile = 8;
 constexpr long long kColumnAlign = 64;
 // Largest GMRES restart the context accepts.
 constexpr int kMaxRestart = 1024;
-
-// Device-side state of one restart cycle's Arnoldi steps.
-struct ArnoldiControl {
-  int col;        // the step the step kernels take (0-based)
-  int completed;  // steps completed in this cycle
-  int columns;    // step limit of this cycle
-  int stop;       // 0 running; 1 stopped (tolerance, breakdown or limit); 2 nonfinite estimate
-  int breakdown;  // the last step's subdiagonal was zero
-  int pad;
-  double tolerance;
-};
 
 // Interior coordinates of compact index t (32-bit arithmetic: solver_create
 // requires 3 (n+1)^3 < 2^31).
@@ -850,6 +840,7 @@ __global__ void arnoldi_begin_kernel(ArnoldiControl* ctl, int columns, double to
   ctl->columns = columns;
   ctl->stop = 0;
   ctl->breakdown = 0;
+  ctl->failed = 0;
   ctl->tolerance = tolerance;
 }
 
@@ -925,6 +916,13 @@ struct SolverWorkspace {
   };
   MassMap maps[4];
   int next_map = 0;
+  // The resident kernels' plan (resident.cuh), where the grid takes them.
+  bool resident = false;
+  ResidentPlan plan{};
+  unsigned resident_grid = 0;
+  size_t resident_bytes = 0;
+  double* resident_partials = nullptr;
+  unsigned* resident_barrier = nullptr;
 
   double* hessenberg() { return state; }
   double* cosine() { return state + (size_t)restart * (restart + 1); }
@@ -934,6 +932,89 @@ struct SolverWorkspace {
   double* status() { return coefficients() + restart; }
   template <class S> S* basis_col(int c) { return (S*)basis + (size_t)c * ld; }
 };
+
+// The resident kernels of a precision: start and cycle, for A and A^T.
+template <class P>
+struct ResidentKernels {
+  using Kernel = void (*)(ResidentPlan);
+  static Kernel start() { return resident_start_kernel<typename P::EC, typename P::Mass, typename P::Fld, false>; }
+  static Kernel start_transposed() { return resident_start_kernel<typename P::EC, typename P::Mass, typename P::Fld, true>; }
+  static Kernel cycle() { return resident_cycle_kernel<typename P::EC, typename P::Mass, typename P::Fld, false>; }
+  static Kernel cycle_transposed() { return resident_cycle_kernel<typename P::EC, typename P::Mass, typename P::Fld, true>; }
+};
+
+// Tiles of the resident kernels: the smallest tile whose CTAs are all
+// resident at once, so that every SM has nodes and a node has many threads;
+// the basis in shared memory where that tile leaves room for it (FP64 256 x
+// 128 x 1: 325 us a solve with tiles of 128 nodes and the basis in global
+// memory, 410 us with 256 and the basis in shared memory). A grid that needs
+// more than two tiles of 256 nodes an SM keeps the step graph, whose applies
+// stream the mass better: at 400 x 300 x 1 several tiles a CTA took 1.45 ms
+// against its 1.15-1.39 ms, at 64^3 2.07 against 1.17-1.33 ms. Below, resident
+// against step graph, ms a solve (mixed, stencil-major): 1024 x 1 x 1 1.59 / 5.72,
+// 16^3 0.20 / 0.58, 32^3 0.31 / 0.59, 256 x 128 x 1 0.36 / 0.78, 256 x 256 x 1
+// 0.52 / 0.94.
+template <class P>
+void plan_resident(SolverWorkspace* w, int sms) {
+  using K = ResidentKernels<P>;
+  if (w->restart > kResidentRestart || w->smoothing.iterations > 0) return;
+  const Geom& g = w->g;
+  int device = 0, cooperative = 0, limit = 0;
+  if (cudaGetDevice(&device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, device) != cudaSuccess || !cooperative ||
+      cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess)
+    return;
+  const typename K::Kernel kernels[4] = {K::start(), K::start_transposed(), K::cycle(), K::cycle_transposed()};
+  for (auto k : kernels)
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, limit) != cudaSuccess) {
+      cudaGetLastError();
+      return;
+    }
+  auto power = [](int n) {
+    int p = 1;
+    while (p < n) p *= 2;
+    return p;
+  };
+  for (int nodes = 32; nodes <= kResidentNodeThreads; nodes *= 2) {
+    ResidentPlan p{};
+    p.g = g;
+    p.tx = std::min({power(g.nx), 32, nodes});
+    p.ty = std::min(power(g.ny), nodes / p.tx);
+    p.tz = std::min(power(g.nz), nodes / (p.tx * p.ty));
+    while (p.tx * p.ty * p.tz < nodes && p.tx < power(g.nx)) p.tx *= 2;
+    p.nodes = p.tx * p.ty * p.tz;
+    p.parts = kResidentNodeThreads / p.nodes;
+    while ((1 << p.shift) < p.nodes) ++p.shift;
+    p.tiles_x = (g.nx + p.tx - 1) / p.tx;
+    p.tiles_y = (g.ny + p.ty - 1) / p.ty;
+    p.tiles = p.tiles_x * p.tiles_y * ((g.nz + p.tz - 1) / p.tz);
+    p.restart = w->restart;
+    p.delta = w->delta;
+    p.kfac = w->kfac;
+    p.inv_volume = g.inv_volume;
+    for (int shared = 1; shared >= 0; --shared) {
+      p.shared_basis = shared != 0;
+      if (!p.shared_basis && 3LL * p.tiles * p.nodes > w->ld) continue;
+      const size_t bytes = resident_shared(p, sizeof(typename P::EC)).total;
+      if (bytes > size_t(limit)) continue;
+      int per_sm = 2;
+      for (auto k : kernels) {
+        int blocks = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k, kResidentThreads, bytes) != cudaSuccess) {
+          cudaGetLastError();
+          return;
+        }
+        per_sm = std::min(per_sm, blocks);
+      }
+      if (p.tiles > per_sm * sms) continue;
+      w->plan = p;
+      w->resident_grid = unsigned(p.tiles);
+      w->resident_bytes = bytes;
+      w->resident = true;
+      return;
+    }
+  }
+}
 
 SolverWorkspace* solver_create(int precision, const Geom& g, int restart, double dt, double theta,
                                double c, const SmoothingPlan& smoothing, cudaError_t* err) {
@@ -987,6 +1068,16 @@ SolverWorkspace* solver_create(int precision, const Geom& g, int restart, double
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&w->capture, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaMemset(w->input, 0, 3 * g.nodes * sizeof(double));
   if (e == cudaSuccess) e = cudaMemset(w->rhs, 0, 3 * g.nodes * sizeof(double));
+  if (e == cudaSuccess && !w->loop_unavailable) {
+    if (precision == TPICB200_PRECISION_DOUBLE) plan_resident<PDouble>(w, sms);
+    else plan_resident<PMixed>(w, sms);
+  }
+  if (w->resident) {
+    alloc((void**)&w->resident_partials, size_t(kResidentRestart + 2) * w->resident_grid * sizeof(double));
+    alloc((void**)&w->resident_barrier, 2 * sizeof(unsigned));
+    if (e == cudaSuccess) e = cudaMemset(w->resident_barrier, 0, 2 * sizeof(unsigned));
+    if (e == cudaSuccess) e = cudaMemset(w->ctl, 0, sizeof(ArnoldiControl));
+  }
   *err = e;
   if (e != cudaSuccess) {
     solver_destroy(w);
@@ -1001,6 +1092,7 @@ void solver_destroy(SolverWorkspace* w) {
   cudaFree(w->ximage); cudaFree(w->input); cudaFree(w->rhs); cudaFree(w->values);
   cudaFree(w->partials); cudaFree(w->state); cudaFree(w->ctl);
   cudaFree(w->smooth_a); cudaFree(w->smooth_b); cudaFree(w->smooth_image);
+  cudaFree(w->resident_partials); cudaFree(w->resident_barrier);
   for (int t = 0; t < 2; ++t) {
     if (w->loop_exec[t]) cudaGraphExecDestroy(w->loop_exec[t]);
     if (w->loop_graph[t]) cudaGraphDestroy(w->loop_graph[t]);
@@ -1366,11 +1458,88 @@ struct Solve {
     return w->conditional_checked;
   }
 
+  // The resident kernels (resident.cuh): one launch for the start and one per
+  // restart cycle. Not while a wait bound or a stall is set: those act on the
+  // applies of the step graph.
+  bool resident() const { return w->resident && w->wait_polls == 0 && w->stall_stencil < 0; }
+  // Launches one of them and reads its outcome back; false on a failure.
+  bool launch_resident(typename ResidentKernels<P>::Kernel kernel, double controls[2], ArnoldiControl* control) {
+    ResidentPlan p = w->plan;
+    void* args[] = {&p};
+    if (err == cudaSuccess)
+      err = cudaLaunchCooperativeKernel((const void*)kernel, dim3(w->resident_grid), dim3(kResidentThreads), args,
+                                        w->resident_bytes, s);
+    count_launches(1);
+    if (!read_back(w->values, controls, control)) return false;
+    if (control->failed) {
+      // A barrier ran out of polls: the next solve starts from clear counters.
+      cudaMemsetAsync(w->ctl, 0, sizeof(ArnoldiControl), s);
+      cudaMemsetAsync(w->resident_barrier, 0, 2 * sizeof(unsigned), s);
+      err = cudaErrorLaunchTimeout;
+      return false;
+    }
+    return true;
+  }
+  int run_resident(const void* e, const void* bcell, const void* j, const void* mass, double* etheta,
+                   tpicb200_gmres_result* result, int max_iterations, double tolerance, const double* rhs_in) {
+    using K = ResidentKernels<P>;
+    ResidentPlan& p = w->plan;
+    p.mass = mass;
+    p.vector = w->image;
+    p.basis = w->basis;
+    p.x = w->x;
+    p.b = w->b;
+    p.r = w->r;
+    p.values = w->values;
+    p.partials = w->resident_partials;
+    p.ctl = w->ctl;
+    p.barrier = w->resident_barrier;
+    p.e = e;
+    p.bcell = bcell;
+    p.j = j;
+    p.rhs = rhs_in;
+    p.etheta = etheta;
+    p.accept = tolerance;
+    tpicb200_gmres_result res{};
+    double controls[2];
+    ArnoldiControl control{};
+    if (!launch_resident(w->transpose ? K::start_transposed() : K::start(), controls, &control))
+      return TPICB200_BACKEND_FAILURE;
+    if (!std::isfinite(controls[0]) || !std::isfinite(controls[1])) return TPICB200_OVERFLOW;
+    res.residual = res.initial_residual = std::sqrt(controls[0]);
+    res.rhs_norm = std::sqrt(controls[1]);
+    const double scale = res.rhs_norm == 0.0 ? 1.0 : res.rhs_norm;
+    const double atol = scale * tolerance;
+    auto converged = [&] {
+      res.relative_residual = res.residual / scale;
+      res.converged = res.residual <= atol;
+    };
+    converged();
+    while (!res.converged && res.iterations < max_iterations) {
+      p.columns = std::min(w->restart, max_iterations - res.iterations);
+      p.tolerance =
+          refined ? std::max(atol, res.residual * 16.0 * double(std::numeric_limits<S>::epsilon())) : atol;
+      p.accept = atol;
+      if (!launch_resident(w->transpose ? K::cycle_transposed() : K::cycle(), controls, &control))
+        return TPICB200_BACKEND_FAILURE;
+      if (control.stop == 2) return TPICB200_OVERFLOW;
+      if (!std::isfinite(controls[0]) || controls[0] < 0) return TPICB200_OVERFLOW;
+      res.iterations += control.completed;
+      res.residual = std::sqrt(controls[0]);
+      converged();
+      if (control.breakdown && !res.converged) break;
+    }
+    res.host_waits = waits;
+    if (result) *result = res;
+    return res.converged ? TPICB200_SUCCESS : TPICB200_NOT_CONVERGED;
+  }
+
   // With rhs_in (a double node field, the adjoint solve): that right-hand
   // side and a zero initial guess; otherwise the Maxwell RHS from e, bcell
   // and j with the guess E^n.
   int run(const void* e, const void* bcell, const void* j, const void* mass_v, double* etheta,
           tpicb200_gmres_result* result, int max_iterations, double tolerance, const double* rhs_in = nullptr) {
+    if (resident()) return run_resident(e, bcell, j, mass_v, etheta, result, max_iterations, tolerance, rhs_in);
     const Geom& g = w->g;
     const Mass* mass = (const Mass*)mass_v;
     const long long N = w->count;
