@@ -25,7 +25,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
           "-Xptxas", "-warn-spills"]
 PER_FILE = {"mover.cu": ["-fmad=false"], "load.cu": ["-fmad=false"]}
-SOURCES = ["abi.cu", "mover.cu", "sort.cu", "deposit.cu", "fields.cu", "solver.cu", "mass_tc.cu", "cases.cu",
+SOURCES = ["abi.cu", "mover.cu", "sort.cu", "deposit.cu", "fields.cu", "solver.cu", "mass_tc.cu", "moments.cu", "cases.cu",
            "load.cu", "checkpoint.cu", "adjoint.cu", "output.cu", "gauss.cu"]
 
 

@@ -99,12 +99,29 @@ cudaError_t launch_moments(tpicb200_context* ctx, int kind, int ns, const double
                            const tpicb200_particles* const* parts, const uint32_t* const* counts,
                            const uint32_t* const* offsets, const void* b_node, int accumulate, uint32_t* invalid,
                            const SortedCopy* const* copies, cudaStream_t s) {
-  if (kind == TPICB200_MASS_MOMENTS_F64)
-    return launch_deposit_moments_f64(ctx->g, ns, qom, ctx->opt.dt, ctx->opt.c, parts, counts, offsets, b_node,
-                                      (double*)ctx->moments, accumulate, invalid, copies, s);
+  if (kind != TPICB200_MASS_TF32 && kind != TPICB200_MASS_BF16X3)
+    return launch_deposit_moments(ctx->opt.precision, kind, ctx->g, ns, qom, ctx->opt.dt, ctx->opt.c, parts, counts,
+                                  offsets, b_node, ctx->moments, accumulate, invalid, copies, s);
   return launch_deposit_tc(kind, ctx->g, ns, qom, ctx->opt.dt, ctx->opt.c, parts, counts, offsets, b_node,
                            (float*)ctx->moments, accumulate, invalid, copies, s, ctx->wait_polls,
                            ctx->stall_site == TPICB200_STALL_DEPOSIT ? ctx->stall_index : 0u);
+}
+
+// The scalar forms deposit J and the mass of sorted records through the
+// context's moments too, assembled within the call; not while those hold
+// moments that wait for the fold.
+bool sums_by_moments(const tpicb200_context* ctx, const void* j, const void* mass) {
+  return j && mass && !ctx->moments_pending;
+}
+int deposit_through_moments(tpicb200_context* ctx, int kind, int ns, const double* qom,
+                            const tpicb200_particles* const* parts, const uint32_t* const* counts,
+                            const uint32_t* const* offsets, const void* b_node, void* j, void* mass,
+                            uint32_t* invalid, cudaStream_t s) {
+  const int overwrite = j == ctx->cleared_j && mass == ctx->cleared_mass ? 1 : 0;
+  ctx->cleared_j = ctx->cleared_mass = nullptr;
+  cudaError_t e = launch_moments(ctx, kind, ns, qom, parts, counts, offsets, b_node, 0, invalid, nullptr, s);
+  if (e == cudaSuccess) e = launch_assemble_moments(ctx->opt.precision, ctx->g, ctx->moments, j, mass, overwrite, s);
+  return cuda_status(e, "deposition launch failed");
 }
 
 }  // namespace
@@ -374,9 +391,11 @@ int tpicb200_deposit(tpicb200_context* ctx, double qom, const tpicb200_particles
     if (r == TPICB200_SUCCESS) ctx->moments_pending = true;
     return r;
   }
+  if (sums_by_moments(ctx, j, mass) && counts) return deposit_through_moments(ctx, mass_kind, 1, &qom, &p, &counts,
+                                                                              &offsets, b_node, j, mass, inv, s);
   ctx->cleared_j = ctx->cleared_mass = nullptr;
   return cuda_status(launch_deposit(ctx->opt.precision, mass_kind, ctx->g, qom, ctx->opt.dt, ctx->opt.c, p,
-                                    counts, offsets, b_node, j, mass, inv, nullptr, s),
+                                    counts, offsets, b_node, j, mass, inv, s),
                      "deposition launch failed");
 }
 
@@ -533,14 +552,17 @@ int tpicb200_deposit_species(tpicb200_context* ctx, int ns, const double* qom, c
   if (int s = check_ctx(ctx)) return s;
   if (ns < 0 || ns > TPICB200_MAX_SPECIES || (ns > 0 && (!qom || !species || !counts || !offsets)))
     return fail(TPICB200_INVALID_ARGUMENT, "invalid species arrays");
-  if (!moment_form(mass_kind)) {
+  bool sorted = ns > 0;
+  for (int sp = 0; sp < ns; ++sp) sorted = sorted && counts[sp] && offsets[sp];
+  const bool through = !moment_form(mass_kind) && sorted && b_node && sums_by_moments(ctx, j, mass);
+  if (!moment_form(mass_kind) && !through) {
     for (int sp = 0; sp < ns; ++sp)
       if (int r = tpicb200_deposit(ctx, qom[sp], &species[sp], counts[sp], offsets[sp], b_node, j, mass, mass_kind,
                                    invalid, stream))
         return r;
     return TPICB200_SUCCESS;
   }
-  // Moment forms: the per-species checks of tpicb200_deposit, then one
+  // Through moments: the per-species checks of tpicb200_deposit, then one
   // fused pass per species pair.
   if (int r = check_mass_kind(ctx, mass_kind)) return r;
   if (!b_node) return fail(TPICB200_INVALID_ARGUMENT, "deposit needs B nodes");
@@ -554,6 +576,9 @@ int tpicb200_deposit_species(tpicb200_context* ctx, int ns, const double* qom, c
     if (!std::isfinite(qom[sp])) return fail(TPICB200_INVALID_ARGUMENT, "deposit needs finite q/m");
     if (!std::isfinite(qom[sp] * ctx->opt.dt / 2 / ctx->opt.c)) return fail(TPICB200_OVERFLOW, "beta/c is not finite");
   }
+  if (through)
+    return deposit_through_moments(ctx, mass_kind, ns, qom, parts, counts, offsets, b_node, j, mass,
+                                   invalid_or_own(ctx, invalid), (cudaStream_t)stream);
   const int r = cuda_status(launch_moments(ctx, mass_kind, ns, qom, parts, counts, offsets, b_node,
                                            ctx->moments_pending ? 1 : 0, invalid_or_own(ctx, invalid), nullptr,
                                            (cudaStream_t)stream),
@@ -713,20 +738,10 @@ static int deposit_pair(tpicb200_context* ctx, tpicb200_state* st, int first, in
     offsets[i] = st->offsets[sp];
     qom[i] = st->qom[sp];
   }
-  const int kind = st->mass_kind;
-  const int p = ctx->opt.precision;
-  cudaError_t e = cudaSuccess;
-  if (moment_form(kind)) {
-    if (int r = check_mass_kind(ctx, kind)) return r;
-    e = launch_moments(ctx, kind, count, qom, parts, counts, offsets, st->b_node_next, accumulate ? 1 : 0,
-                       ctx->invalid, copies, s);
-    if (e == cudaSuccess) ctx->moments_pending = true;
-  } else {
-    ctx->cleared_j = ctx->cleared_mass = nullptr;
-    for (int i = 0; i < count && e == cudaSuccess; ++i)
-      e = launch_deposit(p, kind, ctx->g, qom[i], ctx->opt.dt, ctx->opt.c, parts[i], counts[i], offsets[i],
-                         st->b_node_next, st->j, st->mass, ctx->invalid, copies[i], s);
-  }
+  if (int r = check_mass_kind(ctx, st->mass_kind)) return r;
+  cudaError_t e = launch_moments(ctx, st->mass_kind, count, qom, parts, counts, offsets, st->b_node_next,
+                                 accumulate ? 1 : 0, ctx->invalid, copies, s);
+  if (e == cudaSuccess) ctx->moments_pending = true;
   for (int i = 0; i < count && e == cudaSuccess; ++i) e = launch_copy_ids(parts[i], copies[i], s);
   if (e != cudaSuccess) return cuda_status(e, "deposition launch failed");
   for (int i = 0; i < count; ++i)
@@ -871,15 +886,12 @@ int tpicb200_cycle(tpicb200_context* ctx, tpicb200_state* st, int ncycles, tpicb
     cudaEventRecord(ev[2], s);
     // Per pair of species: the mover and the sort of each, then one
     // deposition of both with the next B that also writes the sorted records.
-    // The moment forms need no cleared J and mass: the assembly stores
-    // every entry of the unique nodes and the fold copies every other vertex.
-    if (moment_form(kind) && st->ns > 0) {
-      ctx->moments_pending = false;
-      ctx->cleared_j = st->j;
-      ctx->cleared_mass = st->mass;
-    } else if (int r = tpicb200_clear_moments(ctx, st->j, st->mass, stream)) {
-      return r;
-    }
+    // Every form deposits cell moments; they need no cleared J and mass: the
+    // assembly stores every entry of the unique nodes and the fold copies
+    // every other vertex.
+    ctx->moments_pending = false;
+    ctx->cleared_j = st->j;
+    ctx->cleared_mass = st->mass;
     for (int first = 0; first < st->ns; first += 2) {
       const int count = st->ns - first < 2 ? st->ns - first : 2;
       DepositPlan plan[2];

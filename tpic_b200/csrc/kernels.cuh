@@ -117,11 +117,12 @@ cudaError_t launch_copy_ids(const tpicb200_particles* in, const SortedCopy* copy
 cudaError_t launch_sorted_gather(int precision, const uint32_t* perm, const tpicb200_particles* in,
                                  tpicb200_particles* out, cudaStream_t s);
 
-// deposit.cu
+// deposit.cu: per-record and per-cell deposition with atomics, for records
+// without bins, for one output alone, and while moments await their assembly.
 cudaError_t launch_deposit(int precision, int mass_kind, const Geom& g, double qom, double dt,
                            double c, const tpicb200_particles* p, const uint32_t* counts,
                            const uint32_t* offsets, const void* bnode, void* j, void* mass,
-                           uint32_t* invalid, const SortedCopy* copy, cudaStream_t s);
+                           uint32_t* invalid, cudaStream_t s);
 cudaError_t launch_fold(int precision, const Geom& g, void* j, void* mass, cudaStream_t s);
 
 // mass_tc.cu (tcgen05 forms): per-cell moments, then their assembly into J
@@ -139,12 +140,13 @@ cudaError_t launch_deposit_tc(int mass_kind, const Geom& g, int ns, const double
                               const uint32_t* const* offsets, const void* bnode, float* moments, int accumulate,
                               uint32_t* invalid, const SortedCopy* const* copies, cudaStream_t s,
                               uint32_t wait_polls = 0, uint32_t stall_chunk = 0);
-// FP64 CUDA-core form of the same moments (double precision; double moments).
-cudaError_t launch_deposit_moments_f64(const Geom& g, int ns, const double* qom, double dt, double c,
-                                       const tpicb200_particles* const* p, const uint32_t* const* counts,
-                                       const uint32_t* const* offsets, const void* bnode, double* moments,
-                                       int accumulate, uint32_t* invalid, const SortedCopy* const* copies,
-                                       cudaStream_t s);
+// moments.cu: the same moments off the tcgen05 forms. SCALAR in mixed precision
+// takes FP32 arithmetic and sums; the other forms FP64 ones (SCALAR_F64 in
+// mixed precision narrows a cell's moments once, into the float moments).
+cudaError_t launch_deposit_moments(int precision, int mass_kind, const Geom& g, int ns, const double* qom, double dt,
+                                   double c, const tpicb200_particles* const* p, const uint32_t* const* counts,
+                                   const uint32_t* const* offsets, const void* bnode, void* moments, int accumulate,
+                                   uint32_t* invalid, const SortedCopy* const* copies, cudaStream_t s);
 // Moments (float or double, as the precision mode) into J and the mass records.
 cudaError_t launch_assemble_moments(int precision, const Geom& g, const void* moments, void* j, void* mass,
                                     int overwrite, cudaStream_t s);

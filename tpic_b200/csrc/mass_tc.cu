@@ -46,6 +46,7 @@
 // tcgen05.mma.kind::f16 (BF16 inputs, FP32 accumulation, K = 16); B then has
 // 16 columns per cell (N = 64) so each cell's block is whole 16-byte core rows.
 #include "kernels.cuh"
+#include "moments.cuh"
 #include "tcgen05.cuh"
 
 #include <algorithm>
@@ -57,16 +58,8 @@ namespace {
 
 constexpr int kCells = 4;          // cells per CTA group (one per warp)
 constexpr int kChunk = 32;         // particles per chunk (one per lane)
-constexpr int kFuse = 2;           // species per launch
 constexpr int kFacStride = 36;     // floats per factor row (16-byte aligned rows)
 constexpr uint32_t kTmemCols = 128;
-constexpr int kMassMoments = 27 * 9;                  // G[t][c] per cell
-constexpr int kMoments = kMassMoments + 24;           // + J corner sums [a][c]
-// Moment layout: each group of four consecutive cells has one contiguous
-// record of kMoments 16-byte words, word q holding entry q of the four cells.
-__host__ __device__ constexpr long long moment_index(long long cell, int q) {
-  return ((cell >> 2) * kMoments + q) * 4 + (cell & 3);
-}
 constexpr uint32_t kDcol = 64;
 constexpr int kCtasPerSm = 4;      // 4 x 128 tensor-memory columns = all 512
 constexpr int kPermBuf = 256;      // ranks of a cell staged ahead (per warp and group)
@@ -82,11 +75,6 @@ template <bool Bf16> struct Form {
   static constexpr uint32_t tile_bytes = Bf16 ? uint32_t(n / 8) * 512u : 8u * kTf32KChunk;
   static constexpr int tiles = Bf16 ? 2 : 1;         // hi (+ lo)
 };
-
-// Monomial class of the corner pair (a, b).
-__host__ __device__ constexpr int monomial_class(int a, int b) {
-  return ((a & 1) + (b & 1)) + 3 * (((a >> 1) & 1) + ((b >> 1) & 1)) + 9 * (((a >> 2) & 1) + ((b >> 2) & 1));
-}
 
 struct TcSpecies {
   const double* rx;
@@ -1466,214 +1454,6 @@ __global__ void __launch_bounds__(128) assemble_warp_quads_kernel(Geom g, const 
   }
 }
 
-
-
-// ---------------------------------------------------------------------------
-// FP64 form of the moment deposition (double precision).
-//
-// The same per-cell moments as the tensor-core forms, G[t][e] = sum_p m_pt
-// (s_p alpha_p[e]) and H[t][c] = sum_p m_pt j_p[c], accumulated in FP64: a
-// warp per cell; per chunk of 32 records each lane forms one record's B
-// gather, response, s alpha and j (12 values) and its 27 pair-weight products
-// m_t = (X_tx Y_ty) Z_tz into shared memory; then the warp contracts the
-// chunk on the FP64 tensor cores (mma.sync m8n8k4: D[t][e] += sum_k m[k][t]
-// src[k][e], t in four tiles of 8 rows (27 used), e in two of 8 columns (12
-// used), four records per step). The contraction on the CUDA cores (a 3 x 4
-// register block per lane, 7 shared loads per 12 fused multiply-adds) was
-// bound by the shared-memory pipe (93 % of its wavefronts at 64^3); the
-// fragments need 6 shared loads per 4 records and lane (128^3-cell workload:
-// the FP64 deposit stage 20.0 -> 16.1 ms). The flush stores G and the corner
-// currents J_a[c] = sum_b H[t(a,b)][c] into the double moment records, which
-// the assembly adds into J and the mass records as for the tensor-core forms.
-// Per record this is 27 x 12 multiply-adds, where the reference's scalar and
-// matrix-core kernels form the 64 corner-pair products of 9 entries
-// (mass_matrix_scalar_device.hpp:25-97, mass_matrix_mma_device.hpp:58-150).
-struct F64Species {
-  const double* rx;
-  const double* ry;
-  const double* rz;
-  const double* u;
-  const double* v;
-  const double* w;
-  const double* q;
-  const int32_t* key;
-  const uint32_t* counts;
-  const uint32_t* offsets;
-  double beta_over_c;
-  const uint32_t* perm;  // sorted position -> record (null: records in sorted order)
-  double* orx;           // sorted copy (null: none)
-  double* ory;
-  double* orz;
-  double* ou;
-  double* ov;
-  double* ow;
-  double* oq;
-  int32_t* okey;
-};
-
-struct F64Params {
-  F64Species sp[kFuse];
-  int ns;
-  double inv_volume;
-};
-
-// D (8 x 8) += A (8 x 4) B (4 x 8) in FP64 on the tensor cores. Per lane:
-// A[lane >> 2][lane & 3], B[lane & 3][lane >> 2], D[lane >> 2][2 (lane & 3) + i].
-__device__ __forceinline__ void dmma_884(double (&d)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
-}
-
-constexpr int kF64Warps = 4;
-// The products and values are stored by (t or entry, record), 36 records a
-// row: a lane's stores of its record fall in consecutive words, and the 16
-// lanes of a half-warp fragment load (4 rows x 4 records) hit 16 different
-// bank pairs. With record-major rows of 29 and 13 words the fragment loads
-// met 2-way conflicts (C3 FP64 deposit stage 16.2 ms, 15.7 ms with these rows).
-constexpr int kF64Pitch = 36;
-struct F64Warp {
-  double bc[24];                 // B at the cell's corners, [c][a]
-  double m[27][kF64Pitch];       // [t][record]: the 27 pair-weight products
-  double src[12][kF64Pitch];     // [entry][record]: s alpha[9], j[3]
-  double hs[27][3];              // H of the cell at the flush
-};
-
-__global__ void __launch_bounds__(kF64Warps * 32) moments_f64_kernel(Geom g, F64Params fp,
-                                                                     const double* __restrict__ bnode,
-                                                                     double* __restrict__ mom, int accumulate,
-                                                                     uint32_t* invalid) {
-  __shared__ F64Warp shared[kF64Warps];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  F64Warp& S = shared[warp];
-  const int nx = g.nx, ny = g.ny;
-  const long long cells = (long long)nx * ny * g.nz, nn = g.nodes;
-  const int kk = lane & 3, rr = lane >> 2;  // fragment coordinates
-  uint32_t bad = 0;
-  for (long long cell = (long long)blockIdx.x * kF64Warps + warp; cell < cells;
-       cell += (long long)gridDim.x * kF64Warps) {
-    const int ci = int(cell % nx), cj = int((cell / nx) % ny), ck = int(cell / ((long long)nx * ny));
-    const int32_t key = g.encode(ci, cj, ck);
-    if (lane < 24) {
-      const int c = lane >> 3, a = lane & 7;
-      S.bc[lane] = bnode[c * nn + g.node(ci + (a & 1), cj + ((a >> 1) & 1), ck + ((a >> 2) & 1))];
-    }
-    __syncwarp();
-    // D tiles (t: 4 x 8 rows, entry: 2 x 8 columns) of this lane.
-    double acc[4][2][2];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) acc[i][e][0] = acc[i][e][1] = 0.0;
-    for (int si = 0; si < fp.ns; ++si) {
-      const F64Species& sp = fp.sp[si];
-      const uint32_t begin = sp.offsets[key], n = sp.counts[key];
-      for (uint32_t c0 = 0; c0 < n; c0 += 32) {
-        const uint32_t m = n - c0 < 32u ? n - c0 : 32u;
-        if (lane < int(m)) {
-          const uint32_t pos = begin + c0 + lane;
-          const uint32_t r = sp.perm ? sp.perm[pos] : pos;
-          const double fx = sp.rx[r], fy = sp.ry[r], fz = sp.rz[r];
-          const double u = sp.u[r], v = sp.v[r], w = sp.w[r], q = sp.q[r];
-          const int32_t k0 = sp.key[r];
-          if (sp.orx) {
-            sp.orx[pos] = fx; sp.ory[pos] = fy; sp.orz[pos] = fz;
-            sp.ou[pos] = u; sp.ov[pos] = v; sp.ow[pos] = w; sp.oq[pos] = q; sp.okey[pos] = k0;
-          }
-          bool ok = k0 == key && fx >= 0 && fx < 1 && fy >= 0 && fy < 1 && fz >= 0 && fz < 1;
-          if (ok) {
-            double wt[8];
-            cic_weights<double>(fx, fy, fz, wt);
-            double b[3];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-              double val = 0;
-#pragma unroll
-              for (int a = 0; a < 8; ++a) val += wt[a] * S.bc[c * 8 + a];
-              b[c] = val;
-            }
-            const Response<double> resp(b[0], b[1], b[2], sp.beta_over_c);
-            const double scale = sp.beta_over_c * q;
-            double hx, hy, hz;
-            resp.apply(u, v, w, hx, hy, hz);
-            const double qv = q * fp.inv_volume;
-            double sv[12];
-#pragma unroll
-            for (int e = 0; e < 9; ++e) sv[e] = resp.a[e] * scale;
-            sv[9] = qv * hx; sv[10] = qv * hy; sv[11] = qv * hz;
-#pragma unroll
-            for (int e = 0; e < 12; ++e) {
-              ok = ok && isfinite(sv[e]);
-              S.src[e][lane] = sv[e];
-            }
-            const double cx = 1.0 - fx, cy = 1.0 - fy, cz = 1.0 - fz;
-            const double px[3] = {cx * cx, cx * fx, fx * fx};
-            const double py[3] = {cy * cy, cy * fy, fy * fy};
-            const double pz[3] = {cz * cz, cz * fz, fz * fz};
-#pragma unroll
-            for (int ty = 0; ty < 3; ++ty)
-#pragma unroll
-              for (int tx = 0; tx < 3; ++tx) {
-                const double pxy = px[tx] * py[ty];
-#pragma unroll
-                for (int tz = 0; tz < 3; ++tz) S.m[tx + 3 * ty + 9 * tz][lane] = pxy * pz[tz];
-              }
-          }
-          if (!ok) {
-            ++bad;
-#pragma unroll
-            for (int e = 0; e < 12; ++e) S.src[e][lane] = 0.0;
-#pragma unroll
-            for (int t = 0; t < 27; ++t) S.m[t][lane] = 0.0;
-          }
-        }
-        __syncwarp();
-        for (uint32_t k0 = 0; k0 < m; k0 += 4) {
-          const uint32_t k = k0 + kk;
-          const bool in = k < m;
-          double av[4], bv[2];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) av[i] = in && 8 * i + rr < 27 ? S.m[8 * i + rr][k] : 0.0;
-#pragma unroll
-          for (int e = 0; e < 2; ++e) bv[e] = in && 8 * e + rr < 12 ? S.src[8 * e + rr][k] : 0.0;
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) dmma_884(acc[i][e], av[i], bv[e]);
-        }
-        __syncwarp();
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int e = 0; e < 2; ++e)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int t = 8 * i + rr, entry = 8 * e + 2 * kk + h;
-          if (t >= 27 || entry >= 12) continue;
-          if (entry < 9) {
-            double* dst = mom + moment_index(cell, t * 9 + entry);
-            *dst = accumulate ? *dst + acc[i][e][h] : acc[i][e][h];
-          } else {
-            S.hs[t][entry - 9] = acc[i][e][h];
-          }
-        }
-    __syncwarp();
-    if (lane < 24) {
-      const int a = lane / 3, c = lane % 3;
-      double sum = 0.0;
-#pragma unroll
-      for (int b = 0; b < 8; ++b) sum += S.hs[monomial_class(a, b)][c];
-      double* dst = mom + moment_index(cell, kMassMoments + a * 3 + c);
-      *dst = accumulate ? *dst + sum : sum;
-    }
-    __syncwarp();
-  }
-  bad = warp_sum(bad);
-  if (bad && lane == 0) atomicAdd(invalid, bad);
-}
-
 }  // namespace
 
 cudaError_t launch_assemble_moments(int precision, const Geom& g, const void* moments, void* j, void* mass,
@@ -1701,39 +1481,6 @@ cudaError_t launch_assemble_moments(int precision, const Geom& g, const void* mo
   }
   count_launches(1);
   return cudaGetLastError();
-}
-
-cudaError_t launch_deposit_moments_f64(const Geom& g, int ns, const double* qom, double dt, double c,
-                                       const tpicb200_particles* const* p, const uint32_t* const* counts,
-                                       const uint32_t* const* offsets, const void* bnode, double* moments,
-                                       int accumulate, uint32_t* invalid, const SortedCopy* const* copies,
-                                       cudaStream_t s) {
-  if (!moments || ns < 1) return cudaErrorInvalidValue;
-  const long long cells = (long long)g.nx * g.ny * g.nz;
-  const unsigned blocks = unsigned(std::min<long long>((cells + kF64Warps - 1) / kF64Warps, 148LL * 16));
-  for (int first = 0; first < ns; first += kFuse) {
-    F64Params fp{};
-    fp.ns = std::min(kFuse, ns - first);
-    fp.inv_volume = g.inv_volume;
-    for (int i = 0; i < fp.ns; ++i) {
-      const tpicb200_particles* sp = p[first + i];
-      const SortedCopy* cp = copies ? copies[first + i] : nullptr;
-      const bool copy = cp && cp->perm && cp->out.rx;
-      fp.sp[i] = F64Species{(const double*)sp->rx, (const double*)sp->ry, (const double*)sp->rz,
-                            (const double*)sp->u, (const double*)sp->v, (const double*)sp->w, sp->q, sp->cell,
-                            counts[first + i], offsets[first + i], qom[first + i] * dt / 2 / c,
-                            cp ? cp->perm : nullptr, copy ? (double*)cp->out.rx : nullptr,
-                            copy ? (double*)cp->out.ry : nullptr, copy ? (double*)cp->out.rz : nullptr,
-                            copy ? (double*)cp->out.u : nullptr, copy ? (double*)cp->out.v : nullptr,
-                            copy ? (double*)cp->out.w : nullptr, copy ? cp->out.q : nullptr,
-                            copy ? cp->out.cell : nullptr};
-    }
-    moments_f64_kernel<<<blocks, kF64Warps * 32, 0, s>>>(g, fp, (const double*)bnode, moments,
-                                                        (accumulate || first > 0) ? 1 : 0, invalid);
-    count_launches(1);
-    if (cudaError_t e = cudaGetLastError()) return e;
-  }
-  return cudaSuccess;
 }
 
 }  // namespace tpicb200
