@@ -74,3 +74,29 @@ def test_resident_solve_equals_the_step_graph(torch_cuda, shape, precision, adjo
         assert float((got - want).abs().max()) <= 20 * tol * max(res.rhs_norm, scale)
         ctx.close()
     assert torch.equal(stepped[1], stepped[2]) and torch.equal(stepped[0], stepped[1])
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (3, 1, 1), (70, 1, 1), (5, 3, 1), (40, 24, 1), (1, 33, 1), (150, 90, 1)],
+                         ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("smoothing", [(1, 0.5, 0), (6, 0.5, 0), (3, 0.25, 1), (8, 0.75, 0)])
+def test_resident_smoothed_solve_equals_the_step_graph(torch_cuda, shape, precision, smoothing):
+    """Halos wider than the grid (every pass reads periodic copies of copies) and of several tiles."""
+    import torch
+    from gpu_helpers import StageContext
+    g = GridSpec(*shape, *(0.1 * n for n in shape))
+    rng = np.random.default_rng(sum(shape))
+    tol = 1e-10
+    ctx = StageContext(g, precision=precision, dt=0.1, tol=tol, mass_layout=1, max_iterations=300, restart=20,
+                       smoothing=smoothing)
+    inputs = (ctx.field(periodic_node_field(g, smooth_random_unique(g, rng, 0.01))),
+              ctx.field(periodic_cell_field(g, smooth_random_unique(g, rng, 0.05))),
+              ctx.field(periodic_node_field(g, smooth_random_unique(g, rng, 0.02))),
+              ctx.mass_from_records(random_mass(g, rng, dt=0.1)))
+    got, res = ctx.field_solve(*inputs)
+    _lib.check(ctx.lib.tpicb200_set_wait_limit(ctx.ctx, 1 << 22))
+    want, ref = ctx.field_solve(*inputs)
+    assert res.converged and ref.converged and abs(res.iterations - ref.iterations) <= 1
+    scale = np.abs(interior_nodes(g, want.cpu().numpy())).max()
+    assert float((got - want).abs().max()) <= 20 * tol * max(res.rhs_norm, scale)
+    ctx.close()

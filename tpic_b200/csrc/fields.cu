@@ -2,6 +2,7 @@
 // B, the Maxwell right-hand side, the E/B advance and the energy reductions.
 // All are HBM-streaming stencils, one thread per target sample.
 #include "kernels.cuh"
+#include "smoothing.cuh"
 #include "stencils.cuh"
 
 namespace tpicb200 {
@@ -261,82 +262,98 @@ cudaError_t launch_rhs(int precision, const Geom& g, double delta, double kfac, 
   return cudaGetLastError();
 }
 
-// Energy-conserving smoothing, one pass (node_smoothing_kernel,
-// ecsim/fields/node_smoothing_device.hpp:17-36, with the operator of
-// ecsim/fields/node_smoothing.hpp:24-52): every interior node 0..n of the
-// three components, from a double node field with filled ghosts into a
-// double node field, in arithmetic C with each product and sum rounded on
-// its own (no contraction) in the reference's order. Op 0 Face7: alpha *
-// centre + beta * faces; op 1 Binomial27: (8 centre + 4 faces + 2 edges +
-// corners) * (1/64). A nonfinite result counts in *invalid (when given), as
-// the reference's kernel flags it (node_smoothing_device.hpp:30-36).
-__device__ __forceinline__ float rn_mul(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double rn_mul(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ float rn_add(float a, float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ double rn_add(double a, double b) { return __dadd_rn(a, b); }
+// `passes` smoothing passes of a double node field into another, the tile and
+// its halo in shared memory (blockIdx.x a tile of unique nodes, blockIdx.y a
+// component). Neighbours
+// are read from the unique nodes by their periodic index, and every stored
+// copy of a node is written, so no ghost fill is needed before, between or
+// after. One launch per pass with a ghost fill behind it took 12 launches for
+// the default six passes, some 55 us on 256 x 128 x 1, where the passes
+// themselves are 1 us each; the halo costs (32 + 12)(8 + 12) / (32 x 8) = 3.4
+// times the nodes there. On grids thicker than one cell three passes a launch
+// (tile 16 x 8 x 8) keep that factor at 4.2.
+constexpr int kSmoothThreads = 256;
 
-template <class C, int Op>
-__global__ void __launch_bounds__(256) smooth_kernel(Geom g, C alpha, C beta, const double* __restrict__ src,
-                                                     double* __restrict__ dst, uint32_t* invalid) {
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < 3 * g.interior;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int c = int(t / g.interior);
-    int i, j, k;
-    interior_node_coordinates(g, t - c * g.interior, i, j, k);
-    const double* f = src + c * g.nodes;
-    auto v = [&](int a, int b, int d) { return C(f[g.node(a, b, d)]); };
-    const C face = rn_add(rn_add(rn_add(rn_add(rn_add(v(i - 1, j, k), v(i + 1, j, k)), v(i, j - 1, k)),
-                                        v(i, j + 1, k)), v(i, j, k - 1)), v(i, j, k + 1));
-    C value;
-    if constexpr (Op == 0) {
-      value = rn_add(rn_mul(alpha, v(i, j, k)), rn_mul(beta, face));
-    } else {
-      C edge = rn_add(v(i - 1, j - 1, k), v(i + 1, j - 1, k));
-      edge = rn_add(edge, v(i - 1, j + 1, k)); edge = rn_add(edge, v(i + 1, j + 1, k));
-      edge = rn_add(edge, v(i - 1, j, k - 1)); edge = rn_add(edge, v(i + 1, j, k - 1));
-      edge = rn_add(edge, v(i - 1, j, k + 1)); edge = rn_add(edge, v(i + 1, j, k + 1));
-      edge = rn_add(edge, v(i, j - 1, k - 1)); edge = rn_add(edge, v(i, j + 1, k - 1));
-      edge = rn_add(edge, v(i, j - 1, k + 1)); edge = rn_add(edge, v(i, j + 1, k + 1));
-      C corner = rn_add(v(i - 1, j - 1, k - 1), v(i + 1, j - 1, k - 1));
-      corner = rn_add(corner, v(i - 1, j + 1, k - 1)); corner = rn_add(corner, v(i + 1, j + 1, k - 1));
-      corner = rn_add(corner, v(i - 1, j - 1, k + 1)); corner = rn_add(corner, v(i + 1, j - 1, k + 1));
-      corner = rn_add(corner, v(i - 1, j + 1, k + 1)); corner = rn_add(corner, v(i + 1, j + 1, k + 1));
-      const C sum = rn_add(rn_add(rn_add(rn_mul(C(8), v(i, j, k)), rn_mul(C(4), face)), rn_mul(C(2), edge)), corner);
-      value = rn_mul(sum, C(1) / C(64));
+template <class C>
+__global__ void __launch_bounds__(kSmoothThreads) smooth_tile_kernel(Geom g, SmoothTile t, int tx, int ty, int tz,
+                                                                     int passes, int op, double alpha,
+                                                                     const double* __restrict__ src,
+                                                                     double* __restrict__ dst, uint32_t* invalid) {
+  extern __shared__ __align__(16) uint8_t smooth_smem[];
+  C* a = reinterpret_cast<C*>(smooth_smem);
+  C* b = a + t.size;
+  src += blockIdx.y * g.nodes;
+  dst += blockIdx.y * g.nodes;
+  const int tiles_x = (g.nx + tx - 1) / tx, tiles_y = (g.ny + ty - 1) / ty;
+  const int row = blockIdx.x / tiles_x;
+  const int i0 = (blockIdx.x - row * tiles_x) * tx, j0 = (row % tiles_y) * ty, k0 = (row / tiles_y) * tz;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = kSmoothThreads / 32;
+  const int rows = t.e[1] * t.e[2];
+  for (int r = warp; r < rows; r += warps) {
+    const int z = r / t.e[1], y = r - z * t.e[1];
+    const long long at = g.node(0, wrap_index(j0 - t.h[1] + y, g.ny), wrap_index(k0 - t.h[2] + z, g.nz));
+    for (int x = lane; x < t.e[0]; x += 32) a[r * t.e[0] + x] = C(src[at + wrap_index(i0 - t.h[0] + x, g.nx)]);
+  }
+  __syncthreads();
+  const int nx = min(tx, g.nx - i0), ny = min(ty, g.ny - j0), nz = min(tz, g.nz - k0);
+  const C* out = smooth_passes<C>(t, 1, a, b, passes, op, alpha, warp, warps, [&](int x, int y, int z) {
+    x -= t.h[0];
+    y -= t.h[1];
+    z -= t.h[2];
+    if (invalid && x >= 0 && x < nx && y >= 0 && y < ny && z >= 0 && z < nz) atomicAdd(invalid, 1u);
+  });
+  for (int r = warp; r < ny * nz; r += warps) {
+    const int z = r / ny, y = r - z * ny, j = j0 + y, k = k0 + z;
+    for (int x = lane; x < nx; x += 32) {
+      const int i = i0 + x;
+      const double v = double(out[(x + t.h[0]) + t.e[0] * ((y + t.h[1]) + t.e[1] * (z + t.h[2]))]);
+      // The copies of node i on an axis of n: i + m n within -1 .. n + 1.
+      for (int kk = k - (k + 1) / g.nz * g.nz; kk <= g.nz + 1; kk += g.nz)
+        for (int jj = j - (j + 1) / g.ny * g.ny; jj <= g.ny + 1; jj += g.ny)
+          for (int ii = i - (i + 1) / g.nx * g.nx; ii <= g.nx + 1; ii += g.nx) dst[g.node(ii, jj, kk)] = v;
     }
-    dst[c * g.nodes + g.node(i, j, k)] = double(value);
-    if (invalid && !isfinite(value)) atomicAdd(invalid, 1u);
   }
 }
 
+template <class C>
+cudaError_t launch_smooth_typed(const Geom& g, int niter, int op, double alpha, const double* src, double* out,
+                                double* tmp, uint32_t* invalid, cudaStream_t s) {
+  // Passes a launch: as many as a halo is worth, split evenly.
+  const bool flat = g.nx == 1 || g.ny == 1 || g.nz == 1;
+  const int most = flat ? 8 : 3, launches = (niter + most - 1) / most;
+  const int tx = flat ? 32 : 16, ty = g.ny == 1 ? 1 : 8, tz = g.nz == 1 ? 1 : 8;
+  const long long tiles = (long long)((g.nx + tx - 1) / tx) * ((g.ny + ty - 1) / ty) * ((g.nz + tz - 1) / tz);
+  if (tiles > 0x7fffffffLL) return cudaErrorInvalidValue;
+  int done = 0;
+  for (int l = 0; l < launches; ++l) {
+    const int passes = (niter - done + launches - l - 1) / (launches - l);
+    done += passes;
+    const SmoothTile t(g.nx, g.ny, g.nz, tx, ty, tz, passes);
+    const size_t bytes = size_t(2) * t.size * sizeof(C);
+    const cudaError_t e =
+        cudaFuncSetAttribute(smooth_tile_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
+    if (e != cudaSuccess) return e;
+    double* to = (launches - l) % 2 == 1 ? out : tmp;
+    smooth_tile_kernel<C><<<dim3(unsigned(tiles), 3), kSmoothThreads, bytes, s>>>(g, t, tx, ty, tz, passes, op, alpha, src, to,
+                                                                         invalid);
+    count_launches(1);
+    src = to;
+  }
+  return cudaGetLastError();
+}
+
 // S^n(src) into out with its ghosts filled (complete_smoothing,
-// ecsim/maxwell/maxwell_device.hpp:455-487 on a periodic domain): src's
-// ghosts must be filled; the passes alternate between out and tmp so that
-// the last lands in out, with the ghosts refilled between passes. Neither
-// out nor tmp may alias src. double_arithmetic selects the pass arithmetic
-// (the reference's Arithmetic / Compute::Electric). invalid (may be null)
-// counts nonfinite smoothed values.
+// ecsim/maxwell/maxwell_device.hpp:455-487 on a periodic domain); the launches
+// alternate between out and tmp so that the last lands in out. Neither out
+// nor tmp may alias src. double_arithmetic selects the pass arithmetic (the
+// reference's Arithmetic / Compute::Electric). invalid (may be null) counts
+// nonfinite smoothed values, as the reference's kernel flags them
+// (node_smoothing_device.hpp:30-36).
 cudaError_t launch_smooth(bool double_arithmetic, const Geom& g, int niter, int op, double alpha,
                           const double* src, double* out, double* tmp, uint32_t* invalid, cudaStream_t s) {
   if (niter <= 0 || src == out || src == tmp || out == tmp) return cudaErrorInvalidValue;
-  const unsigned blocks = grid_for(3 * g.interior, 256);
-  const double* from = src;
-  for (int pass = 1; pass <= niter; ++pass) {
-    double* to = (niter - pass) % 2 == 0 ? out : tmp;
-    if (double_arithmetic) {
-      const double beta = (1.0 - alpha) / 6.0;
-      if (op == 0) smooth_kernel<double, 0><<<blocks, 256, 0, s>>>(g, alpha, beta, from, to, invalid);
-      else smooth_kernel<double, 1><<<blocks, 256, 0, s>>>(g, alpha, beta, from, to, invalid);
-    } else {
-      const float a = float(alpha), beta = (1.0f - a) / 6.0f;
-      if (op == 0) smooth_kernel<float, 0><<<blocks, 256, 0, s>>>(g, a, beta, from, to, invalid);
-      else smooth_kernel<float, 1><<<blocks, 256, 0, s>>>(g, a, beta, from, to, invalid);
-    }
-    count_launches(1);
-    launch_node_ghosts(g, to, 3, s);
-    from = to;
-  }
-  return cudaGetLastError();
+  return double_arithmetic ? launch_smooth_typed<double>(g, niter, op, alpha, src, out, tmp, invalid, s)
+                           : launch_smooth_typed<float>(g, niter, op, alpha, src, out, tmp, invalid, s);
 }
 
 // A node field of float or double into double (every entry, ghosts included).

@@ -23,12 +23,20 @@
 // that share the 27 mass blocks: small grids take small tiles, so that every
 // SM has one.
 //
-// Launched cooperatively (all CTAs resident). A barrier that does not
+// With smoothing (grids one cell thick along z) a tile holds passes + 1 more
+// nodes on each side and takes the passes in shared memory: the smoothed
+// vector's mass response goes to a global vector, and after one more barrier
+// the response is smoothed the same way.
+//
+// A grid of at most 16 tiles is launched as one cluster, whose hardware barrier
+// takes the place of the grid barrier. Otherwise the launch is cooperative
+// (all CTAs resident). A barrier that does not
 // complete within its polls makes its CTA set ctl->failed and leave; the
 // others then run out at theirs, and the solve fails.
 #pragma once
 
 #include "common.cuh"
+#include "smoothing.cuh"
 #include "stencils.cuh"
 
 namespace tpicb200 {
@@ -55,6 +63,7 @@ struct ResidentPlan {
   int tx, ty, tz;          // tile, powers of two; tx*ty*tz = nodes
   int nodes, parts, shift; // nodes of a tile, threads per node, log2 nodes
   int tiles_x, tiles_y, tiles;
+  bool cluster;            // the grid is one cluster
   bool shared_basis;       // basis rows in shared memory, else in `basis`
   double delta, kfac, inv_volume;
   const void* mass;
@@ -74,14 +83,22 @@ struct ResidentPlan {
   const void* bcell;
   const void* j;
   const double* rhs;
+  int smooth, smooth_op;   // smoothing passes (0: none), operator
+  double smooth_alpha;
+  double* response;        // [3][unique]: the smoothed vector's mass response
+  uint32_t* invalid;       // counts nonfinite smoothed values
   double* etheta;          // the solution with its ghosts, written when the residual is accepted
 };
 
 // Shared memory of a plan with arithmetic up to double: bytes per array.
 struct ResidentShared {
   int halo, cells;                 // nodes and cells a tile stages
-  size_t vs, cs, part, h, hcol, rot, sums, basis, image, unode, mult, table, ctable, total;
+  size_t vs, cs, part, h, hcol, rot, sums, basis, image, unode, mult, table, ctable, smooth, total;
 };
+// The tile and halo of the smoothing passes (the mass product reads one more node).
+inline __host__ __device__ SmoothTile resident_smooth_tile(const ResidentPlan& p) {
+  return SmoothTile(p.g.nx, p.g.ny, p.g.nz, p.tx, p.ty, p.tz, p.smooth + 1);
+}
 inline __host__ __device__ ResidentShared resident_shared(const ResidentPlan& p, size_t scalar) {
   ResidentShared s;
   s.halo = (p.tx + 2) * (p.ty + 2) * (p.tz + 2);
@@ -106,6 +123,7 @@ inline __host__ __device__ ResidentShared resident_shared(const ResidentPlan& p,
   s.mult = take(size_t(p.nodes) * 4);
   s.table = take(size_t(s.halo) * 4);
   s.ctable = take(size_t(s.cells) * 4);
+  s.smooth = take(p.smooth ? size_t(6) * resident_smooth_tile(p).size * 8 : 0);
   s.total = at;
   return s;
 }
@@ -121,7 +139,7 @@ __device__ __forceinline__ uint32_t load_acquire(const unsigned* p) {
   return v;
 }
 
-template <class S, class Mass, class Fld, bool kTranspose>
+template <class S, class Mass, class Fld, bool kTranspose, bool kSmooth>
 struct Resident {
   const ResidentPlan& p;
   uint8_t* smem;
@@ -148,6 +166,10 @@ struct Resident {
 
   // All CTAs of the grid. False when it gave up (for every thread of the CTA).
   __device__ bool grid_barrier() {
+    if (p.cluster) {
+      asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+      return true;
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
       arrivals += gridDim.x;
@@ -165,7 +187,7 @@ struct Resident {
   }
   // The last CTA to leave zeroes the barrier for the next launch.
   __device__ void leave() {
-    if (threadIdx.x == 0 && !failed && atomicAdd(p.barrier + 1, 1u) == gridDim.x - 1) {
+    if (threadIdx.x == 0 && !p.cluster && !failed && atomicAdd(p.barrier + 1, 1u) == gridDim.x - 1) {
       p.barrier[0] = 0;
       p.barrier[1] = 0;
     }
@@ -206,12 +228,11 @@ struct Resident {
     return i < p.g.nx && j < p.g.ny && k < p.g.nz;
   }
 
-  // The operator on the tile's nodes in arithmetic C: stage() reads the vector
-  // load(component, unique index) over the tile and its halo (the node
-  // threads; a CTA barrier follows), image() calls store(node in tile, its
-  // coordinates, the three values) from the first thread of each node in the
-  // grid. The products and their order are those of maxwell_apply_kernel where
-  // a node has one thread; with more, their partial sums are added in order.
+  // The operator in arithmetic C: stage() reads the vector load(component,
+  // unique index) over the tile and its halo (the node threads; a CTA barrier
+  // follows), image() forms its rows. The products and their order are those
+  // of maxwell_apply_kernel where a node has one thread; with more, their
+  // partial sums are added in order.
   template <class C, class Load>
   __device__ __forceinline__ void stage(Load&& load) {
     if (threadIdx.x >= kResidentNodeThreads) return;
@@ -223,16 +244,16 @@ struct Resident {
 #pragma unroll
       for (int c = 0; c < 3; ++c) vs[c * VN + n] = u >= 0 ? C(load(c, u)) : C(0);
     }
+    if constexpr (kSmooth) stage_region<C>(resident_smooth_tile(p), load);
   }
-  template <class C, class Store>
-  __device__ __forceinline__ void image(Store&& store) {
-    const Geom& g = p.g;
-    C* vs = at<C>(L.vs);
+  // The cell curls of the staged vector.
+  template <class C>
+  __device__ __forceinline__ void cell_curls() {
+    const C* vs = at<C>(L.vs);
     C* cs = at<C>(L.cs);
     const int* ctable = at<int>(L.ctable);
-    const int vx = p.tx + 2, vxy = vx * (p.ty + 2), cx = p.tx + 1, cxy = cx * (p.ty + 1);
-    const int VN = L.halo, CN = L.cells;
-    const C inv[3] = {C(g.inv[0]), C(g.inv[1]), C(g.inv[2])};
+    const int vx = p.tx + 2, vxy = vx * (p.ty + 2), VN = L.halo, CN = L.cells;
+    const C inv[3] = {C(p.g.inv[0]), C(p.g.inv[1]), C(p.g.inv[2])};
     for (int n = threadIdx.x; n < CN; n += kResidentThreads) {
       const C* v = vs + ctable[n];
       C q[3][8];
@@ -249,11 +270,25 @@ struct Resident {
       cs[CN + n] = dz(q[0]) - dx(q[2]);
       cs[2 * CN + n] = dx(q[1]) - dy(q[0]);
     }
-    const int n = threadIdx.x & (p.nodes - 1), part = threadIdx.x >> p.shift;
-    int i = 0, j = 0, k = 0;
-    const bool live = threadIdx.x < kResidentNodeThreads && node_of(n, i, j, k);
-    const int lx = n & (p.tx - 1), ly = (n / p.tx) & (p.ty - 1), lz = n / (p.tx * p.ty);
-    const int vi = (lx + 1) + vx * (ly + 1) + vxy * (lz + 1);
+  }
+  // This thread's node of the tile and its part of the node's mass blocks.
+  __device__ __forceinline__ bool my_node(int& n, int& part, int& i, int& j, int& k) const {
+    n = threadIdx.x & (p.nodes - 1);
+    part = threadIdx.x >> p.shift;
+    return threadIdx.x < kResidentNodeThreads && node_of(n, i, j, k);
+  }
+  __device__ __forceinline__ void local(int n, int& lx, int& ly, int& lz) const {
+    lx = n & (p.tx - 1);
+    ly = (n / p.tx) & (p.ty - 1);
+    lz = n / (p.tx * p.ty);
+  }
+  // The mass product of node (i, j, k) from v (component stride vn, neighbour
+  // strides sx, sy, sz), complete in the node's first thread. A CTA barrier
+  // is in it.
+  template <class C>
+  __device__ __forceinline__ void mass(bool live, int n, int part, int i, int j, int k, const C* v, int vn, int sx,
+                                       int sy, int sz, C out[3]) {
+    const Geom& g = p.g;
     C x = C(0), y = C(0), z = C(0);
     if (live) {
       // Blocks in stencil order: part r of P takes stencils [14 r / P, 14 (r + 1) / P).
@@ -262,9 +297,9 @@ struct Resident {
       const int s1 = 14 * (part + 1) / p.parts;
       for (int s = 14 * part / p.parts; s < s1; ++s) {
         const int ox = kResidentOffsets[s][0], oy = kResidentOffsets[s][1], oz = kResidentOffsets[s][2];
-        const int vo = ox + vx * oy + vxy * oz;
-        product(mass + g.mass_index(mat, 9 * s), vs + vi + vo, VN, x, y, z);
-        if (s > 0) product(mass + g.mass_index(mat - g.mass_offset(ox, oy, oz), 9 * s), vs + vi - vo, VN, x, y, z);
+        const int vo = ox * sx + oy * sy + oz * sz;
+        product(mass + g.mass_index(mat, 9 * s), v + vo, vn, x, y, z);
+        if (s > 0) product(mass + g.mass_index(mat - g.mass_offset(ox, oy, oz), 9 * s), v - vo, vn, x, y, z);
       }
       if (part > 0) {
         C* sum = at<C>(L.part);
@@ -282,24 +317,105 @@ struct Resident {
         y += sum[kResidentNodeThreads + t];
         z += sum[2 * kResidentNodeThreads + t];
       }
-      C w[3][8];
+    }
+    const C iv = C(p.inv_volume);
+    out[0] = x * iv;
+    out[1] = y * iv;
+    out[2] = z * iv;
+  }
+  // v + delta^2 curl curl v + k m at a node.
+  template <class C>
+  __device__ __forceinline__ void combine(int lx, int ly, int lz, const C m[3], C value[3]) const {
+    const C* vs = at<C>(L.vs);
+    const C* cs = at<C>(L.cs);
+    const int vx = p.tx + 2, vxy = vx * (p.ty + 2), cx = p.tx + 1, cxy = cx * (p.ty + 1);
+    const int VN = L.halo, CN = L.cells;
+    const C inv[3] = {C(p.g.inv[0]), C(p.g.inv[1]), C(p.g.inv[2])};
+    C w[3][8];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const C* f = cs + c * CN + (lx + 1) + cx * (ly + 1) + cxy * (lz + 1);
-        w[c][0] = f[0];        w[c][1] = f[-1];       w[c][2] = f[-cx];       w[c][3] = f[-cxy];
-        w[c][4] = f[-cx - 1];  w[c][5] = f[-cxy - 1]; w[c][6] = f[-cxy - cx]; w[c][7] = f[-cxy - cx - 1];
+    for (int c = 0; c < 3; ++c) {
+      const C* f = cs + c * CN + (lx + 1) + cx * (ly + 1) + cxy * (lz + 1);
+      w[c][0] = f[0];        w[c][1] = f[-1];       w[c][2] = f[-cx];       w[c][3] = f[-cxy];
+      w[c][4] = f[-cx - 1];  w[c][5] = f[-cxy - 1]; w[c][6] = f[-cxy - cx]; w[c][7] = f[-cxy - cx - 1];
+    }
+    auto dx = [&](const C* q) { return C(0.25) * inv[0] * (q[0] - q[1] + (q[3] - q[5]) + (q[2] - q[4]) + (q[6] - q[7])); };
+    auto dy = [&](const C* q) { return C(0.25) * inv[1] * (q[0] - q[2] + (q[3] - q[6]) + (q[1] - q[4]) + (q[5] - q[7])); };
+    auto dz = [&](const C* q) { return C(0.25) * inv[2] * (q[0] - q[3] + (q[1] - q[5]) + (q[2] - q[6]) + (q[4] - q[7])); };
+    const C curl[3] = {dy(w[2]) - dz(w[1]), dz(w[0]) - dx(w[2]), dx(w[1]) - dy(w[0])};
+    const C d2 = C(p.delta * p.delta), kf = C(p.kfac);
+    const int vi = (lx + 1) + vx * (ly + 1) + vxy * (lz + 1);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) value[c] = (vs[c * VN + vi] + d2 * curl[c]) + kf * m[c];
+  }
+
+  // Smoothing: the region of the tile's passes filled from load(component,
+  // unique index), and the passes over it (the passes have CTA barriers).
+  template <class C, class Load>
+  __device__ __forceinline__ void stage_region(const SmoothTile& t, Load&& load) {
+    if (threadIdx.x >= kResidentNodeThreads) return;
+    C* a = at<C>(L.smooth);
+    int i0, j0, k0;
+    origin(i0, j0, k0);
+    const Geom& g = p.g;
+    for (int y = threadIdx.x >> 5; y < t.e[1]; y += kResidentNodeThreads / 32) {
+      const int row = g.nx * wrap_index(j0 - t.h[1] + y, g.ny);
+      for (int x = threadIdx.x & 31; x < t.e[0]; x += 32) {
+        const int u = wrap_index(i0 - t.h[0] + x, g.nx) + row;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) a[c * t.size + y * t.e[0] + x] = C(load(c, u));
       }
-      auto dx = [&](const C* q) { return C(0.25) * inv[0] * (q[0] - q[1] + (q[3] - q[5]) + (q[2] - q[4]) + (q[6] - q[7])); };
-      auto dy = [&](const C* q) { return C(0.25) * inv[1] * (q[0] - q[2] + (q[3] - q[6]) + (q[1] - q[4]) + (q[5] - q[7])); };
-      auto dz = [&](const C* q) { return C(0.25) * inv[2] * (q[0] - q[3] + (q[1] - q[5]) + (q[2] - q[6]) + (q[4] - q[7])); };
-      const C curl[3] = {dy(w[2]) - dz(w[1]), dz(w[0]) - dx(w[2]), dx(w[1]) - dy(w[0])};
-      const C d2 = C(p.delta * p.delta), kf = C(p.kfac), iv = C(p.inv_volume);
-      const C mv[3] = {x * iv, y * iv, z * iv};
-      C value[3];
+    }
+  }
+  template <class C>
+  __device__ __forceinline__ const C* smoothed(const SmoothTile& t) {
+    C* a = at<C>(L.smooth);
+    int i0, j0, k0;
+    origin(i0, j0, k0);
+    return smooth_passes<C>(t, 3, a, a + 3 * t.size, p.smooth, p.smooth_op, p.smooth_alpha, threadIdx.x >> 5,
+                            kResidentThreads / 32, [&](int x, int y, int) {
+                              x -= t.h[0];
+                              y -= t.h[1];
+                              if (x >= 0 && x < p.tx && i0 + x < p.g.nx && y >= 0 && y < p.ty && j0 + y < p.g.ny)
+                                atomicAdd(p.invalid, 1u);
+                            });
+  }
+
+  // The operator on the tile's nodes, after stage() (and, with smoothing,
+  // stage_region()) of the vector and a CTA barrier: store(node in tile, its
+  // coordinates, the three values) from the first thread of each node in the
+  // grid. False when a barrier gave up.
+  template <class C, class Store>
+  __device__ __forceinline__ bool image(Store&& store) {
+    cell_curls<C>();
+    int n, part, i = 0, j = 0, k = 0, lx, ly, lz;
+    const bool live = my_node(n, part, i, j, k);
+    local(n, lx, ly, lz);
+    C m[3];
+    if constexpr (!kSmooth) {
+      const int vx = p.tx + 2, vxy = vx * (p.ty + 2);
+      mass<C>(live, n, part, i, j, k, at<C>(L.vs) + (lx + 1) + vx * (ly + 1) + vxy * (lz + 1), L.halo, 1, vx, vxy, m);
+    } else {
+      const SmoothTile t = resident_smooth_tile(p);
+      const int own = (lx + t.h[0]) + t.e[0] * (ly + t.h[1]);
+      const long long U = unique();
+      const C* v = smoothed<C>(t);
+      mass<C>(live, n, part, i, j, k, v + own, t.size, t.s[0], t.s[1], t.s[2], m);
+      if (live && part == 0)
 #pragma unroll
-      for (int c = 0; c < 3; ++c) value[c] = (vs[c * VN + vi] + d2 * curl[c]) + kf * mv[c];
+        for (int c = 0; c < 3; ++c) p.response[c * U + i + p.g.nx * j] = double(m[c]);
+      if (!grid_barrier()) return false;
+      stage_region<C>(t, [&](int c, int u) { return __ldcg(p.response + c * U + u); });
+      __syncthreads();
+      v = smoothed<C>(t);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) m[c] = live ? v[c * t.size + own] : C(0);
+    }
+    if (live && part == 0) {
+      C value[3];
+      combine<C>(lx, ly, lz, m, value);
       store(n, i, j, k, value);
     }
+    return true;
   }
 
   template <class C>
@@ -364,12 +480,12 @@ struct Resident {
   // r = b - A x over the owned nodes (x read through `load`), the sums of r^2
   // (and of b^2) published.
   template <class Load>
-  __device__ void residual(Load&& load, bool with_rhs) {
+  __device__ bool residual(Load&& load, bool with_rhs) {
     double s0 = 0, s1 = 0;
     const long long U = unique();
     stage<double>(load);
     __syncthreads();
-    image<double>([&](int, int i, int j, int k, const double value[3]) {
+    const bool done = image<double>([&](int, int i, int j, int k, const double value[3]) {
       const int u = i + p.g.nx * (j + p.g.ny * k);
       const double m = (i == 0 ? 2.0 : 1.0) * (j == 0 ? 2.0 : 1.0) * (k == 0 ? 2.0 : 1.0);
 #pragma unroll
@@ -380,8 +496,10 @@ struct Resident {
         s1 += m * (b * b);
       }
     });
+    if (!done) return false;
     __syncthreads();
     publish(s0, s1, 0, with_rhs);
+    return true;
   }
 
   // The solution x with its ghosts into etheta (node field).
@@ -401,16 +519,27 @@ struct Resident {
 
 // The right-hand side, the guess and its residual (values[0] = |r|^2,
 // values[1] = |b|^2).
-template <class S, class Mass, class Fld, bool kTranspose>
+template <class S, class Mass, class Fld, bool kTranspose, bool kSmooth>
 __global__ void __launch_bounds__(kResidentThreads, 2) resident_start_kernel(const __grid_constant__ ResidentPlan p) {
   extern __shared__ __align__(16) uint8_t resident_smem[];
-  using R = Resident<S, Mass, Fld, kTranspose>;
+  using R = Resident<S, Mass, Fld, kTranspose, kSmooth>;
   R r(p, resident_smem);
   r.prepare();
   const Geom& g = p.g;
   const long long U = r.unique();
   const Fld* e = static_cast<const Fld*>(p.e);
   const Fld inv[3] = {Fld(g.inv[0]), Fld(g.inv[1]), Fld(g.inv[2])};
+  // With smoothing the right-hand side has S^n(J), in the field arithmetic.
+  const Fld* smooth_j = nullptr;
+  SmoothTile t = resident_smooth_tile(p);
+  if constexpr (kSmooth) {
+    r.template stage_region<Fld>(t, [&](int c, int u) {
+      const int row = u / g.nx;
+      return static_cast<const Fld*>(p.j)[c * g.nodes + g.node(u - row * g.nx, row, 0)];
+    });
+    __syncthreads();
+    smooth_j = r.template smoothed<Fld>(t);
+  }
   int i, j, k;
   if (int(threadIdx.x) < p.nodes && r.node_of(threadIdx.x, i, j, k)) {
     const int u = i + g.nx * (j + g.ny * k);
@@ -426,18 +555,27 @@ __global__ void __launch_bounds__(kResidentThreads, 2) resident_start_kernel(con
       curl_c2n_at<Fld>(g, static_cast<const Fld*>(p.bcell), i, j, k, inv, cb);
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        const Fld ev = e[c * g.nodes + at], jv = static_cast<const Fld*>(p.j)[c * g.nodes + at];
+        const Fld ev = e[c * g.nodes + at];
+        Fld jv;
+        if constexpr (kSmooth) {
+          int lx, ly, lz;
+          r.local(threadIdx.x, lx, ly, lz);
+          jv = smooth_j[c * t.size + (lx + t.h[0]) + t.e[0] * (ly + t.h[1])];
+        } else {
+          jv = static_cast<const Fld*>(p.j)[c * g.nodes + at];
+        }
         p.x[c * U + u] = double(ev);
         p.b[c * U + u] = double((ev + Fld(p.delta) * cb[c]) + (-Fld(p.kfac)) * jv);
       }
     }
   }
   __syncthreads();
-  r.residual([&](int c, int u) -> double {
-    if (p.rhs) return 0.0;
-    const int row = u / g.nx, k = row / g.ny;
-    return double(e[c * g.nodes + g.node(u - row * g.nx, row - k * g.ny, k)]);
-  }, true);
+  if (!r.residual([&](int c, int u) -> double {
+        if (p.rhs) return 0.0;
+        const int row = u / g.nx, k = row / g.ny;
+        return double(e[c * g.nodes + g.node(u - row * g.nx, row - k * g.ny, k)]);
+      }, true))
+    return;
   if (!r.grid_barrier()) return;
   const double r2 = r.gathered(0), b2 = r.gathered(1);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -451,10 +589,10 @@ __global__ void __launch_bounds__(kResidentThreads, 2) resident_start_kernel(con
 
 // One restart cycle from the residual r (values[0] = |r|^2): at most
 // `columns` Arnoldi steps, the update of x, its residual (values[0]).
-template <class S, class Mass, class Fld, bool kTranspose>
+template <class S, class Mass, class Fld, bool kTranspose, bool kSmooth>
 __global__ void __launch_bounds__(kResidentThreads, 2) resident_cycle_kernel(const __grid_constant__ ResidentPlan p) {
   extern __shared__ __align__(16) uint8_t resident_smem[];
-  using R = Resident<S, Mass, Fld, kTranspose>;
+  using R = Resident<S, Mass, Fld, kTranspose, kSmooth>;
   R r(p, resident_smem);
   constexpr int m = kResidentRestart, kWarps = kResidentThreads / 32;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -500,10 +638,11 @@ __global__ void __launch_bounds__(kResidentThreads, 2) resident_cycle_kernel(con
     __syncthreads();
     stop = int(shared[1]);
     if (stop) break;
-    r.template image<S>([&](int n, int, int, int, const S value[3]) {
+    if (!r.template image<S>([&](int n, int, int, int, const S value[3]) {
 #pragma unroll
-      for (int c = 0; c < 3; ++c) image[c * p.nodes + n] = value[c];
-    });
+          for (int c = 0; c < 3; ++c) image[c * p.nodes + n] = value[c];
+        }))
+      return;
     __syncthreads();
     for (int c = warp; c <= col; c += kWarps) {
       const S* v = r.basis(c);
@@ -595,7 +734,7 @@ __global__ void __launch_bounds__(kResidentThreads, 2) resident_cycle_kernel(con
     p.x[at] = value;
   }
   if (!r.grid_barrier()) return;
-  r.residual([&](int c, int u) { return __ldcg(p.x + c * U + u); }, false);
+  if (!r.residual([&](int c, int u) { return __ldcg(p.x + c * U + u); }, false)) return;
   if (!r.grid_barrier()) return;
   const double r2 = r.gathered(0);
   if (blockIdx.x == 0 && threadIdx.x == 0) {

@@ -42,6 +42,8 @@ constexpr int kDotTile = 8;
 constexpr long long kColumnAlign = 64;
 // Largest GMRES restart the context accepts.
 constexpr int kMaxRestart = 1024;
+constexpr int kResidentSmooth = 8;   // smoothing passes the resident kernels take
+constexpr int kResidentCluster = 16; // CTAs of a cluster
 
 // Interior coordinates of compact index t (32-bit arithmetic: solver_create
 // requires 3 (n+1)^3 < 2^31).
@@ -937,11 +939,43 @@ struct SolverWorkspace {
 template <class P>
 struct ResidentKernels {
   using Kernel = void (*)(ResidentPlan);
-  static Kernel start() { return resident_start_kernel<typename P::EC, typename P::Mass, typename P::Fld, false>; }
-  static Kernel start_transposed() { return resident_start_kernel<typename P::EC, typename P::Mass, typename P::Fld, true>; }
-  static Kernel cycle() { return resident_cycle_kernel<typename P::EC, typename P::Mass, typename P::Fld, false>; }
-  static Kernel cycle_transposed() { return resident_cycle_kernel<typename P::EC, typename P::Mass, typename P::Fld, true>; }
+  template <bool T, bool Sm>
+  static Kernel start() { return resident_start_kernel<typename P::EC, typename P::Mass, typename P::Fld, T, Sm>; }
+  template <bool T, bool Sm>
+  static Kernel cycle() { return resident_cycle_kernel<typename P::EC, typename P::Mass, typename P::Fld, T, Sm>; }
+  // The start and the cycle of A (with smoothing or not) or of A^T.
+  static void pick(bool transpose, bool smooth, Kernel out[2]) {
+    out[0] = smooth ? start<false, true>() : transpose ? start<true, false>() : start<false, false>();
+    out[1] = smooth ? cycle<false, true>() : transpose ? cycle<true, false>() : cycle<false, false>();
+  }
 };
+
+// The launch of `blocks` CTAs as one cluster.
+struct ClusterLaunch {
+  cudaLaunchConfig_t config{};
+  cudaLaunchAttribute attribute[1];
+  ClusterLaunch(unsigned blocks, size_t bytes, cudaStream_t s) {
+    config.gridDim = dim3(blocks);
+    config.blockDim = dim3(kResidentThreads);
+    config.dynamicSmemBytes = bytes;
+    config.stream = s;
+    attribute[0].id = cudaLaunchAttributeClusterDimension;
+    attribute[0].val.clusterDim.x = blocks;
+    attribute[0].val.clusterDim.y = attribute[0].val.clusterDim.z = 1;
+    config.attrs = attribute;
+    config.numAttrs = 1;
+  }
+};
+bool cluster_fits(void (*kernel)(ResidentPlan), int blocks, size_t bytes) {
+  int clusters = 0;
+  const ClusterLaunch launch(unsigned(blocks), bytes, nullptr);
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&clusters, kernel, &launch.config) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return clusters > 0;
+}
 
 // Tiles of the resident kernels: the smallest tile whose CTAs are all
 // resident at once, so that every SM has nodes and a node has many threads;
@@ -957,14 +991,17 @@ struct ResidentKernels {
 template <class P>
 void plan_resident(SolverWorkspace* w, int sms) {
   using K = ResidentKernels<P>;
-  if (w->restart > kResidentRestart || w->smoothing.iterations > 0) return;
   const Geom& g = w->g;
+  const int smooth = w->smoothing.iterations;
+  if (w->restart > kResidentRestart || (smooth > 0 && (g.nz != 1 || smooth > kResidentSmooth))) return;
   int device = 0, cooperative = 0, limit = 0;
   if (cudaGetDevice(&device) != cudaSuccess ||
       cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, device) != cudaSuccess || !cooperative ||
       cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess)
     return;
-  const typename K::Kernel kernels[4] = {K::start(), K::start_transposed(), K::cycle(), K::cycle_transposed()};
+  typename K::Kernel kernels[4];
+  K::pick(false, smooth > 0, kernels);
+  K::pick(smooth == 0, smooth > 0, kernels + 2);  // no adjoint with smoothing
   for (auto k : kernels)
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, limit) != cudaSuccess) {
       cudaGetLastError();
@@ -992,6 +1029,14 @@ void plan_resident(SolverWorkspace* w, int sms) {
     p.delta = w->delta;
     p.kfac = w->kfac;
     p.inv_volume = g.inv_volume;
+    p.smooth = smooth;
+    p.smooth_op = w->smoothing.op;
+    p.smooth_alpha = w->smoothing.alpha;
+    // One cluster, where the smallest tiles fit its 16 CTAs (128 x 1 x 1: 1.15
+    // ms a solve, 1.36 with the grid barrier); larger tiles to make them fit
+    // lost more in threads per node than the barrier costs (1024 x 1 x 1 1.55
+    // against 1.51 ms, 12^3 0.29 against 0.19).
+    p.cluster = p.tiles <= kResidentCluster;
     for (int shared = 1; shared >= 0; --shared) {
       p.shared_basis = shared != 0;
       if (!p.shared_basis && 3LL * p.tiles * p.nodes > w->ld) continue;
@@ -1007,6 +1052,10 @@ void plan_resident(SolverWorkspace* w, int sms) {
         per_sm = std::min(per_sm, blocks);
       }
       if (p.tiles > per_sm * sms) continue;
+      if (p.cluster) {
+        for (auto k : kernels)
+          if (!cluster_fits(k, p.tiles, bytes)) p.cluster = false;
+      }
       w->plan = p;
       w->resident_grid = unsigned(p.tiles);
       w->resident_bytes = bytes;
@@ -1220,7 +1269,6 @@ struct Solve {
       mass_image_kernel<C, Mass><<<grid_for(g.interior, kThreads), kThreads, 0, st>>>(g, C(iv), mass, w->smooth_a,
                                                                                      w->smooth_image);
       count_launches(1);
-      launch_node_ghosts(g, w->smooth_image, 3, st);
       if (err == cudaSuccess)
         err = launch_smooth(dbl, g, sp.iterations, sp.op, sp.alpha, w->smooth_image, w->smooth_a, w->smooth_b, w->invalid, st);
       response = w->smooth_a;
@@ -1466,9 +1514,13 @@ struct Solve {
   bool launch_resident(typename ResidentKernels<P>::Kernel kernel, double controls[2], ArnoldiControl* control) {
     ResidentPlan p = w->plan;
     void* args[] = {&p};
-    if (err == cudaSuccess)
+    if (err == cudaSuccess && p.cluster) {
+      const ClusterLaunch launch(w->resident_grid, w->resident_bytes, s);
+      err = cudaLaunchKernelExC(&launch.config, (const void*)kernel, args);
+    } else if (err == cudaSuccess) {
       err = cudaLaunchCooperativeKernel((const void*)kernel, dim3(w->resident_grid), dim3(kResidentThreads), args,
                                         w->resident_bytes, s);
+    }
     count_launches(1);
     if (!read_back(w->values, controls, control)) return false;
     if (control->failed) {
@@ -1498,12 +1550,16 @@ struct Solve {
     p.bcell = bcell;
     p.j = j;
     p.rhs = rhs_in;
+    p.response = w->smooth_image;
+    p.invalid = w->invalid;
     p.etheta = etheta;
     p.accept = tolerance;
     tpicb200_gmres_result res{};
     double controls[2];
     ArnoldiControl control{};
-    if (!launch_resident(w->transpose ? K::start_transposed() : K::start(), controls, &control))
+    typename K::Kernel kernels[2];
+    K::pick(w->transpose, w->smoothing.iterations > 0, kernels);
+    if (!launch_resident(kernels[0], controls, &control))
       return TPICB200_BACKEND_FAILURE;
     if (!std::isfinite(controls[0]) || !std::isfinite(controls[1])) return TPICB200_OVERFLOW;
     res.residual = res.initial_residual = std::sqrt(controls[0]);
@@ -1520,7 +1576,7 @@ struct Solve {
       p.tolerance =
           refined ? std::max(atol, res.residual * 16.0 * double(std::numeric_limits<S>::epsilon())) : atol;
       p.accept = atol;
-      if (!launch_resident(w->transpose ? K::cycle_transposed() : K::cycle(), controls, &control))
+      if (!launch_resident(kernels[1], controls, &control))
         return TPICB200_BACKEND_FAILURE;
       if (control.stop == 2) return TPICB200_OVERFLOW;
       if (!std::isfinite(controls[0]) || controls[0] < 0) return TPICB200_OVERFLOW;
@@ -1556,11 +1612,9 @@ struct Solve {
     pack_storage_kernel<Fld><<<blocks(), kThreads, 0, s>>>(g, (const Fld*)e, w->x);
     if (w->smoothing.iterations > 0) {
       // RHS with S^n(J-hat) (complete_rhs, maxwell_device.hpp:152-172): the
-      // current widened to double with its ghosts refilled, then smoothed in
-      // the field arithmetic.
+      // current widened to double, then smoothed in the field arithmetic.
       const SmoothingPlan& sp = w->smoothing;
       if (err == cudaSuccess) err = launch_widen(P::id, g, j, w->smooth_image, s);
-      launch_node_ghosts(g, w->smooth_image, 3, s);
       if (err == cudaSuccess)
         err = launch_smooth(P::id == TPICB200_PRECISION_DOUBLE, g, sp.iterations, sp.op, sp.alpha, w->smooth_image,
                             w->smooth_a, w->smooth_b, w->invalid, s);
