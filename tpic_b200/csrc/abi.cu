@@ -238,6 +238,7 @@ int tpicb200_create(const tpicb200_grid* grid, const tpicb200_options* options, 
   alloc((void**)&ctx->moments, moment_floats(ctx->g) * (options->precision == TPICB200_PRECISION_MIXED ? 4 : 8));
   if (e == cudaSuccess) e = cudaMallocHost((void**)&ctx->pinned, (2 + 5 * TPICB200_MAX_SPECIES + 2) * 8);
   if (e == cudaSuccess) e = cudaMemset(ctx->invalid, 0, 4);
+  if (e == cudaSuccess) e = binned_reset(binned_scratch(ctx->g, ctx->binned, ctx->codes));
   if (e == cudaSuccess && ctx->solver) solver_set_invalid(ctx->solver, ctx->invalid);
   for (auto& ev : ctx->events)
     if (e == cudaSuccess) e = cudaEventCreate(&ev);
@@ -688,8 +689,7 @@ static int move_and_sort(tpicb200_context* ctx, tpicb200_state* st, int sp, uint
     return TPICB200_SUCCESS;
   }
   const BinnedScratch b = binned_scratch(ctx->g, ctx->binned, ctx->codes);
-  cudaError_t e = binned_begin(ctx->g, b, st->counts[sp], st->offsets[sp], true, s);
-  if (e == cudaSuccess) e = binned_validate(ctx->g, b, in->count, s);
+  cudaError_t e = binned_begin(ctx->g, b, in->count, st->counts[sp], st->offsets[sp], true, s);
   const bool ranks = st->ranks[sp] != nullptr;
   if (ranks) {
     // Out of place: the moved records, in the previous sorted order, go live.
@@ -838,21 +838,25 @@ int tpicb200_read_invalid(tpicb200_context* ctx, uint32_t* count, int clear, tpi
 // The cycle's energy report: the field energies of the committed fields and
 // the species scalars the movers accumulated (the values tpicb200_energy
 // computes from the live slots, summed in the movers' block order).
-static int cycle_energy(tpicb200_context* ctx, const tpicb200_state* st, double* out, cudaStream_t s) {
+// With the invalid counter, read back by the same wait.
+static int cycle_energy(tpicb200_context* ctx, const tpicb200_state* st, double* out, uint32_t* invalid,
+                        cudaStream_t s) {
   const int blocks = ctx->energy_blocks;
   cudaError_t err = launch_field_energy(ctx->opt.precision, ctx->g, st->e, st->b_cell, ctx->partials, blocks, s);
-  if (err == cudaSuccess) err = launch_reduce_rows(ctx->partials, ctx->reduced, 2, blocks, blocks, 2, s);
-  for (int sp = 0; sp < st->ns && err == cudaSuccess; ++sp)
-    err = launch_reduce_rows(ctx->mover_partials + size_t(kMoverPartials) * 5 * sp, ctx->reduced + 2 + 5 * sp, 5,
-                             kMoverPartials, ctx->mover_written[sp], ctx->mover_written[sp] > 0 ? 5 : 0, s);
+  ReportRows report{ctx->partials, blocks, ctx->mover_partials, {}};
+  for (int sp = 0; sp < st->ns; ++sp) report.written[sp] = ctx->mover_written[sp];
+  if (err == cudaSuccess) err = launch_reduce_report(report, st->ns, ctx->reduced, s);
   const int rows = 2 + 5 * st->ns;
   if (err == cudaSuccess) err = cudaMemcpyAsync(ctx->pinned, ctx->reduced, rows * 8, cudaMemcpyDeviceToHost, s);
+  if (err == cudaSuccess) err = cudaMemcpyAsync(ctx->pinned + rows, ctx->invalid, 4, cudaMemcpyDeviceToHost, s);
+  if (err == cudaSuccess) err = cudaEventRecord(ctx->events[4], s);
   if (err == cudaSuccess) err = cudaStreamSynchronize(s);
   if (err != cudaSuccess) return cuda_status(err, "energy reduction failed");
   const double norm = ctx->g.volume / (8 * 3.14159265358979323846);
   out[0] = norm * ctx->pinned[0];
   out[1] = norm * ctx->pinned[1];
   for (int r = 2; r < rows; ++r) out[r] = ctx->pinned[r];
+  std::memcpy(invalid, ctx->pinned + rows, 4);
   return TPICB200_SUCCESS;
 }
 
@@ -910,9 +914,10 @@ int tpicb200_cycle(tpicb200_context* ctx, tpicb200_state* st, int ncycles, tpicb
     cudaEventRecord(ev[3], s);
     std::swap(st->b_cell, st->b_cell_next);
     std::swap(st->b_node, st->b_node_next);
+    uint32_t bad = 0;
     if (reports) {
       double out[2 + 5 * TPICB200_MAX_SPECIES];
-      if (int r = cycle_energy(ctx, st, out, s)) return r;
+      if (int r = cycle_energy(ctx, st, out, &bad, s)) return r;
       report.field_energy[0] = out[0];
       report.field_energy[1] = out[1];
       report.total_energy = out[0] + out[1];
@@ -921,9 +926,10 @@ int tpicb200_cycle(tpicb200_context* ctx, tpicb200_state* st, int ncycles, tpicb
         report.total_energy += out[2 + 5 * sp];
       }
     }
-    cudaEventRecord(ev[4], s);
-    uint32_t bad = 0;
-    if (int r = read_invalid(ctx, s, &bad)) return r;
+    if (!reports) {
+      cudaEventRecord(ev[4], s);
+      if (int r = read_invalid(ctx, s, &bad)) return r;
+    }
     if (bad) return fail(TPICB200_INVALID_DATA, "the cycle raised the invalid-data flag");
     // Stage times: solve, move, advance, sort, deposit, fold + diagnostics.
     float t = 0.0f;

@@ -205,6 +205,18 @@ __global__ void __launch_bounds__(256) reduce_rows_kernel(const double* __restri
   if (threadIdx.x == 0) out[row] = sum;
 }
 
+__global__ void __launch_bounds__(256) reduce_report_kernel(ReportRows rows, double* out) {
+  __shared__ double scratch[8];
+  const int row = blockIdx.x, sp = (row - 2) / 5;
+  const double* from = row < 2 ? rows.fields + (long long)row * rows.blocks
+                               : rows.movers + (long long)(row - 2) * kMoverPartials;
+  const int count = row < 2 ? rows.blocks : rows.written[sp];
+  double sum = 0;
+  for (int i = threadIdx.x; i < count; i += blockDim.x) sum += from[i];
+  sum = block_sum<256>(sum, scratch);
+  if (threadIdx.x == 0) out[row] = sum;
+}
+
 template <class T>
 __global__ void __launch_bounds__(256) copy_node_kernel(long long total, const T* __restrict__ in,
                                                         double* __restrict__ out) {
@@ -422,6 +434,12 @@ cudaError_t launch_reduce_rows(const double* partials, double* out, int rows, in
     return launch_programmatic(reduce_rows_kernel, unsigned(rows), 256, 0, s, partials, out, row_stride, count,
                                filled);
   reduce_rows_kernel<<<rows, 256, 0, s>>>(partials, out, row_stride, count, filled);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_reduce_report(const ReportRows& rows, int ns, double* out, cudaStream_t s) {
+  reduce_report_kernel<<<2 + 5 * ns, 256, 0, s>>>(rows, out);
+  count_launches(1);
   return cudaGetLastError();
 }
 

@@ -57,10 +57,12 @@ cudaError_t launch_sort(int precision, const Geom& g, const tpicb200_particles* 
 // Sort of records grouped by the bins (in_counts, in_offsets) of an earlier
 // sort, keys updated since: neighbour moves go through the transfer-count
 // path, anything else through the general sort (same stable order).
+// The state is zero between sorts: the last kernel of a sort that raised a flag
+// clears it (binned_reset at the context's creation).
 struct BinnedState {
-  uint32_t fallback;         // nonzero: the general sort produces the output
-  uint32_t bins_bad;         // nonzero: the old bins do not tile the records
-  unsigned long long total;  // records in the old bins
+  uint32_t fallback;    // nonzero: the general sort produces the output
+  uint32_t bins_bad;    // nonzero: the old bins do not tile the records
+  uint32_t barrier[2];  // grid barrier of the cooperative kernels
 };
 struct BinnedScratch {
   BinnedState* state;
@@ -72,17 +74,16 @@ struct BinnedScratch {
 size_t binned_scratch_words(const Geom& g);
 bool binned_sort_applies(const Geom& g);
 BinnedScratch binned_scratch(const Geom& g, uint32_t* words, uint16_t* codes);
-// Copies the input's bins and clears the state (and the transfer counts when
-// the mover will add into them).
-cudaError_t binned_begin(const Geom& g, const BinnedScratch& b, const uint32_t* in_counts,
+cudaError_t binned_reset(const BinnedScratch& b);
+// Copies the input's bins, checks that they tile the n records in key order
+// (else raises bins_bad and fallback) and clears the transfer counts when the
+// mover will add into them.
+cudaError_t binned_begin(const Geom& g, const BinnedScratch& b, uint32_t n, const uint32_t* in_counts,
                          const uint32_t* in_offsets, bool zero_transfer, cudaStream_t s);
-// Checks that the old bins tile the n records in key order (else raises
-// bins_bad and fallback).
-cudaError_t binned_validate(const Geom& g, const BinnedScratch& b, uint32_t n, cudaStream_t s);
 // (Classification when `classify`), counts, scan, bases, the ranks (perm:
 // sorted position -> input record), the gather of the sorted records when
 // `materialize`, and the gated general sort (which always writes `out` and
-// the same perm); binned_validate must have run.
+// the same perm); binned_begin must have run.
 cudaError_t binned_finish(int precision, const Geom& g, const BinnedScratch& b, bool classify, bool materialize,
                           const tpicb200_particles* in, tpicb200_particles* out, uint32_t* counts,
                           uint32_t* offsets, uint32_t* cursor, uint32_t* perm, uint32_t* scan_scratch,
@@ -171,6 +172,15 @@ cudaError_t launch_rhs(int precision, const Geom& g, double delta, double kfac, 
 cudaError_t launch_field_advance(int precision, const Geom& g, double theta_value, double faraday,
                                  void* e, const void* bcell, const double* etheta, void* bnext,
                                  uint32_t* invalid, cudaStream_t s);
+// A cycle's report in one launch: rows 0-1 the field energies' partials (`blocks`
+// each), then per species five rows of the movers' partials.
+struct ReportRows {
+  const double* fields;
+  int blocks;
+  const double* movers;  // kMoverPartials a row, five rows a species
+  int written[TPICB200_MAX_SPECIES];
+};
+cudaError_t launch_reduce_report(const ReportRows& rows, int ns, double* out, cudaStream_t s);
 cudaError_t launch_field_energy(int precision, const Geom& g, const void* e, const void* bcell,
                                 double* partials, int blocks, cudaStream_t s);
 cudaError_t launch_species_scalars(int precision, const tpicb200_particles* p, double qom,

@@ -11,13 +11,15 @@
 //   2. exclusive scan of the bins,
 //   3. placement by warp-aggregated atomic cursors (stable within a warp),
 //   4. per-bin fix-up: each bin's source indices are sorted ascending, which
-//      restores the input order among equal keys (warp bitonic sort in shared
-//      memory; block merge-path sort for large bins),
+//      restores the input order among equal keys (a warp ranks them by
+//      counting; block bitonic or merge-path sorts for large bins),
 //   5. one fused gather of every attribute through the permutation.
 // An out-of-range key stops the sort after step 1 (the kernels of steps 2-5
 // test the sort's own flag) and is reported through *invalid.
+#include "grid_barrier.cuh"
 #include "kernels.cuh"
 
+#include <algorithm>
 #include <cuda.h>
 #include <mutex>
 
@@ -55,28 +57,18 @@ __device__ __forceinline__ void aggregated_add(uint32_t* base, int32_t key, bool
   }
 }
 
-// `gate`: the kernels of the general path run only when it is null or holds a
-// nonzero word (the binned sort's fallback flag).
-__device__ __forceinline__ bool closed(const uint32_t* gate) { return gate && *gate == 0; }
-
-__global__ void __launch_bounds__(256) fill_kernel(uint32_t* out, long long n, uint32_t value,
-                                                   const uint32_t* gate) {
-  if (closed(gate)) return;
+__global__ void __launch_bounds__(256) fill_kernel(uint32_t* out, long long n, uint32_t value) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     out[i] = value;
 }
 
-__global__ void __launch_bounds__(256) copy_kernel(uint32_t* out, const uint32_t* __restrict__ in, long long n,
-                                                   const uint32_t* gate) {
-  if (closed(gate)) return;
+__global__ void __launch_bounds__(256) copy_kernel(uint32_t* out, const uint32_t* __restrict__ in, long long n) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     out[i] = in[i];
 }
 
-__global__ void __launch_bounds__(256) histogram_kernel(Geom g, const int32_t* __restrict__ keys,
-                                                        uint32_t count, uint32_t* counts,
-                                                        uint32_t* flag, const uint32_t* gate) {
-  if (closed(gate)) return;
+__device__ __forceinline__ void histogram(const Geom& g, const int32_t* __restrict__ keys, uint32_t count,
+                                          uint32_t* counts, uint32_t* flag) {
   const uint32_t stride = gridDim.x * blockDim.x;
   for (uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < count; base += stride) {
     const uint32_t i = base + (threadIdx.x & 31);
@@ -88,12 +80,16 @@ __global__ void __launch_bounds__(256) histogram_kernel(Geom g, const int32_t* _
     aggregated_add(counts, key, in_range && ok, unused);
   }
 }
+__global__ void __launch_bounds__(256) histogram_kernel(Geom g, const int32_t* __restrict__ keys, uint32_t count,
+                                                        uint32_t* counts, uint32_t* flag) {
+  histogram(g, keys, count, counts, flag);
+}
 
 __global__ void __launch_bounds__(kScanThreads) scan_reduce_kernel(const uint32_t* __restrict__ counts,
                                                                    long long bins, uint32_t* block_sums,
-                                                                   const uint32_t* flag, const uint32_t* gate) {
+                                                                   const uint32_t* flag) {
   __shared__ uint32_t scratch[kScanThreads / 32];
-  if (closed(gate) || *flag) return;
+  if (*flag) return;
   const long long base = (long long)blockIdx.x * kScanTile;
   uint32_t sum = 0;
 #pragma unroll
@@ -107,9 +103,9 @@ __global__ void __launch_bounds__(kScanThreads) scan_reduce_kernel(const uint32_
 
 // Exclusive scan of the block sums by one block of 1024 threads.
 __global__ void __launch_bounds__(1024) scan_block_sums_kernel(uint32_t* block_sums, int nblocks,
-                                                               const uint32_t* flag, const uint32_t* gate) {
+                                                               const uint32_t* flag) {
   __shared__ uint32_t warp_totals[32];
-  if (closed(gate) || *flag) return;
+  if (*flag) return;
   const int per = (nblocks + 1023) / 1024;
   const int first = threadIdx.x * per;
   uint32_t local = 0;
@@ -148,10 +144,9 @@ __global__ void __launch_bounds__(1024) scan_block_sums_kernel(uint32_t* block_s
 __global__ void __launch_bounds__(kScanThreads) scan_down_kernel(const uint32_t* __restrict__ counts,
                                                                  long long bins,
                                                                  const uint32_t* __restrict__ block_sums,
-                                                                 uint32_t* offsets, const uint32_t* flag,
-                                                                 const uint32_t* gate) {
+                                                                 uint32_t* offsets, const uint32_t* flag) {
   __shared__ uint32_t warp_totals[kScanThreads / 32];
-  if (closed(gate) || *flag) return;
+  if (*flag) return;
   const long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanItems;
   uint32_t items[kScanItems];
   uint32_t local = 0;
@@ -181,10 +176,8 @@ __global__ void __launch_bounds__(kScanThreads) scan_down_kernel(const uint32_t*
   if (bins == 0 && blockIdx.x == 0 && threadIdx.x == 0) offsets[0] = 0;
 }
 
-__global__ void __launch_bounds__(256) place_kernel(const int32_t* __restrict__ keys, uint32_t count,
-                                                    uint32_t* cursor, uint32_t* perm,
-                                                    const uint32_t* flag, const uint32_t* gate) {
-  if (closed(gate) || *flag) return;
+__device__ __forceinline__ void place(const int32_t* __restrict__ keys, uint32_t count, uint32_t* cursor,
+                                      uint32_t* perm) {
   const uint32_t stride = gridDim.x * blockDim.x;
   for (uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < count; base += stride) {
     const uint32_t i = base + (threadIdx.x & 31);
@@ -195,31 +188,37 @@ __global__ void __launch_bounds__(256) place_kernel(const int32_t* __restrict__ 
     if (valid) perm[position] = i;
   }
 }
-
-// Warp-level bitonic sort of up to kWarpBinCapacity indices in shared memory.
-__device__ __forceinline__ void warp_bitonic(uint32_t* s, int size) {
-  const int lane = threadIdx.x & 31;
-  for (int k = 2; k <= size; k <<= 1)
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int t = lane; t < size; t += 32) {
-        const int partner = t ^ j;
-        if (partner > t) {
-          const uint32_t a = s[t], b = s[partner];
-          const bool up = (t & k) == 0;
-          if ((a > b) == up) { s[t] = b; s[partner] = a; }
-        }
-      }
-      __syncwarp();
-    }
+__global__ void __launch_bounds__(256) place_kernel(const int32_t* __restrict__ keys, uint32_t count,
+                                                    uint32_t* cursor, uint32_t* perm, const uint32_t* flag) {
+  if (*flag) return;
+  place(keys, count, cursor, perm);
 }
 
-__global__ void __launch_bounds__(256) fixup_small_kernel(const uint32_t* __restrict__ counts,
-                                                          const uint32_t* __restrict__ offsets,
-                                                          long long bins, uint32_t* perm,
-                                                          uint32_t* large_count, uint32_t* large_bins,
-                                                          const uint32_t* flag, const uint32_t* gate) {
-  __shared__ uint32_t buffer[8][kWarpBinCapacity];
-  if (closed(gate) || *flag) return;
+// The n <= kWarpBinCapacity distinct indices in s, written in increasing order
+// to `to` by one warp: an index's place is the number of smaller ones. Every
+// lane holds up to eight of them and compares each of the n with all eight.
+__device__ __forceinline__ void warp_rank_sort(const uint32_t* s, uint32_t n, uint32_t* to) {
+  constexpr int kOwn = kWarpBinCapacity / 32;
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t own[kOwn], rank[kOwn];
+#pragma unroll
+  for (int r = 0; r < kOwn; ++r) {
+    own[r] = 32 * r + lane < n ? s[32 * r + lane] : 0xffffffffu;
+    rank[r] = 0;
+  }
+  for (uint32_t t = 0; t < n; ++t) {
+    const uint32_t other = s[t];
+#pragma unroll
+    for (int r = 0; r < kOwn; ++r) rank[r] += other < own[r] ? 1u : 0u;
+  }
+#pragma unroll
+  for (int r = 0; r < kOwn; ++r)
+    if (32 * r + lane < n) to[rank[r]] = own[r];
+}
+
+__device__ __forceinline__ void fixup_small(const uint32_t* counts, const uint32_t* offsets, long long bins,
+                                            uint32_t* perm, uint32_t* large_count, uint32_t* large_bins,
+                                            uint32_t (*buffer)[kWarpBinCapacity]) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t* s = buffer[warp];
   const long long warps = (long long)gridDim.x * 8;
@@ -238,27 +237,26 @@ __global__ void __launch_bounds__(256) fixup_small_kernel(const uint32_t* __rest
       if (t > 0 && perm[first + t - 1] > value) sorted = false;
     }
     if (__all_sync(0xffffffffu, sorted)) continue;
-    int size = 1;
-    while (size < (int)n) size <<= 1;
-    for (int t = n + lane; t < size; t += 32) s[t] = 0xffffffffu;
     __syncwarp();
-    warp_bitonic(s, size);
-    for (uint32_t t = lane; t < n; t += 32) perm[first + t] = s[t];
+    warp_rank_sort(s, n, perm + first);
     __syncwarp();
   }
+}
+
+__global__ void __launch_bounds__(256) fixup_small_kernel(const uint32_t* counts, const uint32_t* offsets,
+                                                          long long bins, uint32_t* perm, uint32_t* large_count,
+                                                          uint32_t* large_bins, const uint32_t* flag) {
+  __shared__ uint32_t buffer[8][kWarpBinCapacity];
+  if (*flag) return;
+  fixup_small(counts, offsets, bins, perm, large_count, large_bins, buffer);
 }
 
 // One block per large bin. Up to kBlockBinCapacity entries sort in shared
 // memory; larger bins merge runs in global memory with merge-path splits,
 // ping-ponging with `scratch` (a free array of the output records).
-__global__ void __launch_bounds__(1024) fixup_large_kernel(const uint32_t* __restrict__ counts,
-                                                           const uint32_t* __restrict__ offsets,
-                                                           uint32_t* perm, uint32_t* scratch,
-                                                           const uint32_t* large_count,
-                                                           const uint32_t* large_bins,
-                                                           const uint32_t* flag, const uint32_t* gate) {
-  __shared__ uint32_t s[kBlockBinCapacity];
-  if (closed(gate) || *flag) return;
+__device__ __forceinline__ void fixup_large(const uint32_t* counts, const uint32_t* offsets, uint32_t* perm,
+                                            uint32_t* scratch, const uint32_t* large_count,
+                                            const uint32_t* large_bins, uint32_t* s) {
   const uint32_t nlarge = *large_count;
   for (uint32_t item = blockIdx.x; item < nlarge; item += gridDim.x) {
     const uint32_t bin = large_bins[item];
@@ -314,27 +312,71 @@ __global__ void __launch_bounds__(1024) fixup_large_kernel(const uint32_t* __res
   }
 }
 
-template <class Vel>
-__global__ void __launch_bounds__(256) gather_kernel(const uint32_t* __restrict__ perm, uint32_t count,
-    const double* __restrict__ irx, const double* __restrict__ iry, const double* __restrict__ irz,
-    const Vel* __restrict__ iu, const Vel* __restrict__ iv, const Vel* __restrict__ iw,
-    const double* __restrict__ iq, const int32_t* __restrict__ ikey, const uint64_t* __restrict__ iid,
-    double* __restrict__ orx, double* __restrict__ ory, double* __restrict__ orz,
-    Vel* __restrict__ ou, Vel* __restrict__ ov, Vel* __restrict__ ow, double* __restrict__ oq,
-    int32_t* __restrict__ okey, uint64_t* __restrict__ oid, const uint32_t* flag, const uint32_t* gate) {
-  if (closed(gate) || (flag && *flag)) return;
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < count; p += gridDim.x * blockDim.x) {
-    const uint32_t s = perm[p];
-    orx[p] = irx[s]; ory[p] = iry[s]; orz[p] = irz[s];
-    ou[p] = iu[s]; ov[p] = iv[s]; ow[p] = iw[s];
-    oq[p] = iq[s];
-    okey[p] = ikey[s];
-    if (oid) oid[p] = iid[s];
-  }
+__global__ void __launch_bounds__(1024) fixup_large_kernel(const uint32_t* counts, const uint32_t* offsets,
+                                                           uint32_t* perm, uint32_t* scratch,
+                                                           const uint32_t* large_count, const uint32_t* large_bins,
+                                                           const uint32_t* flag) {
+  __shared__ uint32_t s[kBlockBinCapacity];
+  if (*flag) return;
+  fixup_large(counts, offsets, perm, scratch, large_count, large_bins, s);
 }
 
-__global__ void report_kernel(const uint32_t* flag, uint32_t* invalid, const uint32_t* gate) {
-  if (closed(gate)) return;
+// The records of both sides of a gather.
+template <class Vel>
+struct SortRecords {
+  const double *irx, *iry, *irz;
+  const Vel *iu, *iv, *iw;
+  const double* iq;
+  const int32_t* ikey;
+  const uint64_t* iid;
+  double *orx, *ory, *orz;
+  Vel *ou, *ov, *ow;
+  double* oq;
+  int32_t* okey;
+  uint64_t* oid;  // null: no ids
+  SortRecords(const tpicb200_particles* in, tpicb200_particles* out)
+      : irx((const double*)in->rx), iry((const double*)in->ry), irz((const double*)in->rz), iu((const Vel*)in->u),
+        iv((const Vel*)in->v), iw((const Vel*)in->w), iq(in->q), ikey(in->cell), iid(in->id), orx((double*)out->rx),
+        ory((double*)out->ry), orz((double*)out->rz), ou((Vel*)out->u), ov((Vel*)out->v), ow((Vel*)out->w),
+        oq(out->q), okey(out->cell), oid(in->id ? out->id : nullptr) {}
+};
+template <class Vel>
+__device__ __forceinline__ void gather(const uint32_t* perm, uint32_t count, const SortRecords<Vel>& r) {
+  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < count; p += gridDim.x * blockDim.x) {
+    const uint32_t s = perm[p];
+    const double x = __ldg(r.irx + s), y = __ldg(r.iry + s), z = __ldg(r.irz + s), q = __ldg(r.iq + s);
+    const Vel u = __ldg(r.iu + s), v = __ldg(r.iv + s), w = __ldg(r.iw + s);
+    const int32_t key = __ldg(r.ikey + s);
+    r.orx[p] = x;
+    r.ory[p] = y;
+    r.orz[p] = z;
+    r.ou[p] = u;
+    r.ov[p] = v;
+    r.ow[p] = w;
+    r.oq[p] = q;
+    r.okey[p] = key;
+    if (r.oid) r.oid[p] = r.iid[s];
+  }
+}
+template <class Vel>
+__global__ void __launch_bounds__(256) gather_kernel(const uint32_t* __restrict__ perm, uint32_t count,
+                                                     SortRecords<Vel> r, const uint32_t* flag) {
+  if (flag && *flag) return;
+  gather(perm, count, r);
+}
+cudaError_t launch_gather(int precision, const uint32_t* perm, const tpicb200_particles* in, tpicb200_particles* out,
+                          const uint32_t* flag, cudaStream_t s) {
+  const uint32_t n = in->count;
+  const unsigned blocks = grid_for(n, 256, 148u * 8u);
+  if (precision == TPICB200_PRECISION_DOUBLE)
+    gather_kernel<double><<<blocks, 256, 0, s>>>(perm, n, SortRecords<double>(in, out), flag);
+  else
+    gather_kernel<float><<<blocks, 256, 0, s>>>(perm, n, SortRecords<float>(in, out), flag);
+  count_launches(1);
+  return cudaGetLastError();
+}
+
+__global__ void report_kernel(const uint32_t* flag, uint32_t* invalid) {
   if (*flag && invalid) atomicAdd(invalid, 1u);
 }
 
@@ -347,10 +389,10 @@ size_t sort_scan_words(long long bins) {
 
 namespace {
 
-// The general sort; with a gate, every step runs only when *gate != 0.
+// The general sort.
 cudaError_t enqueue_general(int precision, const Geom& g, const tpicb200_particles* in, tpicb200_particles* out,
                             uint32_t* counts, uint32_t* offsets, uint32_t* cursor, uint32_t* perm,
-                            uint32_t* scan_scratch, uint32_t* invalid, const uint32_t* gate, cudaStream_t s) {
+                            uint32_t* scan_scratch, uint32_t* invalid, cudaStream_t s) {
   const long long bins = g.bins;
   const int nblocks = int((bins + kScanTile - 1) / kScanTile);
   ScanScratch sc{scan_scratch, scan_scratch + nblocks, scan_scratch + nblocks + 1,
@@ -358,37 +400,160 @@ cudaError_t enqueue_general(int precision, const Geom& g, const tpicb200_particl
   const uint32_t n = in->count;
   cudaError_t e;
   if ((e = cudaMemsetAsync(sc.flag, 0, 2 * sizeof(uint32_t), s)) != cudaSuccess) return e;
-  fill_kernel<<<grid_for(bins, 256, 148u * 8u), 256, 0, s>>>(counts, bins, 0u, gate);
-  if (n) histogram_kernel<<<grid_for(n, 256, 148u * 8u), 256, 0, s>>>(g, in->cell, n, counts, sc.flag, gate);
-  scan_reduce_kernel<<<nblocks, kScanThreads, 0, s>>>(counts, bins, sc.block_sums, sc.flag, gate);
-  scan_block_sums_kernel<<<1, 1024, 0, s>>>(sc.block_sums, nblocks, sc.flag, gate);
-  scan_down_kernel<<<nblocks, kScanThreads, 0, s>>>(counts, bins, sc.block_sums, offsets, sc.flag, gate);
-  copy_kernel<<<grid_for(bins, 256, 148u * 8u), 256, 0, s>>>(cursor, offsets, bins, gate);
+  fill_kernel<<<grid_for(bins, 256, 148u * 8u), 256, 0, s>>>(counts, bins, 0u);
+  if (n) histogram_kernel<<<grid_for(n, 256, 148u * 8u), 256, 0, s>>>(g, in->cell, n, counts, sc.flag);
+  scan_reduce_kernel<<<nblocks, kScanThreads, 0, s>>>(counts, bins, sc.block_sums, sc.flag);
+  scan_block_sums_kernel<<<1, 1024, 0, s>>>(sc.block_sums, nblocks, sc.flag);
+  scan_down_kernel<<<nblocks, kScanThreads, 0, s>>>(counts, bins, sc.block_sums, offsets, sc.flag);
+  copy_kernel<<<grid_for(bins, 256, 148u * 8u), 256, 0, s>>>(cursor, offsets, bins);
   int launches = 7;
   if (n) {
-    place_kernel<<<grid_for(n, 256, 148u * 8u), 256, 0, s>>>(in->cell, n, cursor, perm, sc.flag, gate);
-    fixup_small_kernel<<<grid_for(bins, 256, 148u * 16u), 256, 0, s>>>(
-        counts, offsets, bins, perm, sc.large_count, sc.large_bins, sc.flag, gate);
-    fixup_large_kernel<<<148, 1024, 0, s>>>(counts, offsets, perm, (uint32_t*)out->cell,
-                                            sc.large_count, sc.large_bins, sc.flag, gate);
-    const unsigned gb = grid_for(n, 256, 148u * 8u);
-    if (precision == TPICB200_PRECISION_DOUBLE)
-      gather_kernel<double><<<gb, 256, 0, s>>>(perm, n, (const double*)in->rx, (const double*)in->ry,
-          (const double*)in->rz, (const double*)in->u, (const double*)in->v, (const double*)in->w,
-          in->q, in->cell, in->id, (double*)out->rx, (double*)out->ry, (double*)out->rz,
-          (double*)out->u, (double*)out->v, (double*)out->w, out->q, out->cell,
-          in->id ? out->id : nullptr, sc.flag, gate);
-    else
-      gather_kernel<float><<<gb, 256, 0, s>>>(perm, n, (const double*)in->rx, (const double*)in->ry,
-          (const double*)in->rz, (const float*)in->u, (const float*)in->v, (const float*)in->w,
-          in->q, in->cell, in->id, (double*)out->rx, (double*)out->ry, (double*)out->rz,
-          (float*)out->u, (float*)out->v, (float*)out->w, out->q, out->cell,
-          in->id ? out->id : nullptr, sc.flag, gate);
-    launches += 4;
+    place_kernel<<<grid_for(n, 256, 148u * 8u), 256, 0, s>>>(in->cell, n, cursor, perm, sc.flag);
+    fixup_small_kernel<<<grid_for(bins, 256, 148u * 16u), 256, 0, s>>>(counts, offsets, bins, perm, sc.large_count,
+                                                                      sc.large_bins, sc.flag);
+    fixup_large_kernel<<<148, 1024, 0, s>>>(counts, offsets, perm, (uint32_t*)out->cell, sc.large_count,
+                                            sc.large_bins, sc.flag);
+    launches += 3;
+    if ((e = launch_gather(precision, perm, in, out, sc.flag, s)) != cudaSuccess) return e;
   }
-  report_kernel<<<1, 1, 0, s>>>(sc.flag, invalid, gate);
+  report_kernel<<<1, 1, 0, s>>>(sc.flag, invalid);
   count_launches(launches + 1);
   return cudaGetLastError();
+}
+
+// ---- The binned sort's cooperative kernels ----
+
+// Exclusive scan of counts[0, bins) into offsets[0, bins] (and cursor, when
+// given) by all CTAs: each takes a contiguous range, whose sum it has stored
+// in sums[blockIdx.x]; the other CTAs' sums are read after a grid barrier.
+constexpr int kCoopThreads = 256;
+__device__ __forceinline__ void coop_range(long long bins, long long& b0, long long& b1) {
+  const long long each = (bins + gridDim.x - 1) / gridDim.x;
+  b0 = min(blockIdx.x * each, bins);
+  b1 = min(b0 + each, bins);
+}
+__device__ __forceinline__ void coop_scan(const uint32_t* counts, long long bins, const uint32_t* sums,
+                                          uint32_t* offsets, uint32_t* cursor) {
+  __shared__ uint32_t scratch[kCoopThreads / 32];
+  __shared__ uint32_t warp_totals[kCoopThreads / 32];
+  constexpr int kItems = 4;
+  uint32_t before = 0;
+  for (unsigned b = threadIdx.x; b < blockIdx.x; b += kCoopThreads) before += __ldcg(sums + b);
+  uint32_t running = block_sum<kCoopThreads>(before, scratch);
+  long long b0, b1;
+  coop_range(bins, b0, b1);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (long long tile = b0; tile < b1; tile += kItems * kCoopThreads) {
+    const long long at = tile + (long long)threadIdx.x * kItems;
+    uint32_t items[kItems], local = 0;
+#pragma unroll
+    for (int r = 0; r < kItems; ++r) {
+      items[r] = at + r < b1 ? __ldcg(counts + at + r) : 0u;
+      local += items[r];
+    }
+    uint32_t inclusive = local;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, inclusive, o);
+      if (lane >= o) inclusive += t;
+    }
+    __syncthreads();
+    if (lane == 31) warp_totals[warp] = inclusive;
+    __syncthreads();
+    uint32_t prefix = running, total = 0;
+#pragma unroll
+    for (int w = 0; w < kCoopThreads / 32; ++w) {
+      if (w < warp) prefix += warp_totals[w];
+      total += warp_totals[w];
+    }
+    prefix += inclusive - local;
+#pragma unroll
+    for (int r = 0; r < kItems; ++r) {
+      if (at + r < b1) {
+        offsets[at + r] = prefix;
+        if (cursor) cursor[at + r] = prefix;
+      }
+      prefix += items[r];
+    }
+    running += total;
+  }
+  if (b1 == bins && b0 < b1 && threadIdx.x == 0) offsets[bins] = running;
+}
+
+// A grid barrier that gave up counts 1 << 22 in *invalid.
+__device__ __forceinline__ bool coop_wait(GridBarrier& barrier, uint32_t* invalid) {
+  if (barrier.wait()) return true;
+  if (threadIdx.x == 0 && invalid) atomicAdd(invalid, 1u << 22);
+  return false;
+}
+
+// The general sort in one launch, for the binned sort's fallback: enqueued
+// behind every binned sort and leaving at once unless the fallback flag is up.
+// As the general sort's eleven kernels it cost 25 us of empty launches per
+// species and cycle. Its steps are separated by grid barriers; at the end the
+// flags are cleared for the next sort.
+template <class Vel>
+__global__ void __launch_bounds__(kCoopThreads, 2) fallback_sort_kernel(Geom g, uint32_t n, SortRecords<Vel> r,
+                                                                        uint32_t* counts, uint32_t* offsets,
+                                                                        uint32_t* cursor, uint32_t* perm,
+                                                                        ScanScratch sc, uint32_t* invalid,
+                                                                        BinnedState* state) {
+  __shared__ uint32_t buffer[kBlockBinCapacity];
+  __shared__ uint32_t scratch[kCoopThreads / 32];
+  if (state->fallback == 0) return;
+  GridBarrier barrier(state->barrier);
+  uint32_t* sums = sc.large_bins;  // free until the fix-up
+  for (long long b = blockIdx.x * (long long)kCoopThreads + threadIdx.x; b < g.bins;
+       b += (long long)gridDim.x * kCoopThreads)
+    counts[b] = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *sc.flag = *sc.large_count = 0;
+  if (!coop_wait(barrier, invalid)) return;
+  histogram(g, r.ikey, n, counts, sc.flag);
+  if (!coop_wait(barrier, invalid)) return;
+  const bool bad = __ldcg(sc.flag) != 0;
+  if (!bad) {
+    long long b0, b1;
+    coop_range(g.bins, b0, b1);
+    uint32_t sum = 0;
+    for (long long b = b0 + threadIdx.x; b < b1; b += kCoopThreads) sum += __ldcg(counts + b);
+    sum = block_sum<kCoopThreads>(sum, scratch);
+    if (threadIdx.x == 0) sums[blockIdx.x] = sum;
+    if (!coop_wait(barrier, invalid)) return;
+    coop_scan(counts, g.bins, sums, offsets, cursor);
+    if (!coop_wait(barrier, invalid)) return;
+    place(r.ikey, n, cursor, perm);
+    if (!coop_wait(barrier, invalid)) return;
+    fixup_small(counts, offsets, g.bins, perm, sc.large_count, sc.large_bins,
+                reinterpret_cast<uint32_t (*)[kWarpBinCapacity]>(buffer));
+    if (!coop_wait(barrier, invalid)) return;
+    fixup_large(counts, offsets, perm, (uint32_t*)r.okey, sc.large_count, sc.large_bins, buffer);
+    if (!coop_wait(barrier, invalid)) return;
+    gather(perm, n, r);
+  } else if (blockIdx.x == 0 && threadIdx.x == 0 && invalid) {
+    atomicAdd(invalid, 1u);
+  }
+  if (!coop_wait(barrier, invalid)) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) state->fallback = state->bins_bad = 0;
+  barrier.leave();
+}
+
+template <class Vel>
+cudaError_t launch_fallback(const Geom& g, const tpicb200_particles* in, tpicb200_particles* out, uint32_t* counts,
+                            uint32_t* offsets, uint32_t* cursor, uint32_t* perm, uint32_t* scan_scratch,
+                            uint32_t* invalid, BinnedState* state, cudaStream_t s) {
+  const int nblocks = int((g.bins + kScanTile - 1) / kScanTile);
+  ScanScratch sc{scan_scratch, scan_scratch + nblocks, scan_scratch + nblocks + 1, scan_scratch + nblocks + 2};
+  Geom geom = g;
+  uint32_t n = in->count;
+  SortRecords<Vel> r(in, out);
+  // Two CTAs an SM, fewer for little work (a barrier costs with their number);
+  // their sums must fit the bins' scratch.
+  const long long work = std::max<long long>(g.bins, n);
+  const unsigned blocks = unsigned(std::min<long long>(grid_for(work, 4 * kCoopThreads, 148u * 2u), g.bins));
+  void* args[] = {&geom, &n, &r, &counts, &offsets, &cursor, &perm, &sc, &invalid, &state};
+  count_launches(1);
+  return cudaLaunchCooperativeKernel((const void*)fallback_sort_kernel<Vel>, dim3(blocks), dim3(kCoopThreads), args, 0,
+                                     s);
 }
 
 // ---- Binned sort: the input is grouped by the bins of an earlier sort ----
@@ -464,45 +629,32 @@ __device__ __forceinline__ int key_move_code(const Geom& g, int i, int j, int k,
   return move_code(g, i, j, k, a, b, c);
 }
 
-// The old bins must tile the records in key order: disjoint ranges in
-// increasing key order, records only in interior cells, n records in all.
-__global__ void __launch_bounds__(256) validate_bins_kernel(Geom g, uint32_t n,
-                                                            const uint32_t* __restrict__ old_counts,
-                                                            const uint32_t* __restrict__ old_offsets,
-                                                            BinnedState* state) {
-  __shared__ unsigned long long partial[8];
+// The old bins copied (the new ones may overwrite them in place), checked, and
+// the transfer counts cleared when the mover will add into them. The bins must
+// tile the n records in key order: each starts where the one before it ends,
+// the first at 0, the last ending at n, records only in interior cells.
+__global__ void __launch_bounds__(256) binned_begin_kernel(Geom g, uint32_t n, const uint32_t* in_counts,
+                                                           const uint32_t* in_offsets, uint32_t* old_counts,
+                                                           uint32_t* old_offsets, uint32_t* transfer,
+                                                           long long transfer_words, BinnedState* state) {
+  const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
   bool bad = false;
-  unsigned long long total = 0;
-  for (long long b = blockIdx.x * (long long)blockDim.x + threadIdx.x; b < g.bins;
-       b += (long long)gridDim.x * blockDim.x) {
-    const uint32_t off = old_offsets[b], cnt = old_counts[b];
-    if ((unsigned long long)off + cnt > old_offsets[b + 1]) bad = true;
+  for (long long b = first; b < g.bins; b += stride) {
+    const uint32_t off = in_offsets[b], cnt = in_counts[b], next = in_offsets[b + 1];
+    bad = bad || (unsigned long long)off + cnt != next || (b == 0 && off != 0) || (b + 1 == g.bins && next != n);
     if (cnt) {
       int i, j, k;
       g.decode(int32_t(b), i, j, k);
-      if (!g.interior_cell(i, j, k)) bad = true;
+      bad = bad || !g.interior_cell(i, j, k);
     }
-    total += cnt;
+    old_counts[b] = cnt;
+    old_offsets[b] = off;
+    if (b + 1 == g.bins) old_offsets[g.bins] = next;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0 && old_offsets[g.bins] > n) bad = true;
-  total = warp_sum(total);
-  if ((threadIdx.x & 31) == 0) partial[threadIdx.x >> 5] = total;
-  const bool any_bad = __syncthreads_or(bad);
-  if (threadIdx.x == 0) {
-    unsigned long long block_total = 0;
-    for (int w = 0; w < 8; ++w) block_total += partial[w];
-    atomicAdd(&state->total, block_total);
-    if (any_bad) {
-      atomicExch(&state->bins_bad, 1u);
-      atomicExch(&state->fallback, 1u);
-    }
-  }
-}
-
-__global__ void decide_kernel(uint32_t n, BinnedState* state) {
-  if (state->total != (unsigned long long)n) {
-    state->bins_bad = 1;
-    state->fallback = 1;
+  for (long long t = first; t < transfer_words; t += stride) transfer[t] = 0;
+  if (__syncthreads_or(bad) && threadIdx.x == 0) {
+    atomicExch(&state->bins_bad, 1u);
+    atomicExch(&state->fallback, 1u);
   }
 }
 
@@ -565,34 +717,30 @@ __global__ void __launch_bounds__(kBinnedThreads) classify_kernel(Geom g, const 
   if (__syncthreads_or(bad) && threadIdx.x == 0) atomicExch(&state->fallback, 1u);
 }
 
-__global__ void __launch_bounds__(256) binned_counts_kernel(Geom g, const uint32_t* __restrict__ transfer,
-                                                            uint32_t* counts, const BinnedState* state) {
-  if (state->fallback) return;
+// Records that bin b receives.
+__device__ __forceinline__ uint32_t binned_count(const Geom& g, const uint32_t* __restrict__ transfer, long long b) {
   const int nx = g.nx, ny = g.ny, nz = g.nz;
   const long long cells = (long long)nx * ny * nz;
-  for (long long b = blockIdx.x * (long long)blockDim.x + threadIdx.x; b < g.bins;
-       b += (long long)gridDim.x * blockDim.x) {
-    int i, j, k;
-    g.decode(int32_t(b), i, j, k);
-    uint32_t sum = 0;
-    if (g.interior_cell(i, j, k)) {
+  int i, j, k;
+  g.decode(int32_t(b), i, j, k);
+  uint32_t sum = 0;
+  if (g.interior_cell(i, j, k)) {
 #pragma unroll
-      for (int dz = -1; dz <= 1; ++dz)
+    for (int dz = -1; dz <= 1; ++dz)
 #pragma unroll
-        for (int dy = -1; dy <= 1; ++dy)
+      for (int dy = -1; dy <= 1; ++dy)
 #pragma unroll
-          for (int dx = -1; dx <= 1; ++dx) {
-            // Neighbour offsets are -1..1: a conditional wrap (no modulo).
-            int si = i - dx, sj = j - dy, sk = k - dz;
-            si = si < 0 ? si + nx : (si >= nx ? si - nx : si);
-            sj = sj < 0 ? sj + ny : (sj >= ny ? sj - ny : sj);
-            sk = sk < 0 ? sk + nz : (sk >= nz ? sk - nz : sk);
-            const int d = (dx + 1) + 3 * (dy + 1) + 9 * (dz + 1);
-            sum += transfer[d * cells + si + (long long)nx * (sj + (long long)ny * sk)];
-          }
-    }
-    counts[b] = sum;
+        for (int dx = -1; dx <= 1; ++dx) {
+          // Neighbour offsets are -1..1: a conditional wrap (no modulo).
+          int si = i - dx, sj = j - dy, sk = k - dz;
+          si = si < 0 ? si + nx : (si >= nx ? si - nx : si);
+          sj = sj < 0 ? sj + ny : (sj >= ny ? sj - ny : sj);
+          sk = sk < 0 ? sk + nz : (sk >= nz ? sk - nz : sk);
+          const int d = (dx + 1) + 3 * (dy + 1) + 9 * (dz + 1);
+          sum += transfer[d * cells + si + (long long)nx * (sj + (long long)ny * sk)];
+        }
   }
+  return sum;
 }
 
 // Directions along one axis in increasing source coordinate: the sources of
@@ -603,9 +751,7 @@ __device__ __forceinline__ void source_order(int x, int n, int (&d)[3]) {
   else { d[0] = 1; d[1] = 0; d[2] = -1; }
 }
 
-__global__ void __launch_bounds__(256) binned_bases_kernel(Geom g, const uint32_t* __restrict__ offsets,
-                                                           uint32_t* transfer, const BinnedState* state) {
-  if (state->fallback) return;
+__device__ __forceinline__ void binned_bases(const Geom& g, const uint32_t* offsets, uint32_t* transfer) {
   const int nx = g.nx, ny = g.ny, nz = g.nz;
   const long long cells = (long long)nx * ny * nz;
   for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < cells;
@@ -642,6 +788,33 @@ __global__ void __launch_bounds__(256) binned_bases_kernel(Geom g, const uint32_
       base += count[e];
     }
   }
+}
+
+// Counts, their scan and the bases in one launch, the passes separated by grid
+// barriers. As five kernels they were launch latency on small grids (127 x 65
+// x 1 FP64 particle stage 125 us, 111 us with one) and no faster on large ones
+// (128^3 cycle 27.1 ms, 26.8 ms with one).
+__global__ void __launch_bounds__(kCoopThreads, 2) binned_plan_kernel(Geom g, uint32_t* transfer, uint32_t* counts,
+                                                                      uint32_t* offsets, uint32_t* sums,
+                                                                      uint32_t* invalid, BinnedState* state) {
+  __shared__ uint32_t scratch[kCoopThreads / 32];
+  if (state->fallback) return;
+  GridBarrier barrier(state->barrier);
+  long long b0, b1;
+  coop_range(g.bins, b0, b1);
+  uint32_t sum = 0;
+  for (long long b = b0 + threadIdx.x; b < b1; b += kCoopThreads) {
+    const uint32_t count = binned_count(g, transfer, b);
+    counts[b] = count;
+    sum += count;
+  }
+  sum = block_sum<kCoopThreads>(sum, scratch);
+  if (threadIdx.x == 0) sums[blockIdx.x] = sum;
+  if (!coop_wait(barrier, invalid)) return;
+  coop_scan(counts, g.bins, sums, offsets, nullptr);
+  if (!coop_wait(barrier, invalid)) return;
+  binned_bases(g, offsets, transfer);
+  barrier.leave();
 }
 
 // The lane mask of a live lane's slot: the live lanes with the same slot
@@ -730,28 +903,14 @@ cudaError_t launch_sort(int precision, const Geom& g, const tpicb200_particles* 
                         uint32_t* cursor, uint32_t* perm, uint32_t* scan_scratch,
                         uint32_t* invalid, cudaStream_t s) {
   out->count = in->count;
-  return enqueue_general(precision, g, in, out, counts, offsets, cursor, perm, scan_scratch, invalid, nullptr, s);
+  return enqueue_general(precision, g, in, out, counts, offsets, cursor, perm, scan_scratch, invalid, s);
 }
 
 cudaError_t launch_sorted_gather(int precision, const uint32_t* perm, const tpicb200_particles* in,
                                  tpicb200_particles* out, cudaStream_t s) {
-  const uint32_t n = in->count;
-  out->count = n;
-  if (!n) return cudaSuccess;
-  const unsigned gb = grid_for(n, 256, 148u * 8u);
-  const uint32_t* zero = nullptr;  // no stop flag
-  if (precision == TPICB200_PRECISION_DOUBLE)
-    gather_kernel<double><<<gb, 256, 0, s>>>(perm, n, (const double*)in->rx, (const double*)in->ry,
-        (const double*)in->rz, (const double*)in->u, (const double*)in->v, (const double*)in->w, in->q, in->cell,
-        in->id, (double*)out->rx, (double*)out->ry, (double*)out->rz, (double*)out->u, (double*)out->v,
-        (double*)out->w, out->q, out->cell, in->id ? out->id : nullptr, zero, nullptr);
-  else
-    gather_kernel<float><<<gb, 256, 0, s>>>(perm, n, (const double*)in->rx, (const double*)in->ry,
-        (const double*)in->rz, (const float*)in->u, (const float*)in->v, (const float*)in->w, in->q, in->cell,
-        in->id, (double*)out->rx, (double*)out->ry, (double*)out->rz, (float*)out->u, (float*)out->v,
-        (float*)out->w, out->q, out->cell, in->id ? out->id : nullptr, zero, nullptr);
-  count_launches(1);
-  return cudaGetLastError();
+  out->count = in->count;
+  if (!in->count) return cudaSuccess;
+  return launch_gather(precision, perm, in, out, nullptr, s);
 }
 
 size_t binned_scratch_words(const Geom& g) {
@@ -775,26 +934,14 @@ BinnedScratch binned_scratch(const Geom& g, uint32_t* words, uint16_t* codes) {
   return b;
 }
 
-cudaError_t binned_begin(const Geom& g, const BinnedScratch& b, const uint32_t* in_counts,
-                         const uint32_t* in_offsets, bool zero_transfer, cudaStream_t s) {
-  // The old bins are copied first: the new ones may overwrite them in place.
-  cudaError_t e;
-  if ((e = cudaMemsetAsync(b.state, 0, sizeof(BinnedState), s)) != cudaSuccess) return e;
-  if ((e = cudaMemcpyAsync(b.old_counts, in_counts, size_t(g.bins) * 4, cudaMemcpyDeviceToDevice, s)) !=
-      cudaSuccess)
-    return e;
-  if ((e = cudaMemcpyAsync(b.old_offsets, in_offsets, size_t(g.bins + 1) * 4, cudaMemcpyDeviceToDevice, s)) !=
-      cudaSuccess)
-    return e;
-  if (zero_transfer)
-    e = cudaMemsetAsync(b.transfer, 0, size_t(27) * size_t((long long)g.nx * g.ny * g.nz) * 4, s);
-  return e;
-}
+cudaError_t binned_reset(const BinnedScratch& b) { return cudaMemset(b.state, 0, sizeof(BinnedState)); }
 
-cudaError_t binned_validate(const Geom& g, const BinnedScratch& b, uint32_t n, cudaStream_t s) {
-  validate_bins_kernel<<<grid_for(g.bins, 256, 148u * 8u), 256, 0, s>>>(g, n, b.old_counts, b.old_offsets, b.state);
-  decide_kernel<<<1, 1, 0, s>>>(n, b.state);
-  count_launches(2);
+cudaError_t binned_begin(const Geom& g, const BinnedScratch& b, uint32_t n, const uint32_t* in_counts,
+                         const uint32_t* in_offsets, bool zero_transfer, cudaStream_t s) {
+  const long long words = zero_transfer ? 27LL * g.nx * g.ny * g.nz : 0;
+  binned_begin_kernel<<<grid_for(std::max(g.bins, words / 4), 256, 148u * 8u), 256, 0, s>>>(
+      g, n, in_counts, in_offsets, b.old_counts, b.old_offsets, b.transfer, words, b.state);
+  count_launches(1);
   return cudaGetLastError();
 }
 
@@ -803,52 +950,40 @@ cudaError_t binned_finish(int precision, const Geom& g, const BinnedScratch& b, 
                           uint32_t* offsets, uint32_t* cursor, uint32_t* perm, uint32_t* scan_scratch,
                           uint32_t* invalid, cudaStream_t s) {
   const long long bins = g.bins;
-  const long long cells = (long long)g.nx * g.ny * g.nz;
   const uint32_t n = in->count;
   out->count = n;
   // One warp per run (up to 32 cells of an x-row).
   const unsigned runs_grid = grid_for(run_count(g) * 32, kBinnedThreads, 148u * 8u);
-  int launches = 0;
   if (classify) {
     classify_kernel<<<runs_grid, kBinnedThreads, 0, s>>>(g, in->cell, n, b.old_counts, b.old_offsets, b.transfer,
                                                         b.code, b.state);
-    ++launches;
+    count_launches(1);
   }
-  binned_counts_kernel<<<grid_for(bins, 256, 148u * 16u), 256, 0, s>>>(g, b.transfer, counts, b.state);
   const int nblocks = int((bins + kScanTile - 1) / kScanTile);
-  // The scan kernels take the fallback flag as their stop flag: they run only
-  // when it is clear.
   ScanScratch sc{scan_scratch, scan_scratch + nblocks, scan_scratch + nblocks + 1, scan_scratch + nblocks + 2};
-  scan_reduce_kernel<<<nblocks, kScanThreads, 0, s>>>(counts, bins, sc.block_sums, &b.state->fallback, nullptr);
-  scan_block_sums_kernel<<<1, 1024, 0, s>>>(sc.block_sums, nblocks, &b.state->fallback, nullptr);
-  scan_down_kernel<<<nblocks, kScanThreads, 0, s>>>(counts, bins, sc.block_sums, offsets, &b.state->fallback,
-                                                    nullptr);
-  binned_bases_kernel<<<grid_for(cells, 256, 148u * 16u), 256, 0, s>>>(g, offsets, b.transfer, b.state);
+  cudaError_t e = cudaSuccess;
+  {
+    Geom geom = g;
+    uint32_t *transfer = b.transfer, *sums = sc.large_bins;
+    BinnedState* state = b.state;
+    void* args[] = {&geom, &transfer, &counts, &offsets, &sums, &invalid, &state};
+    const unsigned blocks = unsigned(std::min<long long>(grid_for(bins, kCoopThreads, 148u * 2u), bins));
+    e = cudaLaunchCooperativeKernel((const void*)binned_plan_kernel, dim3(blocks), dim3(kCoopThreads), args, 0, s);
+    count_launches(1);
+  }
+  if (e != cudaSuccess) return e;
   binned_rank_kernel<<<runs_grid, kBinnedThreads, 0, s>>>(g, n, b.old_counts, b.old_offsets, b.transfer, b.code,
                                                            in->cell, perm, b.state);
+  count_launches(1);
   // The gather writes the records unless a check raised the fallback flag
   // (without `materialize` the caller reads the records through perm).
-  if (n && materialize) {
-    const unsigned gb = grid_for(n, 256, 148u * 8u);
-    if (precision == TPICB200_PRECISION_DOUBLE)
-      gather_kernel<double><<<gb, 256, 0, s>>>(perm, n, (const double*)in->rx, (const double*)in->ry,
-          (const double*)in->rz, (const double*)in->u, (const double*)in->v, (const double*)in->w,
-          in->q, in->cell, in->id, (double*)out->rx, (double*)out->ry, (double*)out->rz,
-          (double*)out->u, (double*)out->v, (double*)out->w, out->q, out->cell,
-          in->id ? out->id : nullptr, &b.state->fallback, nullptr);
-    else
-      gather_kernel<float><<<gb, 256, 0, s>>>(perm, n, (const double*)in->rx, (const double*)in->ry,
-          (const double*)in->rz, (const float*)in->u, (const float*)in->v, (const float*)in->w,
-          in->q, in->cell, in->id, (double*)out->rx, (double*)out->ry, (double*)out->rz,
-          (float*)out->u, (float*)out->v, (float*)out->w, out->q, out->cell,
-          in->id ? out->id : nullptr, &b.state->fallback, nullptr);
-    ++launches;
-  }
-  count_launches(launches + 6);
-  if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) return e;
-  // General sort, gated on the fallback flag: it rewrites every output.
-  return enqueue_general(precision, g, in, out, counts, offsets, cursor, perm, scan_scratch, invalid,
-                         &b.state->fallback, s);
+  if (n && materialize) e = launch_gather(precision, perm, in, out, &b.state->fallback, s);
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  // The general sort behind the fallback flag: it rewrites every output.
+  return precision == TPICB200_PRECISION_DOUBLE
+             ? launch_fallback<double>(g, in, out, counts, offsets, cursor, perm, scan_scratch, invalid, b.state, s)
+             : launch_fallback<float>(g, in, out, counts, offsets, cursor, perm, scan_scratch, invalid, b.state, s);
 }
 
 cudaError_t launch_sort_binned(int precision, const Geom& g, const tpicb200_particles* in,
@@ -857,8 +992,7 @@ cudaError_t launch_sort_binned(int precision, const Geom& g, const tpicb200_part
                                uint32_t* scan_scratch, uint32_t* binned_words, uint16_t* codes,
                                uint32_t* invalid, cudaStream_t s) {
   const BinnedScratch b = binned_scratch(g, binned_words, codes);
-  if (cudaError_t e = binned_begin(g, b, in_counts, in_offsets, false, s); e != cudaSuccess) return e;
-  if (cudaError_t e = binned_validate(g, b, in->count, s); e != cudaSuccess) return e;
+  if (cudaError_t e = binned_begin(g, b, in->count, in_counts, in_offsets, false, s); e != cudaSuccess) return e;
   return binned_finish(precision, g, b, true, true, in, out, counts, offsets, cursor, perm, scan_scratch, invalid,
                        s);
 }
@@ -967,7 +1101,7 @@ cudaError_t launch_sort_static(int precision, const Geom& g, const tpicb200_part
   // flags and large-bin count (memset), the counts (fill); the cursors are
   // copied from the offsets and the permutation is fully written.
   out->count = in->count;
-  return enqueue_general(precision, g, in, out, counts, offsets, cursor, perm, scan, invalid, nullptr, s);
+  return enqueue_general(precision, g, in, out, counts, offsets, cursor, perm, scan, invalid, s);
 }
 
 }  // namespace tpicb200
