@@ -131,6 +131,61 @@ __device__ __forceinline__ bool record_values(const MomentRecord<Vel>& r, bool v
   return ok;
 }
 
+// A warp's walk over cells: the records of a cell's two species form one
+// stream (species 0 first), so that a cell has at most one chunk that is not
+// full.
+struct MomentCell {
+  int32_t key;
+  uint32_t begin[kFuse], n[kFuse], total;
+};
+template <class Vel>
+struct MomentWalk {
+  const Geom& g;
+  const MomentParams<Vel>& mp;
+  uint32_t nx, ny, cells;
+  __device__ __forceinline__ MomentWalk(const Geom& geom, const MomentParams<Vel>& params)
+      : g(geom), mp(params), nx(geom.nx), ny(geom.ny), cells(uint32_t(geom.nx) * geom.ny * geom.nz) {}
+  __device__ __forceinline__ void coordinates(uint32_t cell, int& i, int& j, int& k) const {
+    const uint32_t row = cell / nx;
+    i = int(cell - row * nx);
+    j = int(row % ny);
+    k = int(row / ny);
+  }
+  __device__ __forceinline__ MomentCell info(uint32_t cell) const {
+    MomentCell c{};
+    if (cell >= cells) return c;
+    int i, j, k;
+    coordinates(cell, i, j, k);
+    c.key = g.encode(i, j, k);
+#pragma unroll
+    for (int s = 0; s < kFuse; ++s)
+      if (s < mp.ns) {
+        c.begin[s] = mp.sp[s].offsets[c.key];
+        c.n[s] = mp.sp[s].counts[c.key];
+      }
+    c.total = c.n[0] + c.n[1];
+    return c;
+  }
+  __device__ __forceinline__ int species(const MomentCell& c, uint32_t at) const { return at >= c.n[0] ? 1 : 0; }
+  // Record o + lane of the cell.
+  __device__ __forceinline__ void load(const MomentCell& c, uint32_t o, MomentRecord<Vel>& r) const {
+    const uint32_t at = o + (threadIdx.x & 31u);
+    if (at >= c.total) return;
+    const int s = species(c, at);
+    r.load(mp.sp[s], (s ? c.begin[1] - c.n[0] : c.begin[0]) + at);
+  }
+  // B at the corners of a cell, [c][a], by the first 24 lanes.
+  template <class F, class C>
+  __device__ __forceinline__ void corners(uint32_t cell, const F* __restrict__ bnode, C* bc) const {
+    const int lane = threadIdx.x & 31;
+    if (lane >= 24) return;
+    int i, j, k;
+    coordinates(cell, i, j, k);
+    const int c = lane >> 3, a = lane & 7;
+    bc[lane] = C(bnode[c * g.nodes + g.node(i + (a & 1), j + ((a >> 1) & 1), k + ((a >> 2) & 1))]);
+  }
+};
+
 // A moment as it is stored: zero, and counted, when its sum is not finite.
 template <class T>
 __device__ __forceinline__ T checked(T value, uint32_t& bad) {
@@ -181,44 +236,11 @@ __global__ void __launch_bounds__(kF32Warps * 32, 4) moments_f32_kernel(Geom g, 
   extern __shared__ __align__(16) uint8_t f32_smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   F32Warp& S = reinterpret_cast<F32Warp*>(f32_smem)[warp];
-  const uint32_t nx = uint32_t(g.nx), ny = uint32_t(g.ny);
-  const uint32_t cells = nx * ny * uint32_t(g.nz);
+  const MomentWalk<float> walk(g, mp);
+  const uint32_t cells = walk.cells;
   const uint32_t warps = gridDim.x * kF32Warps;
   const int quarter = lane >> 3, tg = lane & 3, eg = (lane >> 2) & 1;
   uint32_t bad = 0;
-
-  struct Cell {
-    int32_t key;
-    uint32_t begin[kFuse], n[kFuse], total;
-  };
-  auto coordinates = [&](uint32_t cell, int& i, int& j, int& k) {
-    const uint32_t row = cell / nx;
-    i = int(cell - row * nx);
-    j = int(row % ny);
-    k = int(row / ny);
-  };
-  auto info = [&](uint32_t cell) {
-    Cell c{};
-    if (cell >= cells) return c;
-    int i, j, k;
-    coordinates(cell, i, j, k);
-    c.key = g.encode(i, j, k);
-#pragma unroll
-    for (int s = 0; s < kFuse; ++s)
-      if (s < mp.ns) {
-        c.begin[s] = mp.sp[s].offsets[c.key];
-        c.n[s] = mp.sp[s].counts[c.key];
-      }
-    c.total = c.n[0] + c.n[1];
-    return c;
-  };
-  // Record o + lane of the cell (species 0 first).
-  auto load = [&](const Cell& c, uint32_t o, MomentRecord<float>& r) {
-    const uint32_t at = o + lane;
-    if (at >= c.total) return;
-    const int s = at >= c.n[0] ? 1 : 0;
-    r.load(mp.sp[s], (s ? c.begin[1] - c.n[0] : c.begin[0]) + at);
-  };
   // The cell after `cell` in this warp's order (batches strided by the grid).
   auto following = [&](uint32_t cell) {
     const uint32_t next = cell + 1;
@@ -226,33 +248,28 @@ __global__ void __launch_bounds__(kF32Warps * 32, 4) moments_f32_kernel(Geom g, 
   };
 
   uint32_t cell = (blockIdx.x * kF32Warps + warp) * batch;
-  Cell cur = info(cell);
+  MomentCell cur = walk.info(cell);
   MomentRecord<float> next;
-  load(cur, 0, next);
+  walk.load(cur, 0, next);
   while (cell < cells) {
     const uint32_t cell_next = following(cell);
-    const Cell after = info(cell_next);
-    int ci, cj, ck;
-    coordinates(cell, ci, cj, ck);
+    const MomentCell after = walk.info(cell_next);
     __syncwarp();
-    if (lane < 24) {
-      const int c = lane >> 3, a = lane & 7;
-      S.bc[lane] = bnode[c * g.nodes + g.node(ci + (a & 1), cj + ((a >> 1) & 1), ck + ((a >> 2) & 1))];
-    }
+    walk.corners(cell, bnode, S.bc);
     __syncwarp();
     float2 acc[7][3];
 #pragma unroll
     for (int i = 0; i < 7; ++i)
 #pragma unroll
       for (int e = 0; e < 3; ++e) acc[i][e] = make_float2(0.0f, 0.0f);
-    if (cur.total == 0) load(after, 0, next);
+    if (cur.total == 0) walk.load(after, 0, next);
     for (uint32_t o = 0; o < cur.total; o += 32) {
       const uint32_t m = min(cur.total - o, 32u);
       const MomentRecord<float> r = next;
-      if (o + 32 < cur.total) load(cur, o + 32, next);
-      else load(after, 0, next);
+      if (o + 32 < cur.total) walk.load(cur, o + 32, next);
+      else walk.load(after, 0, next);
       const bool active = lane < int(m);
-      const int sp = active && o + lane >= cur.n[0] ? 1 : 0;
+      const int sp = active ? walk.species(cur, o + lane) : 0;
       // Zeros from the lanes without a record fill the rows past m.
       float* row = S.rec[lane];
       float value[12], prod[28];
@@ -391,25 +408,25 @@ struct F64Warp {
 };
 
 template <class Vel, class Fld, class Mom>
-__global__ void __launch_bounds__(kF64Warps * 32) moments_f64_kernel(Geom g, MomentParams<Vel> mp,
+__global__ void __launch_bounds__(kF64Warps * 32, 4) moments_f64_kernel(Geom g, MomentParams<Vel> mp,
                                                                      const Fld* __restrict__ bnode,
                                                                      Mom* __restrict__ mom, int accumulate,
                                                                      uint32_t* invalid) {
   __shared__ F64Warp shared[kF64Warps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   F64Warp& S = shared[warp];
-  const int nx = g.nx, ny = g.ny;
-  const long long cells = (long long)nx * ny * g.nz, nn = g.nodes;
+  const MomentWalk<Vel> walk(g, mp);
+  const uint32_t stride = gridDim.x * kF64Warps;
   const int kk = lane & 3, rr = lane >> 2;  // fragment coordinates
   uint32_t bad = 0;
-  for (long long cell = (long long)blockIdx.x * kF64Warps + warp; cell < cells;
-       cell += (long long)gridDim.x * kF64Warps) {
-    const int ci = int(cell % nx), cj = int((cell / nx) % ny), ck = int(cell / ((long long)nx * ny));
-    const int32_t key = g.encode(ci, cj, ck);
-    if (lane < 24) {
-      const int c = lane >> 3, a = lane & 7;
-      S.bc[lane] = double(bnode[c * nn + g.node(ci + (a & 1), cj + ((a >> 1) & 1), ck + ((a >> 2) & 1))]);
-    }
+  uint32_t cell = blockIdx.x * kF64Warps + warp;
+  MomentCell cur = walk.info(cell);
+  MomentRecord<Vel> next;
+  walk.load(cur, 0, next);
+  while (cell < walk.cells) {
+    const uint32_t cell_next = cell + stride;
+    const MomentCell after = walk.info(cell_next);
+    walk.corners(cell, bnode, S.bc);
     __syncwarp();
     // D tiles (t: 4 x 8 rows, entry: 2 x 8 columns) of this lane.
     double acc[4][2][2];
@@ -417,43 +434,41 @@ __global__ void __launch_bounds__(kF64Warps * 32) moments_f64_kernel(Geom g, Mom
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int e = 0; e < 2; ++e) acc[i][e][0] = acc[i][e][1] = 0.0;
-    for (int si = 0; si < mp.ns; ++si) {
-      const MomentSpecies<Vel>& sp = mp.sp[si];
-      const uint32_t begin = sp.offsets[key], n = sp.counts[key];
-      for (uint32_t c0 = 0; c0 < n; c0 += 32) {
-        const uint32_t m = n - c0 < 32u ? n - c0 : 32u;
-        if (lane < int(m)) {
-          MomentRecord<Vel> r;
-          r.load(sp, begin + c0 + lane);
-          bool ok = r.valid(key);
-          if (ok)
-            ok = record_values<double, false>(r, true, S.bc, sp.beta_over_c, mp.inv_volume,
-                                              [&](int e, double v) { S.src[e][lane] = v; },
-                                              [&](int t, double v) { S.m[t][lane] = v; });
-          if (!ok) {
-            ++bad;
+    if (cur.total == 0) walk.load(after, 0, next);
+    for (uint32_t o = 0; o < cur.total; o += 32) {
+      const uint32_t m = min(cur.total - o, 32u);
+      const MomentRecord<Vel> r = next;
+      if (o + 32 < cur.total) walk.load(cur, o + 32, next);
+      else walk.load(after, 0, next);
+      if (lane < int(m)) {
+        bool ok = r.valid(cur.key);
+        if (ok)
+          ok = record_values<double, false>(r, true, S.bc, mp.sp[walk.species(cur, o + lane)].beta_over_c,
+                                            mp.inv_volume, [&](int e, double v) { S.src[e][lane] = v; },
+                                            [&](int t, double v) { S.m[t][lane] = v; });
+        if (!ok) {
+          ++bad;
 #pragma unroll
-            for (int e = 0; e < 12; ++e) S.src[e][lane] = 0.0;
+          for (int e = 0; e < 12; ++e) S.src[e][lane] = 0.0;
 #pragma unroll
-            for (int t = 0; t < 27; ++t) S.m[t][lane] = 0.0;
-          }
+          for (int t = 0; t < 27; ++t) S.m[t][lane] = 0.0;
         }
-        __syncwarp();
-        for (uint32_t k0 = 0; k0 < m; k0 += 4) {
-          const uint32_t k = k0 + kk;
-          const bool in = k < m;
-          double av[4], bv[2];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) av[i] = in && 8 * i + rr < 27 ? S.m[8 * i + rr][k] : 0.0;
-#pragma unroll
-          for (int e = 0; e < 2; ++e) bv[e] = in && 8 * e + rr < 12 ? S.src[8 * e + rr][k] : 0.0;
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) dmma_884(acc[i][e], av[i], bv[e]);
-        }
-        __syncwarp();
       }
+      __syncwarp();
+      for (uint32_t k0 = 0; k0 < m; k0 += 4) {
+        const uint32_t k = k0 + kk;
+        const bool in = k < m;
+        double av[4], bv[2];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) av[i] = in && 8 * i + rr < 27 ? S.m[8 * i + rr][k] : 0.0;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) bv[e] = in && 8 * e + rr < 12 ? S.src[8 * e + rr][k] : 0.0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) dmma_884(acc[i][e], av[i], bv[e]);
+      }
+      __syncwarp();
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -482,6 +497,8 @@ __global__ void __launch_bounds__(kF64Warps * 32) moments_f64_kernel(Geom g, Mom
       *dst = accumulate ? *dst + value : value;
     }
     __syncwarp();
+    cell = cell_next;
+    cur = after;
   }
   bad = warp_sum(bad);
   if (bad && lane == 0) atomicAdd(invalid, bad);
@@ -526,7 +543,7 @@ cudaError_t launch_deposit_moments(int precision, int mass_kind, const Geom& g, 
                                                int(bytes));
     if (e != cudaSuccess) return e;
   }
-  const unsigned f64_blocks = unsigned(std::min<long long>((cells + kF64Warps - 1) / kF64Warps, 148LL * 16));
+  const unsigned f64_blocks = unsigned(std::min<long long>((cells + kF64Warps - 1) / kF64Warps, 148LL * 4));
   // Batches of four cells once each resident warp has one.
   const int batch = cells >= 4LL * 148 * 4 * kF32Warps ? 4 : 1;
   const long long batches = (cells + batch - 1) / batch;
