@@ -3,7 +3,7 @@
 // On grids of up to some ten thousand nodes an Arnoldi step is short work
 // behind nine launches: 36 us a step on a 1024 x 1 x 1 grid, 55 us on 256 x
 // 128 x 1, where the mass matrix and the vectors stay in L2. Here every CTA
-// owns the unique nodes of one tile for the whole cycle, keeps its rows of the
+// owns the unique nodes of its tiles for the whole cycle, keeps its rows of the
 // Krylov basis in shared memory where they fit, and the CTAs meet at two grid
 // barriers a step:
 //   A  the operator on the last vector (neighbours' rows read from one global
@@ -19,7 +19,8 @@
 // counts twice per such axis in the dots and norms, which are then those over
 // the interior nodes. All sums run in a fixed order.
 //
-// A tile of TN (32..256, a power of two) nodes has 256 / TN threads a node
+// A CTA has one tile, or several on grids of more tiles than CTAs fit. A tile of
+// TN (32..256, a power of two) nodes has 256 / TN threads a node
 // that share the 27 mass blocks: small grids take small tiles, so that every
 // SM has one.
 //
@@ -36,6 +37,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "grid_barrier.cuh"
 #include "smoothing.cuh"
 #include "stencils.cuh"
 
@@ -55,20 +57,20 @@ struct ArnoldiControl {
 
 constexpr int kResidentNodeThreads = 256;
 constexpr int kResidentThreads = kResidentNodeThreads + 32;  // and the warp that rotates the Hessenberg column
-constexpr int kResidentRestart = 32;                         // longest restart cycle
-constexpr uint32_t kResidentPolls = 1u << 22;
+constexpr int kResidentRestart = 32;                         // longest restart cycle (four columns a warp)
 
 struct ResidentPlan {
   Geom g;
   int tx, ty, tz;          // tile, powers of two; tx*ty*tz = nodes
   int nodes, parts, shift; // nodes of a tile, threads per node, log2 nodes
   int tiles_x, tiles_y, tiles;
+  int slots;               // tiles per CTA: tile blockIdx.x + slot * gridDim.x
   bool cluster;            // the grid is one cluster
   bool shared_basis;       // basis rows in shared memory, else in `basis`
   double delta, kfac, inv_volume;
   const void* mass;
   void* vector;            // [3][unique] S: the last unnormalized vector
-  void* basis;             // owner-private rows, 3 * nodes of each CTA per column
+  void* basis;             // owner-private rows, slots * 3 * nodes of each CTA per column
   double* x;               // [3][unique]
   double* b;
   double* r;
@@ -93,7 +95,7 @@ struct ResidentPlan {
 // Shared memory of a plan with arithmetic up to double: bytes per array.
 struct ResidentShared {
   int halo, cells;                 // nodes and cells a tile stages
-  size_t vs, cs, part, h, hcol, rot, sums, basis, image, unode, mult, table, ctable, smooth, total;
+  size_t vs, cs, part, h, hcol, rot, sums, basis, image, unode, mult, table, ctable, offsets, smooth, total;
 };
 // The tile and halo of the smoothing passes (the mass product reads one more node).
 inline __host__ __device__ SmoothTile resident_smooth_tile(const ResidentPlan& p) {
@@ -117,12 +119,13 @@ inline __host__ __device__ ResidentShared resident_shared(const ResidentPlan& p,
   s.hcol = take(size_t(m + 1) * 8);
   s.rot = take(size_t(4) * (m + 1) * 8);  // cosines, sines, right-hand side, coefficients
   s.sums = take(size_t(kResidentThreads / 32 + 2) * 2 * 8);  // per warp, then the step's diagonal and decision
-  s.basis = take(p.shared_basis ? size_t(p.restart + 1) * 3 * p.nodes * scalar : 0);
-  s.image = take(size_t(3) * p.nodes * scalar);
-  s.unode = take(size_t(p.nodes) * 4);
-  s.mult = take(size_t(p.nodes) * 4);
+  s.basis = take(p.shared_basis ? size_t(p.restart + 1) * p.slots * 3 * p.nodes * scalar : 0);
+  s.image = take(size_t(p.slots) * 3 * p.nodes * scalar);
+  s.unode = take(size_t(p.slots) * p.nodes * 4);
+  s.mult = take(size_t(p.slots) * p.nodes);
   s.table = take(size_t(s.halo) * 4);
   s.ctable = take(size_t(s.cells) * 4);
+  s.offsets = take(size_t(14) * sizeof(int2));
   s.smooth = take(p.smooth ? size_t(6) * resident_smooth_tile(p).size * 8 : 0);
   s.total = at;
   return s;
@@ -133,31 +136,26 @@ __constant__ int8_t kResidentOffsets[14][3] = {{0, 0, 0},  {1, 0, 0},  {0, 1, 0}
                                                {1, -1, 0}, {1, 0, 1},  {1, 0, -1}, {0, 1, 1},  {0, 1, -1},
                                                {1, -1, 1}, {1, 1, -1}, {-1, 1, 1}, {1, 1, 1}};
 
-__device__ __forceinline__ uint32_t load_acquire(const unsigned* p) {
-  uint32_t v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
 template <class S, class Mass, class Fld, bool kTranspose, bool kSmooth>
 struct Resident {
   const ResidentPlan& p;
   uint8_t* smem;
   const ResidentShared L;
-  uint32_t arrivals = 0;
-  bool failed = false;
+  GridBarrier barrier;
 
-  __device__ Resident(const ResidentPlan& plan, uint8_t* s) : p(plan), smem(s), L(resident_shared(plan, sizeof(S))) {}
+  __device__ Resident(const ResidentPlan& plan, uint8_t* s)
+      : p(plan), smem(s), L(resident_shared(plan, sizeof(S))), barrier(plan.barrier) {}
 
   template <class T> __device__ __forceinline__ T* at(size_t offset) const { return reinterpret_cast<T*>(smem + offset); }
   __device__ __forceinline__ long long unique() const { return (long long)p.g.nx * p.g.ny * p.g.nz; }
   __device__ __forceinline__ S* basis(int col) const {
-    const int rows = 3 * p.nodes;
+    const int rows = p.slots * 3 * p.nodes;
     return p.shared_basis ? at<S>(L.basis) + col * rows
                           : static_cast<S*>(p.basis) + ((long long)col * gridDim.x + blockIdx.x) * rows;
   }
-  __device__ __forceinline__ void origin(int& i0, int& j0, int& k0) const {
-    const int tile = blockIdx.x, row = tile / p.tiles_x;
+  __device__ __forceinline__ int tile_of(int slot) const { return int(blockIdx.x) + slot * int(gridDim.x); }
+  __device__ __forceinline__ void origin(int slot, int& i0, int& j0, int& k0) const {
+    const int tile = tile_of(slot), row = tile / p.tiles_x;
     i0 = (tile - row * p.tiles_x) * p.tx;
     k0 = row / p.tiles_y;
     j0 = (row - k0 * p.tiles_y) * p.ty;
@@ -170,38 +168,22 @@ struct Resident {
       asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
       return true;
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      arrivals += gridDim.x;
-      // The CTA's writes are ordered before the arrival (the barrier above and
-      // the release), the others' before what follows the acquire.
-      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p.barrier) : "memory");
-      uint32_t poll = 0;
-      while (load_acquire(p.barrier) < arrivals && poll < kResidentPolls) ++poll;
-      if (poll == kResidentPolls) {
-        failed = true;
-        p.ctl->failed = 1;
-      }
-    }
-    return !__syncthreads_or(failed);
+    if (barrier.wait()) return true;
+    if (threadIdx.x == 0) p.ctl->failed = 1;
+    return false;
   }
-  // The last CTA to leave zeroes the barrier for the next launch.
   __device__ void leave() {
-    if (threadIdx.x == 0 && !p.cluster && !failed && atomicAdd(p.barrier + 1, 1u) == gridDim.x - 1) {
-      p.barrier[0] = 0;
-      p.barrier[1] = 0;
-    }
+    if (!p.cluster) barrier.leave();
   }
 
-  // Tables of the tile: the unique index of every staged node (-1 beyond the
-  // grid's halo) and the staged base node of every cell.
-  __device__ void tables() {
-    const int vx = p.tx + 2, vy = p.ty + 2, cx = p.tx + 1, cy = p.ty + 1;
+  // Table of a slot's tile: the unique index of every staged node (-1 beyond
+  // the grid's halo).
+  __device__ void tables(int slot) {
+    const int vx = p.tx + 2, vy = p.ty + 2;
     int i0, j0, k0;
-    origin(i0, j0, k0);
+    origin(slot, i0, j0, k0);
     const Geom& g = p.g;
     int* table = at<int>(L.table);
-    int* ctable = at<int>(L.ctable);
     for (int n = threadIdx.x; n < L.halo; n += kResidentThreads) {
       const int row = n / vx, i = i0 - 1 + n - row * vx, j = j0 - 1 + row % vy, k = k0 - 1 + row / vy;
       int u = -1;
@@ -212,20 +194,37 @@ struct Resident {
       }
       table[n] = u;
     }
+  }
+  // The tables that hold for every tile: the staged base node of a cell, the
+  // stencils' distances.
+  __device__ void fixed_tables() {
+    const int vx = p.tx + 2, vy = p.ty + 2, cx = p.tx + 1, cy = p.ty + 1;
+    const Geom& g = p.g;
+    int* ctable = at<int>(L.ctable);
+    if (threadIdx.x < 14) {
+      // A stencil's distance in the array the mass product reads, and in the mass.
+      const int ox = kResidentOffsets[threadIdx.x][0], oy = kResidentOffsets[threadIdx.x][1],
+                oz = kResidentOffsets[threadIdx.x][2];
+      // On an axis of one cell the fold's copies hold the node's own blocks.
+      const SmoothTile t = resident_smooth_tile(p);
+      at<int2>(L.offsets)[threadIdx.x] =
+          make_int2(kSmooth ? ox * t.s[0] + oy * t.s[1] + oz * t.s[2] : ox + vx * (oy + vy * oz),
+                    int(g.mass_offset(g.nx > 1 ? ox : 0, g.ny > 1 ? oy : 0, g.nz > 1 ? oz : 0) * g.mvs));
+    }
     for (int n = threadIdx.x; n < L.cells; n += kResidentThreads) {
       const int row = n / cx;
       ctable[n] = (n - row * cx) + vx * (row % cy + vy * (row / cy));
     }
   }
 
-  // Node n of the tile: coordinates, and whether it is in the grid.
-  __device__ __forceinline__ bool node_of(int n, int& i, int& j, int& k) const {
-    origin(i, j, k);
+  // Node n of a slot's tile: coordinates, and whether it is in the grid.
+  __device__ __forceinline__ bool node_of(int slot, int n, int& i, int& j, int& k) const {
+    origin(slot, i, j, k);
     i += n & (p.tx - 1);
     const int row = n / p.tx;
     j += row & (p.ty - 1);
     k += row / p.ty;
-    return i < p.g.nx && j < p.g.ny && k < p.g.nz;
+    return tile_of(slot) < p.tiles && i < p.g.nx && j < p.g.ny && k < p.g.nz;
   }
 
   // The operator in arithmetic C: stage() reads the vector load(component,
@@ -239,10 +238,21 @@ struct Resident {
     C* vs = at<C>(L.vs);
     const int* table = at<int>(L.table);
     const int VN = L.halo;
-    for (int n = threadIdx.x; n < VN; n += kResidentNodeThreads) {
-      const int u = table[n];
+    // Two nodes' values at a time: the loads wait for L2 once for both.
+    for (int n = threadIdx.x; n < VN; n += 2 * kResidentNodeThreads) {
+      const int other = n + kResidentNodeThreads;
+      const int u = table[n], w = other < VN ? table[other] : -1;
+      C v[2][3];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) vs[c * VN + n] = u >= 0 ? C(load(c, u)) : C(0);
+      for (int c = 0; c < 3; ++c) {
+        v[0][c] = u >= 0 ? C(load(c, u)) : C(0);
+        v[1][c] = w >= 0 ? C(load(c, w)) : C(0);
+      }
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        vs[c * VN + n] = v[0][c];
+        if (other < VN) vs[c * VN + other] = v[1][c];
+      }
     }
     if constexpr (kSmooth) stage_region<C>(resident_smooth_tile(p), load);
   }
@@ -272,34 +282,43 @@ struct Resident {
     }
   }
   // This thread's node of the tile and its part of the node's mass blocks.
-  __device__ __forceinline__ bool my_node(int& n, int& part, int& i, int& j, int& k) const {
+  __device__ __forceinline__ bool my_node(int slot, int& n, int& part, int& i, int& j, int& k) const {
     n = threadIdx.x & (p.nodes - 1);
     part = threadIdx.x >> p.shift;
-    return threadIdx.x < kResidentNodeThreads && node_of(n, i, j, k);
+    return threadIdx.x < kResidentNodeThreads && node_of(slot, n, i, j, k);
   }
   __device__ __forceinline__ void local(int n, int& lx, int& ly, int& lz) const {
     lx = n & (p.tx - 1);
     ly = (n / p.tx) & (p.ty - 1);
     lz = n / (p.tx * p.ty);
   }
-  // The mass product of node (i, j, k) from v (component stride vn, neighbour
-  // strides sx, sy, sz), complete in the node's first thread. A CTA barrier
+  // The mass product of node (i, j, k) from v (component stride vn), complete in the node's first thread. A CTA barrier
   // is in it.
   template <class C>
-  __device__ __forceinline__ void mass(bool live, int n, int part, int i, int j, int k, const C* v, int vn, int sx,
-                                       int sy, int sz, C out[3]) {
+  __device__ __forceinline__ void mass(bool live, int n, int part, int i, int j, int k, const C* v, int vn, C out[3]) {
     const Geom& g = p.g;
     C x = C(0), y = C(0), z = C(0);
     if (live) {
       // Blocks in stencil order: part r of P takes stencils [14 r / P, 14 (r + 1) / P).
-      const Mass* mass = static_cast<const Mass*>(p.mass);
-      const long long mat = g.mass_vertex(i, j, k);
+      const Mass* mass = static_cast<const Mass*>(p.mass) + g.mass_vertex(i, j, k) * g.mvs;
+      const int2* offsets = at<int2>(L.offsets);
       const int s1 = 14 * (part + 1) / p.parts;
       for (int s = 14 * part / p.parts; s < s1; ++s) {
-        const int ox = kResidentOffsets[s][0], oy = kResidentOffsets[s][1], oz = kResidentOffsets[s][2];
-        const int vo = ox * sx + oy * sy + oz * sz;
-        product(mass + g.mass_index(mat, 9 * s), v + vo, vn, x, y, z);
-        if (s > 0) product(mass + g.mass_index(mat - g.mass_offset(ox, oy, oz), 9 * s), v - vo, vn, x, y, z);
+        const int2 o = offsets[s];
+        const Mass* b = mass + 9 * s * g.mes;
+        if (p.slots > 1 && s + 1 < s1) {
+          // Grids whose mass L2 does not hold: the next stencil's rows are
+          // requested while this one's are applied, as in the step's apply.
+          const Mass* next = b + 9 * g.mes;
+          const int back = offsets[s + 1].y;
+#pragma unroll
+          for (int e = 0; e < 9; ++e) {
+            prefetch_l2(next + e * g.mes);
+            prefetch_l2(next + e * g.mes - back);
+          }
+        }
+        product(b, v + o.x, vn, x, y, z);
+        if (s > 0) product(b - o.y, v - o.x, vn, x, y, z);
       }
       if (part > 0) {
         C* sum = at<C>(L.part);
@@ -355,7 +374,7 @@ struct Resident {
     if (threadIdx.x >= kResidentNodeThreads) return;
     C* a = at<C>(L.smooth);
     int i0, j0, k0;
-    origin(i0, j0, k0);
+    origin(0, i0, j0, k0);
     const Geom& g = p.g;
     for (int y = threadIdx.x >> 5; y < t.e[1]; y += kResidentNodeThreads / 32) {
       const int row = g.nx * wrap_index(j0 - t.h[1] + y, g.ny);
@@ -370,7 +389,7 @@ struct Resident {
   __device__ __forceinline__ const C* smoothed(const SmoothTile& t) {
     C* a = at<C>(L.smooth);
     int i0, j0, k0;
-    origin(i0, j0, k0);
+    origin(0, i0, j0, k0);
     return smooth_passes<C>(t, 3, a, a + 3 * t.size, p.smooth, p.smooth_op, p.smooth_alpha, threadIdx.x >> 5,
                             kResidentThreads / 32, [&](int x, int y, int) {
                               x -= t.h[0];
@@ -385,21 +404,21 @@ struct Resident {
   // coordinates, the three values) from the first thread of each node in the
   // grid. False when a barrier gave up.
   template <class C, class Store>
-  __device__ __forceinline__ bool image(Store&& store) {
+  __device__ __forceinline__ bool image(int slot, Store&& store) {
     cell_curls<C>();
     int n, part, i = 0, j = 0, k = 0, lx, ly, lz;
-    const bool live = my_node(n, part, i, j, k);
+    const bool live = my_node(slot, n, part, i, j, k);
     local(n, lx, ly, lz);
     C m[3];
     if constexpr (!kSmooth) {
       const int vx = p.tx + 2, vxy = vx * (p.ty + 2);
-      mass<C>(live, n, part, i, j, k, at<C>(L.vs) + (lx + 1) + vx * (ly + 1) + vxy * (lz + 1), L.halo, 1, vx, vxy, m);
+      mass<C>(live, n, part, i, j, k, at<C>(L.vs) + (lx + 1) + vx * (ly + 1) + vxy * (lz + 1), L.halo, m);
     } else {
       const SmoothTile t = resident_smooth_tile(p);
       const int own = (lx + t.h[0]) + t.e[0] * (ly + t.h[1]);
       const long long U = unique();
       const C* v = smoothed<C>(t);
-      mass<C>(live, n, part, i, j, k, v + own, t.size, t.s[0], t.s[1], t.s[2], m);
+      mass<C>(live, n, part, i, j, k, v + own, t.size, m);
       if (live && part == 0)
 #pragma unroll
         for (int c = 0; c < 3; ++c) p.response[c * U + i + p.g.nx * j] = double(m[c]);
@@ -460,20 +479,57 @@ struct Resident {
     for (unsigned t = threadIdx.x & 31; t < gridDim.x; t += 32) total += __ldcg(from + t);
     return warp_sum(total);
   }
+  // Sums over a warp's columns first, first + step, ... <= last (at most four,
+  // each lane's share from term(column)), to sink(column, sum) in lane 0. The
+  // columns' loads and shuffles run side by side: one after the other their
+  // latencies were a third of a step on small grids.
+  template <class Term, class Sink>
+  __device__ __forceinline__ void column_sums(int first, int step, int last, Term&& term, Sink&& sink) const {
+    double sum[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) sum[r] = first + r * step <= last ? term(first + r * step) : 0.0;
+    if (first + step <= last) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], o);
+    } else {
+      sum[0] = warp_sum(sum[0]);
+    }
+    if ((threadIdx.x & 31) == 0)
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        if (first + r * step <= last) sink(first + r * step, sum[r]);
+  }
 
   // What the nodes keep: unique indexes, multiplicities and the tables.
   __device__ void prepare() {
     int* unode = at<int>(L.unode);
-    float* mult = at<float>(L.mult);
-    for (int t = threadIdx.x; t < p.nodes; t += kResidentThreads) {
+    uint8_t* mult = at<uint8_t>(L.mult);
+    for (int t = threadIdx.x; t < p.slots * p.nodes; t += kResidentThreads) {
       int i, j, k;
-      const bool live = node_of(t, i, j, k);
+      const bool live = node_of(t >> p.shift, t & (p.nodes - 1), i, j, k);
       unode[t] = live ? i + p.g.nx * (j + p.g.ny * k) : -1;
-      mult[t] = live ? float((i == 0 ? 2 : 1) * (j == 0 ? 2 : 1) * (k == 0 ? 2 : 1)) : 0.0f;
+      mult[t] = live ? uint8_t((i == 0 ? 2 : 1) * (j == 0 ? 2 : 1) * (k == 0 ? 2 : 1)) : uint8_t(0);
     }
     S* last = at<S>(L.image);
-    for (int t = threadIdx.x; t < 3 * p.nodes; t += kResidentThreads) last[t] = S(0);
-    tables();
+    for (int t = threadIdx.x; t < p.slots * 3 * p.nodes; t += kResidentThreads) last[t] = S(0);
+    fixed_tables();
+    tables(0);
+    __syncthreads();
+  }
+  // With several slots the table holds the slot in hand, whose centre blocks
+  // are requested ahead.
+  __device__ __forceinline__ void enter(int slot) {
+    if (p.slots == 1) return;
+    __syncthreads();
+    tables(slot);
+    int i, j, k;
+    if (threadIdx.x < kResidentNodeThreads && node_of(slot, threadIdx.x & (p.nodes - 1), i, j, k)) {
+      const Mass* b = static_cast<const Mass*>(p.mass) + p.g.mass_vertex(i, j, k) * p.g.mvs;
+#pragma unroll
+      for (int e = 0; e < 9; ++e) prefetch_l2(b + e * p.g.mes);
+    }
     __syncthreads();
   }
 
@@ -483,20 +539,23 @@ struct Resident {
   __device__ bool residual(Load&& load, bool with_rhs) {
     double s0 = 0, s1 = 0;
     const long long U = unique();
-    stage<double>(load);
-    __syncthreads();
-    const bool done = image<double>([&](int, int i, int j, int k, const double value[3]) {
-      const int u = i + p.g.nx * (j + p.g.ny * k);
-      const double m = (i == 0 ? 2.0 : 1.0) * (j == 0 ? 2.0 : 1.0) * (k == 0 ? 2.0 : 1.0);
+    for (int slot = 0; slot < p.slots && tile_of(slot) < p.tiles; ++slot) {
+      enter(slot);
+      stage<double>(load);
+      __syncthreads();
+      const bool done = image<double>(slot, [&](int, int i, int j, int k, const double value[3]) {
+        const int u = i + p.g.nx * (j + p.g.ny * k);
+        const double m = (i == 0 ? 2.0 : 1.0) * (j == 0 ? 2.0 : 1.0) * (k == 0 ? 2.0 : 1.0);
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const double b = p.b[c * U + u], r = b - value[c];
-        p.r[c * U + u] = r;
-        s0 += m * (r * r);
-        s1 += m * (b * b);
-      }
-    });
-    if (!done) return false;
+        for (int c = 0; c < 3; ++c) {
+          const double b = p.b[c * U + u], r = b - value[c];
+          p.r[c * U + u] = r;
+          s0 += m * (r * r);
+          s1 += m * (b * b);
+        }
+      });
+      if (!done) return false;
+    }
     __syncthreads();
     publish(s0, s1, 0, with_rhs);
     return true;
@@ -540,8 +599,9 @@ __global__ void __launch_bounds__(kResidentThreads, 2) resident_start_kernel(con
     __syncthreads();
     smooth_j = r.template smoothed<Fld>(t);
   }
-  int i, j, k;
-  if (int(threadIdx.x) < p.nodes && r.node_of(threadIdx.x, i, j, k)) {
+  for (int slot = 0; slot < p.slots; ++slot) {
+    int i, j, k;
+    if (int(threadIdx.x) >= p.nodes || !r.node_of(slot, threadIdx.x, i, j, k)) continue;
     const int u = i + g.nx * (j + g.ny * k);
     const long long at = g.node(i, j, k);
     if (p.rhs) {
@@ -597,7 +657,7 @@ __global__ void __launch_bounds__(kResidentThreads, 2) resident_cycle_kernel(con
   constexpr int m = kResidentRestart, kWarps = kResidentThreads / 32;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long U = r.unique();
-  const int rows = 3 * p.nodes;
+  const int rows = p.slots * 3 * p.nodes;
   double* H = r.template at<double>(r.L.h);      // column c at c * (m + 1)
   double* hcol = r.template at<double>(r.L.hcol);
   double* cosine = r.template at<double>(r.L.rot);
@@ -607,13 +667,14 @@ __global__ void __launch_bounds__(kResidentThreads, 2) resident_cycle_kernel(con
   double* shared = r.template at<double>(r.L.sums) + 2 * kWarps;  // diagonal, decision, breakdown
   S* image = r.template at<S>(r.L.image);
   const int* unode = r.template at<int>(r.L.unode);
-  const float* mult = r.template at<float>(r.L.mult);
+  const uint8_t* mult = r.template at<uint8_t>(r.L.mult);
   S* vector = static_cast<S*>(p.vector);
   r.prepare();
   // Row t of the owned rows: its node and its place in a [3][unique] vector.
   auto place = [&](int t, int& n) -> long long {
-    n = t & (p.nodes - 1);
-    return (t >> p.shift) * U + unode[n];
+    const int slot = p.slots == 1 ? 0 : t / (3 * p.nodes), rest = t - slot * 3 * p.nodes;
+    n = slot * p.nodes + (rest & (p.nodes - 1));
+    return (rest >> p.shift) * U + unode[n];
   };
   const double first = p.values[0];
   double scale = first > 0.0 ? 1.0 / sqrt(first) : 0.0;
@@ -633,31 +694,43 @@ __global__ void __launch_bounds__(kResidentThreads, 2) resident_cycle_kernel(con
   while (true) {
     // A: image = A v_col; its dots with columns 0..col. The decision on the
     // last step is formed by the other warp while the vector is staged.
-    if (col == 0) r.template stage<S>([&](int c, int u) { return S(__ldcg(p.r + c * U + u) * scale); });
-    else r.template stage<S>([&](int c, int u) { return S(double(__ldcg(vector + c * U + u)) * scale); });
-    __syncthreads();
-    stop = int(shared[1]);
-    if (stop) break;
-    if (!r.template image<S>([&](int n, int, int, int, const S value[3]) {
+    for (int slot = 0; slot < p.slots && r.tile_of(slot) < p.tiles; ++slot) {
+      r.enter(slot);
+      if (col == 0) r.template stage<S>([&](int c, int u) { return S(__ldcg(p.r + c * U + u) * scale); });
+      else r.template stage<S>([&](int c, int u) { return S(double(__ldcg(vector + c * U + u)) * scale); });
+      __syncthreads();
+      stop = int(shared[1]);
+      if (stop) break;
+      S* out = image + slot * 3 * p.nodes;
+      if (!r.template image<S>(slot, [&](int n, int, int, int, const S value[3]) {
 #pragma unroll
-          for (int c = 0; c < 3; ++c) image[c * p.nodes + n] = value[c];
-        }))
-      return;
-    __syncthreads();
-    for (int c = warp; c <= col; c += kWarps) {
-      const S* v = r.basis(c);
-      double sum = 0;
-      for (int t = lane; t < rows; t += 32)
-        sum += double(v[t]) * (double(image[t]) * double(mult[t & (p.nodes - 1)]));
-      sum = warp_sum(sum);
-      if (lane == 0) p.partials[(long long)c * gridDim.x + blockIdx.x] = sum;
+            for (int c = 0; c < 3; ++c) out[c * p.nodes + n] = value[c];
+          }))
+        return;
     }
+    if (stop) break;
+    __syncthreads();
+    r.column_sums(warp, kWarps, col,
+                  [&](int c) {
+                    const S* v = r.basis(c);
+                    double sum = 0;
+                    for (int slot = 0, t0 = 0; slot < p.slots; ++slot, t0 += 3 * p.nodes)
+                      for (int t = lane; t < 3 * p.nodes; t += 32)
+                        sum += double(v[t0 + t]) *
+                               (double(image[t0 + t]) * double(mult[slot * p.nodes + (t & (p.nodes - 1))]));
+                    return sum;
+                  },
+                  [&](int c, double sum) { p.partials[(long long)c * gridDim.x + blockIdx.x] = sum; });
     if (!r.grid_barrier()) return;
     // B: Gram-Schmidt of the owned rows.
-    for (int c = warp; c <= col; c += kWarps) {
-      const double sum = r.gathered(c);
-      if (lane == 0) hcol[c] = sum;
-    }
+    r.column_sums(warp, kWarps, col,
+                  [&](int c) {
+                    const double* from = p.partials + (long long)c * gridDim.x;
+                    double sum = 0;
+                    for (unsigned t = lane; t < gridDim.x; t += 32) sum += __ldcg(from + t);
+                    return sum;
+                  },
+                  [&](int c, double sum) { hcol[c] = sum; });
     __syncthreads();
     double norm2 = 0;
     if (threadIdx.x < kResidentNodeThreads) {

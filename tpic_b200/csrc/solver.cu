@@ -981,13 +981,10 @@ bool cluster_fits(void (*kernel)(ResidentPlan), int blocks, size_t bytes) {
 // resident at once, so that every SM has nodes and a node has many threads;
 // the basis in shared memory where that tile leaves room for it (FP64 256 x
 // 128 x 1: 325 us a solve with tiles of 128 nodes and the basis in global
-// memory, 410 us with 256 and the basis in shared memory). A grid that needs
-// more than two tiles of 256 nodes an SM keeps the step graph, whose applies
-// stream the mass better: at 400 x 300 x 1 several tiles a CTA took 1.45 ms
-// against its 1.15-1.39 ms, at 64^3 2.07 against 1.17-1.33 ms. Below, resident
-// against step graph, ms a solve (mixed, stencil-major): 1024 x 1 x 1 1.59 / 5.72,
-// 16^3 0.20 / 0.58, 32^3 0.31 / 0.59, 256 x 128 x 1 0.36 / 0.78, 256 x 256 x 1
-// 0.52 / 0.94.
+// memory, 410 us with 256 and the basis in shared memory). Resident against
+// step graph, ms a solve (mixed, stencil-major): 1024 x 1 x 1 1.51 / 5.72, 16^3
+// 0.19 / 0.58, 32^3 0.29 / 0.59, 40^3 0.44 / 0.70, 256 x 128 x 1 0.34 / 0.78,
+// 256 x 256 x 1 0.44 / 0.94.
 template <class P>
 void plan_resident(SolverWorkspace* w, int sms) {
   using K = ResidentKernels<P>;
@@ -1015,16 +1012,28 @@ void plan_resident(SolverWorkspace* w, int sms) {
   for (int nodes = 32; nodes <= kResidentNodeThreads; nodes *= 2) {
     ResidentPlan p{};
     p.g = g;
-    p.tx = std::min({power(g.nx), 32, nodes});
-    p.ty = std::min(power(g.ny), nodes / p.tx);
-    p.tz = std::min(power(g.nz), nodes / (p.tx * p.ty));
-    while (p.tx * p.ty * p.tz < nodes && p.tx < power(g.nx)) p.tx *= 2;
+    // The shape with the fewest tiles, the widest x of those.
+    for (int x = 32; x >= 8; x /= 2) {
+      int t[3] = {std::min({power(g.nx), x, nodes}), 1, 1};
+      int rest = nodes / t[0];
+      t[1] = 1;
+      while (t[1] < power(g.ny) && t[1] < rest && (g.nz == 1 || t[1] * t[1] < rest)) t[1] *= 2;
+      t[2] = std::min(power(g.nz), rest / t[1]);
+      while (t[0] * t[1] * t[2] < nodes && t[1] < power(g.ny)) t[1] *= 2;
+      while (t[0] * t[1] * t[2] < nodes && t[0] < power(g.nx)) t[0] *= 2;
+      const int tiles_x = (g.nx + t[0] - 1) / t[0], tiles_y = (g.ny + t[1] - 1) / t[1];
+      const int tiles = tiles_x * tiles_y * ((g.nz + t[2] - 1) / t[2]);
+      if (p.tiles && tiles * t[0] * t[1] * t[2] >= p.tiles * p.tx * p.ty * p.tz) continue;
+      p.tx = t[0];
+      p.ty = t[1];
+      p.tz = t[2];
+      p.tiles_x = tiles_x;
+      p.tiles_y = tiles_y;
+      p.tiles = tiles;
+    }
     p.nodes = p.tx * p.ty * p.tz;
     p.parts = kResidentNodeThreads / p.nodes;
     while ((1 << p.shift) < p.nodes) ++p.shift;
-    p.tiles_x = (g.nx + p.tx - 1) / p.tx;
-    p.tiles_y = (g.ny + p.ty - 1) / p.ty;
-    p.tiles = p.tiles_x * p.tiles_y * ((g.nz + p.tz - 1) / p.tz);
     p.restart = w->restart;
     p.delta = w->delta;
     p.kfac = w->kfac;
@@ -1037,9 +1046,19 @@ void plan_resident(SolverWorkspace* w, int sms) {
     // lost more in threads per node than the barrier costs (1024 x 1 x 1 1.55
     // against 1.51 ms, 12^3 0.29 against 0.19).
     p.cluster = p.tiles <= kResidentCluster;
-    for (int shared = 1; shared >= 0; --shared) {
-      p.shared_basis = shared != 0;
-      if (!p.shared_basis && 3LL * p.tiles * p.nodes > w->ld) continue;
+    // Several tiles a CTA only with the largest tile, the basis then in global
+    // memory: up to four on flat grids and two on boxes, in FP64 up to four
+    // there too when at least 85 % of the CTAs' tiles are used. Beyond, the
+    // step graph's applies stream the mass better. Resident / step graph (its
+    // TMA apply on the tiled layout), ms a solve: 512 x 512 x 1 mixed 1.81 /
+    // 2.18 (1.87), FP64 1.83 / 2.93 (2.44); 48^3 0.75 / 0.84 (0.75) and 0.86 /
+    // 1.19 (0.94); 64^3 FP64 1.53 / 1.72 (1.55), mixed 1.48 / 1.31 (1.17);
+    // 56^3 FP64 (77 % of three tiles a CTA) 1.48 / 1.34 (1.26).
+    const int slots = nodes == kResidentNodeThreads && smooth == 0 ? 4 : 1;
+    for (int choice = 0; choice <= slots; ++choice) {
+      p.shared_basis = choice == 0;
+      p.slots = std::max(choice, 1);
+      const int grid = (p.tiles + p.slots - 1) / p.slots;
       const size_t bytes = resident_shared(p, sizeof(typename P::EC)).total;
       if (bytes > size_t(limit)) continue;
       int per_sm = 2;
@@ -1051,13 +1070,15 @@ void plan_resident(SolverWorkspace* w, int sms) {
         }
         per_sm = std::min(per_sm, blocks);
       }
-      if (p.tiles > per_sm * sms) continue;
-      if (p.cluster) {
+      if (grid > per_sm * sms) continue;
+      if (p.slots > 2 && g.nz > 1 &&
+          (sizeof(typename P::EC) == 4 || 100LL * p.tiles < 85LL * p.slots * per_sm * sms))
+        break;
+      if (p.cluster)
         for (auto k : kernels)
-          if (!cluster_fits(k, p.tiles, bytes)) p.cluster = false;
-      }
+          if (!cluster_fits(k, grid, bytes)) p.cluster = false;
       w->plan = p;
-      w->resident_grid = unsigned(p.tiles);
+      w->resident_grid = unsigned(grid);
       w->resident_bytes = bytes;
       w->resident = true;
       return;
@@ -1101,7 +1122,13 @@ SolverWorkspace* solver_create(int precision, const Geom& g, int restart, double
     alloc((void**)&w->smooth_b, 3 * g.nodes * sizeof(double));
     alloc((void**)&w->smooth_image, 3 * g.nodes * sizeof(double));
   }
-  alloc(&w->basis, (size_t)(restart + 1) * w->ld * w->scalar_bytes);
+  if (!w->loop_unavailable) {
+    if (precision == TPICB200_PRECISION_DOUBLE) plan_resident<PDouble>(w, sms);
+    else plan_resident<PMixed>(w, sms);
+  }
+  // The resident kernels' rows are padded to whole tiles.
+  const long long padded = 3LL * w->resident_grid * w->plan.slots * w->plan.nodes;
+  alloc(&w->basis, (size_t)(restart + 1) * std::max(w->ld, padded) * w->scalar_bytes);
   alloc(&w->image, (size_t)w->count * w->scalar_bytes);
   alloc((void**)&w->x, w->count * sizeof(double));
   alloc((void**)&w->b, w->count * sizeof(double));
@@ -1117,10 +1144,6 @@ SolverWorkspace* solver_create(int precision, const Geom& g, int restart, double
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&w->capture, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaMemset(w->input, 0, 3 * g.nodes * sizeof(double));
   if (e == cudaSuccess) e = cudaMemset(w->rhs, 0, 3 * g.nodes * sizeof(double));
-  if (e == cudaSuccess && !w->loop_unavailable) {
-    if (precision == TPICB200_PRECISION_DOUBLE) plan_resident<PDouble>(w, sms);
-    else plan_resident<PMixed>(w, sms);
-  }
   if (w->resident) {
     alloc((void**)&w->resident_partials, size_t(kResidentRestart + 2) * w->resident_grid * sizeof(double));
     alloc((void**)&w->resident_barrier, 2 * sizeof(unsigned));
