@@ -143,14 +143,24 @@ __device__ __forceinline__ void response_gradient(const double om[3], const doub
   }
 }
 
-// Adds a cell's corner total into the unique node of component n of `field`.
-__device__ __forceinline__ void add_corner(const Geom& g, double* __restrict__ field, int32_t key, int a, int n,
-                                           double total) {
-  int i, j, k;
-  g.decode(key, i, j, k);
-  const int ci = i + (a & 1), cj = j + ((a >> 1) & 1), ck = k + ((a >> 2) & 1);
-  atomicAdd(field + n * g.nodes + g.node(ci == g.nx ? 0 : ci, cj == g.ny ? 0 : cj, ck == g.nz ? 0 : ck), total);
-}
+// Adds a cell's corner totals into the unique nodes: components 0-2 of `first`,
+// 3-5 (where there are) of `second`.
+struct AdjointSink {
+  const Geom& g;
+  double* first;
+  double* second;
+  __device__ __forceinline__ long long node(int32_t key, int a) const {
+    int i, j, k;
+    g.decode(key, i, j, k);
+    i += a & 1;
+    j += (a >> 1) & 1;
+    k += (a >> 2) & 1;
+    return g.node(i == g.nx ? 0 : i, j == g.ny ? 0 : j, k == g.nz ? 0 : k);
+  }
+  __device__ __forceinline__ void add(long long at, int n, double total) const {
+    atomicAdd((n < 3 ? first : second) + (n < 3 ? n : n - 3) * g.nodes + at, total);
+  }
+};
 
 template <class P>
 __device__ __forceinline__ void load_record(const Geom& g, const AdjointRecords& r, uint32_t n, bool active,
@@ -198,7 +208,7 @@ __global__ void __launch_bounds__(kAdjointThreads) adjoint_theta_scatter_kernel(
   const uint32_t lane = threadIdx.x & 31u;
   uint32_t first, last;
   warp_segment(r.count, first, last);
-  auto sink = [&](int32_t key, int a, int n, double total) { add_corner(g, etheta_bar, key, a, n, total); };
+  const AdjointSink sink{g, etheta_bar, nullptr};
   Sums sums;
   sums.begin();
   for (uint32_t base = first; base < last; base += 32) {
@@ -249,10 +259,7 @@ __global__ void __launch_bounds__(kRecordThreads, kRecordBlocks) adjoint_record_
   uint32_t first, last;
   warp_segment(r.count, first, last);
   const long long nid = r.nid;
-  auto sink = [&](int32_t key, int a, int n, double total) {
-    if (kScatterTheta && n >= 3) add_corner(g, etheta_bar, key, a, n - 3, total);
-    else add_corner(g, bnode_bar, key, a, n, total);
-  };
+  const AdjointSink sink{g, bnode_bar, etheta_bar};
   Sums sums;
   sums.begin();
   for (uint32_t base = first; base < last; base += 32) {

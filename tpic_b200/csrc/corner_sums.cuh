@@ -45,17 +45,19 @@ struct CornerSums {
     for (int t = 0; t < kTiles; ++t) c[t][0] = c[t][1] = 0.0;
   }
 
-  // Hands the totals held to sink(key, corner, n, total), this lane's share.
+  // Hands the totals held to sink.add(node, n, total), this lane's share, with
+  // node = sink.node(key, corner).
   template <class Sink>
   __device__ __forceinline__ void flush(Sink&& sink) {
     if (key < 0) return;
     const int lane = threadIdx.x & 31;
+    const auto node = sink.node(key, lane >> 2);
 #pragma unroll
     for (int t = 0; t < kTiles; ++t)
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int n = 8 * t + 2 * (lane & 3) + h;
-        if (n < N) sink(key, lane >> 2, n, c[t][h]);
+        if (n < N) sink.add(node, n, c[t][h]);
       }
     begin();
   }

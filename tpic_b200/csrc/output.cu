@@ -70,6 +70,28 @@ struct OutputRecord {
   }
 };
 
+// Adds a cell's totals at its corners' unique nodes.
+struct MomentSink {
+  const Geom& g;
+  double* rho;
+  double* j;
+  double* pressure;
+  __device__ __forceinline__ long long node(int32_t key, int a) const {
+    int i, jj, k;
+    g.decode(key, i, jj, k);
+    i += a & 1;
+    jj += (a >> 1) & 1;
+    k += (a >> 2) & 1;
+    return (i == g.nx ? 0 : i) + (long long)g.nx * ((jj == g.ny ? 0 : jj) + (long long)g.ny * (k == g.nz ? 0 : k));
+  }
+  __device__ __forceinline__ void add(long long at, int n, double total) const {
+    double* out = n == 0 ? rho : n < 4 ? j : pressure;
+    if (!out || total == 0.0) return;
+    const long long unique = (long long)g.nx * g.ny * g.nz;
+    atomicAdd(out + (n == 0 ? 0 : n < 4 ? n - 1 : n - 4) * unique + at, total);
+  }
+};
+
 template <class V, int N>
 __global__ void __launch_bounds__(kMomentThreads) output_moments_kernel(Geom g, tpicb200_particles p,
                                                                       double inverse_volume, double inverse_qom,
@@ -80,20 +102,10 @@ __global__ void __launch_bounds__(kMomentThreads) output_moments_kernel(Geom g, 
   using Sums = CornerSums<N>;
   __shared__ typename Sums::Stage stages[kMomentThreads / 32];
   typename Sums::Stage& stage = stages[threadIdx.x / 32];
-  const long long unique = (long long)g.nx * g.ny * g.nz;
   const uint32_t lane = threadIdx.x & 31u;
   uint32_t first, last;
   warp_segment(p.count, first, last);
-  auto sink = [&](int32_t key, int a, int n, double total) {
-    double* out = n == 0 ? rho : n < 4 ? (j ? j + (n - 1) * unique : nullptr)
-                                       : (pressure ? pressure + (n - 4) * unique : nullptr);
-    if (!out || total == 0.0) return;
-    int ci, cj, ck;
-    g.decode(key, ci, cj, ck);
-    const int i = wrap_index(ci + (a & 1), g.nx), jj = wrap_index(cj + ((a >> 1) & 1), g.ny),
-              k = wrap_index(ck + ((a >> 2) & 1), g.nz);
-    atomicAdd(out + i + (long long)g.nx * (jj + (long long)g.ny * k), total);
-  };
+  const MomentSink sink{g, rho, j, pressure};
   Sums sums;
   sums.begin();
   OutputRecord<V> next;
@@ -106,7 +118,8 @@ __global__ void __launch_bounds__(kMomentThreads) output_moments_kernel(Geom g, 
 #pragma unroll
     for (int n = 0; n < N; ++n) amount[n] = 0.0;
     bool ok = active && r.key >= 0 && (long long)r.key < g.bins;
-    if (ok) {
+    // The cell summed at the moment has been checked.
+    if (ok && r.key != sums.key) {
       int ci, cj, ck;
       g.decode(r.key, ci, cj, ck);
       ok = g.interior_cell(ci, cj, ck);
