@@ -453,7 +453,6 @@ int tpicb200_field_advance(tpicb200_context* ctx, void* e, const void* b_cell, c
   const int p = ctx->opt.precision;
   cudaError_t err = launch_field_advance(p, ctx->g, ctx->opt.theta, -ctx->opt.c * ctx->opt.dt, e, b_cell, e_theta,
                                          b_cell_next, ctx->invalid, s);
-  if (err == cudaSuccess) err = launch_cell_ghosts(p, ctx->g, b_cell_next, s);
   if (err == cudaSuccess) err = launch_cell_to_node(p, ctx->g, b_cell_next, b_node_next, s);
   return cuda_status(err, "field advance failed");
 }

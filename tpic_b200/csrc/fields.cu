@@ -61,21 +61,23 @@ __global__ void __launch_bounds__(256) cell_fill_kernel(Geom g, T* __restrict__ 
 }
 
 // cell_to_node_average in Compute::Magnetic (ecsim/fields/cell_to_node.hpp:19-32,
-// ecsim/fields/cell_to_node_device.hpp:17-38), interior nodes.
+// ecsim/fields/cell_to_node_device.hpp:17-38) at every stored node, duplicates
+// and ghosts as their unique node (no ghost fill behind it); component
+// blockIdx.y.
 template <class C, class T>
 __global__ void __launch_bounds__(256) cell_to_node_kernel(Geom g, const T* __restrict__ cellf, T* __restrict__ node) {
-  const long long total = 3 * g.interior;
-  for (long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x; t0 < total;
-       t0 += (long long)gridDim.x * blockDim.x) {
-    const long long c = t0 / g.interior;
-    int i, j, k;
-    interior_node_coordinates(g, t0 - c * g.interior, i, j, k);
-    const T* f = cellf + c * g.cells;
+  const T* f = cellf + blockIdx.y * g.cells;
+  T* out = node + blockIdx.y * g.nodes;
+  const uint32_t total = uint32_t(g.nodes), NX = uint32_t(g.NX), NY = uint32_t(g.NY);
+  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+    const uint32_t row = t / NX;
+    const int i = wrap_index(int(t - row * NX) - 1, g.nx), j = wrap_index(int(row % NY) - 1, g.ny),
+              k = wrap_index(int(row / NY) - 1, g.nz);
     const C v = (C(f[g.cell(i - 1, j - 1, k - 1)]) + C(f[g.cell(i, j - 1, k - 1)]) +
                  C(f[g.cell(i - 1, j, k - 1)]) + C(f[g.cell(i, j, k - 1)]) +
                  C(f[g.cell(i - 1, j - 1, k)]) + C(f[g.cell(i, j - 1, k)]) +
                  C(f[g.cell(i - 1, j, k)]) + C(f[g.cell(i, j, k)])) * C(0.125);
-    node[c * g.nodes + g.node(i, j, k)] = T(v);
+    out[t] = T(v);
   }
 }
 
@@ -101,44 +103,48 @@ __global__ void __launch_bounds__(256) rhs_kernel(Geom g, C delta, C kfac, const
   }
 }
 
-// E update over interior nodes (field_vector_linear_combination, two terms).
+// The field advance: the E update over the interior nodes
+// (field_vector_linear_combination, two terms) and Faraday's
+// next = 1*B + faraday*curl_N2C(theta) in Compute::Magnetic over all cells
+// (faraday_update_kernel, ecsim/maxwell/field_update_device.hpp:25-44), each
+// cell stored at its periodic copies too.
 template <class C, class T>
-__global__ void __launch_bounds__(256) e_update_kernel(Geom g, C a, C b, bool copy, T* __restrict__ e,
-                                                       const double* __restrict__ th, uint32_t* invalid) {
-  const long long total = 3 * g.interior;
-  for (long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x; t0 < total;
-       t0 += (long long)gridDim.x * blockDim.x) {
-    const long long c = t0 / g.interior;
+__global__ void __launch_bounds__(256) advance_kernel(Geom g, C a, C b, bool copy, T* __restrict__ e, C faraday,
+                                                      const T* __restrict__ bcell, const double* __restrict__ th,
+                                                      T* __restrict__ next, uint32_t* invalid) {
+  const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
+  for (long long t = first; t < g.interior; t += stride) {
     int i, j, k;
-    interior_node_coordinates(g, t0 - c * g.interior, i, j, k);
-    const long long p = c * g.nodes + g.node(i, j, k);
-    const T value = copy ? T(th[p]) : T(a * C(th[p]) + b * C(e[p]));
-    e[p] = value;
-    if (!isfinite(value)) atomicAdd(invalid, 1u);
+    interior_node_coordinates(g, t, i, j, k);
+    const long long at = g.node(i, j, k);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const long long p = c * g.nodes + at;
+      const T value = copy ? T(th[p]) : T(a * C(th[p]) + b * C(e[p]));
+      e[p] = value;
+      if (!isfinite(value)) atomicAdd(invalid, 1u);
+    }
   }
-}
-
-// Faraday: next = 1*B + faraday*curl_N2C(theta) in Compute::Magnetic over all
-// cells (faraday_update_kernel, ecsim/maxwell/field_update_device.hpp:25-44).
-template <class C, class T>
-__global__ void __launch_bounds__(256) faraday_kernel(Geom g, C faraday, const T* __restrict__ b,
-                                                      const double* __restrict__ th, T* __restrict__ next,
-                                                      uint32_t* invalid) {
   const C inv[3] = {C(g.inv[0]), C(g.inv[1]), C(g.inv[2])};
   const long long cells = (long long)g.nx * g.ny * g.nz;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < cells;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int i = int(t % g.nx), j = int((t / g.nx) % g.ny), k = int(t / ((long long)g.nx * g.ny));
+  for (long long t = first; t < cells; t += stride) {
+    const uint32_t u = uint32_t(t), nx = uint32_t(g.nx), row = u / nx;
+    const int i = int(u - row * nx), j = int(row % uint32_t(g.ny)), k = int(row / uint32_t(g.ny));
     C cu[3];
     curl_n2c_at<C>(g, th, i, j, k, inv, cu);
     const long long at = g.cell(i, j, k);
+    T value[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      const long long p = c * g.cells + at;
-      const T value = T(C(1) * C(b[p]) + faraday * cu[c]);
-      next[p] = value;
-      if (!isfinite(value)) atomicAdd(invalid, 1u);
+      value[c] = T(C(1) * C(bcell[c * g.cells + at]) + faraday * cu[c]);
+      if (!isfinite(value[c])) atomicAdd(invalid, 1u);
     }
+    // The copies of cell i on an axis of n: i + m n within -1 .. n.
+    for (int kk = k - (k + 1) / g.nz * g.nz; kk <= g.nz; kk += g.nz)
+      for (int jj = j - (j + 1) / g.ny * g.ny; jj <= g.ny; jj += g.ny)
+        for (int ii = i - (i + 1) / g.nx * g.nx; ii <= g.nx; ii += g.nx)
+#pragma unroll
+          for (int c = 0; c < 3; ++c) next[c * g.cells + g.cell(ii, jj, kk)] = value[c];
   }
 }
 
@@ -246,15 +252,13 @@ cudaError_t launch_cell_ghosts(int precision, const Geom& g, void* f, cudaStream
 }
 
 cudaError_t launch_cell_to_node(int precision, const Geom& g, const void* cellf, void* node, cudaStream_t s) {
-  const unsigned blocks = grid_for(3 * g.interior, 256);
-  if (precision == TPICB200_PRECISION_DOUBLE) {
+  if (g.nodes >= (1LL << 32)) return cudaErrorInvalidValue;
+  const dim3 blocks(grid_for(g.nodes, 256), 3);
+  if (precision == TPICB200_PRECISION_DOUBLE)
     cell_to_node_kernel<double, double><<<blocks, 256, 0, s>>>(g, (const double*)cellf, (double*)node);
-    node_fill_kernel<double><<<dim3(grid_for(shell_count(g), 256), 3), 256, 0, s>>>(g, (double*)node);
-  } else {
+  else
     cell_to_node_kernel<float, float><<<blocks, 256, 0, s>>>(g, (const float*)cellf, (float*)node);
-    node_fill_kernel<float><<<dim3(grid_for(shell_count(g), 256), 3), 256, 0, s>>>(g, (float*)node);
-  }
-  count_launches(2);
+  count_launches(1);
   return cudaGetLastError();
 }
 
@@ -387,21 +391,18 @@ cudaError_t launch_field_advance(int precision, const Geom& g, double theta_valu
                                  void* e, const void* bcell, const double* etheta, void* bnext,
                                  uint32_t* invalid, cudaStream_t s) {
   const bool copy = fabs(theta_value - 1.0) < 1e-10;
-  const unsigned eb = grid_for(3 * g.interior, 256);
-  const unsigned fb = grid_for((long long)g.nx * g.ny * g.nz, 256);
+  const unsigned blocks = grid_for(g.interior, 256);
   if (precision == TPICB200_PRECISION_DOUBLE) {
     const double a = 1.0 / theta_value, b = -(1.0 - theta_value) / theta_value;
-    e_update_kernel<double, double><<<eb, 256, 0, s>>>(g, a, b, copy, (double*)e, etheta, invalid);
-    faraday_kernel<double, double><<<fb, 256, 0, s>>>(g, faraday, (const double*)bcell, etheta,
-                                                     (double*)bnext, invalid);
+    advance_kernel<double, double><<<blocks, 256, 0, s>>>(g, a, b, copy, (double*)e, faraday, (const double*)bcell,
+                                                         etheta, (double*)bnext, invalid);
   } else {
     const float th = float(theta_value);
     const float a = 1.0f / th, b = -(1.0f - th) / th;
-    e_update_kernel<float, float><<<eb, 256, 0, s>>>(g, a, b, copy, (float*)e, etheta, invalid);
-    faraday_kernel<float, float><<<fb, 256, 0, s>>>(g, float(faraday), (const float*)bcell, etheta,
-                                                   (float*)bnext, invalid);
+    advance_kernel<float, float><<<blocks, 256, 0, s>>>(g, a, b, copy, (float*)e, float(faraday), (const float*)bcell,
+                                                       etheta, (float*)bnext, invalid);
   }
-  count_launches(2);
+  count_launches(1);
   return cudaGetLastError();
 }
 

@@ -165,10 +165,12 @@ cudaError_t launch_smooth(bool double_arithmetic, const Geom& g, int niter, int 
                           const double* src, double* out, double* tmp, uint32_t* invalid, cudaStream_t s);
 cudaError_t launch_widen(int precision, const Geom& g, const void* in, double* out, cudaStream_t s);
 cudaError_t launch_cell_ghosts(int precision, const Geom& g, void* f, cudaStream_t s);
+// At every stored node, ghosts included (the cells' ghosts must be filled).
 cudaError_t launch_cell_to_node(int precision, const Geom& g, const void* cellf, void* node,
                                 cudaStream_t s);
 cudaError_t launch_rhs(int precision, const Geom& g, double delta, double kfac, const void* e,
                        const void* bcell, const void* j, double* rhs, cudaStream_t s, bool j_double = false);
+// E in place, the next B with its ghosts.
 cudaError_t launch_field_advance(int precision, const Geom& g, double theta_value, double faraday,
                                  void* e, const void* bcell, const double* etheta, void* bnext,
                                  uint32_t* invalid, cudaStream_t s);

@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(256, TPICB200_MOVER_MIN_BLOCKS) mover_kernel(G
 }
 
 // Runs of up to g.run_len cells of one x-row; records grouped by the bins
-// (old_counts, old_offsets), which validate_bins has checked (the kernel
+// (old_counts, old_offsets), which binned_begin has checked (the kernel
 // returns at once when they do not tile the records).
 constexpr int kRunWarps = 4;
 // Resident blocks of the run mover: eight (64 registers) in the mixed form,
@@ -507,7 +507,7 @@ cudaError_t launch(const Geom& g, double qom, double dt, double c, tpicb200_part
     if (scalars) *scalars->written = int(blocks);
     return cudaGetLastError();
   }
-  // Bins checked by validate_bins: the run mover; otherwise the per-record
+  // Bins checked by binned_begin: the run mover; otherwise the per-record
   // mover moves every record. Exactly one of the two works (the choice
   // depends only on the bins, not on flags the movers themselves raise).
   MoveCodes mc{binned->code, binned->transfer, &binned->state->fallback, &binned->state->bins_bad,

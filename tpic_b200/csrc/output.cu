@@ -46,7 +46,7 @@ constexpr double kFourPi = 4.0 * 3.14159265358979323846;
 // (64^3 cells, two species, mixed), bound by the atomics' rate. Snapshots write
 // sorted records, so a warp walks consecutive records and sums a cell's
 // amounts over its corners on the FP64 tensor cores (corner_sums.cuh), with
-// one set of atomics per cell of a warp: 0.74 ms. The next chunk's records
+// one set of atomics per cell of a warp: 0.99 ms. The next chunk's records
 // are loaded before this one is summed.
 constexpr int kMomentThreads = 256;
 
