@@ -282,9 +282,15 @@ __global__ void __launch_bounds__(TX * TY * TZ, sizeof(C) == 4 ? 4 : 3) maxwell_
 // Per stencil s = (ox, oy, oz) one 4-D box of the mass tensor (x, y, z,
 // entry) holds the stencil's 9 entries over the tile plus a one-node halo
 // on the side of -s: x elements i0 .. i0+35 (nodes i0-1 .. i0+34; element
-// i0 is 16-byte aligned), y nodes j0 - max(oy,0) .. + TY, z likewise. The
-// forward block of a node (at the node) and its backward block (at the
-// node - s) are both in that box. The boxes stream through S stages with one
+// i0 is 16-byte aligned), y nodes j0 .. j0 + TY - 1 with the row before for
+// oy = 1 and the row behind for oy = -1, z likewise. The forward block of a
+// node (at the node) and its backward block (at the node - s) are both in that
+// box. The halos come from L2 and its rate to the SMs bounds the kernel, so
+// only the stencils that reach along y or z fetch a halo there (one tensor map
+// per box shape): 172 of the 210 rows that 14 boxes with both halos hold.
+// Solve of 128^3, ms: 5.65 -> 5.53 mixed, 9.67 -> 9.23 FP64 (larger tiles hold
+// fewer halo rows still, but in half as many CTAs: 64 x 4 x 2 nodes 6.12
+// mixed, 32 x 8 x 2 6.16, 32 x 4 x 4 6.13). The boxes stream through S stages with one
 // mbarrier each; one thread issues the copies (after the kernel's
 // predecessor has completed), every thread waits (bounded) for a stage's
 // copy, and the stage is refilled with stencil s + S after a CTA barrier. The
@@ -300,11 +306,18 @@ constexpr int kBoxX = 36;
 // of it, so the box holds that plane alone and the products are unchanged bit
 // for bit, with half the mass bytes read.
 template <int TY, int TZ, class M, bool Flat = false> struct TmaBox {
-  static constexpr int X = kBoxX, Y = TY + 1, Z = Flat ? 1 : TZ + 1;
-  static constexpr int entry = X * Y * Z;              // elements of one entry's box
-  static constexpr int elems = 9 * entry;              // one stencil's box
-  static constexpr int bytes = elems * int(sizeof(M));
-  static constexpr int stage = (bytes + 1023) / 1024 * 1024;  // 1024-byte aligned stages
+  static constexpr int X = kBoxX;
+  // Rows, planes, one entry's elements and all bytes of a stencil's box.
+  static __device__ __forceinline__ constexpr int y(int oy) { return TY + (oy != 0); }
+  static __device__ __forceinline__ constexpr int z(int oz) { return Flat ? 1 : TZ + (oz != 0); }
+  static __device__ __forceinline__ constexpr int entry(int oy, int oz) { return X * y(oy) * z(oz); }
+  static __device__ __forceinline__ constexpr int bytes(int oy, int oz) { return 9 * entry(oy, oz) * int(sizeof(M)); }
+  static constexpr int largest = 9 * X * (TY + 1) * (Flat ? 1 : TZ + 1) * int(sizeof(M));
+  static constexpr int stage = (largest + 1023) / 1024 * 1024;  // 1024-byte aligned stages
+};
+// The mass tensor with a box per halo: [halo along y][halo along z].
+struct MassMaps {
+  CUtensorMap box[2][2];
 };
 
 template <class C, class M, int TX, int TY, int TZ, int S, bool Flat = false>
@@ -320,7 +333,7 @@ struct TmaApplyShared {
 
 template <class C, class M, class Out, int TX, int TY, int TZ, int S, bool kTranspose, bool kFlat>
 __global__ void __launch_bounds__(TX * TY * TZ, sizeof(C) == 4 ? 4 : 2)
-    maxwell_apply_tma_kernel(const __grid_constant__ CUtensorMap map, Geom g, C d2, C kfac, C inv_volume,
+    maxwell_apply_tma_kernel(const __grid_constant__ MassMaps maps, Geom g, C d2, C kfac, C inv_volume,
                              const double* __restrict__ v, Out* __restrict__ out, uint32_t* invalid,
                              uint32_t polls, int stall) {
   static_assert(!kFlat || TZ == 1, "flat boxes hold one z plane");
@@ -339,8 +352,8 @@ __global__ void __launch_bounds__(TX * TY * TZ, sizeof(C) == 4 ? 4 : 2)
   auto issue = [&](int s) {
     const int oy = stencil_offset(s, 1), oz = stencil_offset(s, 2);
     uint64_t* bar = &bars[s % S];
-    tc::mbar_arrive_expect_tx(bar, uint32_t(Box::bytes));
-    tc::tma_load_4d(tma_smem + (s % S) * Box::stage, &map, i0, j0 + 1 - (oy > 0 ? oy : 0),
+    tc::mbar_arrive_expect_tx(bar, uint32_t(Box::bytes(oy, oz)));
+    tc::tma_load_4d(tma_smem + (s % S) * Box::stage, &maps.box[oy != 0][oz != 0], i0, j0 + 1 - (oy > 0 ? oy : 0),
                     kFlat ? k0 + 1 : k0 + 1 - (oz > 0 ? oz : 0), 9 * s, bar);
   };
   if (threadIdx.x == 0) {
@@ -425,16 +438,17 @@ __global__ void __launch_bounds__(TX * TY * TZ, sizeof(C) == 4 ? 4 : 2)
       const M* box = reinterpret_cast<const M*>(tma_smem + (s % S) * Box::stage);
       const int ox = stencil_offset(s, 0), oy = stencil_offset(s, 1), oz = stencil_offset(s, 2);
       const int my = oy > 0 ? oy : 0, mz = oz > 0 ? oz : 0;
-      const int fwd = (lx + 1) + Box::X * ((ly + my) + Box::Y * (kFlat ? 0 : lz + mz));
+      const int rows = Box::y(oy), entry = Box::entry(oy, oz);
+      const int fwd = (lx + 1) + Box::X * ((ly + my) + rows * (kFlat ? 0 : lz + mz));
       if (s == 0) {
-        block_product<C, M, kTranspose>(box + fwd, Box::entry, vv(0, 0, 0, 0), vv(1, 0, 0, 0), vv(2, 0, 0, 0), x, y, z);
+        block_product<C, M, kTranspose>(box + fwd, entry, vv(0, 0, 0, 0), vv(1, 0, 0, 0), vv(2, 0, 0, 0), x, y, z);
       } else {
-        const int bwd = (lx + 1 - ox) + Box::X * ((ly - oy + my) + Box::Y * (kFlat ? 0 : lz - oz + mz));
+        const int bwd = (lx + 1 - ox) + Box::X * ((ly - oy + my) + rows * (kFlat ? 0 : lz - oz + mz));
         C bx, by, bz;
-        block_product<C, M, kTranspose>(box + fwd, Box::entry, vv(0, ox, oy, oz), vv(1, ox, oy, oz),
+        block_product<C, M, kTranspose>(box + fwd, entry, vv(0, ox, oy, oz), vv(1, ox, oy, oz),
                                         vv(2, ox, oy, oz), bx, by, bz);
         x += bx; y += by; z += bz;
-        block_product<C, M, kTranspose>(box + bwd, Box::entry, vv(0, -ox, -oy, -oz), vv(1, -ox, -oy, -oz),
+        block_product<C, M, kTranspose>(box + bwd, entry, vv(0, -ox, -oy, -oz), vv(1, -ox, -oy, -oz),
                                         vv(2, -ox, -oy, -oz), bx, by, bz);
         x += bx; y += by; z += bz;
       }
@@ -911,7 +925,7 @@ struct SolverWorkspace {
   // Tensor maps of mass buffers for the TMA-staged apply, per mass pointer
   // and tile shape (0: 32x4x2, 1: thin 32x8x1); built on first use.
   struct MassMap {
-    CUtensorMap map;
+    MassMaps maps;
     const void* mass = nullptr;
     int tile = -1;
     bool usable = false;
@@ -1197,18 +1211,18 @@ TensorMapEncodeTiled tensor_map_encoder() {
   return f;
 }
 
-// The tensor map of a mass buffer as a 4-D tensor (x pitch MX, y NY, z NZ,
-// 126 entries) with the apply's box {36, TY+1, TZ+1, 9}, or nullptr when the
+// The tensor maps of a mass buffer as a 4-D tensor (x pitch MX, y NY, z NZ,
+// 126 entries) with the apply's boxes {36, TY (+1), TZ (+1), 9}, or nullptr when the
 // buffer does not meet the copies' alignment rules (vertex stride 1, the
 // base, the row pitch and the entry-plane stride multiples of 16 bytes):
 // those buffers take maxwell_apply_kernel.
 template <class M>
-const CUtensorMap* mass_tensor_map(SolverWorkspace* w, const M* mass, bool thin) {
+const MassMaps* mass_tensor_maps(SolverWorkspace* w, const M* mass, bool thin) {
   const Geom& g = w->g;
   const bool flat = thin;  // thin tiles are on grids one cell thick along z
   const int tile = thin ? 1 : 0;
   for (auto& m : w->maps)
-    if (m.mass == mass && m.tile == tile) return m.usable ? &m.map : nullptr;
+    if (m.mass == mass && m.tile == tile) return m.usable ? &m.maps : nullptr;
   auto& m = w->maps[w->next_map];
   w->next_map = (w->next_map + 1) % 4;
   m.mass = mass;
@@ -1222,21 +1236,25 @@ const CUtensorMap* mass_tensor_map(SolverWorkspace* w, const M* mass, bool thin)
   if (!encode) return nullptr;
   const cuuint64_t dims[4] = {cuuint64_t(g.MX), cuuint64_t(g.NY), cuuint64_t(g.NZ), 126};
   const cuuint64_t strides[3] = {cuuint64_t(g.MX) * es, cuuint64_t(g.MX) * g.NY * es, cuuint64_t(g.mes) * es};
-  const cuuint32_t box[4] = {cuuint32_t(kBoxX), cuuint32_t((thin ? kThinTY : kTY) + 1),
-                             cuuint32_t(flat ? 1 : kTZ + 1), 9};
   const cuuint32_t unit[4] = {1, 1, 1, 1};
-  const CUresult r = encode(&m.map, es == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
-                            const_cast<M*>(mass), dims, strides, box, unit, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  m.usable = r == CUDA_SUCCESS;
-  return m.usable ? &m.map : nullptr;
+  m.usable = true;
+  for (int y = 0; y < 2; ++y)
+    for (int z = 0; z < 2; ++z) {
+      const cuuint32_t box[4] = {cuuint32_t(kBoxX), cuuint32_t((thin ? kThinTY : kTY) + y),
+                                 cuuint32_t(flat ? 1 : kTZ + z), 9};
+      m.usable = m.usable &&
+                 encode(&m.maps.box[y][z], es == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
+                        4, const_cast<M*>(mass), dims, strides, box, unit, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    }
+  return m.usable ? &m.maps : nullptr;
 }
 
 // Launches the TMA-staged apply; the kernel's dynamic shared memory limit is
 // raised once per device.
 template <class C, class M, class Out, int TY, int TZ, bool kTranspose, bool kFlat = false>
-cudaError_t launch_apply_tma(const CUtensorMap& map, unsigned tiles, cudaStream_t st, const Geom& g, C d2, C kf,
+cudaError_t launch_apply_tma(const MassMaps& maps, unsigned tiles, cudaStream_t st, const Geom& g, C d2, C kf,
                              C civ, const double* in, Out* out, uint32_t* invalid, uint32_t polls, int stall) {
   // Two stages: four CTAs per SM in the float apply (three in the mixed
   // residual apply); three stages gave three (two) and a slower solve.
@@ -1254,7 +1272,7 @@ cudaError_t launch_apply_tma(const CUtensorMap& map, unsigned tiles, cudaStream_
     if (e != cudaSuccess) return e;
     ready.fetch_or(bit);
   }
-  return launch_programmatic(kernel, tiles, kTX * TY * TZ, bytes, st, map, g, d2, kf, civ, in, out, invalid,
+  return launch_programmatic(kernel, tiles, kTX * TY * TZ, bytes, st, maps, g, d2, kf, civ, in, out, invalid,
                              polls ? polls : kDefaultWaitPolls, stall);
 }
 
@@ -1308,23 +1326,23 @@ struct Solve {
                                            ((g.nz + kTZ - 1) / kTZ));
     const C d2 = C(w->delta * w->delta), kf = C(w->kfac), civ = C(iv);
     const double* in = w->input;
-    const CUtensorMap* map = response ? nullptr : mass_tensor_map(w, mass, thin);
-    if (map) {
+    const MassMaps* maps = response ? nullptr : mass_tensor_maps(w, mass, thin);
+    if (maps) {
       const uint32_t polls = w->wait_polls;
       const int stall = w->stall_stencil;
       cudaError_t e;
       // Thin tiles are on grids one cell thick along z: flat boxes.
       if (w->transpose && thin)
-        e = launch_apply_tma<C, Mass, Out, kThinTY, 1, true, true>(*map, tiles, st, g, d2, kf, civ, in, out,
+        e = launch_apply_tma<C, Mass, Out, kThinTY, 1, true, true>(*maps, tiles, st, g, d2, kf, civ, in, out,
                                                                    w->invalid, polls, stall);
       else if (w->transpose)
-        e = launch_apply_tma<C, Mass, Out, kTY, kTZ, true>(*map, tiles, st, g, d2, kf, civ, in, out, w->invalid,
+        e = launch_apply_tma<C, Mass, Out, kTY, kTZ, true>(*maps, tiles, st, g, d2, kf, civ, in, out, w->invalid,
                                                            polls, stall);
       else if (thin)
-        e = launch_apply_tma<C, Mass, Out, kThinTY, 1, false, true>(*map, tiles, st, g, d2, kf, civ, in, out,
+        e = launch_apply_tma<C, Mass, Out, kThinTY, 1, false, true>(*maps, tiles, st, g, d2, kf, civ, in, out,
                                                                     w->invalid, polls, stall);
       else
-        e = launch_apply_tma<C, Mass, Out, kTY, kTZ, false>(*map, tiles, st, g, d2, kf, civ, in, out, w->invalid,
+        e = launch_apply_tma<C, Mass, Out, kTY, kTZ, false>(*maps, tiles, st, g, d2, kf, civ, in, out, w->invalid,
                                                             polls, stall);
       if (err == cudaSuccess) err = e;
     } else if (w->transpose) {
