@@ -24,6 +24,13 @@
 // that share the 27 mass blocks: small grids take small tiles, so that every
 // SM has one.
 //
+// With one CTA an SM, the rest of its shared memory keeps the mass blocks of its
+// threads through the cycle, as many as fit, and the sums over columns run side
+// by side: a step is bound by the latencies of its phases, and the 4 dependent
+// block loads of a thread took a quarter of it. With two CTAs an SM, which hide
+// each other's latencies and share L1, both made steps longer (40^3 mixed 528
+// against 444 us a solve, 512 x 512 x 1 2.03 against 1.81 ms).
+//
 // With smoothing (grids one cell thick along z) a tile holds passes + 1 more
 // nodes on each side and takes the passes in shared memory: the smoothed
 // vector's mass response goes to a global vector, and after one more barrier
@@ -67,6 +74,7 @@ struct ResidentPlan {
   int slots;               // tiles per CTA: tile blockIdx.x + slot * gridDim.x
   bool cluster;            // the grid is one cluster
   bool shared_basis;       // basis rows in shared memory, else in `basis`
+  int kept;                // stencils of each thread whose mass blocks a cycle keeps in shared memory
   double delta, kfac, inv_volume;
   const void* mass;
   void* vector;            // [3][unique] S: the last unnormalized vector
@@ -95,7 +103,7 @@ struct ResidentPlan {
 // Shared memory of a plan with arithmetic up to double: bytes per array.
 struct ResidentShared {
   int halo, cells;                 // nodes and cells a tile stages
-  size_t vs, cs, part, h, hcol, rot, sums, basis, image, unode, mult, table, ctable, offsets, smooth, total;
+  size_t vs, cs, part, h, hcol, rot, sums, basis, image, unode, mult, table, ctable, offsets, smooth, mass, total;
 };
 // The tile and halo of the smoothing passes (the mass product reads one more node).
 inline __host__ __device__ SmoothTile resident_smooth_tile(const ResidentPlan& p) {
@@ -127,6 +135,7 @@ inline __host__ __device__ ResidentShared resident_shared(const ResidentPlan& p,
   s.ctable = take(size_t(s.cells) * 4);
   s.offsets = take(size_t(14) * sizeof(int2));
   s.smooth = take(p.smooth ? size_t(6) * resident_smooth_tile(p).size * 8 : 0);
+  s.mass = take(size_t(p.kept) * 18 * kResidentNodeThreads * scalar);  // [stencil][18 entries][thread]
   s.total = at;
   return s;
 }
@@ -136,7 +145,8 @@ __constant__ int8_t kResidentOffsets[14][3] = {{0, 0, 0},  {1, 0, 0},  {0, 1, 0}
                                                {1, -1, 0}, {1, 0, 1},  {1, 0, -1}, {0, 1, 1},  {0, 1, -1},
                                                {1, -1, 1}, {1, 1, -1}, {-1, 1, 1}, {1, 1, 1}};
 
-template <class S, class Mass, class Fld, bool kTranspose, bool kSmooth>
+// kCtas: the CTAs an SM holds, which sets a thread's registers.
+template <class S, class Mass, class Fld, bool kTranspose, bool kSmooth, int kCtas>
 struct Resident {
   const ResidentPlan& p;
   uint8_t* smem;
@@ -281,6 +291,24 @@ struct Resident {
       cs[2 * CN + n] = dx(q[1]) - dy(q[0]);
     }
   }
+  // Keeps the mass blocks of the thread's first p.kept stencils for the steps
+  // of a cycle (with one tile a CTA).
+  int kept = 0;
+  __device__ __forceinline__ void keep_mass() {
+    kept = p.kept;
+    int n, part, i, j, k;
+    if (!kept || !my_node(0, n, part, i, j, k)) return;
+    const Mass* mass = static_cast<const Mass*>(p.mass) + p.g.mass_vertex(i, j, k) * p.g.mvs;
+    const int s0 = 14 * part / p.parts, s1 = min(s0 + kept, 14 * (part + 1) / p.parts);
+    Mass* own = at<Mass>(L.mass) + threadIdx.x;
+    for (int s = s0; s < s1; ++s, own += 18 * kResidentNodeThreads) {
+      Mass m[18];
+      load_blocks(mass, s, at<int2>(L.offsets)[s].y, m);
+#pragma unroll
+      for (int e = 0; e < 18; ++e)
+        if (e < 9 || s > 0) own[e * kResidentNodeThreads] = m[e];
+    }
+  }
   // This thread's node of the tile and its part of the node's mass blocks.
   __device__ __forceinline__ bool my_node(int slot, int& n, int& part, int& i, int& j, int& k) const {
     n = threadIdx.x & (p.nodes - 1);
@@ -302,23 +330,46 @@ struct Resident {
       // Blocks in stencil order: part r of P takes stencils [14 r / P, 14 (r + 1) / P).
       const Mass* mass = static_cast<const Mass*>(p.mass) + g.mass_vertex(i, j, k) * g.mvs;
       const int2* offsets = at<int2>(L.offsets);
-      const int s1 = 14 * (part + 1) / p.parts;
-      for (int s = 14 * part / p.parts; s < s1; ++s) {
-        const int2 o = offsets[s];
-        const Mass* b = mass + 9 * s * g.mes;
-        if (p.slots > 1 && s + 1 < s1) {
-          // Grids whose mass L2 does not hold: the next stencil's rows are
-          // requested while this one's are applied, as in the step's apply.
-          const Mass* next = b + 9 * g.mes;
-          const int back = offsets[s + 1].y;
-#pragma unroll
-          for (int e = 0; e < 9; ++e) {
-            prefetch_l2(next + e * g.mes);
-            prefetch_l2(next + e * g.mes - back);
-          }
+      const int s0 = 14 * part / p.parts, s1 = 14 * (part + 1) / p.parts;
+      if constexpr (kCtas == 1) {
+        // The stencils kept, then the others, each loaded while the last one
+        // is applied.
+        const int loaded = min(s0 + kept, s1);
+        Mass next[18];
+        if (loaded < s1) load_blocks(mass, loaded, offsets[loaded].y, next);
+        const Mass* own = at<Mass>(L.mass) + threadIdx.x;
+        for (int s = s0; s < loaded; ++s, own += 18 * kResidentNodeThreads) {
+          const int o = offsets[s].x;
+          product<C>([&](int e) { return own[e * kResidentNodeThreads]; }, v + o, vn, x, y, z);
+          if (s > 0) product<C>([&](int e) { return own[(9 + e) * kResidentNodeThreads]; }, v - o, vn, x, y, z);
         }
-        product(b, v + o.x, vn, x, y, z);
-        if (s > 0) product(b - o.y, v - o.x, vn, x, y, z);
+        for (int s = loaded; s < s1; ++s) {
+          const int o = offsets[s].x;
+          Mass m[18];
+#pragma unroll
+          for (int e = 0; e < 18; ++e) m[e] = next[e];
+          if (s + 1 < s1) load_blocks(mass, s + 1, offsets[s + 1].y, next);
+          product<C>([&](int e) { return m[e]; }, v + o, vn, x, y, z);
+          if (s > 0) product<C>([&](int e) { return m[9 + e]; }, v - o, vn, x, y, z);
+        }
+      } else {
+        for (int s = s0; s < s1; ++s) {
+          const int2 o = offsets[s];
+          const Mass* b = mass + 9 * s * g.mes;
+          if (p.slots > 1 && s + 1 < s1) {
+            // Grids whose mass L2 does not hold: the next stencil's rows are
+            // requested while this one's are applied, as in the step's apply.
+            const Mass* next = b + 9 * g.mes;
+            const int back = offsets[s + 1].y;
+#pragma unroll
+            for (int e = 0; e < 9; ++e) {
+              prefetch_l2(next + e * g.mes);
+              prefetch_l2(next + e * g.mes - back);
+            }
+          }
+          product<C>([&](int e) { return __ldg(b + e * g.mes); }, v + o.x, vn, x, y, z);
+          if (s > 0) product<C>([&](int e) { return __ldg(b - o.y + e * g.mes); }, v - o.x, vn, x, y, z);
+        }
       }
       if (part > 0) {
         C* sum = at<C>(L.part);
@@ -437,12 +488,20 @@ struct Resident {
     return true;
   }
 
-  template <class C>
-  __device__ __forceinline__ void product(const Mass* __restrict__ b, const C* v, int VN, C& x, C& y, C& z) {
-    const long long es = p.g.mes;
+  // The blocks of stencil s at a node (m[0..8]) and at the node - s (m[9..17]).
+  __device__ __forceinline__ void load_blocks(const Mass* __restrict__ mass, int s, int back, Mass (&m)[18]) const {
+    const Mass* b = mass + 9 * s * p.g.mes;
+#pragma unroll
+    for (int e = 0; e < 9; ++e) m[e] = __ldg(b + e * p.g.mes);
+    if (s > 0)
+#pragma unroll
+      for (int e = 0; e < 9; ++e) m[9 + e] = __ldg(b - back + e * p.g.mes);
+  }
+  template <class C, class Entry>
+  __device__ __forceinline__ void product(Entry&& entry, const C* v, int VN, C& x, C& y, C& z) const {
     C m[9];
 #pragma unroll
-    for (int e = 0; e < 9; ++e) m[e] = C(__ldg(b + e * es));
+    for (int e = 0; e < 9; ++e) m[e] = C(entry(e));
     const C v0 = v[0], v1 = v[VN], v2 = v[2 * VN];
     if constexpr (kTranspose) {
       x += v0 * m[0] + v1 * m[3] + v2 * m[6];
@@ -479,15 +538,12 @@ struct Resident {
     for (unsigned t = threadIdx.x & 31; t < gridDim.x; t += 32) total += __ldcg(from + t);
     return warp_sum(total);
   }
-  // Sums over a warp's columns first, first + step, ... <= last (at most four,
-  // each lane's share from term(column)), to sink(column, sum) in lane 0. The
-  // columns' loads and shuffles run side by side: one after the other their
-  // latencies were a third of a step on small grids.
-  template <class Term, class Sink>
-  __device__ __forceinline__ void column_sums(int first, int step, int last, Term&& term, Sink&& sink) const {
-    double sum[4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) sum[r] = first + r * step <= last ? term(first + r * step) : 0.0;
+  // Sums over the lanes of a warp's columns first, first + step, ... <= last (at
+  // most four), to sink(column, sum) in lane 0. The columns' terms and shuffles
+  // run side by side: one after the other their latencies were a third of a
+  // step on small grids.
+  template <class Sink>
+  __device__ __forceinline__ void column_sums(int first, int step, int last, double (&sum)[4], Sink&& sink) const {
     if (first + step <= last) {
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1)
@@ -578,10 +634,10 @@ struct Resident {
 
 // The right-hand side, the guess and its residual (values[0] = |r|^2,
 // values[1] = |b|^2).
-template <class S, class Mass, class Fld, bool kTranspose, bool kSmooth>
-__global__ void __launch_bounds__(kResidentThreads, 2) resident_start_kernel(const __grid_constant__ ResidentPlan p) {
+template <class S, class Mass, class Fld, bool kTranspose, bool kSmooth, int kCtas>
+__global__ void __launch_bounds__(kResidentThreads, kCtas) resident_start_kernel(const __grid_constant__ ResidentPlan p) {
   extern __shared__ __align__(16) uint8_t resident_smem[];
-  using R = Resident<S, Mass, Fld, kTranspose, kSmooth>;
+  using R = Resident<S, Mass, Fld, kTranspose, kSmooth, kCtas>;
   R r(p, resident_smem);
   r.prepare();
   const Geom& g = p.g;
@@ -649,10 +705,10 @@ __global__ void __launch_bounds__(kResidentThreads, 2) resident_start_kernel(con
 
 // One restart cycle from the residual r (values[0] = |r|^2): at most
 // `columns` Arnoldi steps, the update of x, its residual (values[0]).
-template <class S, class Mass, class Fld, bool kTranspose, bool kSmooth>
-__global__ void __launch_bounds__(kResidentThreads, 2) resident_cycle_kernel(const __grid_constant__ ResidentPlan p) {
+template <class S, class Mass, class Fld, bool kTranspose, bool kSmooth, int kCtas>
+__global__ void __launch_bounds__(kResidentThreads, kCtas) resident_cycle_kernel(const __grid_constant__ ResidentPlan p) {
   extern __shared__ __align__(16) uint8_t resident_smem[];
-  using R = Resident<S, Mass, Fld, kTranspose, kSmooth>;
+  using R = Resident<S, Mass, Fld, kTranspose, kSmooth, kCtas>;
   R r(p, resident_smem);
   constexpr int m = kResidentRestart, kWarps = kResidentThreads / 32;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -669,7 +725,9 @@ __global__ void __launch_bounds__(kResidentThreads, 2) resident_cycle_kernel(con
   const int* unode = r.template at<int>(r.L.unode);
   const uint8_t* mult = r.template at<uint8_t>(r.L.mult);
   S* vector = static_cast<S*>(p.vector);
+  constexpr bool kSideBySide = kCtas == 1;
   r.prepare();
+  r.keep_mass();
   // Row t of the owned rows: its node and its place in a [3][unique] vector.
   auto place = [&](int t, int& n) -> long long {
     const int slot = p.slots == 1 ? 0 : t / (3 * p.nodes), rest = t - slot * 3 * p.nodes;
@@ -710,27 +768,51 @@ __global__ void __launch_bounds__(kResidentThreads, 2) resident_cycle_kernel(con
     }
     if (stop) break;
     __syncthreads();
-    r.column_sums(warp, kWarps, col,
-                  [&](int c) {
-                    const S* v = r.basis(c);
-                    double sum = 0;
-                    for (int slot = 0, t0 = 0; slot < p.slots; ++slot, t0 += 3 * p.nodes)
-                      for (int t = lane; t < 3 * p.nodes; t += 32)
-                        sum += double(v[t0 + t]) *
-                               (double(image[t0 + t]) * double(mult[slot * p.nodes + (t & (p.nodes - 1))]));
-                    return sum;
-                  },
+    // A warp's columns one after the other with two CTAs an SM, which hide
+    // each other's latency; else side by side.
+    double dots[4] = {0.0, 0.0, 0.0, 0.0};
+    if (kSideBySide && warp <= col) {
+      const S* v = r.basis(warp);
+      const long long next = r.basis(kWarps) - r.basis(0);
+      const int columns = (col - warp) / kWarps + 1;
+      for (int slot = 0, t0 = 0; slot < p.slots; ++slot, t0 += 3 * p.nodes)
+#pragma unroll 2
+        for (int t = lane; t < 3 * p.nodes; t += 32) {
+          const double w = double(image[t0 + t]) * double(mult[slot * p.nodes + (t & (p.nodes - 1))]);
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            if (c < columns) dots[c] += double(v[c * next + t0 + t]) * w;
+        }
+    } else if (!kSideBySide) {
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        if (warp + c * kWarps > col) continue;
+        const S* v = r.basis(warp + c * kWarps);
+        for (int slot = 0, t0 = 0; slot < p.slots; ++slot, t0 += 3 * p.nodes)
+          for (int t = lane; t < 3 * p.nodes; t += 32)
+            dots[c] += double(v[t0 + t]) *
+                       (double(image[t0 + t]) * double(mult[slot * p.nodes + (t & (p.nodes - 1))]));
+      }
+    }
+    r.column_sums(warp, kWarps, col, dots,
                   [&](int c, double sum) { p.partials[(long long)c * gridDim.x + blockIdx.x] = sum; });
     if (!r.grid_barrier()) return;
     // B: Gram-Schmidt of the owned rows.
-    r.column_sums(warp, kWarps, col,
-                  [&](int c) {
-                    const double* from = p.partials + (long long)c * gridDim.x;
-                    double sum = 0;
-                    for (unsigned t = lane; t < gridDim.x; t += 32) sum += __ldcg(from + t);
-                    return sum;
-                  },
-                  [&](int c, double sum) { hcol[c] = sum; });
+    double totals[4] = {0.0, 0.0, 0.0, 0.0};
+    const double* from = p.partials + (long long)warp * gridDim.x;
+    if (kSideBySide) {
+#pragma unroll 2
+      for (unsigned t = lane; t < gridDim.x; t += 32)
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          if (warp + c * kWarps <= col) totals[c] += __ldcg(from + (long long)c * kWarps * gridDim.x + t);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        if (warp + c * kWarps <= col)
+          for (unsigned t = lane; t < gridDim.x; t += 32) totals[c] += __ldcg(from + (long long)c * kWarps * gridDim.x + t);
+    }
+    r.column_sums(warp, kWarps, col, totals, [&](int c, double sum) { hcol[c] = sum; });
     __syncthreads();
     double norm2 = 0;
     if (threadIdx.x < kResidentNodeThreads) {

@@ -44,6 +44,7 @@ constexpr long long kColumnAlign = 64;
 constexpr int kMaxRestart = 1024;
 constexpr int kResidentSmooth = 8;   // smoothing passes the resident kernels take
 constexpr int kResidentCluster = 16; // CTAs of a cluster
+constexpr int kOneCtaNodes = 128;    // largest tile for which one CTA an SM comes first
 
 // Interior coordinates of compact index t (32-bit arithmetic: solver_create
 // requires 3 (n+1)^3 < 2^31).
@@ -937,6 +938,7 @@ struct SolverWorkspace {
   ResidentPlan plan{};
   unsigned resident_grid = 0;
   size_t resident_bytes = 0;
+  int resident_ctas = 1;
   double* resident_partials = nullptr;
   unsigned* resident_barrier = nullptr;
 
@@ -953,14 +955,22 @@ struct SolverWorkspace {
 template <class P>
 struct ResidentKernels {
   using Kernel = void (*)(ResidentPlan);
-  template <bool T, bool Sm>
-  static Kernel start() { return resident_start_kernel<typename P::EC, typename P::Mass, typename P::Fld, T, Sm>; }
-  template <bool T, bool Sm>
-  static Kernel cycle() { return resident_cycle_kernel<typename P::EC, typename P::Mass, typename P::Fld, T, Sm>; }
-  // The start and the cycle of A (with smoothing or not) or of A^T.
+  template <bool T, bool Sm, int Ctas>
+  static void pair(Kernel out[2]) {
+    out[0] = resident_start_kernel<typename P::EC, typename P::Mass, typename P::Fld, T, Sm, Ctas>;
+    out[1] = resident_cycle_kernel<typename P::EC, typename P::Mass, typename P::Fld, T, Sm, Ctas>;
+  }
+  template <int Ctas>
   static void pick(bool transpose, bool smooth, Kernel out[2]) {
-    out[0] = smooth ? start<false, true>() : transpose ? start<true, false>() : start<false, false>();
-    out[1] = smooth ? cycle<false, true>() : transpose ? cycle<true, false>() : cycle<false, false>();
+    if (smooth) pair<false, true, Ctas>(out);
+    else if (transpose) pair<true, false, Ctas>(out);
+    else pair<false, false, Ctas>(out);
+  }
+  // The start and the cycle of A (with smoothing or not) or of A^T, for one
+  // CTA an SM or two.
+  static void pick(bool transpose, bool smooth, int ctas, Kernel out[2]) {
+    if (ctas == 1) pick<1>(transpose, smooth, out);
+    else pick<2>(transpose, smooth, out);
   }
 };
 
@@ -992,11 +1002,19 @@ bool cluster_fits(void (*kernel)(ResidentPlan), int blocks, size_t bytes) {
 }
 
 // Tiles of the resident kernels: the smallest tile whose CTAs are all
-// resident at once, so that every SM has nodes and a node has many threads;
-// the basis in shared memory where that tile leaves room for it (FP64 256 x
+// resident at once, so that every SM has nodes and a node has many threads,
+// but one CTA an SM where a tile has at least two threads a node: its shared
+// memory then keeps the mass blocks of the threads (all of them in FP32)
+// through a restart cycle. Without that a step of a 1024 x 1 x 1 grid spent
+// 4,800 of its 18,600 cycles on the mass product, most of it waiting for L2.
+// Solves, us, one CTA an SM first / the smallest tile first: 1024 x 1 x 1
+// 1,281 / 1,514 mixed, 1,301 / 1,547 FP64; 96 x 96 x 1 235 / 279, 200 / 240;
+// 128 x 128 x 1 255 / 276, 227 / 250; 24^3 237 / 264 mixed, 245 / 245 FP64;
+// but 20^3 FP64 229 / 218, so FP64 boxes take the smallest tile. The basis is
+// in shared memory where that tile leaves room for it (FP64 256 x
 // 128 x 1: 325 us a solve with tiles of 128 nodes and the basis in global
 // memory, 410 us with 256 and the basis in shared memory). Resident against
-// step graph, ms a solve (mixed, stencil-major): 1024 x 1 x 1 1.51 / 5.72, 16^3
+// step graph, ms a solve (mixed, stencil-major): 1024 x 1 x 1 1.28 / 5.72, 16^3
 // 0.19 / 0.58, 32^3 0.29 / 0.59, 40^3 0.44 / 0.70, 256 x 128 x 1 0.34 / 0.78,
 // 256 x 256 x 1 0.44 / 0.94.
 template <class P>
@@ -1010,10 +1028,14 @@ void plan_resident(SolverWorkspace* w, int sms) {
       cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, device) != cudaSuccess || !cooperative ||
       cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess)
     return;
-  typename K::Kernel kernels[4];
-  K::pick(false, smooth > 0, kernels);
-  K::pick(smooth == 0, smooth > 0, kernels + 2);  // no adjoint with smoothing
-  for (auto k : kernels)
+  // [CTAs an SM - 1]
+  typename K::Kernel kernels[2][4];
+  for (int c = 0; c < 2; ++c) {
+    K::pick(false, smooth > 0, c + 1, kernels[c]);
+    K::pick(smooth == 0, smooth > 0, c + 1, kernels[c] + 2);  // no adjoint with smoothing
+  }
+  for (auto k : {kernels[0][0], kernels[0][1], kernels[0][2], kernels[0][3], kernels[1][0], kernels[1][1], kernels[1][2],
+                 kernels[1][3]})
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, limit) != cudaSuccess) {
       cudaGetLastError();
       return;
@@ -1023,7 +1045,13 @@ void plan_resident(SolverWorkspace* w, int sms) {
     while (p < n) p *= 2;
     return p;
   };
-  for (int nodes = 32; nodes <= kResidentNodeThreads; nodes *= 2) {
+  // The tile sizes in the order they are tried; the first ones only with one
+  // CTA an SM.
+  const bool fp64_box = sizeof(typename P::EC) == 8 && g.nz > 1;
+  const int sizes[] = {32, 64, kOneCtaNodes, 32, 64, 128, kResidentNodeThreads};
+  for (int n = smooth > 0 || fp64_box ? 3 : 0; n < 7; ++n) {
+    const int nodes = sizes[n];
+    const bool alone = n < 3;
     ResidentPlan p{};
     p.g = g;
     // The shape with the fewest tiles, the widest x of those.
@@ -1075,8 +1103,9 @@ void plan_resident(SolverWorkspace* w, int sms) {
       const int grid = (p.tiles + p.slots - 1) / p.slots;
       const size_t bytes = resident_shared(p, sizeof(typename P::EC)).total;
       if (bytes > size_t(limit)) continue;
-      int per_sm = 2;
-      for (auto k : kernels) {
+      const int ctas = grid <= sms ? 1 : 2;
+      int per_sm = ctas;
+      for (auto k : kernels[ctas - 1]) {
         int blocks = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k, kResidentThreads, bytes) != cudaSuccess) {
           cudaGetLastError();
@@ -1085,15 +1114,26 @@ void plan_resident(SolverWorkspace* w, int sms) {
         per_sm = std::min(per_sm, blocks);
       }
       if (grid > per_sm * sms) continue;
+      if (alone && grid > sms) continue;
       if (p.slots > 2 && g.nz > 1 &&
           (sizeof(typename P::EC) == 4 || 100LL * p.tiles < 85LL * p.slots * per_sm * sms))
         break;
+      // The rest of the shared memory keeps mass blocks.
+      size_t used = bytes;
+      if (p.slots == 1 && ctas == 1) {
+        const size_t budget = size_t(limit);
+        const size_t stencil = size_t(18) * kResidentNodeThreads * sizeof(typename P::EC);
+        const int most = (14 + p.parts - 1) / p.parts;
+        if (budget > bytes) p.kept = std::min(most, int((budget - bytes) / stencil));
+        used = resident_shared(p, sizeof(typename P::EC)).total;
+      }
       if (p.cluster)
-        for (auto k : kernels)
-          if (!cluster_fits(k, grid, bytes)) p.cluster = false;
+        for (auto k : kernels[ctas - 1])
+          if (!cluster_fits(k, grid, used)) p.cluster = false;
+      w->resident_ctas = ctas;
       w->plan = p;
       w->resident_grid = unsigned(grid);
-      w->resident_bytes = bytes;
+      w->resident_bytes = used;
       w->resident = true;
       return;
     }
@@ -1599,7 +1639,7 @@ struct Solve {
     double controls[2];
     ArnoldiControl control{};
     typename K::Kernel kernels[2];
-    K::pick(w->transpose, w->smoothing.iterations > 0, kernels);
+    K::pick(w->transpose, w->smoothing.iterations > 0, w->resident_ctas, kernels);
     if (!launch_resident(kernels[0], controls, &control))
       return TPICB200_BACKEND_FAILURE;
     if (!std::isfinite(controls[0]) || !std::isfinite(controls[1])) return TPICB200_OVERFLOW;
