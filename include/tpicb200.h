@@ -97,11 +97,12 @@ enum { TPICB200_MASS_LAYOUT_RECORDS = 0, TPICB200_MASS_LAYOUT_STENCIL_MAJOR = 1,
 /* Mass-matrix assembly forms, the extended `--mass-matrix` selection
  * (TPIC: scalar | matrix-core, config/numerics_options.hpp:31-47). */
 enum {
-  TPICB200_MASS_SCALAR = 0,     /* CUDA cores, the precision mode's compute type */
-  TPICB200_MASS_SCALAR_F64 = 1, /* CUDA cores, FP64 cell sums, narrowed once at the flush */
+  TPICB200_MASS_SCALAR = 0,     /* the precision mode's compute type: FP32 cell sums on CUDA cores, or
+                                   FP64 on the FP64 tensor cores */
+  TPICB200_MASS_SCALAR_F64 = 1, /* FP64 cell sums, narrowed once at the flush */
   TPICB200_MASS_TF32 = 2,       /* tcgen05 tensor cores, TF32 operands, FP32 accumulation */
   TPICB200_MASS_BF16X3 = 3,     /* tcgen05, BF16 hi/lo split products, FP32 accumulation */
-  TPICB200_MASS_MOMENTS_F64 = 4 /* CUDA cores, FP64 per-cell moments (27 pair-weight classes x
+  TPICB200_MASS_MOMENTS_F64 = 4 /* FP64 tensor cores, FP64 per-cell moments (27 pair-weight classes x
                                    (9 response + 3 current) entries), then a per-node assembly;
                                    DOUBLE precision only */
 };
@@ -307,7 +308,9 @@ int tpicb200_read_invalid(tpicb200_context* ctx, uint32_t* count, int clear, tpi
  *   its CTA wait (with the default bound) for its copies in flight and
  *   return without writing its rows; the apply adds 1 << 21 to the invalid
  *   counter.
- * tpicb200_cycle then returns TPICB200_INVALID_DATA. */
+ * tpicb200_cycle then returns TPICB200_INVALID_DATA. The grid barriers of the
+ * binned sort's cooperative kernels have the default bound: one that gives up
+ * adds 1 << 22 to the invalid counter. */
 int tpicb200_set_wait_limit(tpicb200_context* ctx, uint32_t polls);
 
 /* Test of the bounded waits (tpicb200_set_wait_limit) without a fault: with
@@ -329,9 +332,11 @@ int tpicb200_clear_moments(tpicb200_context* ctx, void* j, void* mass, tpicb200_
  * tensor-core forms (TF32, BF16X3; mixed precision, sorted bins) keep the
  * cell moments of every species deposited since tpicb200_clear_moments in
  * the context and tpicb200_fold_periodic adds them into j and mass, with no
- * atomics and a fixed summation order. With counts/offsets (the
- * bins of p, from tpicb200_sort) the sorted cell-tile kernels run; with NULL
- * bins the per-particle kernels run (scalar forms only). Replaces
+ * atomics and a fixed summation order. The scalar forms with counts/offsets
+ * (the bins of p, from tpicb200_sort) and both j and mass sum the same cell
+ * moments and add them into j and mass within the call; with only one of the
+ * two, or while a moment form's moments wait for the fold, the sorted
+ * cell-tile kernels run; with NULL bins the per-particle kernels run. Replaces
  * enqueue_sorted_current / enqueue_unsorted_current
  * (ecsim/deposition/current_deposition_device.hpp:340-421) and
  * enqueue_sorted_mass_matrix<Kernel> / enqueue_unsorted_mass_matrix
@@ -371,11 +376,16 @@ int tpicb200_mass_apply(tpicb200_context* ctx, const void* mass, const double* i
  * A(v) = v + delta^2 curl_C2N curl_N2C v + k M v / V from the guess E; writes
  * E_theta (interior nodes and ghosts) when converged. Host-blocking like
  * Gmres::host_blocking_solve (ecsim/gmres/gmres_device.hpp:353-454), which
- * reads two scalars back per Arnoldi step; here the steps of a restart cycle
- * run as one CUDA graph (a WHILE node) and the host waits once per restart
- * cycle plus once for the initial residual. With the environment variable
- * TPICB200_STEP_GRAPH=0 when the context is created, the host steps the loop
- * (one wait per step). b_cell needs filled ghosts. */
+ * reads two scalars back per Arnoldi step; here the host waits once per
+ * restart cycle plus once for the initial residual. A restart cycle is one
+ * cooperative kernel that keeps its vectors on the chip where the grid fits
+ * (restart at most 32), else one CUDA graph (a WHILE node over the step's
+ * kernels). The step's kernels run, whatever the grid, while a wait limit or
+ * a stall is set (those act on their operator apply), and with the environment
+ * variable TPICB200_STEP_GRAPH=0 when the context is created, which has the
+ * host step the loop (one wait per step). A cooperative kernel whose bounded
+ * grid barrier gives up returns TPICB200_BACKEND_FAILURE. b_cell needs filled
+ * ghosts. */
 int tpicb200_field_solve(tpicb200_context* ctx, const void* e, const void* b_cell, const void* j,
                          const void* mass, double* e_theta, tpicb200_gmres_result* result,
                          tpicb200_stream stream);
