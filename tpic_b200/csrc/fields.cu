@@ -286,8 +286,11 @@ cudaError_t launch_rhs(int precision, const Geom& g, double delta, double kfac, 
 // after. One launch per pass with a ghost fill behind it took 12 launches for
 // the default six passes, some 55 us on 256 x 128 x 1, where the passes
 // themselves are 1 us each; the halo costs (32 + 12)(8 + 12) / (32 x 8) = 3.4
-// times the nodes there. On grids thicker than one cell three passes a launch
-// (tile 16 x 8 x 8) keep that factor at 4.2.
+// times the nodes there. Grids thicker than one cell
+// on every axis take smooth_pass_kernel: halos all around cost more than a
+// launch a pass (smoothed FP32 solve of 64^3 with three passes on 16 x 8 x 8
+// tiles 7.0 ms, with one or two 9.1 and 7.2, with passes and ghost fills 4.4,
+// now 3.9).
 constexpr int kSmoothThreads = 256;
 
 template <class C>
@@ -331,13 +334,48 @@ __global__ void __launch_bounds__(kSmoothThreads) smooth_tile_kernel(Geom g, Smo
   }
 }
 
+// One pass at every stored node, ghosts as their unique node (blockIdx.y a
+// component), so no ghost fill follows.
+template <class C>
+__global__ void __launch_bounds__(kSmoothThreads) smooth_pass_kernel(Geom g, int op, C alpha, C beta,
+                                                                     const double* __restrict__ src,
+                                                                     double* __restrict__ dst, uint32_t* invalid) {
+  src += blockIdx.y * g.nodes;
+  dst += blockIdx.y * g.nodes;
+  const uint32_t total = uint32_t(g.nodes), NX = uint32_t(g.NX), NY = uint32_t(g.NY);
+  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+    const uint32_t row = t / NX;
+    const int a = int(t - row * NX) - 1, b = int(row % NY) - 1, c = int(row / NY) - 1;
+    const int i = wrap_index(a, g.nx), j = wrap_index(b, g.ny), k = wrap_index(c, g.nz);
+    // The neighbours' unique indexes along each axis.
+    const int x[3] = {i == 0 ? g.nx - 1 : i - 1, i, i + 1 == g.nx ? 0 : i + 1};
+    const int y[3] = {j == 0 ? g.ny - 1 : j - 1, j, j + 1 == g.ny ? 0 : j + 1};
+    const int z[3] = {k == 0 ? g.nz - 1 : k - 1, k, k + 1 == g.nz ? 0 : k + 1};
+    const C value = smooth_sum<C>([&](int dx, int dy, int dz) { return C(src[g.node(x[dx + 1], y[dy + 1], z[dz + 1])]); },
+                                  op, alpha, beta);
+    dst[t] = double(value);
+    if (invalid && a == i && b == j && c == k && !isfinite(value)) atomicAdd(invalid, 1u);
+  }
+}
+
 template <class C>
 cudaError_t launch_smooth_typed(const Geom& g, int niter, int op, double alpha, const double* src, double* out,
                                 double* tmp, uint32_t* invalid, cudaStream_t s) {
+  if (g.nx > 1 && g.ny > 1 && g.nz > 1) {
+    if (g.nodes >= (1LL << 32)) return cudaErrorInvalidValue;
+    const C a = C(alpha), beta = (C(1) - a) / C(6);
+    for (int left = niter; left > 0; --left) {
+      double* to = left % 2 == 1 ? out : tmp;
+      smooth_pass_kernel<C><<<dim3(grid_for(g.nodes, kSmoothThreads), 3), kSmoothThreads, 0, s>>>(g, op, a, beta, src,
+                                                                                                  to, invalid);
+      count_launches(1);
+      src = to;
+    }
+    return cudaGetLastError();
+  }
   // Passes a launch: as many as a halo is worth, split evenly.
-  const bool flat = g.nx == 1 || g.ny == 1 || g.nz == 1;
-  const int most = flat ? 8 : 3, launches = (niter + most - 1) / most;
-  const int tx = flat ? 32 : 16, ty = g.ny == 1 ? 1 : 8, tz = g.nz == 1 ? 1 : 8;
+  const int most = 8, launches = (niter + most - 1) / most;
+  const int tx = 32, ty = g.ny == 1 ? 1 : 8, tz = g.nz == 1 ? 1 : 8;
   const long long tiles = (long long)((g.nx + tx - 1) / tx) * ((g.ny + ty - 1) / ty) * ((g.nz + tz - 1) / tz);
   if (tiles > 0x7fffffffLL) return cudaErrorInvalidValue;
   int done = 0;

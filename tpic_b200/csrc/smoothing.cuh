@@ -16,10 +16,9 @@ __device__ __forceinline__ double rn_mul(double a, double b) { return __dmul_rn(
 __device__ __forceinline__ float rn_add(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ double rn_add(double a, double b) { return __dadd_rn(a, b); }
 
-// The pass at f[0]; sx, sy, sz are the neighbours' distances.
-template <class C>
-__device__ __forceinline__ C smooth_value(const C* f, int sx, int sy, int sz, int op, C alpha, C beta) {
-  auto v = [&](int a, int b, int c) { return f[a * sx + b * sy + c * sz]; };
+// The pass at a node, its neighbours v(dx, dy, dz).
+template <class C, class V>
+__device__ __forceinline__ C smooth_sum(V&& v, int op, C alpha, C beta) {
   const C face = rn_add(rn_add(rn_add(rn_add(rn_add(v(-1, 0, 0), v(1, 0, 0)), v(0, -1, 0)), v(0, 1, 0)), v(0, 0, -1)),
                         v(0, 0, 1));
   if (op == 0) return rn_add(rn_mul(alpha, v(0, 0, 0)), rn_mul(beta, face));
@@ -35,6 +34,11 @@ __device__ __forceinline__ C smooth_value(const C* f, int sx, int sy, int sz, in
   corner = rn_add(corner, v(-1, 1, 1)); corner = rn_add(corner, v(1, 1, 1));
   const C sum = rn_add(rn_add(rn_add(rn_mul(C(8), v(0, 0, 0)), rn_mul(C(4), face)), rn_mul(C(2), edge)), corner);
   return rn_mul(sum, C(1) / C(64));
+}
+// The pass at f[0]; sx, sy, sz are the neighbours' distances.
+template <class C>
+__device__ __forceinline__ C smooth_value(const C* f, int sx, int sy, int sz, int op, C alpha, C beta) {
+  return smooth_sum<C>([&](int a, int b, int c) { return f[a * sx + b * sy + c * sz]; }, op, alpha, beta);
 }
 
 // A tile of unique nodes with `halo` more on each side. An axis of one cell is
