@@ -939,6 +939,7 @@ struct SolverWorkspace {
   unsigned resident_grid = 0;
   size_t resident_bytes = 0;
   int resident_ctas = 1;
+  bool adjoint_kernels = false;  // the kernels of A^T have their limits
   double* resident_partials = nullptr;
   unsigned* resident_barrier = nullptr;
 
@@ -1001,6 +1002,16 @@ bool cluster_fits(void (*kernel)(ResidentPlan), int blocks, size_t bytes) {
   return clusters > 0;
 }
 
+// Raises the kernels' dynamic shared memory limit.
+bool allow_shared(void (*const (&kernels)[2])(ResidentPlan), int limit) {
+  for (auto k : kernels)
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, limit) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+  return true;
+}
+
 // Tiles of the resident kernels: the smallest tile whose CTAs are all
 // resident at once, so that every SM has nodes and a node has many threads,
 // but one CTA an SM where a tile has at least two threads a node: its shared
@@ -1028,18 +1039,13 @@ void plan_resident(SolverWorkspace* w, int sms) {
       cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, device) != cudaSuccess || !cooperative ||
       cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess)
     return;
-  // [CTAs an SM - 1]
-  typename K::Kernel kernels[2][4];
-  for (int c = 0; c < 2; ++c) {
-    K::pick(false, smooth > 0, c + 1, kernels[c]);
-    K::pick(smooth == 0, smooth > 0, c + 1, kernels[c] + 2);  // no adjoint with smoothing
-  }
-  for (auto k : {kernels[0][0], kernels[0][1], kernels[0][2], kernels[0][3], kernels[1][0], kernels[1][1], kernels[1][2],
-                 kernels[1][3]})
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, limit) != cudaSuccess) {
-      cudaGetLastError();
-      return;
-    }
+  // The kernels of A; those of A^T have the same bounds (adjoint_kernels). A
+  // kernel is loaded when its attributes are set, so only the ones that a tile
+  // asks for.
+  typename K::Kernel kernels[2][2];  // [CTAs an SM - 1]
+  bool loaded[2] = {false, false};
+  K::pick(false, smooth > 0, 1, kernels[0]);
+  K::pick(false, smooth > 0, 2, kernels[1]);
   auto power = [](int n) {
     int p = 1;
     while (p < n) p *= 2;
@@ -1104,7 +1110,10 @@ void plan_resident(SolverWorkspace* w, int sms) {
       const size_t bytes = resident_shared(p, sizeof(typename P::EC)).total;
       if (bytes > size_t(limit)) continue;
       const int ctas = grid <= sms ? 1 : 2;
+      if (alone ? ctas == 2 : grid > 2 * sms) continue;
       int per_sm = ctas;
+      if (!loaded[ctas - 1] && !allow_shared(kernels[ctas - 1], limit)) return;
+      loaded[ctas - 1] = true;
       for (auto k : kernels[ctas - 1]) {
         int blocks = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k, kResidentThreads, bytes) != cudaSuccess) {
@@ -1114,7 +1123,6 @@ void plan_resident(SolverWorkspace* w, int sms) {
         per_sm = std::min(per_sm, blocks);
       }
       if (grid > per_sm * sms) continue;
-      if (alone && grid > sms) continue;
       if (p.slots > 2 && g.nz > 1 &&
           (sizeof(typename P::EC) == 4 || 100LL * p.tiles < 85LL * p.slots * per_sm * sms))
         break;
@@ -1640,6 +1648,16 @@ struct Solve {
     ArnoldiControl control{};
     typename K::Kernel kernels[2];
     K::pick(w->transpose, w->smoothing.iterations > 0, w->resident_ctas, kernels);
+    if (w->transpose && !w->adjoint_kernels) {
+      // Their limits, which the plan raised for the kernels of A.
+      w->adjoint_kernels = allow_shared(kernels, int(w->resident_bytes));
+      for (auto k : kernels)
+        if (p.cluster) w->adjoint_kernels = w->adjoint_kernels && cluster_fits(k, int(w->resident_grid), w->resident_bytes);
+      if (!w->adjoint_kernels) {
+        err = cudaErrorLaunchOutOfResources;
+        return TPICB200_BACKEND_FAILURE;
+      }
+    }
     if (!launch_resident(kernels[0], controls, &control))
       return TPICB200_BACKEND_FAILURE;
     if (!std::isfinite(controls[0]) || !std::isfinite(controls[1])) return TPICB200_OVERFLOW;
