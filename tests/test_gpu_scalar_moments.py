@@ -92,7 +92,7 @@ def test_ragged_cells_match_the_oracle(torch_cuda, shape, nspecies, precision, k
                                                     m.data_ptr(), kind, ctx.invalid.data_ptr(), ctx.stream))
 
     records = int(8 * COUNTS.max() * nspecies / scale)
-    # Cleared buffers are stored into; a second deposition adds.
+    # A second deposition adds.
     _lib.check(ctx.lib.tpicb200_clear_moments(ctx.ctx, j.data_ptr(), m.data_ptr(), ctx.stream))
     deposit()
     ctx.fold(j, m)

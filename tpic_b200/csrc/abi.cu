@@ -36,10 +36,11 @@ struct tpicb200_context {
   cudaEvent_t events[6 + 3 * TPICB200_MAX_SPECIES]{};
   void* moments = nullptr;       // per-cell moments of the moment forms (float: tensor core; double: FP64)
   bool moments_pending = false;  // moments hold deposits not yet assembled
-  // J and mass buffers zeroed by the last tpicb200_clear_moments that nothing
-  // else has deposited into since: the assembly may store instead of add.
-  const void* cleared_j = nullptr;
-  const void* cleared_mass = nullptr;
+  // Set while an entry point that does the whole moment stage itself (the cycle,
+  // prepare, the cycle's backward) runs and has deposited nothing yet: the
+  // assembly then stores J and the mass. In every other call it adds: what a
+  // caller or another context put there since a clear is not known here.
+  bool stores = false;
   uint32_t wait_polls = 0;  // device wait bound of the stream kernel and the TMA apply (0: the default)
   int stall_site = TPICB200_STALL_NONE;  // tpicb200_inject_stall
   uint32_t stall_index = 0;
@@ -107,6 +108,12 @@ cudaError_t launch_moments(tpicb200_context* ctx, int kind, int ns, const double
                            ctx->stall_site == TPICB200_STALL_DEPOSIT ? ctx->stall_index : 0u);
 }
 
+struct StoresMoments {
+  tpicb200_context* ctx;
+  explicit StoresMoments(tpicb200_context* c) : ctx(c) { ctx->stores = true; }
+  ~StoresMoments() { ctx->stores = false; }
+};
+
 // The scalar forms deposit J and the mass of sorted records through the
 // context's moments too, assembled within the call; not while those hold
 // moments that wait for the fold.
@@ -117,8 +124,8 @@ int deposit_through_moments(tpicb200_context* ctx, int kind, int ns, const doubl
                             const tpicb200_particles* const* parts, const uint32_t* const* counts,
                             const uint32_t* const* offsets, const void* b_node, void* j, void* mass,
                             uint32_t* invalid, cudaStream_t s) {
-  const int overwrite = j == ctx->cleared_j && mass == ctx->cleared_mass ? 1 : 0;
-  ctx->cleared_j = ctx->cleared_mass = nullptr;
+  const int overwrite = ctx->stores ? 1 : 0;
+  ctx->stores = false;
   cudaError_t e = launch_moments(ctx, kind, ns, qom, parts, counts, offsets, b_node, 0, invalid, nullptr, s);
   if (e == cudaSuccess) e = launch_assemble_moments(ctx->opt.precision, ctx->g, ctx->moments, j, mass, overwrite, s);
   return cuda_status(e, "deposition launch failed");
@@ -362,8 +369,6 @@ int tpicb200_clear_moments(tpicb200_context* ctx, void* j, void* mass, tpicb200_
   const size_t fb = ctx->opt.precision == TPICB200_PRECISION_DOUBLE ? 8 : 4;
   cudaError_t e = cudaSuccess;
   ctx->moments_pending = false;
-  ctx->cleared_j = j && mass ? j : nullptr;
-  ctx->cleared_mass = j && mass ? mass : nullptr;
   if (j) e = cudaMemsetAsync(j, 0, 3 * size_t(ctx->g.nodes) * fb, (cudaStream_t)stream);
   if (mass && e == cudaSuccess) e = cudaMemsetAsync(mass, 0, 126 * size_t(ctx->g.mnodes) * fb, (cudaStream_t)stream);
   return cuda_status(e, "moment clear failed");
@@ -394,7 +399,7 @@ int tpicb200_deposit(tpicb200_context* ctx, double qom, const tpicb200_particles
   }
   if (sums_by_moments(ctx, j, mass) && counts) return deposit_through_moments(ctx, mass_kind, 1, &qom, &p, &counts,
                                                                               &offsets, b_node, j, mass, inv, s);
-  ctx->cleared_j = ctx->cleared_mass = nullptr;
+  ctx->stores = false;
   return cuda_status(launch_deposit(ctx->opt.precision, mass_kind, ctx->g, qom, ctx->opt.dt, ctx->opt.c, p,
                                     counts, offsets, b_node, j, mass, inv, s),
                      "deposition launch failed");
@@ -405,13 +410,12 @@ int tpicb200_fold_periodic(tpicb200_context* ctx, void* j, void* mass, tpicb200_
   if (ctx->moments_pending) {
     // Cell moments of the moment forms are added into the unique nodes first.
     if (!j || !mass) return fail(TPICB200_INVALID_ARGUMENT, "pending cell moments need J-hat and mass");
-    const int overwrite = j == ctx->cleared_j && mass == ctx->cleared_mass ? 1 : 0;
-    if (int r = cuda_status(launch_assemble_moments(ctx->opt.precision, ctx->g, ctx->moments, j, mass, overwrite,
-                                                    (cudaStream_t)stream),
+    if (int r = cuda_status(launch_assemble_moments(ctx->opt.precision, ctx->g, ctx->moments, j, mass,
+                                                    ctx->stores ? 1 : 0, (cudaStream_t)stream),
                             "moment assembly failed"))
       return r;
     ctx->moments_pending = false;
-    ctx->cleared_j = ctx->cleared_mass = nullptr;
+    ctx->stores = false;
   }
   return cuda_status(launch_fold(ctx->opt.precision, ctx->g, j, mass, (cudaStream_t)stream), "fold launch failed");
 }
@@ -589,6 +593,7 @@ int tpicb200_deposit_species(tpicb200_context* ctx, int ns, const double* qom, c
 
 static int deposit_all(tpicb200_context* ctx, tpicb200_state* st, const void* b_node, cudaStream_t s) {
   if (int r = tpicb200_clear_moments(ctx, st->j, st->mass, (tpicb200_stream)s)) return r;
+  const StoresMoments stores(ctx);
   tpicb200_particles live[TPICB200_MAX_SPECIES];
   const uint32_t* counts[TPICB200_MAX_SPECIES];
   const uint32_t* offsets[TPICB200_MAX_SPECIES];
@@ -893,8 +898,7 @@ int tpicb200_cycle(tpicb200_context* ctx, tpicb200_state* st, int ncycles, tpicb
     // assembly stores every entry of the unique nodes and the fold copies
     // every other vertex.
     ctx->moments_pending = false;
-    ctx->cleared_j = st->j;
-    ctx->cleared_mass = st->mass;
+    const StoresMoments stores(ctx);
     for (int first = 0; first < st->ns; first += 2) {
       const int count = st->ns - first < 2 ? st->ns - first : 2;
       DepositPlan plan[2];
@@ -1152,13 +1156,13 @@ int tpicb200_cycle_backward(tpicb200_context* ctx, tpicb200_tape* tape, tpicb200
   // The cycle's B at the nodes, J and M, deposited again from the tape.
   if (int r = tpicb200_magnetic_to_nodes(ctx, tape->b_cell, adj->b_node, stream)) return r;
   if (int r = tpicb200_clear_moments(ctx, adj->j, adj->mass, stream)) return r;
-  const tpicb200_particles* parts = tape->species;
-  const uint32_t* const* counts = tape->counts;
-  const uint32_t* const* offsets = tape->offsets;
-  if (int r = tpicb200_deposit_species(ctx, tape->ns, tape->qom, parts, counts, offsets, adj->b_node, adj->j,
-                                       adj->mass, tape->mass_kind, nullptr, stream))
-    return r;
-  if (int r = tpicb200_fold_periodic(ctx, adj->j, adj->mass, stream)) return r;
+  {
+    const StoresMoments stores(ctx);
+    if (int r = tpicb200_deposit_species(ctx, tape->ns, tape->qom, tape->species, tape->counts, tape->offsets,
+                                         adj->b_node, adj->j, adj->mass, tape->mass_kind, nullptr, stream))
+      return r;
+    if (int r = tpicb200_fold_periodic(ctx, adj->j, adj->mass, stream)) return r;
+  }
   // Advance backward, then the movers' E_theta gradient.
   cudaError_t err = launch_adjoint_advance(g, ctx->opt.theta, c, dt, adj->e_bar, adj->b_bar, adj->e_theta_bar, s);
   for (int sp = 0; sp < tape->ns && err == cudaSuccess; ++sp)
