@@ -331,8 +331,8 @@ int tpicb200_clear_moments(tpicb200_context* ctx, void* j, void* mass, tpicb200_
  * nodes; call tpicb200_fold_periodic after the last species. The
  * tensor-core forms (TF32, BF16X3; mixed precision, sorted bins) keep the
  * cell moments of every species deposited since tpicb200_clear_moments in
- * the context and tpicb200_fold_periodic adds them into j and mass, with no
- * atomics and a fixed summation order. The scalar forms with counts/offsets
+ * the context and tpicb200_fold_periodic adds them into j and mass: one atomic
+ * addition an entry, of a sum in a fixed order. The scalar forms with counts/offsets
  * (the bins of p, from tpicb200_sort) and both j and mass sum the same cell
  * moments and add them into j and mass within the call; with only one of the
  * two, or while a moment form's moments wait for the fold, the sorted

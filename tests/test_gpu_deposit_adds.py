@@ -7,6 +7,8 @@ An entry's sum over the records is the same number each time and is added in
 one rounding, so the comparisons with the sum added on the host are exact."""
 from __future__ import annotations
 
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -119,3 +121,29 @@ def test_replays_of_the_deposition_alone_add(torch_cuda, precision, kind):
             assert torch.equal(unique(ctx, t), unique(ctx, a) + unique(ctx, a))
         del graph
         ctx.close()
+
+
+def test_two_contexts_on_two_streams_into_the_same_buffers(torch_cuda):
+    """The scalar form's atomic additions of depositions that run at the same time."""
+    import torch
+    g, ctx, bn = setting(0, (23, 21, 20))
+    _, other, _ = setting(0, (23, 21, 20))
+    first, second = Species(ctx, g, 0, 0), Species(ctx, g, 1, 0)
+    alone = [ctx.moments() for _ in range(2)]
+    for s, a in zip((first, second), alone):
+        s.into(ctx, bn, *a, 0)
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    ctx.stream, other.stream = (C.c_void_p(s.cuda_stream) for s in streams)
+    j, m = ctx.moments()
+    torch.cuda.synchronize()
+    rounds = 8
+    for _ in range(rounds):
+        first.into(ctx, bn, j, m, 0)
+        second.into(other, bn, j, m, 0)
+    torch.cuda.synchronize()
+    for t, a, b in zip((j, m), *alone):
+        want = rounds * (a + b)
+        # Sixteen additions of the two sums in any order: 16 eps of their magnitudes.
+        assert float((t - want).abs().max()) <= 16 * 2.0**-52 * rounds * float((a.abs() + b.abs()).max())
+    ctx.close()
+    other.close()

@@ -1244,6 +1244,15 @@ __host__ __device__ constexpr StencilPairs make_stencil_pairs() {
   return r;
 }
 
+// `overwrite` stores a sum (the entry point owns J and M and deposits nothing
+// else); otherwise it is added, atomically: another context may deposit into
+// the same J and M at the same time.
+template <class T>
+__device__ __forceinline__ void put_moment(T* dst, T sum, int overwrite) {
+  if (overwrite) *dst = sum;
+  else atomicAdd(dst, sum);
+}
+
 // One thread per (unique node, stencil): the stencil's nine record entries
 // of the node, each the sum, in increasing corner order, of the moments
 // G[t][e] of the cells holding the pairs (a, a + offset_s); "stencil" 14 is
@@ -1251,8 +1260,7 @@ __host__ __device__ constexpr StencilPairs make_stencil_pairs() {
 // J[a][c] of the cells around the node. The stencil is the block index
 // modulo 15 and each case is unrolled from the compile-time tables, so a thread holds
 // at most nine sums and the loads of a warp are consecutive across its
-// nodes. `overwrite` stores the sums (J and M were cleared and nothing else
-// was deposited); otherwise they are added.
+// nodes.
 template <class T, int S>
 __device__ __forceinline__ void assemble_stencil(const Geom& g, const long long (&cell)[8], long long node,
                                                  long long mvertex, const T* __restrict__ mom,
@@ -1273,7 +1281,7 @@ __device__ __forceinline__ void assemble_stencil(const Geom& g, const long long 
 #pragma unroll
     for (int e = 0; e < 9; ++e) {
       T* dst = M + g.mass_index(mvertex, S * 9 + e);
-      *dst = overwrite ? sum[e] : *dst + sum[e];
+      put_moment(dst, sum[e], overwrite);
     }
   } else {
 #pragma unroll
@@ -1282,7 +1290,7 @@ __device__ __forceinline__ void assemble_stencil(const Geom& g, const long long 
 #pragma unroll
       for (int a = 0; a < 8; ++a) sum += __ldg(mom + moment_index(cell[a], kMassMoments + a * 3 + c));
       T* dst = J + c * g.nodes + node;
-      *dst = overwrite ? sum : *dst + sum;
+      put_moment(dst, sum, overwrite);
     }
   }
 }
@@ -1413,7 +1421,7 @@ __device__ __forceinline__ void assemble_warp_quads(const Geom& g, int m0, int j
 #pragma unroll
     for (int e = 0; e < kEntries; ++e) {
       T* dst = S < 14 ? M + g.mass_index(g.mass_vertex(i, j, k), S * 9 + e) : J + e * g.nodes + node;
-      *dst = overwrite ? stage[e][lane] : *dst + stage[e][lane];
+      put_moment(dst, stage[e][lane], overwrite);
     }
   }
 }
