@@ -76,6 +76,35 @@ def test_resident_solve_equals_the_step_graph(torch_cuda, shape, precision, adjo
     assert torch.equal(stepped[1], stepped[2]) and torch.equal(stepped[0], stepped[1])
 
 
+def system(ctx, g, rng):
+    return (ctx.field(periodic_node_field(g, smooth_random_unique(g, rng, 0.01))),
+            ctx.field(periodic_cell_field(g, smooth_random_unique(g, rng, 0.05))),
+            ctx.field(periodic_node_field(g, smooth_random_unique(g, rng, 0.02))),
+            ctx.mass_from_records(random_mass(g, rng, dt=0.1)))
+
+
+@pytest.mark.parametrize("shapes", [((1024, 1, 1), (2, 1, 1)), ((96, 96, 1), (12, 12, 12)), ((150, 90, 1), (256, 130, 1)),
+                                    ((30, 40, 26), (33, 20, 18))], ids=lambda s: "x".join(map(str, s[0])))
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("adjoint", [False, True])
+def test_two_live_contexts_solve_in_turn(torch_cuda, shapes, precision, adjoint):
+    """The kernels' shared memory limit is one for all contexts: plans of different sizes, forward and adjoint."""
+    import torch
+    from gpu_helpers import StageContext
+    rng = np.random.default_rng(1)
+    pairs = []
+    for shape in shapes:
+        g = GridSpec(*shape, *(0.1 * n for n in shape))
+        ctx = StageContext(g, precision=precision, dt=0.1, tol=1e-10, mass_layout=1, max_iterations=300, restart=20)
+        pairs.append((ctx, system(ctx, g, rng)))
+    first = [solve(ctx, inputs, adjoint)[0] for ctx, inputs in pairs]
+    for order in (0, 1, 1, 0):
+        got, res = solve(*pairs[order], adjoint)
+        assert res.converged and torch.equal(got, first[order])
+    for ctx, _ in pairs:
+        ctx.close()
+
+
 @pytest.mark.parametrize("shape", [(1, 1, 1), (3, 1, 1), (70, 1, 1), (5, 3, 1), (40, 24, 1), (1, 33, 1), (150, 90, 1)],
                          ids=lambda s: "x".join(map(str, s)))
 @pytest.mark.parametrize("precision", [0, 1])
@@ -89,10 +118,7 @@ def test_resident_smoothed_solve_equals_the_step_graph(torch_cuda, shape, precis
     tol = 1e-10
     ctx = StageContext(g, precision=precision, dt=0.1, tol=tol, mass_layout=1, max_iterations=300, restart=20,
                        smoothing=smoothing)
-    inputs = (ctx.field(periodic_node_field(g, smooth_random_unique(g, rng, 0.01))),
-              ctx.field(periodic_cell_field(g, smooth_random_unique(g, rng, 0.05))),
-              ctx.field(periodic_node_field(g, smooth_random_unique(g, rng, 0.02))),
-              ctx.mass_from_records(random_mass(g, rng, dt=0.1)))
+    inputs = system(ctx, g, rng)
     got, res = ctx.field_solve(*inputs)
     _lib.check(ctx.lib.tpicb200_set_wait_limit(ctx.ctx, 1 << 22))
     want, ref = ctx.field_solve(*inputs)

@@ -939,6 +939,7 @@ struct SolverWorkspace {
   unsigned resident_grid = 0;
   size_t resident_bytes = 0;
   int resident_ctas = 1;
+  int shared_limit = 0;          // the device's dynamic shared memory limit of a CTA
   bool adjoint_kernels = false;  // the kernels of A^T have their limits
   double* resident_partials = nullptr;
   unsigned* resident_barrier = nullptr;
@@ -1002,7 +1003,8 @@ bool cluster_fits(void (*kernel)(ResidentPlan), int blocks, size_t bytes) {
   return clusters > 0;
 }
 
-// Raises the kernels' dynamic shared memory limit.
+// Sets the kernels' dynamic shared memory limit, one value a kernel for all
+// contexts: always the device's, so that no context takes another's away.
 bool allow_shared(void (*const (&kernels)[2])(ResidentPlan), int limit) {
   for (auto k : kernels)
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, limit) != cudaSuccess) {
@@ -1139,6 +1141,7 @@ void plan_resident(SolverWorkspace* w, int sms) {
         for (auto k : kernels[ctas - 1])
           if (!cluster_fits(k, grid, used)) p.cluster = false;
       w->resident_ctas = ctas;
+      w->shared_limit = limit;
       w->plan = p;
       w->resident_grid = unsigned(grid);
       w->resident_bytes = used;
@@ -1649,8 +1652,8 @@ struct Solve {
     typename K::Kernel kernels[2];
     K::pick(w->transpose, w->smoothing.iterations > 0, w->resident_ctas, kernels);
     if (w->transpose && !w->adjoint_kernels) {
-      // Their limits, which the plan raised for the kernels of A.
-      w->adjoint_kernels = allow_shared(kernels, int(w->resident_bytes));
+      // Their limits, which the plan set for the kernels of A.
+      w->adjoint_kernels = allow_shared(kernels, w->shared_limit);
       for (auto k : kernels)
         if (p.cluster) w->adjoint_kernels = w->adjoint_kernels && cluster_fits(k, int(w->resident_grid), w->resident_bytes);
       if (!w->adjoint_kernels) {
