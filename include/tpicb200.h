@@ -309,8 +309,13 @@ int tpicb200_read_invalid(tpicb200_context* ctx, uint32_t* count, int clear, tpi
  *   return without writing its rows; the apply adds 1 << 21 to the invalid
  *   counter.
  * tpicb200_cycle then returns TPICB200_INVALID_DATA. The grid barriers of the
- * binned sort's cooperative kernels have the default bound: one that gives up
- * adds 1 << 22 to the invalid counter. */
+ * cooperative kernels keep the default bound (but see tpicb200_inject_stall).
+ * - The binned sort: where a barrier of the plan gives up, the general sort makes
+ *   the output; where one of the general sort does, the bins come out empty
+ *   (counts and offsets zero), the output records are unfinished and the invalid
+ *   counter gets 1 << 22.
+ * - The field solve: TPICB200_BACKEND_FAILURE.
+ * Either way the next call on the context starts from clear barriers. */
 int tpicb200_set_wait_limit(tpicb200_context* ctx, uint32_t polls);
 
 /* Test of the bounded waits (tpicb200_set_wait_limit) without a fault: with
@@ -318,8 +323,19 @@ int tpicb200_set_wait_limit(tpicb200_context* ctx, uint32_t polls);
  * of chunk index - 1 (index >= 1), with TPICB200_STALL_APPLY the TMA apply's
  * wait for the mass box of stencil `index` (0..13) waits instead on an
  * mbarrier that nothing arrives on, so it gives up at its bound and takes
- * the recovery path above. TPICB200_STALL_NONE turns it off. */
-enum { TPICB200_STALL_NONE = 0, TPICB200_STALL_DEPOSIT = 1, TPICB200_STALL_APPLY = 2 };
+ * the recovery path above. With TPICB200_STALL_PLAN, TPICB200_STALL_SORT and
+ * TPICB200_STALL_SOLVE wait number `index` (>= 1) of the first CTA at the grid
+ * barrier of the binned sort's plan, of its general sort and of the resident
+ * solve's kernels is for more CTAs than there are; those waits then have the
+ * bound of tpicb200_set_wait_limit. TPICB200_STALL_NONE turns it off. */
+enum {
+  TPICB200_STALL_NONE = 0,
+  TPICB200_STALL_DEPOSIT = 1,
+  TPICB200_STALL_APPLY = 2,
+  TPICB200_STALL_PLAN = 3,
+  TPICB200_STALL_SORT = 4,
+  TPICB200_STALL_SOLVE = 5
+};
 int tpicb200_inject_stall(tpicb200_context* ctx, int site, uint32_t index);
 
 /* Zero J (node field) and the mass records. Replaces enqueue_clear_mass_matrix

@@ -16,7 +16,7 @@ NOT_CONVERGED, CAPACITY_EXCEEDED, INVALID_DATA = 5, 6, 7
 PRECISION_DOUBLE, PRECISION_MIXED = 0, 1
 MASS_SCALAR, MASS_SCALAR_F64, MASS_TF32, MASS_BF16X3, MASS_MOMENTS_F64 = 0, 1, 2, 3, 4
 MASS_LAYOUT_RECORDS, MASS_LAYOUT_STENCIL_MAJOR, MASS_LAYOUT_TILED = 0, 1, 2
-STALL_NONE, STALL_DEPOSIT, STALL_APPLY = 0, 1, 2
+STALL_NONE, STALL_DEPOSIT, STALL_APPLY, STALL_PLAN, STALL_SORT, STALL_SOLVE = range(6)
 MAX_SPECIES = 8
 
 MASS_KINDS = {"scalar": MASS_SCALAR, "scalar-f64": MASS_SCALAR_F64, "fp64": MASS_SCALAR_F64,

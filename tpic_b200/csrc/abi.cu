@@ -96,6 +96,14 @@ int check_mass_kind(const tpicb200_context* ctx, int kind) {
   return TPICB200_SUCCESS;
 }
 
+BinnedScratch sort_scratch(const tpicb200_context* ctx) {
+  auto waits = [&](int site) {
+    return ctx->stall_site != site ? GridWaits{kGridBarrierPolls, 0}
+                                   : GridWaits{ctx->wait_polls ? ctx->wait_polls : kGridBarrierPolls, ctx->stall_index};
+  };
+  return binned_scratch(ctx->g, ctx->binned, ctx->codes, waits(TPICB200_STALL_PLAN), waits(TPICB200_STALL_SORT));
+}
+
 cudaError_t launch_moments(tpicb200_context* ctx, int kind, int ns, const double* qom,
                            const tpicb200_particles* const* parts, const uint32_t* const* counts,
                            const uint32_t* const* offsets, const void* b_node, int accumulate, uint32_t* invalid,
@@ -245,7 +253,7 @@ int tpicb200_create(const tpicb200_grid* grid, const tpicb200_options* options, 
   alloc((void**)&ctx->moments, moment_floats(ctx->g) * (options->precision == TPICB200_PRECISION_MIXED ? 4 : 8));
   if (e == cudaSuccess) e = cudaMallocHost((void**)&ctx->pinned, (2 + 5 * TPICB200_MAX_SPECIES + 2) * 8);
   if (e == cudaSuccess) e = cudaMemset(ctx->invalid, 0, 4);
-  if (e == cudaSuccess) e = binned_reset(binned_scratch(ctx->g, ctx->binned, ctx->codes));
+  if (e == cudaSuccess) e = binned_reset(sort_scratch(ctx));
   if (e == cudaSuccess && ctx->solver) solver_set_invalid(ctx->solver, ctx->invalid);
   for (auto& ev : ctx->events)
     if (e == cudaSuccess) e = cudaEventCreate(&ev);
@@ -331,7 +339,7 @@ int tpicb200_sort_binned(tpicb200_context* ctx, const tpicb200_particles* in, co
   if (in->count && (in->rx == out->rx || in->cell == out->cell))
     return fail(TPICB200_INVALID_ARGUMENT, "sort input and output alias");
   return cuda_status(launch_sort_binned(ctx->opt.precision, ctx->g, in, in_counts, in_offsets, out, counts, offsets,
-                                        ctx->cursor, ctx->perm, ctx->scan, ctx->binned, ctx->codes,
+                                        ctx->cursor, ctx->perm, ctx->scan, sort_scratch(ctx),
                                         invalid_or_own(ctx, invalid),
                                         (cudaStream_t)stream),
                      "binned sort launch failed");
@@ -692,7 +700,7 @@ static int move_and_sort(tpicb200_context* ctx, tpicb200_state* st, int sp, uint
     *plan = DepositPlan{out, SortedCopy{nullptr, none}, true};
     return TPICB200_SUCCESS;
   }
-  const BinnedScratch b = binned_scratch(ctx->g, ctx->binned, ctx->codes);
+  const BinnedScratch b = sort_scratch(ctx);
   cudaError_t e = binned_begin(ctx->g, b, in->count, st->counts[sp], st->offsets[sp], true, s);
   const bool ranks = st->ranks[sp] != nullptr;
   if (ranks) {
@@ -805,11 +813,16 @@ static int read_invalid(tpicb200_context* ctx, cudaStream_t s, uint32_t* value) 
   return TPICB200_SUCCESS;
 }
 
+static void set_solver_waits(tpicb200_context* ctx) {
+  if (ctx->solver)
+    solver_set_waits(ctx->solver, ctx->wait_polls, ctx->stall_site == TPICB200_STALL_APPLY ? int(ctx->stall_index) : -1,
+                     ctx->stall_site == TPICB200_STALL_SOLVE ? ctx->stall_index : 0u);
+}
+
 int tpicb200_set_wait_limit(tpicb200_context* ctx, uint32_t polls) {
   if (int s = check_ctx(ctx)) return s;
   ctx->wait_polls = polls;
-  if (ctx->solver)
-    solver_set_waits(ctx->solver, polls, ctx->stall_site == TPICB200_STALL_APPLY ? int(ctx->stall_index) : -1);
+  set_solver_waits(ctx);
   return TPICB200_SUCCESS;
 }
 
@@ -821,12 +834,14 @@ int tpicb200_inject_stall(tpicb200_context* ctx, int site, uint32_t index) {
     if (index < 1) return fail(TPICB200_INVALID_ARGUMENT, "the deposition stall index is a chunk >= 1");
   } else if (site == TPICB200_STALL_APPLY) {
     if (index > 13) return fail(TPICB200_INVALID_ARGUMENT, "the apply stall index is a stencil 0..13");
+  } else if (site == TPICB200_STALL_PLAN || site == TPICB200_STALL_SORT || site == TPICB200_STALL_SOLVE) {
+    if (index < 1) return fail(TPICB200_INVALID_ARGUMENT, "the barrier stall index is a wait >= 1");
   } else {
     return fail(TPICB200_INVALID_ARGUMENT, "unknown stall site");
   }
   ctx->stall_site = site;
   ctx->stall_index = index;
-  if (ctx->solver) solver_set_waits(ctx->solver, ctx->wait_polls, site == TPICB200_STALL_APPLY ? int(index) : -1);
+  set_solver_waits(ctx);
   return TPICB200_SUCCESS;
 }
 

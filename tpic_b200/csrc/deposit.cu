@@ -441,8 +441,10 @@ namespace {
 __global__ void __launch_bounds__(256) copy_ids_kernel(const uint32_t* __restrict__ perm,
                                                        const uint64_t* __restrict__ in, uint64_t* __restrict__ out,
                                                        uint32_t count) {
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < count; p += gridDim.x * blockDim.x)
-    out[p] = in[perm[p]];
+  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < count; p += gridDim.x * blockDim.x) {
+    const uint32_t n = perm[p];
+    if (n < count) out[p] = in[n];
+  }
 }
 }  // namespace
 

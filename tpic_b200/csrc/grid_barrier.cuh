@@ -1,8 +1,11 @@
 // A barrier over all CTAs of a cooperative launch, with bounded waits.
 //
-// Two words, zero between launches: arrivals and departures; the last CTA to
-// leave zeroes both. A CTA whose poll runs out reports false to its threads,
-// which leave the kernel; the other CTAs then run out at their next barrier.
+// Three words, zero between launches: arrivals, departures and whether a wait
+// gave up. A CTA whose polls run out reports false to its threads, which go to
+// leave(); the others then run out at their next wait. Every CTA leaves, and the
+// last one to do so zeroes the words, so a launch that failed spoils none after
+// it; that CTA also learns of the failure and can put the outputs in order, all
+// the other CTAs' writes being done.
 #pragma once
 
 #include "common.cuh"
@@ -10,6 +13,13 @@
 namespace tpicb200 {
 
 constexpr uint32_t kGridBarrierPolls = 1u << 22;
+constexpr int kGridBarrierWords = 3;
+
+// The bound of a barrier's waits, and for tests the wait (from 1) at which CTA
+// 0 expects more arrivals than there ever are (0: none).
+struct GridWaits {
+  uint32_t polls, stall;
+};
 
 __device__ __forceinline__ uint32_t load_acquire(const unsigned* p) {
   uint32_t v;
@@ -19,29 +29,44 @@ __device__ __forceinline__ uint32_t load_acquire(const unsigned* p) {
 
 struct GridBarrier {
   unsigned* words;
-  uint32_t arrivals = 0;
+  GridWaits waits;
+  uint32_t arrivals = 0, number = 0;
   bool failed = false;
-  __device__ explicit GridBarrier(unsigned* w) : words(w) {}
+  __device__ GridBarrier(unsigned* w, GridWaits limits) : words(w), waits(limits) {}
 
   // Every thread of every CTA; false when it gave up (for the whole CTA).
   __device__ __forceinline__ bool wait() {
     __syncthreads();
     if (threadIdx.x == 0) {
       arrivals += gridDim.x;
+      ++number;
+      const uint32_t expected = number == waits.stall && blockIdx.x == 0 ? 0xffffffffu : arrivals;
       // The CTA's writes are ordered before the arrival (the barrier above and
       // the release), the others' before what follows the acquire.
       asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(words) : "memory");
       uint32_t poll = 0;
-      while (load_acquire(words) < arrivals && poll < kGridBarrierPolls) ++poll;
-      failed = poll == kGridBarrierPolls;
+      while (load_acquire(words) < expected && poll < waits.polls) ++poll;
+      failed = poll == waits.polls;
     }
     return !__syncthreads_or(failed);
   }
-  __device__ __forceinline__ void leave() {
-    if (threadIdx.x == 0 && !failed && atomicAdd(words + 1, 1u) == gridDim.x - 1) {
-      words[0] = 0;
-      words[1] = 0;
+
+  // Every thread of every CTA, once, on every way out of the kernel.
+  enum Exit { kOther, kLast, kLastOfFailed };
+  __device__ __forceinline__ Exit leave() {
+    __syncthreads();
+    int exit = kOther;
+    if (threadIdx.x == 0) {
+      if (failed) atomicExch(words + 2, 1u);
+      __threadfence();
+      if (atomicAdd(words + 1, 1u) == gridDim.x - 1) {
+        __threadfence();
+        exit = load_acquire(words + 2) ? kLastOfFailed : kLast;
+        words[0] = words[1] = words[2] = 0;
+      }
     }
+    const bool last = __syncthreads_or(exit != kOther), any_failed = __syncthreads_or(exit == kLastOfFailed);
+    return any_failed ? kLastOfFailed : last ? kLast : kOther;
   }
 };
 

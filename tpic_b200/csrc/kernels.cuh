@@ -3,6 +3,7 @@
 
 #include "cases.cuh"
 #include "common.cuh"
+#include "grid_barrier.cuh"
 
 #include <string>
 
@@ -60,9 +61,10 @@ cudaError_t launch_sort(int precision, const Geom& g, const tpicb200_particles* 
 // The state is zero between sorts: the last kernel of a sort that raised a flag
 // clears it (binned_reset at the context's creation).
 struct BinnedState {
-  uint32_t fallback;    // nonzero: the general sort produces the output
-  uint32_t bins_bad;    // nonzero: the old bins do not tile the records
-  uint32_t barrier[2];  // grid barrier of the cooperative kernels
+  uint32_t fallback;                    // nonzero: the general sort produces the output
+  uint32_t bins_bad;                    // nonzero: the old bins do not tile the records
+  uint32_t barrier[kGridBarrierWords];  // grid barrier of the cooperative kernels
+  uint32_t pad[3];
 };
 struct BinnedScratch {
   BinnedState* state;
@@ -70,10 +72,12 @@ struct BinnedScratch {
   uint32_t* old_offsets;
   uint32_t* transfer;     // [27][interior cells]: counts, then output bases
   uint16_t* code;         // run code per record (direction, cell in run; kNoMove)
+  GridWaits plan_waits, sort_waits;  // of the cooperative kernels
 };
 size_t binned_scratch_words(const Geom& g);
 bool binned_sort_applies(const Geom& g);
-BinnedScratch binned_scratch(const Geom& g, uint32_t* words, uint16_t* codes);
+BinnedScratch binned_scratch(const Geom& g, uint32_t* words, uint16_t* codes, GridWaits plan_waits,
+                             GridWaits sort_waits);
 cudaError_t binned_reset(const BinnedScratch& b);
 // Copies the input's bins, checks that they tile the n records in key order
 // (else raises bins_bad and fallback) and clears the transfer counts when the
@@ -83,7 +87,10 @@ cudaError_t binned_begin(const Geom& g, const BinnedScratch& b, uint32_t n, cons
 // (Classification when `classify`), counts, scan, bases, the ranks (perm:
 // sorted position -> input record), the gather of the sorted records when
 // `materialize`, and the gated general sort (which always writes `out` and
-// the same perm); binned_begin must have run.
+// the same perm); binned_begin must have run. A grid barrier of the counts, scan
+// and bases that gives up raises the fallback flag; one of the general sort adds
+// 1 << 22 to *invalid and empties the bins (counts and offsets zero), since perm
+// and the output records are then unfinished: perm may hold anything.
 cudaError_t binned_finish(int precision, const Geom& g, const BinnedScratch& b, bool classify, bool materialize,
                           const tpicb200_particles* in, tpicb200_particles* out, uint32_t* counts,
                           uint32_t* offsets, uint32_t* cursor, uint32_t* perm, uint32_t* scan_scratch,
@@ -91,8 +98,7 @@ cudaError_t binned_finish(int precision, const Geom& g, const BinnedScratch& b, 
 cudaError_t launch_sort_binned(int precision, const Geom& g, const tpicb200_particles* in,
                                const uint32_t* in_counts, const uint32_t* in_offsets, tpicb200_particles* out,
                                uint32_t* counts, uint32_t* offsets, uint32_t* cursor, uint32_t* perm,
-                               uint32_t* scan_scratch, uint32_t* binned_words, uint16_t* codes,
-                               uint32_t* invalid, cudaStream_t s);
+                               uint32_t* scan_scratch, const BinnedScratch& b, uint32_t* invalid, cudaStream_t s);
 
 // Context-free sort on the file-scope scratch array (no allocation): the
 // first call on a device resolves the array's address (sort_static_setup).
@@ -111,10 +117,12 @@ struct SortedCopy {
   tpicb200_particles out;
 };
 // Writes out.id[p] = in.id[perm[p]] for the records a fused deposition
-// copied (the deposition kernels copy every other attribute).
+// copied (the deposition kernels copy every other attribute); entries of perm
+// that are no record (a failed sort's) are passed over.
 cudaError_t launch_copy_ids(const tpicb200_particles* in, const SortedCopy* copy, cudaStream_t s);
 
-// Sorted records: out[p] = in[perm[p]] for every attribute (ids included).
+// Sorted records: out[p] = in[perm[p]] for every attribute (ids included);
+// entries of perm that are no record (a failed sort's) are passed over.
 cudaError_t launch_sorted_gather(int precision, const uint32_t* perm, const tpicb200_particles* in,
                                  tpicb200_particles* out, cudaStream_t s);
 
@@ -249,8 +257,10 @@ int solver_solve_adjoint(SolverWorkspace* w, const double* rhs, const void* mass
 void solver_set_invalid(SolverWorkspace* w, uint32_t* invalid);
 // Bound of the TMA apply's copy waits (0: kDefaultWaitPolls); stall_stencil
 // in 0..13 makes the wait for that stencil's box wait on an mbarrier that
-// nothing arrives on (a test of the bound), -1 none.
-void solver_set_waits(SolverWorkspace* w, uint32_t polls, int stall_stencil);
+// nothing arrives on (a test of the bound), -1 none. stall_barrier: the wait of
+// the resident kernels' grid barrier that is to give up, at the bound `polls`
+// (0: none).
+void solver_set_waits(SolverWorkspace* w, uint32_t polls, int stall_stencil, uint32_t stall_barrier);
 int solver_solve(SolverWorkspace* w, const void* e, const void* bcell, const void* j,
                  const void* mass, double* etheta, tpicb200_gmres_result* result,
                  int max_iterations, double tol, cudaStream_t s, cudaError_t* err);

@@ -324,6 +324,10 @@ __global__ void __launch_bounds__(256, TPICB200_MOVER_MIN_BLOCKS) mover_kernel(G
   const Records<P>& r = io.in;
   for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < count; p += gridDim.x * blockDim.x) {
     const uint32_t n = io.ranks ? io.ranks[p] : p;
+    if (n >= count) {  // ranks of a sort that failed
+      atomicAdd(invalid, 1u);
+      continue;
+    }
     const int32_t k0 = r.key[n];
     const double charge = r.q[n];
     const Pos fx = r.rx[n], fy = r.ry[n], fz = r.rz[n];

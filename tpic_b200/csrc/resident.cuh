@@ -38,9 +38,11 @@
 //
 // A grid of at most 16 tiles is launched as one cluster, whose hardware barrier
 // takes the place of the grid barrier. Otherwise the launch is cooperative
-// (all CTAs resident). A barrier that does not
+// (all CTAs resident). A grid barrier that does not
 // complete within its polls makes its CTA set ctl->failed and leave; the
-// others then run out at theirs, and the solve fails.
+// others then run out at theirs, and the solve fails. The cluster barrier is
+// the hardware's: a cluster's CTAs start together, and one that has left is not
+// waited for.
 #pragma once
 
 #include "common.cuh"
@@ -85,7 +87,8 @@ struct ResidentPlan {
   double* values;          // |r|^2 and (start) |b|^2
   double* partials;        // kResidentRestart + 2 rows of gridDim.x
   ArnoldiControl* ctl;
-  unsigned* barrier;       // arrivals, departures (zero between launches)
+  unsigned* barrier;       // kGridBarrierWords
+  GridWaits waits;
   int restart, columns;
   double tolerance;        // of this cycle's residual estimate
   double accept;           // start: the relative tolerance; cycle: the absolute one
@@ -154,7 +157,7 @@ struct Resident {
   GridBarrier barrier;
 
   __device__ Resident(const ResidentPlan& plan, uint8_t* s)
-      : p(plan), smem(s), L(resident_shared(plan, sizeof(S))), barrier(plan.barrier) {}
+      : p(plan), smem(s), L(resident_shared(plan, sizeof(S))), barrier(plan.barrier, plan.waits) {}
 
   template <class T> __device__ __forceinline__ T* at(size_t offset) const { return reinterpret_cast<T*>(smem + offset); }
   __device__ __forceinline__ long long unique() const { return (long long)p.g.nx * p.g.ny * p.g.nz; }
@@ -172,7 +175,8 @@ struct Resident {
     k0 *= p.tz;
   }
 
-  // All CTAs of the grid. False when it gave up (for every thread of the CTA).
+  // All CTAs of the grid. False when it gave up (for every thread of the CTA),
+  // which has then left and ends.
   __device__ bool grid_barrier() {
     if (p.cluster) {
       asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
@@ -180,6 +184,7 @@ struct Resident {
     }
     if (barrier.wait()) return true;
     if (threadIdx.x == 0) p.ctl->failed = 1;
+    barrier.leave();
     return false;
   }
   __device__ void leave() {

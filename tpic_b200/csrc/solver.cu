@@ -886,6 +886,7 @@ struct SolverWorkspace {
   bool transpose = false;       // applies use A^T (every mass block transposed): the adjoint solve
   uint32_t* invalid = nullptr;  // the context's invalid counter (smoothing passes, TMA apply waits)
   uint32_t wait_polls = 0;      // TMA apply wait bound (0: kDefaultWaitPolls)
+  uint32_t stall_barrier = 0;   // the same for the resident kernels' grid barrier
   int stall_stencil = -1;       // a test of that bound: the stencil whose wait targets no copy
   Geom g;
   int restart;
@@ -1211,8 +1212,8 @@ SolverWorkspace* solver_create(int precision, const Geom& g, int restart, double
   if (e == cudaSuccess) e = cudaMemset(w->rhs, 0, 3 * g.nodes * sizeof(double));
   if (w->resident) {
     alloc((void**)&w->resident_partials, size_t(kResidentRestart + 2) * w->resident_grid * sizeof(double));
-    alloc((void**)&w->resident_barrier, 2 * sizeof(unsigned));
-    if (e == cudaSuccess) e = cudaMemset(w->resident_barrier, 0, 2 * sizeof(unsigned));
+    alloc((void**)&w->resident_barrier, kGridBarrierWords * sizeof(unsigned));
+    if (e == cudaSuccess) e = cudaMemset(w->resident_barrier, 0, kGridBarrierWords * sizeof(unsigned));
     if (e == cudaSuccess) e = cudaMemset(w->ctl, 0, sizeof(ArnoldiControl));
   }
   *err = e;
@@ -1599,9 +1600,9 @@ struct Solve {
   }
 
   // The resident kernels (resident.cuh): one launch for the start and one per
-  // restart cycle. Not while a wait bound or a stall is set: those act on the
-  // applies of the step graph.
-  bool resident() const { return w->resident && w->wait_polls == 0 && w->stall_stencil < 0; }
+  // restart cycle. Not while a wait bound or an apply's stall is set: those act on
+  // the applies of the step graph; with a stall of the barriers the bound is theirs.
+  bool resident() const { return w->resident && (w->stall_barrier || w->wait_polls == 0) && w->stall_stencil < 0; }
   // Launches one of them and reads its outcome back; false on a failure.
   bool launch_resident(typename ResidentKernels<P>::Kernel kernel, double controls[2], ArnoldiControl* control) {
     ResidentPlan p = w->plan;
@@ -1616,9 +1617,8 @@ struct Solve {
     count_launches(1);
     if (!read_back(w->values, controls, control)) return false;
     if (control->failed) {
-      // A barrier ran out of polls: the next solve starts from clear counters.
+      // A barrier ran out of polls; its words are clear again (GridBarrier).
       cudaMemsetAsync(w->ctl, 0, sizeof(ArnoldiControl), s);
-      cudaMemsetAsync(w->resident_barrier, 0, 2 * sizeof(unsigned), s);
       err = cudaErrorLaunchTimeout;
       return false;
     }
@@ -1638,6 +1638,7 @@ struct Solve {
     p.partials = w->resident_partials;
     p.ctl = w->ctl;
     p.barrier = w->resident_barrier;
+    p.waits = GridWaits{w->wait_polls ? w->wait_polls : kGridBarrierPolls, w->stall_barrier};
     p.e = e;
     p.bcell = bcell;
     p.j = j;
@@ -1816,7 +1817,8 @@ int solver_solve(SolverWorkspace* w, const void* e, const void* bcell, const voi
 
 void solver_set_invalid(SolverWorkspace* w, uint32_t* invalid) { w->invalid = invalid; }
 
-void solver_set_waits(SolverWorkspace* w, uint32_t polls, int stall_stencil) {
+void solver_set_waits(SolverWorkspace* w, uint32_t polls, int stall_stencil, uint32_t stall_barrier) {
+  w->stall_barrier = stall_barrier;
   if (polls == w->wait_polls && stall_stencil == w->stall_stencil) return;
   w->wait_polls = polls;
   w->stall_stencil = stall_stencil;

@@ -341,28 +341,26 @@ struct SortRecords {
         oq(out->q), okey(out->cell), oid(in->id ? out->id : nullptr) {}
 };
 template <class Vel>
-__device__ __forceinline__ void gather(const uint32_t* perm, uint32_t count, const SortRecords<Vel>& r) {
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < count; p += gridDim.x * blockDim.x) {
-    const uint32_t s = perm[p];
-    const double x = __ldg(r.irx + s), y = __ldg(r.iry + s), z = __ldg(r.irz + s), q = __ldg(r.iq + s);
-    const Vel u = __ldg(r.iu + s), v = __ldg(r.iv + s), w = __ldg(r.iw + s);
-    const int32_t key = __ldg(r.ikey + s);
-    r.orx[p] = x;
-    r.ory[p] = y;
-    r.orz[p] = z;
-    r.ou[p] = u;
-    r.ov[p] = v;
-    r.ow[p] = w;
-    r.oq[p] = q;
-    r.okey[p] = key;
-    if (r.oid) r.oid[p] = r.iid[s];
-  }
+__device__ __forceinline__ void gather(uint32_t s, uint32_t p, const SortRecords<Vel>& r) {
+  const double x = __ldg(r.irx + s), y = __ldg(r.iry + s), z = __ldg(r.irz + s), q = __ldg(r.iq + s);
+  const Vel u = __ldg(r.iu + s), v = __ldg(r.iv + s), w = __ldg(r.iw + s);
+  const int32_t key = __ldg(r.ikey + s);
+  r.orx[p] = x;
+  r.ory[p] = y;
+  r.orz[p] = z;
+  r.ou[p] = u;
+  r.ov[p] = v;
+  r.ow[p] = w;
+  r.oq[p] = q;
+  r.okey[p] = key;
+  if (r.oid) r.oid[p] = r.iid[s];
 }
 template <class Vel>
 __global__ void __launch_bounds__(256) gather_kernel(const uint32_t* __restrict__ perm, uint32_t count,
                                                      SortRecords<Vel> r, const uint32_t* flag) {
   if (flag && *flag) return;
-  gather(perm, count, r);
+  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < count; p += gridDim.x * blockDim.x)
+    if (perm[p] < count) gather(perm[p], p, r);
 }
 cudaError_t launch_gather(int precision, const uint32_t* perm, const tpicb200_particles* in, tpicb200_particles* out,
                           const uint32_t* flag, cudaStream_t s) {
@@ -480,36 +478,20 @@ __device__ __forceinline__ void coop_scan(const uint32_t* counts, long long bins
   if (b1 == bins && b0 < b1 && threadIdx.x == 0) offsets[bins] = running;
 }
 
-// A grid barrier that gave up counts 1 << 22 in *invalid.
-__device__ __forceinline__ bool coop_wait(GridBarrier& barrier, uint32_t* invalid) {
-  if (barrier.wait()) return true;
-  if (threadIdx.x == 0 && invalid) atomicAdd(invalid, 1u << 22);
-  return false;
-}
-
-// The general sort in one launch, for the binned sort's fallback: enqueued
-// behind every binned sort and leaving at once unless the fallback flag is up.
-// As the general sort's eleven kernels it cost 25 us of empty launches per
-// species and cycle. Its steps are separated by grid barriers; at the end the
-// flags are cleared for the next sort.
+// The steps of the general sort by all CTAs; returns early where a barrier gives up.
 template <class Vel>
-__global__ void __launch_bounds__(kCoopThreads, 2) fallback_sort_kernel(Geom g, uint32_t n, SortRecords<Vel> r,
-                                                                        uint32_t* counts, uint32_t* offsets,
-                                                                        uint32_t* cursor, uint32_t* perm,
-                                                                        ScanScratch sc, uint32_t* invalid,
-                                                                        BinnedState* state) {
-  __shared__ uint32_t buffer[kBlockBinCapacity];
-  __shared__ uint32_t scratch[kCoopThreads / 32];
-  if (state->fallback == 0) return;
-  GridBarrier barrier(state->barrier);
+__device__ __forceinline__ void fallback_sort(const Geom& g, uint32_t n, const SortRecords<Vel>& r, uint32_t* counts,
+                                              uint32_t* offsets, uint32_t* cursor, uint32_t* perm,
+                                              const ScanScratch& sc, uint32_t* invalid, GridBarrier& barrier,
+                                              uint32_t* buffer, uint32_t* scratch) {
   uint32_t* sums = sc.large_bins;  // free until the fix-up
   for (long long b = blockIdx.x * (long long)kCoopThreads + threadIdx.x; b < g.bins;
        b += (long long)gridDim.x * kCoopThreads)
     counts[b] = 0;
   if (blockIdx.x == 0 && threadIdx.x == 0) *sc.flag = *sc.large_count = 0;
-  if (!coop_wait(barrier, invalid)) return;
+  if (!barrier.wait()) return;
   histogram(g, r.ikey, n, counts, sc.flag);
-  if (!coop_wait(barrier, invalid)) return;
+  if (!barrier.wait()) return;
   const bool bad = __ldcg(sc.flag) != 0;
   if (!bad) {
     long long b0, b1;
@@ -518,29 +500,56 @@ __global__ void __launch_bounds__(kCoopThreads, 2) fallback_sort_kernel(Geom g, 
     for (long long b = b0 + threadIdx.x; b < b1; b += kCoopThreads) sum += __ldcg(counts + b);
     sum = block_sum<kCoopThreads>(sum, scratch);
     if (threadIdx.x == 0) sums[blockIdx.x] = sum;
-    if (!coop_wait(barrier, invalid)) return;
+    if (!barrier.wait()) return;
     coop_scan(counts, g.bins, sums, offsets, cursor);
-    if (!coop_wait(barrier, invalid)) return;
+    if (!barrier.wait()) return;
     place(r.ikey, n, cursor, perm);
-    if (!coop_wait(barrier, invalid)) return;
+    if (!barrier.wait()) return;
     fixup_small(counts, offsets, g.bins, perm, sc.large_count, sc.large_bins,
                 reinterpret_cast<uint32_t (*)[kWarpBinCapacity]>(buffer));
-    if (!coop_wait(barrier, invalid)) return;
+    if (!barrier.wait()) return;
     fixup_large(counts, offsets, perm, (uint32_t*)r.okey, sc.large_count, sc.large_bins, buffer);
-    if (!coop_wait(barrier, invalid)) return;
-    gather(perm, n, r);
+    if (!barrier.wait()) return;
+    for (uint32_t p = blockIdx.x * kCoopThreads + threadIdx.x; p < n; p += gridDim.x * kCoopThreads)
+      gather(perm[p], p, r);
   } else if (blockIdx.x == 0 && threadIdx.x == 0 && invalid) {
     atomicAdd(invalid, 1u);
   }
-  if (!coop_wait(barrier, invalid)) return;
-  if (blockIdx.x == 0 && threadIdx.x == 0) state->fallback = state->bins_bad = 0;
-  barrier.leave();
+}
+
+// The general sort in one launch, for the binned sort's fallback: enqueued
+// behind every binned sort and leaving at once unless the fallback flag is up.
+// As the general sort's eleven kernels it cost 25 us of empty launches per
+// species and cycle. Its steps are separated by grid barriers; the last CTA to
+// leave clears the flags for the next sort. Where a barrier gave up, perm and the
+// records are unfinished: that CTA then empties the bins, so that nothing reads
+// through them, and counts 1 << 22 in *invalid.
+template <class Vel>
+__global__ void __launch_bounds__(kCoopThreads, 2) fallback_sort_kernel(Geom g, uint32_t n, SortRecords<Vel> r,
+                                                                        uint32_t* counts, uint32_t* offsets,
+                                                                        uint32_t* cursor, uint32_t* perm,
+                                                                        ScanScratch sc, uint32_t* invalid,
+                                                                        BinnedState* state, GridWaits waits) {
+  __shared__ uint32_t buffer[kBlockBinCapacity];
+  __shared__ uint32_t scratch[kCoopThreads / 32];
+  if (state->fallback == 0) return;
+  GridBarrier barrier(state->barrier, waits);
+  fallback_sort(g, n, r, counts, offsets, cursor, perm, sc, invalid, barrier, buffer, scratch);
+  const GridBarrier::Exit exit = barrier.leave();
+  if (exit == GridBarrier::kLastOfFailed) {
+    for (long long b = threadIdx.x; b <= g.bins; b += kCoopThreads) {
+      if (b < g.bins) counts[b] = 0;
+      offsets[b] = 0;
+    }
+    if (threadIdx.x == 0 && invalid) atomicAdd(invalid, 1u << 22);
+  }
+  if (exit != GridBarrier::kOther && threadIdx.x == 0) state->fallback = state->bins_bad = 0;
 }
 
 template <class Vel>
 cudaError_t launch_fallback(const Geom& g, const tpicb200_particles* in, tpicb200_particles* out, uint32_t* counts,
                             uint32_t* offsets, uint32_t* cursor, uint32_t* perm, uint32_t* scan_scratch,
-                            uint32_t* invalid, BinnedState* state, cudaStream_t s) {
+                            uint32_t* invalid, BinnedState* state, GridWaits waits, cudaStream_t s) {
   const int nblocks = int((g.bins + kScanTile - 1) / kScanTile);
   ScanScratch sc{scan_scratch, scan_scratch + nblocks, scan_scratch + nblocks + 1, scan_scratch + nblocks + 2};
   Geom geom = g;
@@ -550,7 +559,7 @@ cudaError_t launch_fallback(const Geom& g, const tpicb200_particles* in, tpicb20
   // their sums must fit the bins' scratch.
   const long long work = std::max<long long>(g.bins, n);
   const unsigned blocks = unsigned(std::min<long long>(grid_for(work, 4 * kCoopThreads, 148u * 2u), g.bins));
-  void* args[] = {&geom, &n, &r, &counts, &offsets, &cursor, &perm, &sc, &invalid, &state};
+  void* args[] = {&geom, &n, &r, &counts, &offsets, &cursor, &perm, &sc, &invalid, &state, &waits};
   count_launches(1);
   return cudaLaunchCooperativeKernel((const void*)fallback_sort_kernel<Vel>, dim3(blocks), dim3(kCoopThreads), args, 0,
                                      s);
@@ -790,16 +799,9 @@ __device__ __forceinline__ void binned_bases(const Geom& g, const uint32_t* offs
   }
 }
 
-// Counts, their scan and the bases in one launch, the passes separated by grid
-// barriers. As five kernels they were launch latency on small grids (127 x 65
-// x 1 FP64 particle stage 125 us, 111 us with one) and no faster on large ones
-// (128^3 cycle 27.1 ms, 26.8 ms with one).
-__global__ void __launch_bounds__(kCoopThreads, 2) binned_plan_kernel(Geom g, uint32_t* transfer, uint32_t* counts,
-                                                                      uint32_t* offsets, uint32_t* sums,
-                                                                      uint32_t* invalid, BinnedState* state) {
-  __shared__ uint32_t scratch[kCoopThreads / 32];
-  if (state->fallback) return;
-  GridBarrier barrier(state->barrier);
+// The plan by all CTAs; returns early where a barrier gives up.
+__device__ __forceinline__ void binned_plan(const Geom& g, uint32_t* transfer, uint32_t* counts, uint32_t* offsets,
+                                            uint32_t* sums, GridBarrier& barrier, uint32_t* scratch) {
   long long b0, b1;
   coop_range(g.bins, b0, b1);
   uint32_t sum = 0;
@@ -810,11 +812,25 @@ __global__ void __launch_bounds__(kCoopThreads, 2) binned_plan_kernel(Geom g, ui
   }
   sum = block_sum<kCoopThreads>(sum, scratch);
   if (threadIdx.x == 0) sums[blockIdx.x] = sum;
-  if (!coop_wait(barrier, invalid)) return;
+  if (!barrier.wait()) return;
   coop_scan(counts, g.bins, sums, offsets, nullptr);
-  if (!coop_wait(barrier, invalid)) return;
+  if (!barrier.wait()) return;
   binned_bases(g, offsets, transfer);
-  barrier.leave();
+}
+
+// Counts, their scan and the bases in one launch, the passes separated by grid
+// barriers; where one gives up the last CTA to leave raises the fallback flag.
+// As five kernels they were launch latency on small grids (127 x 65
+// x 1 FP64 particle stage 125 us, 111 us with one) and no faster on large ones
+// (128^3 cycle 27.1 ms, 26.8 ms with one).
+__global__ void __launch_bounds__(kCoopThreads, 2) binned_plan_kernel(Geom g, uint32_t* transfer, uint32_t* counts,
+                                                                      uint32_t* offsets, uint32_t* sums,
+                                                                      BinnedState* state, GridWaits waits) {
+  __shared__ uint32_t scratch[kCoopThreads / 32];
+  if (state->fallback) return;
+  GridBarrier barrier(state->barrier, waits);
+  binned_plan(g, transfer, counts, offsets, sums, barrier, scratch);
+  if (barrier.leave() == GridBarrier::kLastOfFailed && threadIdx.x == 0) state->fallback = 1;
 }
 
 // The lane mask of a live lane's slot: the live lanes with the same slot
@@ -915,7 +931,7 @@ cudaError_t launch_sorted_gather(int precision, const uint32_t* perm, const tpic
 
 size_t binned_scratch_words(const Geom& g) {
   const long long cells = (long long)g.nx * g.ny * g.nz;
-  return 4 + size_t(2 * g.bins + 1) + size_t(27 * cells);
+  return sizeof(BinnedState) / 4 + size_t(2 * g.bins + 1) + size_t(27 * cells);
 }
 
 // Every periodic grid: on an axis of one or two cells each (source, destination)
@@ -924,10 +940,13 @@ size_t binned_scratch_words(const Geom& g) {
 // directions sharing a source.
 bool binned_sort_applies(const Geom& g) { return g.nx >= 1 && g.ny >= 1 && g.nz >= 1; }
 
-BinnedScratch binned_scratch(const Geom& g, uint32_t* words, uint16_t* codes) {
+BinnedScratch binned_scratch(const Geom& g, uint32_t* words, uint16_t* codes, GridWaits plan_waits,
+                             GridWaits sort_waits) {
   BinnedScratch b;
-  b.state = reinterpret_cast<BinnedState*>(words);  // 4 words, 8-byte aligned
-  b.old_counts = words + 4;
+  b.plan_waits = plan_waits;
+  b.sort_waits = sort_waits;
+  b.state = reinterpret_cast<BinnedState*>(words);
+  b.old_counts = words + sizeof(BinnedState) / 4;
   b.old_offsets = b.old_counts + g.bins;
   b.transfer = b.old_offsets + g.bins + 1;
   b.code = codes;
@@ -966,7 +985,8 @@ cudaError_t binned_finish(int precision, const Geom& g, const BinnedScratch& b, 
     Geom geom = g;
     uint32_t *transfer = b.transfer, *sums = sc.large_bins;
     BinnedState* state = b.state;
-    void* args[] = {&geom, &transfer, &counts, &offsets, &sums, &invalid, &state};
+    GridWaits waits = b.plan_waits;
+    void* args[] = {&geom, &transfer, &counts, &offsets, &sums, &state, &waits};
     const unsigned blocks = unsigned(std::min<long long>(grid_for(bins, kCoopThreads, 148u * 2u), bins));
     e = cudaLaunchCooperativeKernel((const void*)binned_plan_kernel, dim3(blocks), dim3(kCoopThreads), args, 0, s);
     count_launches(1);
@@ -982,16 +1002,16 @@ cudaError_t binned_finish(int precision, const Geom& g, const BinnedScratch& b, 
   if (e != cudaSuccess) return e;
   // The general sort behind the fallback flag: it rewrites every output.
   return precision == TPICB200_PRECISION_DOUBLE
-             ? launch_fallback<double>(g, in, out, counts, offsets, cursor, perm, scan_scratch, invalid, b.state, s)
-             : launch_fallback<float>(g, in, out, counts, offsets, cursor, perm, scan_scratch, invalid, b.state, s);
+             ? launch_fallback<double>(g, in, out, counts, offsets, cursor, perm, scan_scratch, invalid, b.state,
+                                       b.sort_waits, s)
+             : launch_fallback<float>(g, in, out, counts, offsets, cursor, perm, scan_scratch, invalid, b.state,
+                                      b.sort_waits, s);
 }
 
 cudaError_t launch_sort_binned(int precision, const Geom& g, const tpicb200_particles* in,
                                const uint32_t* in_counts, const uint32_t* in_offsets, tpicb200_particles* out,
                                uint32_t* counts, uint32_t* offsets, uint32_t* cursor, uint32_t* perm,
-                               uint32_t* scan_scratch, uint32_t* binned_words, uint16_t* codes,
-                               uint32_t* invalid, cudaStream_t s) {
-  const BinnedScratch b = binned_scratch(g, binned_words, codes);
+                               uint32_t* scan_scratch, const BinnedScratch& b, uint32_t* invalid, cudaStream_t s) {
   if (cudaError_t e = binned_begin(g, b, in->count, in_counts, in_offsets, false, s); e != cudaSuccess) return e;
   return binned_finish(precision, g, b, true, true, in, out, counts, offsets, cursor, perm, scan_scratch, invalid,
                        s);
