@@ -27,19 +27,21 @@ def stall(lib, ctx, site, index):
     _lib.check(lib.tpicb200_inject_stall(ctx, site, index))
 
 
-def sort_case(torch, shape, n, precision, far, rng, ctx):
+def sort_case(torch, n, precision, far, rng, ctx, crowded=False):
     g = ctx.g
-    d = records(g, n, rng, precision, False)
+    d = records(g, n, rng, precision, crowded)
     counts, offsets = (torch.from_numpy(a).cuda() for a in bins_of(g, d["cell"]))
-    d["cell"] = moved(g, d["cell"], rng, False)
+    if not crowded:
+        d["cell"] = moved(g, d["cell"], rng, False)
     if far:  # bins that do not describe the records
         counts[int(counts.argmax())] -= 1
     return d, ctx.upload_particles(d), counts, offsets
 
 
-@pytest.mark.parametrize("shape,n", [((4, 3, 1), 37), ((9, 8, 7), 20000), ((60, 52, 51), 300000)])
+@pytest.mark.parametrize("shape,n,crowded", [((4, 3, 1), 37, False), ((9, 8, 7), 20000, False),
+                                             ((60, 52, 51), 300000, False), ((61, 1, 1), 50000, True)])
 @pytest.mark.parametrize("precision", [0, 1])
-def test_sort_barriers_that_give_up(torch_cuda, shape, n, precision):
+def test_sort_barriers_that_give_up(torch_cuda, shape, n, crowded, precision):
     import torch
     from gpu_helpers import StageContext
     g = GridSpec(*shape, *(1.0 * m for m in shape))
@@ -48,7 +50,7 @@ def test_sort_barriers_that_give_up(torch_cuda, shape, n, precision):
     assert ctx.lib.tpicb200_inject_stall(ctx.ctx, _lib.STALL_SORT, 0) == _lib.INVALID_ARGUMENT
 
     def sorted_right(far):
-        d, src, c, o = sort_case(torch, shape, n, precision, far, rng, ctx)
+        d, src, c, o = sort_case(torch, n, precision, far, rng, ctx, crowded and far)
         out, counts, offsets = ctx.sort_binned(src, n, c, o)
         assert ctx.invalid_count() == 0
         check(g, d, out, counts, offsets, n)
@@ -60,8 +62,9 @@ def test_sort_barriers_that_give_up(torch_cuda, shape, n, precision):
         sorted_right(False)
     bn = ctx.field(periodic_node_field(g, smooth_random_unique(g, rng, 0.1)))
     j, m = ctx.moments()
-    for wait in range(1, 8):  # the general sort's
-        d, src, c, o = sort_case(torch, shape, n, precision, True, rng, ctx)
+    # The general sort's: seven, and one a merge pass of the 40,000 records of one cell and one behind them.
+    for wait in range(1, 12 if crowded else 8):
+        d, src, c, o = sort_case(torch, n, precision, True, rng, ctx, crowded)
         stall(ctx.lib, ctx.ctx, _lib.STALL_SORT, wait)
         out, counts, offsets = ctx.sort_binned(src, n, c, o)
         assert ctx.invalid_count() == SORT_BIT, wait

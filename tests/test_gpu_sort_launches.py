@@ -90,6 +90,29 @@ def test_binned_sorts_in_a_row(torch_cuda, shape, n, heavy, precision):
     ctx.close()
 
 
+@pytest.mark.parametrize("cells", [(8192,), (8193,), (16384, 300), (16385, 8192, 257, 256, 1), (0, 70000, 33000, 8200, 12),
+                                   (32769, 9000, 65536, 20000), (300,) * 700], ids=lambda c: f"{c[0]}of{len(c)}")
+def test_fallback_of_crowded_cells(torch_cuda, cells):
+    """Bins on both sides of what a warp, a block and the merge passes of all blocks take, of several pass
+    counts in one sort, scrambled by a far move."""
+    import torch
+    from gpu_helpers import StageContext
+    g = GridSpec(len(cells), 1, 1, 1.0 * len(cells), 1.0, 1.0)
+    rng = np.random.default_rng(len(cells))
+    n = int(sum(cells))
+    d = records(g, n, rng, 1, False)
+    d["cell"] = np.sort(d["cell"])  # the old cells: evenly
+    counts, offsets = (torch.from_numpy(a).cuda() for a in bins_of(g, d["cell"]))
+    counts[int(d["cell"][0])] -= 1  # bins that do not describe the records
+    d["cell"] = rng.permutation(np.repeat(g.encode(np.arange(len(cells)), 0, 0), cells)).astype(np.int32)
+    ctx = StageContext(g, precision=1, max_particles=n)
+    for _ in range(2):
+        out, c, o = ctx.sort_binned(ctx.upload_particles(d), n, counts, offsets)
+        assert ctx.invalid_count() == 0
+        check(g, d, out, c, o, n)
+    ctx.close()
+
+
 def test_binned_sort_in_a_graph(torch_cuda):
     import torch
     from gpu_helpers import StageContext

@@ -1,7 +1,7 @@
 // A barrier over all CTAs of a cooperative launch, with bounded waits.
 //
-// Three words, zero between launches: arrivals, departures and whether a wait
-// gave up. A CTA whose polls run out reports false to its threads, which go to
+// Two words, zero between launches: arrivals, and departures with those of
+// CTAs that gave up counted in the upper half. A CTA whose polls run out reports false to its threads, which go to
 // leave(); the others then run out at their next wait. Every CTA leaves, and the
 // last one to do so zeroes the words, so a launch that failed spoils none after
 // it; that CTA also learns of the failure and can put the outputs in order, all
@@ -13,7 +13,7 @@
 namespace tpicb200 {
 
 constexpr uint32_t kGridBarrierPolls = 1u << 22;
-constexpr int kGridBarrierWords = 3;
+constexpr int kGridBarrierWords = 2;
 
 // The bound of a barrier's waits, and for tests the wait (from 1) at which CTA
 // 0 expects more arrivals than there ever are (0: none).
@@ -28,6 +28,7 @@ __device__ __forceinline__ uint32_t load_acquire(const unsigned* p) {
 }
 
 struct GridBarrier {
+  static constexpr uint32_t kFailed = 1u << 16;  // above any number of CTAs resident at once
   unsigned* words;
   GridWaits waits;
   uint32_t arrivals = 0, number = 0;
@@ -51,19 +52,23 @@ struct GridBarrier {
     return !__syncthreads_or(failed);
   }
 
-  // Every thread of every CTA, once, on every way out of the kernel.
   enum Exit { kOther, kLast, kLastOfFailed };
+  // One thread of every CTA, once, on every way out of the kernel.
+  __device__ __forceinline__ Exit depart() {
+    const uint32_t before = atomicAdd(words + 1, failed ? kFailed + 1 : 1u);
+    if (before % kFailed != gridDim.x - 1) return kOther;
+    words[0] = words[1] = 0;
+    return failed || before >= kFailed ? kLastOfFailed : kLast;
+  }
+  // The same by every thread, all of which get the answer; what the CTAs have
+  // written is then done where the last one goes on.
   __device__ __forceinline__ Exit leave() {
     __syncthreads();
-    int exit = kOther;
+    Exit exit = kOther;
     if (threadIdx.x == 0) {
-      if (failed) atomicExch(words + 2, 1u);
       __threadfence();
-      if (atomicAdd(words + 1, 1u) == gridDim.x - 1) {
-        __threadfence();
-        exit = load_acquire(words + 2) ? kLastOfFailed : kLast;
-        words[0] = words[1] = words[2] = 0;
-      }
+      exit = depart();
+      __threadfence();
     }
     const bool last = __syncthreads_or(exit != kOther), any_failed = __syncthreads_or(exit == kLastOfFailed);
     return any_failed ? kLastOfFailed : last ? kLast : kOther;

@@ -64,7 +64,6 @@ struct BinnedState {
   uint32_t fallback;                    // nonzero: the general sort produces the output
   uint32_t bins_bad;                    // nonzero: the old bins do not tile the records
   uint32_t barrier[kGridBarrierWords];  // grid barrier of the cooperative kernels
-  uint32_t pad[3];
 };
 struct BinnedScratch {
   BinnedState* state;

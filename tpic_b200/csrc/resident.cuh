@@ -183,12 +183,14 @@ struct Resident {
       return true;
     }
     if (barrier.wait()) return true;
-    if (threadIdx.x == 0) p.ctl->failed = 1;
-    barrier.leave();
+    if (threadIdx.x == 0) {
+      p.ctl->failed = 1;
+      barrier.depart();
+    }
     return false;
   }
   __device__ void leave() {
-    if (!p.cluster) barrier.leave();
+    if (!p.cluster && threadIdx.x == 0) barrier.depart();
   }
 
   // Table of a slot's tile: the unique index of every staged node (-1 beyond

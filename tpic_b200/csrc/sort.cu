@@ -216,17 +216,23 @@ __device__ __forceinline__ void warp_rank_sort(const uint32_t* s, uint32_t n, ui
     if (32 * r + lane < n) to[rank[r]] = own[r];
 }
 
+// Bins above kWarpBinCapacity are listed in large_bins; with huge_count those
+// above kBlockBinCapacity from its end.
 __device__ __forceinline__ void fixup_small(const uint32_t* counts, const uint32_t* offsets, long long bins,
                                             uint32_t* perm, uint32_t* large_count, uint32_t* large_bins,
-                                            uint32_t (*buffer)[kWarpBinCapacity]) {
+                                            uint32_t* huge_count, uint32_t (*buffer)[kWarpBinCapacity]) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t* s = buffer[warp];
-  const long long warps = (long long)gridDim.x * 8;
-  for (long long bin = (long long)blockIdx.x * 8 + warp; bin < bins; bin += warps) {
+  const int block_warps = blockDim.x / 32;
+  const long long warps = (long long)gridDim.x * block_warps;
+  for (long long bin = (long long)blockIdx.x * block_warps + warp; bin < bins; bin += warps) {
     const uint32_t n = counts[bin];
     if (n <= 1) continue;
     if (n > (uint32_t)kWarpBinCapacity) {
-      if (lane == 0) large_bins[atomicAdd(large_count, 1u)] = (uint32_t)bin;
+      if (lane == 0) {
+        if (huge_count && n > (uint32_t)kBlockBinCapacity) large_bins[bins - 1 - atomicAdd(huge_count, 1u)] = (uint32_t)bin;
+        else large_bins[atomicAdd(large_count, 1u)] = (uint32_t)bin;
+      }
       continue;
     }
     const uint32_t first = offsets[bin];
@@ -248,7 +254,47 @@ __global__ void __launch_bounds__(256) fixup_small_kernel(const uint32_t* counts
                                                           uint32_t* large_bins, const uint32_t* flag) {
   __shared__ uint32_t buffer[8][kWarpBinCapacity];
   if (*flag) return;
-  fixup_small(counts, offsets, bins, perm, large_count, large_bins, buffer);
+  fixup_small(counts, offsets, bins, perm, large_count, large_bins, nullptr, buffer);
+}
+
+// The n <= kBlockBinCapacity distinct indices at p in increasing order, by one
+// block (bitonic, in shared memory).
+__device__ __forceinline__ void block_sort(uint32_t* p, uint32_t n, uint32_t* s) {
+  int size = 1;
+  while (size < (int)n) size <<= 1;
+  for (int t = threadIdx.x; t < size; t += blockDim.x) s[t] = t < (int)n ? p[t] : 0xffffffffu;
+  __syncthreads();
+  for (int k = 2; k <= size; k <<= 1)
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      for (int t = threadIdx.x; t < size; t += blockDim.x) {
+        const int partner = t ^ j;
+        if (partner > t) {
+          const uint32_t a = s[t], b = s[partner];
+          const bool up = (t & k) == 0;
+          if ((a > b) == up) { s[t] = b; s[partner] = a; }
+        }
+      }
+      __syncthreads();
+    }
+  for (int t = threadIdx.x; t < (int)n; t += blockDim.x) p[t] = s[t];
+  __syncthreads();
+}
+
+// Entry t after runs of `width` sorted indices in src[0, n) are merged in pairs
+// (merge path: i entries of the first run and d - i of the second precede
+// output d).
+__device__ __forceinline__ uint32_t merged(const uint32_t* src, uint32_t n, uint32_t width, uint32_t t) {
+  const uint32_t run = uint32_t(t / (2ull * width) * (2ull * width));
+  const uint32_t a0 = run, a1 = min(uint32_t(n - run), width) + run, b1 = uint32_t(min(run + 2ull * width, (unsigned long long)n));
+  const uint32_t la = a1 - a0, lb = b1 - a1, d = t - run;
+  uint32_t lo = d > lb ? d - lb : 0, hi = d < la ? d : la;
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (src[a0 + mid] < src[a1 + d - mid - 1]) lo = mid + 1;
+    else hi = mid;
+  }
+  const uint32_t i = lo, jb = d - i;
+  return i < la && (jb >= lb || src[a0 + i] < src[a1 + jb]) ? src[a0 + i] : src[a1 + jb];
 }
 
 // One block per large bin. Up to kBlockBinCapacity entries sort in shared
@@ -262,47 +308,13 @@ __device__ __forceinline__ void fixup_large(const uint32_t* counts, const uint32
     const uint32_t bin = large_bins[item];
     const uint32_t n = counts[bin], first = offsets[bin];
     if (n <= (uint32_t)kBlockBinCapacity) {
-      int size = 1;
-      while (size < (int)n) size <<= 1;
-      for (int t = threadIdx.x; t < size; t += blockDim.x) s[t] = t < (int)n ? perm[first + t] : 0xffffffffu;
-      __syncthreads();
-      for (int k = 2; k <= size; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1) {
-          for (int t = threadIdx.x; t < size; t += blockDim.x) {
-            const int partner = t ^ j;
-            if (partner > t) {
-              const uint32_t a = s[t], b = s[partner];
-              const bool up = (t & k) == 0;
-              if ((a > b) == up) { s[t] = b; s[partner] = a; }
-            }
-          }
-          __syncthreads();
-        }
-      for (int t = threadIdx.x; t < (int)n; t += blockDim.x) perm[first + t] = s[t];
-      __syncthreads();
+      block_sort(perm + first, n, s);
       continue;
     }
-    // Bottom-up merge sort in global memory, width doubling.
     uint32_t* src = perm + first;
     uint32_t* dst = scratch + first;
-    for (uint32_t width = 1; width < n; width <<= 1) {
-      for (uint32_t t = threadIdx.x; t < n; t += blockDim.x) {
-        const uint32_t run = t / (2 * width) * (2 * width);
-        const uint32_t a0 = run, a1 = min(run + width, n), b1 = min(run + 2 * width, n);
-        const uint32_t la = a1 - a0, lb = b1 - a1, d = t - run;
-        // Merge path: i elements from A and d - i from B precede output d.
-        uint32_t lo = d > lb ? d - lb : 0, hi = d < la ? d : la;
-        while (lo < hi) {
-          const uint32_t mid = (lo + hi) >> 1;
-          if (src[a0 + mid] < src[a1 + d - mid - 1]) lo = mid + 1;
-          else hi = mid;
-        }
-        const uint32_t i = lo, jb = d - i;
-        uint32_t value;
-        if (i < la && (jb >= lb || src[a0 + i] < src[a1 + jb])) value = src[a0 + i];
-        else value = src[a1 + jb];
-        dst[t] = value;
-      }
+    for (unsigned long long width = 1; width < n; width <<= 1) {
+      for (uint32_t t = threadIdx.x; t < n; t += blockDim.x) dst[t] = merged(src, n, uint32_t(width), t);
       __syncthreads();
       uint32_t* tmp = src; src = dst; dst = tmp;
     }
@@ -310,6 +322,65 @@ __device__ __forceinline__ void fixup_large(const uint32_t* counts, const uint32
       for (uint32_t t = threadIdx.x; t < n; t += blockDim.x) perm[first + t] = src[t];
     __syncthreads();
   }
+}
+
+// The same for bins above kBlockBinCapacity (listed from the end of the
+// large-bin list) by all blocks of a cooperative launch: sorted runs of
+// kBlockBinCapacity, then one merge pass over all those bins between two
+// barriers, so that a wait is for one pass over the records and never for
+// a whole bin: by one block a bin of ten million would outlast the barrier's
+// bound. Whole sorts of two bins of 150,000 records 11.0 -> 2.6 ms (separate
+// launches of one block a bin: 5.3), of 64 of 20,000 2.7 -> 1.07 (1.07).
+// False when a barrier gave up.
+__device__ __forceinline__ bool fixup_huge(const uint32_t* counts, const uint32_t* offsets, uint32_t* perm,
+                                           uint32_t* scratch, uint32_t nhuge, const uint32_t* last,
+                                           uint32_t* s, GridBarrier& barrier) {
+  constexpr uint32_t kRun = kBlockBinCapacity;
+  uint32_t longest = 0, run = 0;
+  for (uint32_t h = 0; h < nhuge; ++h) {
+    const uint32_t bin = *(last - h), n = counts[bin], first = offsets[bin];
+    longest = max(longest, n);
+    for (uint32_t r = 0; r < n; r += min(kRun, n - r), ++run)
+      if (run % gridDim.x == blockIdx.x) block_sort(perm + first + r, min(kRun, n - r), s);
+  }
+  // f(first, n, begin, end) for this block's share of every bin [first, first + n):
+  // chunks of the bins in turn, the bins staged in shared memory.
+  auto each_chunk = [&](auto&& f) {
+    constexpr uint32_t kBatch = kBlockBinCapacity / 2;
+    const uint32_t size = 2 * blockDim.x;
+    unsigned long long chunk = 0;
+    for (uint32_t h0 = 0; h0 < nhuge; h0 += kBatch) {
+      const uint32_t batch = min(kBatch, nhuge - h0);
+      __syncthreads();
+      for (uint32_t i = threadIdx.x; i < batch; i += blockDim.x) {
+        const uint32_t bin = *(last - h0 - i);
+        s[2 * i] = offsets[bin];
+        s[2 * i + 1] = counts[bin];
+      }
+      __syncthreads();
+      for (uint32_t i = 0; i < batch; ++i) {
+        const uint32_t first = s[2 * i], n = s[2 * i + 1], chunks = n / size + (n % size ? 1 : 0);
+        for (unsigned long long c = (blockIdx.x + gridDim.x - chunk % gridDim.x) % gridDim.x; c < chunks; c += gridDim.x)
+          f(first, n, uint32_t(c * size), uint32_t(min((c + 1) * size, (unsigned long long)n)));
+        chunk += chunks;
+      }
+    }
+  };
+  // Pass m goes from perm to scratch for even m and back for odd m; a bin that was
+  // one run after an odd number of passes is copied back in the pass behind them.
+  bool odd = false;
+  for (unsigned long long width = kRun; width < longest || odd; width <<= 1, odd = !odd) {
+    if (!barrier.wait()) return false;
+    each_chunk([&](uint32_t first, uint32_t n, uint32_t begin, uint32_t end) {
+      const uint32_t* src = (odd ? scratch : perm) + first;
+      uint32_t* dst = (odd ? perm : scratch) + first;
+      if (n > width)
+        for (uint32_t t = begin + threadIdx.x; t < end; t += blockDim.x) dst[t] = merged(src, n, uint32_t(width), t);
+      else if (odd && 2ull * n > width)
+        for (uint32_t t = begin + threadIdx.x; t < end; t += blockDim.x) dst[t] = src[t];
+    });
+  }
+  return true;
 }
 
 __global__ void __launch_bounds__(1024) fixup_large_kernel(const uint32_t* counts, const uint32_t* offsets,
@@ -355,21 +426,25 @@ __device__ __forceinline__ void gather(uint32_t s, uint32_t p, const SortRecords
   r.okey[p] = key;
   if (r.oid) r.oid[p] = r.iid[s];
 }
-template <class Vel>
+// Unless a flag is raised, or with no flag through ranks that may be a failed sort's.
+template <class Vel, bool kFlag>
 __global__ void __launch_bounds__(256) gather_kernel(const uint32_t* __restrict__ perm, uint32_t count,
                                                      SortRecords<Vel> r, const uint32_t* flag) {
-  if (flag && *flag) return;
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < count; p += gridDim.x * blockDim.x)
-    if (perm[p] < count) gather(perm[p], p, r);
+  if (kFlag && *flag) return;
+  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < count; p += gridDim.x * blockDim.x) {
+    const uint32_t s = perm[p];
+    if (kFlag || s < count) gather(s, p, r);
+  }
 }
 cudaError_t launch_gather(int precision, const uint32_t* perm, const tpicb200_particles* in, tpicb200_particles* out,
                           const uint32_t* flag, cudaStream_t s) {
   const uint32_t n = in->count;
   const unsigned blocks = grid_for(n, 256, 148u * 8u);
+  auto go = [&](auto kernel, auto records) { kernel<<<blocks, 256, 0, s>>>(perm, n, records, flag); };
   if (precision == TPICB200_PRECISION_DOUBLE)
-    gather_kernel<double><<<blocks, 256, 0, s>>>(perm, n, SortRecords<double>(in, out), flag);
+    go(flag ? gather_kernel<double, true> : gather_kernel<double, false>, SortRecords<double>(in, out));
   else
-    gather_kernel<float><<<blocks, 256, 0, s>>>(perm, n, SortRecords<float>(in, out), flag);
+    go(flag ? gather_kernel<float, true> : gather_kernel<float, false>, SortRecords<float>(in, out));
   count_launches(1);
   return cudaGetLastError();
 }
@@ -425,23 +500,27 @@ cudaError_t enqueue_general(int precision, const Geom& g, const tpicb200_particl
 // given) by all CTAs: each takes a contiguous range, whose sum it has stored
 // in sums[blockIdx.x]; the other CTAs' sums are read after a grid barrier.
 constexpr int kCoopThreads = 256;
+// One CTA of 1,024 threads an SM: 64 bins of 5,000 records, a block's sort each, 308
+// us, with two of 512 382, with two of 256 480 (as separate launches 349).
+constexpr int kFallbackThreads = 1024;
 __device__ __forceinline__ void coop_range(long long bins, long long& b0, long long& b1) {
   const long long each = (bins + gridDim.x - 1) / gridDim.x;
   b0 = min(blockIdx.x * each, bins);
   b1 = min(b0 + each, bins);
 }
+template <int kThreads>
 __device__ __forceinline__ void coop_scan(const uint32_t* counts, long long bins, const uint32_t* sums,
                                           uint32_t* offsets, uint32_t* cursor) {
-  __shared__ uint32_t scratch[kCoopThreads / 32];
-  __shared__ uint32_t warp_totals[kCoopThreads / 32];
+  __shared__ uint32_t scratch[kThreads / 32];
+  __shared__ uint32_t warp_totals[kThreads / 32];
   constexpr int kItems = 4;
   uint32_t before = 0;
-  for (unsigned b = threadIdx.x; b < blockIdx.x; b += kCoopThreads) before += __ldcg(sums + b);
-  uint32_t running = block_sum<kCoopThreads>(before, scratch);
+  for (unsigned b = threadIdx.x; b < blockIdx.x; b += kThreads) before += __ldcg(sums + b);
+  uint32_t running = block_sum<kThreads>(before, scratch);
   long long b0, b1;
   coop_range(bins, b0, b1);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (long long tile = b0; tile < b1; tile += kItems * kCoopThreads) {
+  for (long long tile = b0; tile < b1; tile += kItems * kThreads) {
     const long long at = tile + (long long)threadIdx.x * kItems;
     uint32_t items[kItems], local = 0;
 #pragma unroll
@@ -460,7 +539,7 @@ __device__ __forceinline__ void coop_scan(const uint32_t* counts, long long bins
     __syncthreads();
     uint32_t prefix = running, total = 0;
 #pragma unroll
-    for (int w = 0; w < kCoopThreads / 32; ++w) {
+    for (int w = 0; w < kThreads / 32; ++w) {
       if (w < warp) prefix += warp_totals[w];
       total += warp_totals[w];
     }
@@ -485,10 +564,11 @@ __device__ __forceinline__ void fallback_sort(const Geom& g, uint32_t n, const S
                                               const ScanScratch& sc, uint32_t* invalid, GridBarrier& barrier,
                                               uint32_t* buffer, uint32_t* scratch) {
   uint32_t* sums = sc.large_bins;  // free until the fix-up
-  for (long long b = blockIdx.x * (long long)kCoopThreads + threadIdx.x; b < g.bins;
-       b += (long long)gridDim.x * kCoopThreads)
+  constexpr int kThreads = kFallbackThreads;
+  uint32_t* huge_count = sc.block_sums;
+  for (long long b = blockIdx.x * (long long)kThreads + threadIdx.x; b < g.bins; b += (long long)gridDim.x * kThreads)
     counts[b] = 0;
-  if (blockIdx.x == 0 && threadIdx.x == 0) *sc.flag = *sc.large_count = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *sc.flag = *sc.large_count = *huge_count = 0;
   if (!barrier.wait()) return;
   histogram(g, r.ikey, n, counts, sc.flag);
   if (!barrier.wait()) return;
@@ -497,21 +577,23 @@ __device__ __forceinline__ void fallback_sort(const Geom& g, uint32_t n, const S
     long long b0, b1;
     coop_range(g.bins, b0, b1);
     uint32_t sum = 0;
-    for (long long b = b0 + threadIdx.x; b < b1; b += kCoopThreads) sum += __ldcg(counts + b);
-    sum = block_sum<kCoopThreads>(sum, scratch);
+    for (long long b = b0 + threadIdx.x; b < b1; b += kThreads) sum += __ldcg(counts + b);
+    sum = block_sum<kThreads>(sum, scratch);
     if (threadIdx.x == 0) sums[blockIdx.x] = sum;
     if (!barrier.wait()) return;
-    coop_scan(counts, g.bins, sums, offsets, cursor);
+    coop_scan<kThreads>(counts, g.bins, sums, offsets, cursor);
     if (!barrier.wait()) return;
     place(r.ikey, n, cursor, perm);
     if (!barrier.wait()) return;
-    fixup_small(counts, offsets, g.bins, perm, sc.large_count, sc.large_bins,
+    fixup_small(counts, offsets, g.bins, perm, sc.large_count, sc.large_bins, huge_count,
                 reinterpret_cast<uint32_t (*)[kWarpBinCapacity]>(buffer));
     if (!barrier.wait()) return;
-    fixup_large(counts, offsets, perm, (uint32_t*)r.okey, sc.large_count, sc.large_bins, buffer);
+    uint32_t* free = (uint32_t*)r.okey;
+    fixup_large(counts, offsets, perm, free, sc.large_count, sc.large_bins, buffer);
+    if (!fixup_huge(counts, offsets, perm, free, *huge_count, sc.large_bins + g.bins - 1, buffer, barrier)) return;
     if (!barrier.wait()) return;
-    for (uint32_t p = blockIdx.x * kCoopThreads + threadIdx.x; p < n; p += gridDim.x * kCoopThreads)
-      gather(perm[p], p, r);
+    for (unsigned long long p = blockIdx.x * kThreads + threadIdx.x; p < n; p += gridDim.x * kThreads)
+      gather(perm[p], uint32_t(p), r);
   } else if (blockIdx.x == 0 && threadIdx.x == 0 && invalid) {
     atomicAdd(invalid, 1u);
   }
@@ -520,24 +602,24 @@ __device__ __forceinline__ void fallback_sort(const Geom& g, uint32_t n, const S
 // The general sort in one launch, for the binned sort's fallback: enqueued
 // behind every binned sort and leaving at once unless the fallback flag is up.
 // As the general sort's eleven kernels it cost 25 us of empty launches per
-// species and cycle. Its steps are separated by grid barriers; the last CTA to
+// species and cycle. Its steps are separated by grid barriers, none of which waits
+// for more than a pass over the records or the bins; the last CTA to
 // leave clears the flags for the next sort. Where a barrier gave up, perm and the
 // records are unfinished: that CTA then empties the bins, so that nothing reads
 // through them, and counts 1 << 22 in *invalid.
 template <class Vel>
-__global__ void __launch_bounds__(kCoopThreads, 2) fallback_sort_kernel(Geom g, uint32_t n, SortRecords<Vel> r,
-                                                                        uint32_t* counts, uint32_t* offsets,
-                                                                        uint32_t* cursor, uint32_t* perm,
-                                                                        ScanScratch sc, uint32_t* invalid,
-                                                                        BinnedState* state, GridWaits waits) {
+__global__ void __launch_bounds__(kFallbackThreads, 1)
+    fallback_sort_kernel(Geom g, uint32_t n, SortRecords<Vel> r, uint32_t* counts, uint32_t* offsets, uint32_t* cursor,
+                         uint32_t* perm, ScanScratch sc, uint32_t* invalid, BinnedState* state, GridWaits waits) {
+  static_assert(kFallbackThreads / 32 * kWarpBinCapacity <= kBlockBinCapacity, "the warps' buffers are the block's");
   __shared__ uint32_t buffer[kBlockBinCapacity];
-  __shared__ uint32_t scratch[kCoopThreads / 32];
+  __shared__ uint32_t scratch[kFallbackThreads / 32];
   if (state->fallback == 0) return;
   GridBarrier barrier(state->barrier, waits);
   fallback_sort(g, n, r, counts, offsets, cursor, perm, sc, invalid, barrier, buffer, scratch);
   const GridBarrier::Exit exit = barrier.leave();
   if (exit == GridBarrier::kLastOfFailed) {
-    for (long long b = threadIdx.x; b <= g.bins; b += kCoopThreads) {
+    for (long long b = threadIdx.x; b <= g.bins; b += kFallbackThreads) {
       if (b < g.bins) counts[b] = 0;
       offsets[b] = 0;
     }
@@ -555,14 +637,14 @@ cudaError_t launch_fallback(const Geom& g, const tpicb200_particles* in, tpicb20
   Geom geom = g;
   uint32_t n = in->count;
   SortRecords<Vel> r(in, out);
-  // Two CTAs an SM, fewer for little work (a barrier costs with their number);
+  // One CTA an SM, fewer for little work (a barrier costs with their number);
   // their sums must fit the bins' scratch.
   const long long work = std::max<long long>(g.bins, n);
-  const unsigned blocks = unsigned(std::min<long long>(grid_for(work, 4 * kCoopThreads, 148u * 2u), g.bins));
+  const unsigned blocks = unsigned(std::min<long long>(grid_for(work, kFallbackThreads, 148u), g.bins));
   void* args[] = {&geom, &n, &r, &counts, &offsets, &cursor, &perm, &sc, &invalid, &state, &waits};
   count_launches(1);
-  return cudaLaunchCooperativeKernel((const void*)fallback_sort_kernel<Vel>, dim3(blocks), dim3(kCoopThreads), args, 0,
-                                     s);
+  return cudaLaunchCooperativeKernel((const void*)fallback_sort_kernel<Vel>, dim3(blocks), dim3(kFallbackThreads), args,
+                                     0, s);
 }
 
 // ---- Binned sort: the input is grouped by the bins of an earlier sort ----
@@ -813,7 +895,7 @@ __device__ __forceinline__ void binned_plan(const Geom& g, uint32_t* transfer, u
   sum = block_sum<kCoopThreads>(sum, scratch);
   if (threadIdx.x == 0) sums[blockIdx.x] = sum;
   if (!barrier.wait()) return;
-  coop_scan(counts, g.bins, sums, offsets, nullptr);
+  coop_scan<kCoopThreads>(counts, g.bins, sums, offsets, nullptr);
   if (!barrier.wait()) return;
   binned_bases(g, offsets, transfer);
 }
@@ -830,7 +912,7 @@ __global__ void __launch_bounds__(kCoopThreads, 2) binned_plan_kernel(Geom g, ui
   if (state->fallback) return;
   GridBarrier barrier(state->barrier, waits);
   binned_plan(g, transfer, counts, offsets, sums, barrier, scratch);
-  if (barrier.leave() == GridBarrier::kLastOfFailed && threadIdx.x == 0) state->fallback = 1;
+  if (threadIdx.x == 0 && barrier.depart() == GridBarrier::kLastOfFailed) state->fallback = 1;
 }
 
 // The lane mask of a live lane's slot: the live lanes with the same slot
