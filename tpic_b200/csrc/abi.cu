@@ -33,6 +33,7 @@ struct tpicb200_context {
   double* particle_theta = nullptr;  // S^n(E_theta), the movers' field when smoothing is on
   double* pinned = nullptr;      // host mirror of `reduced` + invalid
   int energy_blocks = 0;
+  int sms = 0;                   // of the device
   cudaEvent_t events[6 + 3 * TPICB200_MAX_SPECIES]{};
   void* moments = nullptr;       // per-cell moments of the moment forms (float: tensor core; double: FP64)
   bool moments_pending = false;  // moments hold deposits not yet assembled
@@ -101,7 +102,8 @@ BinnedScratch sort_scratch(const tpicb200_context* ctx) {
     return ctx->stall_site != site ? GridWaits{kGridBarrierPolls, 0}
                                    : GridWaits{ctx->wait_polls ? ctx->wait_polls : kGridBarrierPolls, ctx->stall_index};
   };
-  return binned_scratch(ctx->g, ctx->binned, ctx->codes, waits(TPICB200_STALL_PLAN), waits(TPICB200_STALL_SORT));
+  return binned_scratch(ctx->g, ctx->binned, ctx->codes, waits(TPICB200_STALL_PLAN), waits(TPICB200_STALL_SORT),
+                        ctx->sms);
 }
 
 cudaError_t launch_moments(tpicb200_context* ctx, int kind, int ns, const double* qom,
@@ -234,6 +236,7 @@ int tpicb200_create(const tpicb200_grid* grid, const tpicb200_options* options, 
                               options->theta, options->c, smoothing, &e);
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  ctx->sms = sms;
   ctx->energy_blocks = 4 * sms;
   auto alloc = [&](void** p, size_t bytes) {
     if (e == cudaSuccess) e = cudaMalloc(p, bytes ? bytes : 4);

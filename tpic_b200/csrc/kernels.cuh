@@ -72,11 +72,12 @@ struct BinnedScratch {
   uint32_t* transfer;     // [27][interior cells]: counts, then output bases
   uint16_t* code;         // run code per record (direction, cell in run; kNoMove)
   GridWaits plan_waits, sort_waits;  // of the cooperative kernels
+  int sms;                           // of the device: all their CTAs must be resident
 };
 size_t binned_scratch_words(const Geom& g);
 bool binned_sort_applies(const Geom& g);
 BinnedScratch binned_scratch(const Geom& g, uint32_t* words, uint16_t* codes, GridWaits plan_waits,
-                             GridWaits sort_waits);
+                             GridWaits sort_waits, int sms);
 cudaError_t binned_reset(const BinnedScratch& b);
 // Copies the input's bins, checks that they tile the n records in key order
 // (else raises bins_bad and fallback) and clears the transfer counts when the

@@ -631,7 +631,7 @@ __global__ void __launch_bounds__(kFallbackThreads, 1)
 template <class Vel>
 cudaError_t launch_fallback(const Geom& g, const tpicb200_particles* in, tpicb200_particles* out, uint32_t* counts,
                             uint32_t* offsets, uint32_t* cursor, uint32_t* perm, uint32_t* scan_scratch,
-                            uint32_t* invalid, BinnedState* state, GridWaits waits, cudaStream_t s) {
+                            uint32_t* invalid, const BinnedScratch& b, cudaStream_t s) {
   const int nblocks = int((g.bins + kScanTile - 1) / kScanTile);
   ScanScratch sc{scan_scratch, scan_scratch + nblocks, scan_scratch + nblocks + 1, scan_scratch + nblocks + 2};
   Geom geom = g;
@@ -640,7 +640,9 @@ cudaError_t launch_fallback(const Geom& g, const tpicb200_particles* in, tpicb20
   // One CTA an SM, fewer for little work (a barrier costs with their number);
   // their sums must fit the bins' scratch.
   const long long work = std::max<long long>(g.bins, n);
-  const unsigned blocks = unsigned(std::min<long long>(grid_for(work, kFallbackThreads, 148u), g.bins));
+  const unsigned blocks = unsigned(std::min<long long>(grid_for(work, kFallbackThreads, unsigned(b.sms)), g.bins));
+  BinnedState* state = b.state;
+  GridWaits waits = b.sort_waits;
   void* args[] = {&geom, &n, &r, &counts, &offsets, &cursor, &perm, &sc, &invalid, &state, &waits};
   count_launches(1);
   return cudaLaunchCooperativeKernel((const void*)fallback_sort_kernel<Vel>, dim3(blocks), dim3(kFallbackThreads), args,
@@ -1023,8 +1025,9 @@ size_t binned_scratch_words(const Geom& g) {
 bool binned_sort_applies(const Geom& g) { return g.nx >= 1 && g.ny >= 1 && g.nz >= 1; }
 
 BinnedScratch binned_scratch(const Geom& g, uint32_t* words, uint16_t* codes, GridWaits plan_waits,
-                             GridWaits sort_waits) {
+                             GridWaits sort_waits, int sms) {
   BinnedScratch b;
+  b.sms = sms;
   b.plan_waits = plan_waits;
   b.sort_waits = sort_waits;
   b.state = reinterpret_cast<BinnedState*>(words);
@@ -1069,7 +1072,7 @@ cudaError_t binned_finish(int precision, const Geom& g, const BinnedScratch& b, 
     BinnedState* state = b.state;
     GridWaits waits = b.plan_waits;
     void* args[] = {&geom, &transfer, &counts, &offsets, &sums, &state, &waits};
-    const unsigned blocks = unsigned(std::min<long long>(grid_for(bins, kCoopThreads, 148u * 2u), bins));
+    const unsigned blocks = unsigned(std::min<long long>(grid_for(bins, kCoopThreads, 2u * unsigned(b.sms)), bins));
     e = cudaLaunchCooperativeKernel((const void*)binned_plan_kernel, dim3(blocks), dim3(kCoopThreads), args, 0, s);
     count_launches(1);
   }
@@ -1084,10 +1087,8 @@ cudaError_t binned_finish(int precision, const Geom& g, const BinnedScratch& b, 
   if (e != cudaSuccess) return e;
   // The general sort behind the fallback flag: it rewrites every output.
   return precision == TPICB200_PRECISION_DOUBLE
-             ? launch_fallback<double>(g, in, out, counts, offsets, cursor, perm, scan_scratch, invalid, b.state,
-                                       b.sort_waits, s)
-             : launch_fallback<float>(g, in, out, counts, offsets, cursor, perm, scan_scratch, invalid, b.state,
-                                      b.sort_waits, s);
+             ? launch_fallback<double>(g, in, out, counts, offsets, cursor, perm, scan_scratch, invalid, b, s)
+             : launch_fallback<float>(g, in, out, counts, offsets, cursor, perm, scan_scratch, invalid, b, s);
 }
 
 cudaError_t launch_sort_binned(int precision, const Geom& g, const tpicb200_particles* in,
