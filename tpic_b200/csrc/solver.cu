@@ -934,8 +934,13 @@ struct SolverWorkspace {
   };
   MassMap maps[4];
   int next_map = 0;
-  // The resident kernels' plan (resident.cuh), where the grid takes them.
+  // The resident kernels' plan (resident.cuh), where the grid takes them: made at
+  // the first solve, which loads the kernels; the context's creation sizes the buffers.
   bool resident = false;
+  bool planned = false;
+  int sms = 0;
+  long long resident_rows = 0;   // of a basis column, padded to whole tiles
+  int resident_most_ctas = 0;
   ResidentPlan plan{};
   unsigned resident_grid = 0;
   size_t resident_bytes = 0;
@@ -1031,24 +1036,15 @@ bool allow_shared(void (*const (&kernels)[2])(ResidentPlan), int limit) {
 // step graph, ms a solve (mixed, stencil-major): 1024 x 1 x 1 1.28 / 5.72, 16^3
 // 0.19 / 0.58, 32^3 0.29 / 0.59, 40^3 0.44 / 0.70, 256 x 128 x 1 0.34 / 0.78,
 // 256 x 256 x 1 0.44 / 0.94.
-template <class P>
-void plan_resident(SolverWorkspace* w, int sms) {
-  using K = ResidentKernels<P>;
+//
+// Calls take(plan, CTAs, CTAs an SM, shared memory bytes) for the tiles in that
+// order until it returns false. Arithmetic alone: no kernel is touched.
+template <class P, class Take>
+void resident_tiles(const SolverWorkspace* w, Take&& take) {
   const Geom& g = w->g;
   const int smooth = w->smoothing.iterations;
   if (w->restart > kResidentRestart || (smooth > 0 && (g.nz != 1 || smooth > kResidentSmooth))) return;
-  int device = 0, cooperative = 0, limit = 0;
-  if (cudaGetDevice(&device) != cudaSuccess ||
-      cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, device) != cudaSuccess || !cooperative ||
-      cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess)
-    return;
-  // The kernels of A; those of A^T have the same bounds (adjoint_kernels). A
-  // kernel is loaded when its attributes are set, so only the ones that a tile
-  // asks for.
-  typename K::Kernel kernels[2][2];  // [CTAs an SM - 1]
-  bool loaded[2] = {false, false};
-  K::pick(false, smooth > 0, 1, kernels[0]);
-  K::pick(false, smooth > 0, 2, kernels[1]);
+  const int sms = w->sms, limit = w->shared_limit;
   auto power = [](int n) {
     int p = 1;
     while (p < n) p *= 2;
@@ -1114,42 +1110,75 @@ void plan_resident(SolverWorkspace* w, int sms) {
       if (bytes > size_t(limit)) continue;
       const int ctas = grid <= sms ? 1 : 2;
       if (alone ? ctas == 2 : grid > 2 * sms) continue;
-      int per_sm = ctas;
-      if (!loaded[ctas - 1] && !allow_shared(kernels[ctas - 1], limit)) return;
-      loaded[ctas - 1] = true;
-      for (auto k : kernels[ctas - 1]) {
-        int blocks = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k, kResidentThreads, bytes) != cudaSuccess) {
-          cudaGetLastError();
-          return;
-        }
-        per_sm = std::min(per_sm, blocks);
-      }
-      if (grid > per_sm * sms) continue;
       if (p.slots > 2 && g.nz > 1 &&
-          (sizeof(typename P::EC) == 4 || 100LL * p.tiles < 85LL * p.slots * per_sm * sms))
+          (sizeof(typename P::EC) == 4 || 100LL * p.tiles < 85LL * p.slots * ctas * sms))
         break;
-      // The rest of the shared memory keeps mass blocks.
-      size_t used = bytes;
-      if (p.slots == 1 && ctas == 1) {
-        const size_t budget = size_t(limit);
-        const size_t stencil = size_t(18) * kResidentNodeThreads * sizeof(typename P::EC);
-        const int most = (14 + p.parts - 1) / p.parts;
-        if (budget > bytes) p.kept = std::min(most, int((budget - bytes) / stencil));
-        used = resident_shared(p, sizeof(typename P::EC)).total;
-      }
-      if (p.cluster)
-        for (auto k : kernels[ctas - 1])
-          if (!cluster_fits(k, grid, used)) p.cluster = false;
-      w->resident_ctas = ctas;
-      w->shared_limit = limit;
-      w->plan = p;
-      w->resident_grid = unsigned(grid);
-      w->resident_bytes = used;
-      w->resident = true;
-      return;
+      if (!take(p, grid, ctas, bytes)) return;
     }
   }
+}
+
+// What any of the tiles needs of the context's buffers.
+template <class P>
+void size_resident(SolverWorkspace* w) {
+  int device = 0, cooperative = 0;
+  if (cudaGetDevice(&device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, device) != cudaSuccess || !cooperative ||
+      cudaDeviceGetAttribute(&w->shared_limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess)
+    return;
+  resident_tiles<P>(w, [&](const ResidentPlan& p, int grid, int, size_t) {
+    w->resident = true;
+    w->resident_rows = std::max(w->resident_rows, 3LL * grid * p.slots * p.nodes);
+    w->resident_most_ctas = std::max(w->resident_most_ctas, grid);
+    return true;
+  });
+}
+
+// The first of the tiles whose CTAs are all resident; none: the step graph.
+template <class P>
+void plan_resident(SolverWorkspace* w) {
+  using K = ResidentKernels<P>;
+  w->planned = true;
+  w->resident = false;
+  // The kernels of A; those of A^T have the same bounds (adjoint_kernels). A
+  // kernel is loaded when its attributes are set, so only the ones that a tile
+  // asks for.
+  typename K::Kernel kernels[2][2];  // [CTAs an SM - 1]
+  bool loaded[2] = {false, false};
+  K::pick(false, w->smoothing.iterations > 0, 1, kernels[0]);
+  K::pick(false, w->smoothing.iterations > 0, 2, kernels[1]);
+  resident_tiles<P>(w, [&](ResidentPlan p, int grid, int ctas, size_t bytes) {
+    int per_sm = ctas;
+    if (!loaded[ctas - 1] && !allow_shared(kernels[ctas - 1], w->shared_limit)) return false;
+    loaded[ctas - 1] = true;
+    for (auto k : kernels[ctas - 1]) {
+      int blocks = 0;
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k, kResidentThreads, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+      }
+      per_sm = std::min(per_sm, blocks);
+    }
+    if (grid > per_sm * w->sms) return true;
+    // The rest of the shared memory keeps mass blocks.
+    size_t used = bytes;
+    if (p.slots == 1 && ctas == 1) {
+      const size_t budget = size_t(w->shared_limit);
+      const size_t stencil = size_t(18) * kResidentNodeThreads * sizeof(typename P::EC);
+      const int most = (14 + p.parts - 1) / p.parts;
+      if (budget > bytes) p.kept = std::min(most, int((budget - bytes) / stencil));
+      used = resident_shared(p, sizeof(typename P::EC)).total;
+    }
+    if (p.cluster)
+      for (auto k : kernels[ctas - 1])
+        if (!cluster_fits(k, grid, used)) p.cluster = false;
+    w->resident_ctas = ctas;
+    w->plan = p;
+    w->resident_grid = unsigned(grid);
+    w->resident_bytes = used;
+    w->resident = true;
+    return false;
+  });
 }
 
 SolverWorkspace* solver_create(int precision, const Geom& g, int restart, double dt, double theta,
@@ -1172,6 +1201,7 @@ SolverWorkspace* solver_create(int precision, const Geom& g, int restart, double
   int device = 0, sms = 148;
   cudaGetDevice(&device);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  w->sms = sms;
   w->rblocks = unsigned(std::min<long long>((w->count + kThreads - 1) / kThreads, 4LL * sms));
   w->batch = std::max(restart, 2);
   // TPICB200_STEP_GRAPH=0 keeps the host-stepped Arnoldi loop (one launch per
@@ -1189,12 +1219,10 @@ SolverWorkspace* solver_create(int precision, const Geom& g, int restart, double
     alloc((void**)&w->smooth_image, 3 * g.nodes * sizeof(double));
   }
   if (!w->loop_unavailable) {
-    if (precision == TPICB200_PRECISION_DOUBLE) plan_resident<PDouble>(w, sms);
-    else plan_resident<PMixed>(w, sms);
+    if (precision == TPICB200_PRECISION_DOUBLE) size_resident<PDouble>(w);
+    else size_resident<PMixed>(w);
   }
-  // The resident kernels' rows are padded to whole tiles.
-  const long long padded = 3LL * w->resident_grid * w->plan.slots * w->plan.nodes;
-  alloc(&w->basis, (size_t)(restart + 1) * std::max(w->ld, padded) * w->scalar_bytes);
+  alloc(&w->basis, (size_t)(restart + 1) * std::max(w->ld, w->resident_rows) * w->scalar_bytes);
   alloc(&w->image, (size_t)w->count * w->scalar_bytes);
   alloc((void**)&w->x, w->count * sizeof(double));
   alloc((void**)&w->b, w->count * sizeof(double));
@@ -1211,7 +1239,7 @@ SolverWorkspace* solver_create(int precision, const Geom& g, int restart, double
   if (e == cudaSuccess) e = cudaMemset(w->input, 0, 3 * g.nodes * sizeof(double));
   if (e == cudaSuccess) e = cudaMemset(w->rhs, 0, 3 * g.nodes * sizeof(double));
   if (w->resident) {
-    alloc((void**)&w->resident_partials, size_t(kResidentRestart + 2) * w->resident_grid * sizeof(double));
+    alloc((void**)&w->resident_partials, size_t(kResidentRestart + 2) * w->resident_most_ctas * sizeof(double));
     alloc((void**)&w->resident_barrier, kGridBarrierWords * sizeof(unsigned));
     if (e == cudaSuccess) e = cudaMemset(w->resident_barrier, 0, kGridBarrierWords * sizeof(unsigned));
     if (e == cudaSuccess) e = cudaMemset(w->ctl, 0, sizeof(ArnoldiControl));
@@ -1698,6 +1726,7 @@ struct Solve {
   // and j with the guess E^n.
   int run(const void* e, const void* bcell, const void* j, const void* mass_v, double* etheta,
           tpicb200_gmres_result* result, int max_iterations, double tolerance, const double* rhs_in = nullptr) {
+    if (resident() && !w->planned) plan_resident<P>(w);
     if (resident()) return run_resident(e, bcell, j, mass_v, etheta, result, max_iterations, tolerance, rhs_in);
     const Geom& g = w->g;
     const Mass* mass = (const Mass*)mass_v;
