@@ -351,8 +351,8 @@ int tpicb200_clear_moments(tpicb200_context* ctx, void* j, void* mass, tpicb200_
  * addition an entry, of a sum in a fixed order. The scalar forms with counts/offsets
  * (the bins of p, from tpicb200_sort) and both j and mass sum the same cell
  * moments and add them into j and mass within the call; with only one of the
- * two, or while a moment form's moments wait for the fold, the sorted
- * cell-tile kernels run; with NULL bins the per-particle kernels run. Replaces
+ * two, with few records a cell, or while a moment form's moments wait for the
+ * fold, the sorted cell-tile kernels run; with NULL bins the per-particle kernels run. Replaces
  * enqueue_sorted_current / enqueue_unsorted_current
  * (ecsim/deposition/current_deposition_device.hpp:340-421) and
  * enqueue_sorted_mass_matrix<Kernel> / enqueue_unsorted_mass_matrix

@@ -3,8 +3,9 @@ right behind tpicb200_clear_moments: values that the caller put there after the
 clear, another context's deposition into the same buffers, and the replays of a
 graph that recorded the deposition and not the clear.
 
-An entry's sum over the records is the same number each time and is added in
-one rounding, so the comparisons with the sum added on the host are exact."""
+There are records enough for the scalar forms to deposit cell moments: an entry's
+sum over the records is the same number each time and is added in one rounding, so
+the comparisons with the sum added on the host are exact."""
 from __future__ import annotations
 
 import ctypes as C
@@ -27,7 +28,7 @@ SHAPES = [(8, 6, 4), (5, 3, 2)]  # the assembly by quads of cells and by nodes
 class Species:
     def __init__(self, ctx, g, s, precision):
         rng = np.random.default_rng(s)
-        d = ragged_species(g, s, rng, precision, 4)
+        d = ragged_species(g, s, rng, precision, 0.5)
         self.n, self.qom = len(d["cell"]), QOM[s]
         self.parts = ctx.upload_particles(d)
         self.bins = bins(ctx, d)

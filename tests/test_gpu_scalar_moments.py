@@ -28,7 +28,7 @@ QOM = (-4.0, 1.0, -1.0)
 
 def ragged_species(g, s, rng, precision, scale):
     cells = g.nx * g.ny * g.nz
-    per = COUNTS[(np.arange(cells) * (3 + 2 * s) + s) % len(COUNTS)] // scale
+    per = (COUNTS[(np.arange(cells) * (3 + 2 * s) + s) % len(COUNTS)] / scale).astype(int)
     lin = np.repeat(np.arange(cells), per)
     n = len(lin)
     vt = np.float64 if precision == 0 else np.float32
@@ -133,3 +133,44 @@ def test_scalar_deposition_leaves_waiting_moments_alone(torch_cuda):
     jg, mg = j.cpu().numpy().astype(np.float64), ctx.records(m)
     assert np.abs(interior_nodes(g, jg) - interior_nodes(g, jw)).max() <= 1e-4 * np.abs(interior_nodes(g, jw)).max()
     assert np.abs(interior_records(g, mg) - interior_records(g, mw)).max() <= 1e-4 * np.abs(mw).max()
+
+
+@pytest.mark.parametrize("shape,per_cell", [((12, 12, 12), 48), ((16, 16, 16), 16), ((16, 16, 16), 1), ((21, 20, 20), 1)])
+@pytest.mark.parametrize("precision,kind", [(0, 0), (1, 0), (1, 1)])
+def test_both_sides_of_the_rule_agree(torch_cuda, shape, per_cell, precision, kind):
+    """With one record less than the rule asks for the cell-tile kernel runs (one launch), else the moments
+    (two): the same deposition within the sums' rounding."""
+    from gpu_helpers import StageContext
+    g = GridSpec(*shape, *(0.1 * n for n in shape))
+    cells = g.nx * g.ny * g.nz
+    rng = np.random.default_rng(per_cell)
+    ctx = StageContext(g, precision=precision, dt=0.2, mass_layout=1)
+    bn = ctx.field(periodic_node_field(g, smooth_random_unique(g, rng, 0.9)))
+    fp32 = precision == 1 and kind == 0
+    least = 48 if cells < 148 * 16 else 16 if fp32 and cells < 8192 else 1
+    vt = np.float64 if precision == 0 else np.float32
+    n = per_cell * cells
+    lin = np.arange(n) // per_cell
+    d = {k: rng.random(n) for k in ("rx", "ry", "rz")}
+    d.update({k: np.abs(0.2 * rng.normal(size=n)).astype(vt) for k in ("u", "v", "w")})
+    d["q"] = 1e-3 * (0.5 + rng.random(n))
+    d["cell"] = g.encode(lin % g.nx, (lin // g.nx) % g.ny, lin // (g.nx * g.ny)).astype(np.int32)
+    results = []
+    for count in (n, n - 1):
+        e = {k: v[:count] for k, v in d.items()}
+        if count == n:  # the last record deposits nothing, so that both calls deposit the same
+            e = {**e, "q": e["q"].copy()}
+            e["q"][-1] = 0.0
+        parts = ctx.upload_particles(e)
+        counts, offsets = bins(ctx, e)
+        j, m = ctx.moments()
+        before = ctx.lib.tpicb200_launch_count()
+        ctx.deposit(-1.0, parts, count, bn, j, m, counts, offsets, kind=kind)
+        assert ctx.lib.tpicb200_launch_count() - before == (2 if count >= least * cells else 1)
+        results.append((j.double(), m.double()))
+    assert ctx.invalid_count() == 0
+    # Sums of 8 cells' records, each term within a few roundings, of terms up to the largest entry's size.
+    rel = (8 * per_cell + 40) * (2.0**-53 if precision == 0 else 2.0**-24)
+    for a, b in zip(*results):
+        assert float((a - b).abs().max()) <= rel * float(b.abs().max())
+    ctx.close()

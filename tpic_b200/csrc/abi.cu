@@ -125,10 +125,26 @@ struct StoresMoments {
 };
 
 // The scalar forms deposit J and the mass of sorted records through the
-// context's moments too, assembled within the call; not while those hold
-// moments that wait for the fold.
-bool sums_by_moments(const tpicb200_context* ctx, const void* j, const void* mass) {
-  return j && mass && !ctx->moments_pending;
+// context's moments too, assembled within the call, where that is faster than the
+// sorted cell-tile kernel; not while the moments wait for the fold. The moments
+// cost a pass over all cells and their assembly, whatever the records, the
+// cell-tile kernel a launch a species and a warp's time a cell. Deposition of one
+// species, us, moments / cell tiles: 64^3 with 0.05, 0.5, 1 and 2 records a cell
+// 333 / 150, 380 / 309, 417 / 407 and 437 / 522 mixed, FP64 with 0.5 545 / 604; where
+// the cells are too few for a warp each on every SM, 1024 x 1 x 1 with 16, 64 and 128
+// 19.5 / 13.1, 21.4 / 20.4, 23.6 / 28.6 mixed and 19.5 / 14.5, 23.4 / 26.6, 27.6 /
+// 40.9 FP64, 8^3 the same; between, 16^3 with 1, 8 and 16 23.6 / 18.3, 25.4 / 22.4,
+// 25.4 / 24.5 mixed, FP64 with 1 25.6 / 28.5. Two species of a pair share the
+// moments' pass and their assembly.
+bool sums_by_moments(const tpicb200_context* ctx, int kind, int ns, unsigned long long records, const void* j,
+                     const void* mass) {
+  if (!j || !mass || ctx->moments_pending) return false;
+  const Geom& g = ctx->g;
+  const unsigned long long cells = (unsigned long long)g.nx * g.ny * g.nz;
+  if (ns > 1) return cells < 8192 || 2 * records >= cells;
+  const bool fp32 = ctx->opt.precision == TPICB200_PRECISION_MIXED && kind == TPICB200_MASS_SCALAR;
+  const unsigned long long least = cells < 148 * 16 ? 48 : fp32 && cells < 8192 ? 16 : 1;
+  return records >= least * cells;
 }
 int deposit_through_moments(tpicb200_context* ctx, int kind, int ns, const double* qom,
                             const tpicb200_particles* const* parts, const uint32_t* const* counts,
@@ -408,8 +424,8 @@ int tpicb200_deposit(tpicb200_context* ctx, double qom, const tpicb200_particles
     if (r == TPICB200_SUCCESS) ctx->moments_pending = true;
     return r;
   }
-  if (sums_by_moments(ctx, j, mass) && counts) return deposit_through_moments(ctx, mass_kind, 1, &qom, &p, &counts,
-                                                                              &offsets, b_node, j, mass, inv, s);
+  if (counts && sums_by_moments(ctx, mass_kind, 1, p->count, j, mass))
+    return deposit_through_moments(ctx, mass_kind, 1, &qom, &p, &counts, &offsets, b_node, j, mass, inv, s);
   ctx->stores = false;
   return cuda_status(launch_deposit(ctx->opt.precision, mass_kind, ctx->g, qom, ctx->opt.dt, ctx->opt.c, p,
                                     counts, offsets, b_node, j, mass, inv, s),
@@ -568,8 +584,13 @@ int tpicb200_deposit_species(tpicb200_context* ctx, int ns, const double* qom, c
   if (ns < 0 || ns > TPICB200_MAX_SPECIES || (ns > 0 && (!qom || !species || !counts || !offsets)))
     return fail(TPICB200_INVALID_ARGUMENT, "invalid species arrays");
   bool sorted = ns > 0;
-  for (int sp = 0; sp < ns; ++sp) sorted = sorted && counts[sp] && offsets[sp];
-  const bool through = !moment_form(mass_kind) && sorted && b_node && sums_by_moments(ctx, j, mass);
+  unsigned long long records = 0;
+  for (int sp = 0; sp < ns; ++sp) {
+    sorted = sorted && counts[sp] && offsets[sp];
+    records += species[sp].count;
+  }
+  const bool through =
+      !moment_form(mass_kind) && sorted && b_node && sums_by_moments(ctx, mass_kind, ns, records, j, mass);
   if (!moment_form(mass_kind) && !through) {
     for (int sp = 0; sp < ns; ++sp)
       if (int r = tpicb200_deposit(ctx, qom[sp], &species[sp], counts[sp], offsets[sp], b_node, j, mass, mass_kind,
