@@ -37,6 +37,7 @@ import pytest
 
 import oracle as O
 from fieldutil import periodic_cell_field, periodic_node_field
+from tpic_b200 import _lib
 from tpic_b200.plasma import Case, FieldInit, GridSpec, SpeciesSpec, generate_species
 
 pytestmark = pytest.mark.gpu
@@ -189,6 +190,50 @@ def test_stage_backwards_compose_to_the_cycle_backward(torch_cuda, precision, ma
         for k in ("x", "v", "q"):
             assert relative(x[k], y[k]) <= 1e-12, (s, k)
     sim.close()
+
+
+@pytest.mark.parametrize("order", ["near", "shuffled"])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_stage_backwards_in_any_record_order(torch_cuda, order, precision):
+    """The records' gradients are the same numbers in any order; a node's sums of m terms agree within m eps
+    of the sum of their magnitudes, for which the largest entry stands (positive fields and velocities)."""
+    import torch
+    from gpu_helpers import StageContext
+    g = GridSpec(7, 5, 3, 0.7, 0.5, 0.3)
+    rng = np.random.default_rng(4)
+    n = 3000
+    vt = np.float64 if precision == 0 else np.float32
+    d = {k: rng.random(n) for k in ("rx", "ry", "rz", "q")}
+    d.update({k: rng.random(n).astype(vt) for k in ("u", "v", "w")})
+    d["cell"] = np.sort(g.encode(*(rng.integers(0, m, n) for m in (g.nx, g.ny, g.nz)))).astype(np.int32)
+    d["id"] = np.arange(n, dtype=np.uint64)
+    at = rng.permutation(n) if order == "shuffled" else np.argsort(np.arange(n) + 60 * rng.random(n))
+    ctx = StageContext(g, precision=precision, dt=0.1)
+    field = lambda: ctx.field(periodic_node_field(g, 0.5 + rng.random((3, g.nz, g.ny, g.nx))), np.float64)
+    theta, jbar, left, right = (field() for _ in range(4))
+    bnode = field().to(ctx.fdt)
+    x0, v0, q0 = (torch.rand(k * n, dtype=torch.float64, device="cuda") for k in (3, 3, 1))
+    results = []
+    for records in (d, {k: v[at] for k, v in d.items()}):
+        parts = ctx.upload_particles(records)
+        p = ctx.struct(parts, n)
+        x, v, q = x0.clone(), v0.clone(), q0.clone()
+        ebar, bbar, bdep = (torch.zeros_like(theta) for _ in range(3))
+        _lib.check(ctx.lib.tpicb200_mover_backward(ctx.ctx, -1.0, C.byref(p), theta.data_ptr(), bnode.data_ptr(), n,
+                                                   x.data_ptr(), v.data_ptr(), ebar.data_ptr(), bbar.data_ptr(),
+                                                   ctx.invalid.data_ptr(), ctx.stream))
+        _lib.check(ctx.lib.tpicb200_deposit_backward(ctx.ctx, -1.0, C.byref(p), bnode.data_ptr(), jbar.data_ptr(), 1.0,
+                                                     left.data_ptr(), right.data_ptr(), 1.0, n, x.data_ptr(),
+                                                     v.data_ptr(), q.data_ptr(), bdep.data_ptr(),
+                                                     ctx.invalid.data_ptr(), ctx.stream))
+        results.append((x, v, q, ebar, bbar, bdep))
+    assert ctx.invalid_count() == 0
+    for k, (a, b) in enumerate(zip(*results)):
+        if k < 3:
+            assert torch.equal(a, b)
+        else:
+            assert float((a - b).abs().max()) <= n * 2.0**-52 * float(a.abs().max())
+    ctx.close()
 
 
 def test_backward_rejects_smoothing_and_missing_ids(torch_cuda):

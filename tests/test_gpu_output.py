@@ -62,7 +62,7 @@ def test_output_moments_and_particles_match_the_oracle(torch_cuda, precision):
 
 
 @pytest.mark.parametrize("count", [1, 31, 33, 700, 20000])
-@pytest.mark.parametrize("order", ["sorted", "shuffled"])
+@pytest.mark.parametrize("order", ["sorted", "near", "shuffled"])
 @pytest.mark.parametrize("wanted", ["rho", "rho+j", "j+p"])
 def test_output_moments_over_record_orders_and_counts(torch_cuda, count, order, wanted):
     """Chunks of 32 records and their remainders, several cells in a chunk and several chunks in a
@@ -76,8 +76,10 @@ def test_output_moments_over_record_orders_and_counts(torch_cuda, count, order, 
     rng = np.random.default_rng(count)
     c = [rng.integers(0, m, count) for m in (g.nx, g.ny, g.nz)]
     key = g.encode(*c).astype(np.int32)
-    if order == "sorted":
+    if order != "shuffled":
         key = np.sort(key)
+    if order == "near":  # more runs of equal keys in a chunk than cells
+        key = key[np.argsort(np.arange(count) + 5 * rng.random(count))]
     d = {k: rng.random(count) for k in ("rx", "ry", "rz")}
     d.update({k: rng.normal(size=count) for k in ("u", "v", "w")}, q=rng.random(count), cell=key)
     good = np.ones(count, bool)

@@ -92,14 +92,14 @@ struct MomentSink {
   }
 };
 
-template <class V, int N>
+template <class V, int N, int kMost>
 __global__ void __launch_bounds__(kMomentThreads) output_moments_kernel(Geom g, tpicb200_particles p,
                                                                       double inverse_volume, double inverse_qom,
                                                                       double rho_scale, double* __restrict__ rho,
                                                                       double* __restrict__ j,
                                                                       double* __restrict__ pressure,
                                                                       uint32_t* invalid) {
-  using Sums = CornerSums<N>;
+  using Sums = CornerSums<N, kMost>;
   __shared__ typename Sums::Stage stages[kMomentThreads / 32];
   typename Sums::Stage& stage = stages[threadIdx.x / 32];
   const uint32_t lane = threadIdx.x & 31u;
@@ -281,20 +281,25 @@ cudaError_t launch_output_moments(int precision, const Geom& g, const tpicb200_p
                                   double rho_scale, double* rho, double* j, double* pressure, uint32_t* invalid,
                                   cudaStream_t s) {
   if (p.count == 0) return cudaSuccess;
-  // One wave of resident blocks (three per SM by their shared memory and
-  // registers); fewer when a warp would get less than a chunk.
-  const unsigned blocks = grid_for(p.count, kMomentThreads, 148u * 3u);
-  auto go = [&](auto kernel) {
+  // One wave of resident blocks (by their shared memory and registers); fewer
+  // when a warp would get less than a chunk.
+  auto go = [&](auto kernel, unsigned per_sm) {
+    const unsigned blocks = grid_for(p.count, kMomentThreads, 148u * per_sm);
     kernel<<<blocks, kMomentThreads, 0, s>>>(g, p, g.inv_volume, 1.0 / qom, rho_scale, rho, j, pressure, invalid);
   };
+  // All ten by groups alone where a chunk of sorted records has at most some four
+  // cells: the look at their number costs sorted records 3 % there (33.6M on 64^3 987
+  // us, 1,017 with it) and gains less than elsewhere (8 a cell, near their place, 512
+  // / 490 us; 2 a cell 198 / 162).
+  const bool few = p.count < 8ull * g.nx * g.ny * g.nz;
   if (precision == TPICB200_PRECISION_DOUBLE) {
-    if (pressure) go(output_moments_kernel<double, 10>);
-    else if (j) go(output_moments_kernel<double, 4>);
-    else go(output_moments_kernel<double, 1>);
+    if (pressure) few ? go(output_moments_kernel<double, 10, 12>, 3) : go(output_moments_kernel<double, 10, 32>, 3);
+    else if (j) go(output_moments_kernel<double, 4, 8>, 4);
+    else go(output_moments_kernel<double, 1, 4>, 4);
   } else {
-    if (pressure) go(output_moments_kernel<float, 10>);
-    else if (j) go(output_moments_kernel<float, 4>);
-    else go(output_moments_kernel<float, 1>);
+    if (pressure) few ? go(output_moments_kernel<float, 10, 12>, 3) : go(output_moments_kernel<float, 10, 32>, 3);
+    else if (j) go(output_moments_kernel<float, 4, 8>, 4);
+    else go(output_moments_kernel<float, 1, 4>, 4);
   }
   count_launches(1);
   return cudaGetLastError();
