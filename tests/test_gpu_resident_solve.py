@@ -9,9 +9,9 @@ applies (per-thread loads, and mass boxes by TMA on the tiled layout) form
 every sum in the same order: bit for bit.
 
 Grids: one cell and two per axis (every neighbour a periodic copy), partial
-tiles on each axis, lines, planes and boxes, a tile of every size (1 to 8
-threads a node), bases in shared memory and out of it, and one grid too large
-for the resident kernels.
+tiles on each axis, lines, planes and boxes, tiles of every size (1 to 256
+threads a node), bases in shared memory and out of it, one to three tiles a CTA,
+and grids too large for the resident kernels.
 """
 from __future__ import annotations
 
@@ -26,7 +26,7 @@ from test_gpu_tiled_apply import random_mass
 pytestmark = pytest.mark.gpu
 
 SHAPES = [(1, 1, 1), (2, 1, 1), (3, 2, 1), (2, 2, 2), (33, 1, 1), (200, 1, 1), (1, 70, 1), (31, 9, 1), (40, 24, 1),
-          (150, 90, 1), (256, 130, 1), (5, 6, 7), (17, 16, 15), (33, 20, 18), (30, 40, 26), (48, 44, 40)]
+          (150, 90, 1), (256, 130, 1), (5, 6, 7), (17, 16, 15), (33, 20, 18), (30, 40, 26), (48, 44, 40), (64, 38, 63)]
 
 
 def solve(ctx, inputs, adjoint):

@@ -1020,6 +1020,43 @@ bool allow_shared(void (*const (&kernels)[2])(ResidentPlan), int limit) {
   return true;
 }
 
+// Whether the mass rows of this layout can be fetched by the step graph's TMA apply.
+template <class M>
+bool tma_rows(const Geom& g) {
+  return g.mvs == 1 && g.MX * sizeof(M) % 16 == 0 && g.mes * sizeof(M) % 16 == 0;
+}
+
+// The percentage of the CTAs' tiles that must be in use for several tiles a CTA to
+// be at least as fast as the step graph (101: never). A tile that is not used is
+// time of all the others at the barriers; what it competes with depends on how the
+// step graph reads the mass. Resident / step graph, us a solve, by share in use:
+//   boxes, tiles less than 16 wide, whose mass rows are part lines: 56^3 FP64 (77 %)
+//     1,731 / 1,528, 72 x 56 x 64 (85 %) 2,321 / 2,292, mixed 56 x 48 x 40 (71 %) 1,065 / 956;
+//     FP64 40 x 40 x 48 two a CTA (51 %) 1,101 / 1,297
+//   FP64 boxes, stencil-major: 48 x 40 x 44 (56 %) 984 / 1,006, 64 x 56 x 48 three a CTA
+//     (76 %) 1,369 / 1,515, 60^3 four (76 %) 1,801 / 1,907, 64^3 (86 %) 1,787 / 2,004
+//   FP64 boxes against the TMA apply: 44^3 (61 %) 982 / 1,022, 64 x 52 x 56 three (82 %)
+//     1,457 / 1,457, four: 60^3 (76 %) 1,788 / 1,672, 64^3 (86 %) 1,799 / 1,789, 64 x 72 x 64
+//     (97 %) 1,824 / 1,878
+//   mixed boxes, two a CTA, stencil-major: 48 x 40 x 44 (56 %) 847 / 805, 48 x 48 x 40 (61 %)
+//     848 / 909, 48 x 48 x 64 (97 %) 967 / 1,230; against the TMA apply (81 %) 876 / 850, (97 %)
+//     975 / 1,070; three: 64 x 48 x 60 (81 %) 1,346 / 1,292, four: 64^3 1,693 / 1,508
+//   flat FP64: 700 x 330 (78 %) 1,989 / 2,940, TMA 1,974 / 2,433; flat mixed: 1,847 / 2,032;
+//     TMA, two: 300 x 300 (61 %) 902 / 938, three and four: 500 x 300 (68 %) 1,381 / 1,291,
+//     600 x 400 (80 %) 1,836 / 1,789, 512^2 (86 %) 1,808 / 1,853
+//   records layout: mixed 300 x 300 (61 %) 3,226 / 3,111, 400 x 300 (80 %) 3,529 / 3,849, 700 x 330
+//     (78 %) 6,563 / 6,077, boxes 64 x 40 x 40 (68 %) 3,125 / 2,722, 96 x 32 x 40 (81 %) 3,252 / 3,405;
+//     FP64 flat (78 %) 6,874 / 7,016, boxes 64 x 52 x 56 (82 %) 4,800 / 4,714, 64 x 64 x 48
+//     (86 %) 4,687 / 4,862.
+template <class EC>
+int resident_fill(const Geom& g, const ResidentPlan& p) {
+  const bool fp64 = sizeof(EC) == 8, flat = g.nz == 1, records = g.mes == 1, tma = tma_rows<EC>(g);
+  if (flat) return fp64 ? 0 : records ? 80 : tma ? (p.slots == 2 ? 60 : 85) : 0;
+  if (p.tx < 16) return fp64 && p.slots == 2 && !tma && !records ? 0 : 101;
+  if (fp64) return records ? 85 : tma && p.slots > 3 ? 90 : 0;
+  return p.slots > 2 ? 101 : tma ? 90 : records ? 80 : 60;
+}
+
 // Tiles of the resident kernels: the smallest tile whose CTAs are all
 // resident at once, so that every SM has nodes and a node has many threads,
 // but one CTA an SM where a tile has at least two threads a node: its shared
@@ -1029,7 +1066,9 @@ bool allow_shared(void (*const (&kernels)[2])(ResidentPlan), int limit) {
 // Solves, us, one CTA an SM first / the smallest tile first: 1024 x 1 x 1
 // 1,281 / 1,514 mixed, 1,301 / 1,547 FP64; 96 x 96 x 1 235 / 279, 200 / 240;
 // 128 x 128 x 1 255 / 276, 227 / 250; 24^3 237 / 264 mixed, 245 / 245 FP64;
-// but 20^3 FP64 229 / 218, so FP64 boxes take the smallest tile. The basis is
+// but FP64 boxes, whose tiles hold as many bytes again, gain nothing on the whole:
+// 14 x 15 x 16 196 / 190, 20^3 269 / 257, 24^3 291 / 285, 40 x 12 x 24 278 / 286, 28 x 20 x 24
+// 266 / 289; they take the smallest tile. The basis is
 // in shared memory where that tile leaves room for it (FP64 256 x
 // 128 x 1: 325 us a solve with tiles of 128 nodes and the basis in global
 // memory, 410 us with 256 and the basis in shared memory). Resident against
@@ -1093,14 +1132,8 @@ void resident_tiles(const SolverWorkspace* w, Take&& take) {
     // lost more in threads per node than the barrier costs (1024 x 1 x 1 1.55
     // against 1.51 ms, 12^3 0.29 against 0.19).
     p.cluster = p.tiles <= kResidentCluster;
-    // Several tiles a CTA only with the largest tile, the basis then in global
-    // memory: up to four on flat grids and two on boxes, in FP64 up to four
-    // there too when at least 85 % of the CTAs' tiles are used. Beyond, the
-    // step graph's applies stream the mass better. Resident / step graph (its
-    // TMA apply on the tiled layout), ms a solve: 512 x 512 x 1 mixed 1.81 /
-    // 2.18 (1.87), FP64 1.83 / 2.93 (2.44); 48^3 0.75 / 0.84 (0.75) and 0.86 /
-    // 1.19 (0.94); 64^3 FP64 1.53 / 1.72 (1.55), mixed 1.48 / 1.31 (1.17);
-    // 56^3 FP64 (77 % of three tiles a CTA) 1.48 / 1.34 (1.26).
+    // Several tiles a CTA (up to four) only with the largest tile, the basis then
+    // in global memory, where resident_fill says that it pays.
     const int slots = nodes == kResidentNodeThreads && smooth == 0 ? 4 : 1;
     for (int choice = 0; choice <= slots; ++choice) {
       p.shared_basis = choice == 0;
@@ -1110,9 +1143,7 @@ void resident_tiles(const SolverWorkspace* w, Take&& take) {
       if (bytes > size_t(limit)) continue;
       const int ctas = grid <= sms ? 1 : 2;
       if (alone ? ctas == 2 : grid > 2 * sms) continue;
-      if (p.slots > 2 && g.nz > 1 &&
-          (sizeof(typename P::EC) == 4 || 100LL * p.tiles < 85LL * p.slots * ctas * sms))
-        break;
+      if (p.slots > 1 && 100LL * p.tiles < resident_fill<typename P::EC>(g, p) * 1LL * p.slots * ctas * sms) break;
       if (!take(p, grid, ctas, bytes)) return;
     }
   }
