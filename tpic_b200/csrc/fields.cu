@@ -374,7 +374,11 @@ cudaError_t launch_smooth_typed(const Geom& g, int niter, int op, double alpha, 
     return cudaGetLastError();
   }
   // Passes a launch: as many as a halo is worth, split evenly.
-  const int most = 8, launches = (niter + most - 1) / most;
+  // Two axes of the tile with eight passes' halo fit a kernel's default shared
+  // memory (a raised limit would be one for all contexts).
+  constexpr int most = 8;
+  static_assert(2 * (32 + 2 * most) * (8 + 2 * most) * sizeof(C) <= 48 * 1024, "the tile and its copy");
+  const int launches = (niter + most - 1) / most;
   const int tx = 32, ty = g.ny == 1 ? 1 : 8, tz = g.nz == 1 ? 1 : 8;
   const long long tiles = (long long)((g.nx + tx - 1) / tx) * ((g.ny + ty - 1) / ty) * ((g.nz + tz - 1) / tz);
   if (tiles > 0x7fffffffLL) return cudaErrorInvalidValue;
@@ -384,9 +388,6 @@ cudaError_t launch_smooth_typed(const Geom& g, int niter, int op, double alpha, 
     done += passes;
     const SmoothTile t(g.nx, g.ny, g.nz, tx, ty, tz, passes);
     const size_t bytes = size_t(2) * t.size * sizeof(C);
-    const cudaError_t e =
-        cudaFuncSetAttribute(smooth_tile_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
-    if (e != cudaSuccess) return e;
     double* to = (launches - l) % 2 == 1 ? out : tmp;
     smooth_tile_kernel<C><<<dim3(unsigned(tiles), 3), kSmoothThreads, bytes, s>>>(g, t, tx, ty, tz, passes, op, alpha, src, to,
                                                                          invalid);
