@@ -26,7 +26,8 @@ from test_gpu_tiled_apply import random_mass
 pytestmark = pytest.mark.gpu
 
 SHAPES = [(1, 1, 1), (2, 1, 1), (3, 2, 1), (2, 2, 2), (33, 1, 1), (200, 1, 1), (1, 70, 1), (31, 9, 1), (40, 24, 1),
-          (150, 90, 1), (256, 130, 1), (5, 6, 7), (17, 16, 15), (33, 20, 18), (30, 40, 26), (48, 44, 40), (64, 38, 63)]
+          (150, 90, 1), (256, 130, 1), (5, 6, 7), (17, 16, 15), (33, 20, 18), (30, 40, 26), (48, 44, 40), (48, 48, 44),
+          (64, 38, 63)]
 
 
 def solve(ctx, inputs, adjoint):
