@@ -295,6 +295,14 @@ __device__ __forceinline__ T block_sum(T v, T* scratch /* Threads/32 */) {
   return total;
 }
 
+// D (8 x 8) += A (8 x 4) B (4 x 8) in FP64 on the tensor cores. Per lane:
+// A[lane >> 2][lane & 3], B[lane & 3][lane >> 2], D[lane >> 2][2 (lane & 3) + i].
+__device__ __forceinline__ void dmma_884(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
+}
+
 inline unsigned grid_for(long long n, int threads, unsigned cap = 148u * 16u) {
   long long b = (n + threads - 1) / threads;
   if (b < 1) b = 1;

@@ -23,14 +23,6 @@
 
 namespace tpicb200 {
 
-// D += A B for A 8x4 (row-major), B 4x8: a = A[lane/4][lane%4],
-// b = B[lane%4][lane/4], c = D[lane/4][2*(lane%4) + {0, 1}].
-__device__ __forceinline__ void corner_mma(double& c0, double& c1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-      : "+d"(c0), "+d"(c1)
-      : "d"(a), "d"(b));
-}
-
 template <int N, int kMost>
 struct CornerSums {
   static constexpr int kTiles = (N + 7) / 8;
@@ -132,7 +124,7 @@ struct CornerSums {
 #pragma unroll
         for (int t = 0; t < kTiles; ++t) {
           const int n = 8 * t + row;
-          corner_mma(c[t][0], c[t][1], a, member && n < N ? s.value[n < N ? n : 0][r] : 0.0);
+          dmma_884(c[t], a, member && n < N ? s.value[n < N ? n : 0][r] : 0.0);
         }
       }
     }

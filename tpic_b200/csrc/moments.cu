@@ -384,15 +384,6 @@ __global__ void __launch_bounds__(kF32Warps * 32, 4) moments_f32_kernel(Geom g, 
 // loads per 12 fused multiply-adds) was bound by the shared-memory pipe (93 %
 // of its wavefronts at 64^3); the fragments need 6 shared loads per 4 records
 // and lane (128^3-cell workload: the FP64 deposit stage 20.0 -> 16.1 ms).
-//
-// D (8 x 8) += A (8 x 4) B (4 x 8) in FP64 on the tensor cores. Per lane:
-// A[lane >> 2][lane & 3], B[lane & 3][lane >> 2], D[lane >> 2][2 (lane & 3) + i].
-__device__ __forceinline__ void dmma_884(double (&d)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
-}
-
 constexpr int kF64Warps = 4;
 // The products and values are stored by (t or entry, record), 36 records a
 // row: a lane's stores of its record fall in consecutive words, and the 16
