@@ -323,11 +323,12 @@ int tpicb200_set_wait_limit(tpicb200_context* ctx, uint32_t polls);
  * of chunk index - 1 (index >= 1), with TPICB200_STALL_APPLY the TMA apply's
  * wait for the mass box of stencil `index` (0..13) waits instead on an
  * mbarrier that nothing arrives on, so it gives up at its bound and takes
- * the recovery path above. With TPICB200_STALL_PLAN, TPICB200_STALL_SORT and
- * TPICB200_STALL_SOLVE wait number `index` (>= 1) of the first CTA at the grid
- * barrier of the binned sort's plan, of its general sort and of the resident
- * solve's kernels is for more CTAs than there are; those waits then have the
- * bound of tpicb200_set_wait_limit. TPICB200_STALL_NONE turns it off. */
+ * the recovery path above. With TPICB200_STALL_PLAN and TPICB200_STALL_SORT wait
+ * number `index` (>= 1) of the first CTA at the grid barrier of the binned sort's
+ * plan and of its general sort is for more CTAs than there are; with
+ * TPICB200_STALL_SOLVE the first wait of a resident solve's launch `index` (1: the
+ * start, then one a restart cycle). Those kernels' waits then have the bound of
+ * tpicb200_set_wait_limit. TPICB200_STALL_NONE turns it off. */
 enum {
   TPICB200_STALL_NONE = 0,
   TPICB200_STALL_DEPOSIT = 1,

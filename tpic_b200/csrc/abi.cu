@@ -859,7 +859,7 @@ int tpicb200_inject_stall(tpicb200_context* ctx, int site, uint32_t index) {
   } else if (site == TPICB200_STALL_APPLY) {
     if (index > 13) return fail(TPICB200_INVALID_ARGUMENT, "the apply stall index is a stencil 0..13");
   } else if (site == TPICB200_STALL_PLAN || site == TPICB200_STALL_SORT || site == TPICB200_STALL_SOLVE) {
-    if (index < 1) return fail(TPICB200_INVALID_ARGUMENT, "the barrier stall index is a wait >= 1");
+    if (index < 1) return fail(TPICB200_INVALID_ARGUMENT, "the barrier stall index counts from 1");
   } else {
     return fail(TPICB200_INVALID_ARGUMENT, "unknown stall site");
   }

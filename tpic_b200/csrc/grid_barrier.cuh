@@ -1,11 +1,13 @@
 // A barrier over all CTAs of a cooperative launch, with bounded waits.
 //
 // Two words, zero between launches: arrivals, and departures with those of
-// CTAs that gave up counted in the upper half. A CTA whose polls run out reports false to its threads, which go to
-// leave(); the others then run out at their next wait. Every CTA leaves, and the
-// last one to do so zeroes the words, so a launch that failed spoils none after
-// it; that CTA also learns of the failure and can put the outputs in order, all
-// the other CTAs' writes being done.
+// CTAs that gave up counted in the upper half. A CTA whose polls run out reports
+// false to its threads, which do no more work; the others then run out at their
+// next wait. Where every CTA departs on every way out, the last one to do so zeroes
+// the words, so a launch that failed spoils none after it; that CTA also learns of
+// the failure and, by leave(), can put the outputs in order, all the other CTAs'
+// writes being done. A kernel whose host reads of the failure may end without
+// departing: the host then clears the words.
 #pragma once
 
 #include "common.cuh"
@@ -27,6 +29,8 @@ __device__ __forceinline__ uint32_t load_acquire(const unsigned* p) {
   return v;
 }
 
+// kStall: the waits look at the stall.
+template <bool kStall>
 struct GridBarrier {
   static constexpr uint32_t kFailed = 1u << 16;  // above any number of CTAs resident at once
   unsigned* words;
@@ -40,8 +44,8 @@ struct GridBarrier {
     __syncthreads();
     if (threadIdx.x == 0) {
       arrivals += gridDim.x;
-      ++number;
-      const uint32_t expected = number == waits.stall && blockIdx.x == 0 ? 0xffffffffu : arrivals;
+      uint32_t expected = arrivals;
+      if (kStall && ++number == waits.stall && blockIdx.x == 0) expected = 0xffffffffu;
       // The CTA's writes are ordered before the arrival (the barrier above and
       // the release), the others' before what follows the acquire.
       asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(words) : "memory");

@@ -257,9 +257,8 @@ int solver_solve_adjoint(SolverWorkspace* w, const double* rhs, const void* mass
 void solver_set_invalid(SolverWorkspace* w, uint32_t* invalid);
 // Bound of the TMA apply's copy waits (0: kDefaultWaitPolls); stall_stencil
 // in 0..13 makes the wait for that stencil's box wait on an mbarrier that
-// nothing arrives on (a test of the bound), -1 none. stall_barrier: the wait of
-// the resident kernels' grid barrier that is to give up, at the bound `polls`
-// (0: none).
+// nothing arrives on (a test of the bound), -1 none. stall_barrier: the launch of
+// a resident solve whose grid barrier is to give up, at the bound `polls` (0: none).
 void solver_set_waits(SolverWorkspace* w, uint32_t polls, int stall_stencil, uint32_t stall_barrier);
 int solver_solve(SolverWorkspace* w, const void* e, const void* bcell, const void* j,
                  const void* mass, double* etheta, tpicb200_gmres_result* result,

@@ -88,7 +88,7 @@ struct ResidentPlan {
   double* partials;        // kResidentRestart + 2 rows of gridDim.x
   ArnoldiControl* ctl;
   unsigned* barrier;       // kGridBarrierWords
-  GridWaits waits;
+  uint32_t polls;          // of its waits
   int restart, columns;
   double tolerance;        // of this cycle's residual estimate
   double accept;           // start: the relative tolerance; cycle: the absolute one
@@ -154,10 +154,10 @@ struct Resident {
   const ResidentPlan& p;
   uint8_t* smem;
   const ResidentShared L;
-  GridBarrier barrier;
+  GridBarrier<false> barrier;
 
   __device__ Resident(const ResidentPlan& plan, uint8_t* s)
-      : p(plan), smem(s), L(resident_shared(plan, sizeof(S))), barrier(plan.barrier, plan.waits) {}
+      : p(plan), smem(s), L(resident_shared(plan, sizeof(S))), barrier(plan.barrier, GridWaits{plan.polls, 0}) {}
 
   template <class T> __device__ __forceinline__ T* at(size_t offset) const { return reinterpret_cast<T*>(smem + offset); }
   __device__ __forceinline__ long long unique() const { return (long long)p.g.nx * p.g.ny * p.g.nz; }
@@ -176,17 +176,14 @@ struct Resident {
   }
 
   // All CTAs of the grid. False when it gave up (for every thread of the CTA),
-  // which has then left and ends.
+  // which then ends; the host, which reads ctl->failed, clears the words.
   __device__ bool grid_barrier() {
     if (p.cluster) {
       asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
       return true;
     }
     if (barrier.wait()) return true;
-    if (threadIdx.x == 0) {
-      p.ctl->failed = 1;
-      barrier.depart();
-    }
+    if (threadIdx.x == 0) p.ctl->failed = 1;
     return false;
   }
   __device__ void leave() {

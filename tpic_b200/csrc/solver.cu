@@ -886,7 +886,7 @@ struct SolverWorkspace {
   bool transpose = false;       // applies use A^T (every mass block transposed): the adjoint solve
   uint32_t* invalid = nullptr;  // the context's invalid counter (smoothing passes, TMA apply waits)
   uint32_t wait_polls = 0;      // TMA apply wait bound (0: kDefaultWaitPolls)
-  uint32_t stall_barrier = 0;   // the same for the resident kernels' grid barrier
+  uint32_t stall_barrier = 0;   // the same for the grid barrier: the resident launch of a solve (0: none)
   int stall_stencil = -1;       // a test of that bound: the stencil whose wait targets no copy
   Geom g;
   int restart;
@@ -1662,10 +1662,16 @@ struct Solve {
   // restart cycle. Not while a wait bound or an apply's stall is set: those act on
   // the applies of the step graph; with a stall of the barriers the bound is theirs.
   bool resident() const { return w->resident && (w->stall_barrier || w->wait_polls == 0) && w->stall_stencil < 0; }
+  uint32_t resident_launches = 0;  // of this solve
   // Launches one of them and reads its outcome back; false on a failure.
   bool launch_resident(typename ResidentKernels<P>::Kernel kernel, double controls[2], ArnoldiControl* control) {
     ResidentPlan p = w->plan;
     void* args[] = {&p};
+    // A test of the barriers' bound: this launch's arrivals start one short, so
+    // that its first wait gives up. (A wait number in the kernels, as the sort's
+    // have, made a step of 1024 x 1 x 1 1.5 % longer.)
+    if (err == cudaSuccess && ++resident_launches == w->stall_barrier)
+      err = cudaMemsetAsync(w->resident_barrier, 0xff, sizeof(unsigned), s);
     if (err == cudaSuccess && p.cluster) {
       const ClusterLaunch launch(w->resident_grid, w->resident_bytes, s);
       err = cudaLaunchKernelExC(&launch.config, (const void*)kernel, args);
@@ -1676,8 +1682,9 @@ struct Solve {
     count_launches(1);
     if (!read_back(w->values, controls, control)) return false;
     if (control->failed) {
-      // A barrier ran out of polls; its words are clear again (GridBarrier).
+      // A barrier ran out of polls: the next solve starts from clear counters.
       cudaMemsetAsync(w->ctl, 0, sizeof(ArnoldiControl), s);
+      cudaMemsetAsync(w->resident_barrier, 0, kGridBarrierWords * sizeof(unsigned), s);
       err = cudaErrorLaunchTimeout;
       return false;
     }
@@ -1697,7 +1704,7 @@ struct Solve {
     p.partials = w->resident_partials;
     p.ctl = w->ctl;
     p.barrier = w->resident_barrier;
-    p.waits = GridWaits{w->wait_polls ? w->wait_polls : kGridBarrierPolls, w->stall_barrier};
+    p.polls = w->wait_polls ? w->wait_polls : kGridBarrierPolls;
     p.e = e;
     p.bcell = bcell;
     p.j = j;

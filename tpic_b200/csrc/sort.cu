@@ -26,6 +26,8 @@
 namespace tpicb200 {
 namespace {
 
+using CoopBarrier = GridBarrier<true>;
+
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 16;
 constexpr int kScanTile = kScanThreads * kScanItems;
@@ -334,7 +336,7 @@ __device__ __forceinline__ void fixup_large(const uint32_t* counts, const uint32
 // False when a barrier gave up.
 __device__ __forceinline__ bool fixup_huge(const uint32_t* counts, const uint32_t* offsets, uint32_t* perm,
                                            uint32_t* scratch, uint32_t nhuge, const uint32_t* last,
-                                           uint32_t* s, GridBarrier& barrier) {
+                                           uint32_t* s, CoopBarrier& barrier) {
   constexpr uint32_t kRun = kBlockBinCapacity;
   uint32_t longest = 0, run = 0;
   for (uint32_t h = 0; h < nhuge; ++h) {
@@ -561,7 +563,7 @@ __device__ __forceinline__ void coop_scan(const uint32_t* counts, long long bins
 template <class Vel>
 __device__ __forceinline__ void fallback_sort(const Geom& g, uint32_t n, const SortRecords<Vel>& r, uint32_t* counts,
                                               uint32_t* offsets, uint32_t* cursor, uint32_t* perm,
-                                              const ScanScratch& sc, uint32_t* invalid, GridBarrier& barrier,
+                                              const ScanScratch& sc, uint32_t* invalid, CoopBarrier& barrier,
                                               uint32_t* buffer, uint32_t* scratch) {
   uint32_t* sums = sc.large_bins;  // free until the fix-up
   constexpr int kThreads = kFallbackThreads;
@@ -615,17 +617,17 @@ __global__ void __launch_bounds__(kFallbackThreads, 1)
   __shared__ uint32_t buffer[kBlockBinCapacity];
   __shared__ uint32_t scratch[kFallbackThreads / 32];
   if (state->fallback == 0) return;
-  GridBarrier barrier(state->barrier, waits);
+  CoopBarrier barrier(state->barrier, waits);
   fallback_sort(g, n, r, counts, offsets, cursor, perm, sc, invalid, barrier, buffer, scratch);
-  const GridBarrier::Exit exit = barrier.leave();
-  if (exit == GridBarrier::kLastOfFailed) {
+  const CoopBarrier::Exit exit = barrier.leave();
+  if (exit == CoopBarrier::kLastOfFailed) {
     for (long long b = threadIdx.x; b <= g.bins; b += kFallbackThreads) {
       if (b < g.bins) counts[b] = 0;
       offsets[b] = 0;
     }
     if (threadIdx.x == 0 && invalid) atomicAdd(invalid, 1u << 22);
   }
-  if (exit != GridBarrier::kOther && threadIdx.x == 0) state->fallback = state->bins_bad = 0;
+  if (exit != CoopBarrier::kOther && threadIdx.x == 0) state->fallback = state->bins_bad = 0;
 }
 
 template <class Vel>
@@ -885,7 +887,7 @@ __device__ __forceinline__ void binned_bases(const Geom& g, const uint32_t* offs
 
 // The plan by all CTAs; returns early where a barrier gives up.
 __device__ __forceinline__ void binned_plan(const Geom& g, uint32_t* transfer, uint32_t* counts, uint32_t* offsets,
-                                            uint32_t* sums, GridBarrier& barrier, uint32_t* scratch) {
+                                            uint32_t* sums, CoopBarrier& barrier, uint32_t* scratch) {
   long long b0, b1;
   coop_range(g.bins, b0, b1);
   uint32_t sum = 0;
@@ -912,9 +914,9 @@ __global__ void __launch_bounds__(kCoopThreads, 2) binned_plan_kernel(Geom g, ui
                                                                       BinnedState* state, GridWaits waits) {
   __shared__ uint32_t scratch[kCoopThreads / 32];
   if (state->fallback) return;
-  GridBarrier barrier(state->barrier, waits);
+  CoopBarrier barrier(state->barrier, waits);
   binned_plan(g, transfer, counts, offsets, sums, barrier, scratch);
-  if (threadIdx.x == 0 && barrier.depart() == GridBarrier::kLastOfFailed) state->fallback = 1;
+  if (threadIdx.x == 0 && barrier.depart() == CoopBarrier::kLastOfFailed) state->fallback = 1;
 }
 
 // The lane mask of a live lane's slot: the live lanes with the same slot
