@@ -225,9 +225,9 @@ __device__ __forceinline__ void fixup_small(const uint32_t* counts, const uint32
                                             uint32_t* huge_count, uint32_t (*buffer)[kWarpBinCapacity]) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t* s = buffer[warp];
-  const int block_warps = blockDim.x / 32;
-  const long long warps = (long long)gridDim.x * block_warps;
-  for (long long bin = (long long)blockIdx.x * block_warps + warp; bin < bins; bin += warps) {
+  // Neighbouring bins to different blocks: the cells of a line are neighbours.
+  const long long warps = (long long)gridDim.x * (blockDim.x / 32);
+  for (long long bin = (long long)gridDim.x * warp + blockIdx.x; bin < bins; bin += warps) {
     const uint32_t n = counts[bin];
     if (n <= 1) continue;
     if (n > (uint32_t)kWarpBinCapacity) {
