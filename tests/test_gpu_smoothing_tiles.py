@@ -2,7 +2,8 @@
 oracle bit for bit, ghosts and duplicates included, where tiles, halos and
 launches meet the grid: axes of one to three cells (a halo wraps several
 times), partial tiles, exact tiles, flat grids and boxes, pass counts on both
-sides of what one launch takes (8 passes flat, 3 else)."""
+sides of what one launch takes (8 passes, one on grids thicker than a cell on
+every axis)."""
 from __future__ import annotations
 
 import ctypes as C

@@ -1,8 +1,8 @@
-"""The binned sort's cooperative kernels: the plan (counts, scan, bases) on both
-sides of the grid size that chooses it, and the fallback sort, on one context
+"""The binned sort's cooperative kernels: the plan (counts, scan, bases) on grids
+of one CTA to several tiles of the scan a CTA, and the fallback sort, on one context
 one after the other (each must leave the flags and the barrier as it found
 them): neighbour moves, far moves, bins that do not describe the records, an
-invalid key, bins of one record to more than a block sorts in shared memory;
+invalid key, bins of one record to several merge passes of all CTAs;
 and both recorded in a CUDA graph. Against a stable sort on the host, bit for
 bit."""
 from __future__ import annotations
