@@ -232,8 +232,8 @@ __device__ __forceinline__ void fixup_small(const uint32_t* counts, const uint32
     if (n <= 1) continue;
     if (n > (uint32_t)kWarpBinCapacity) {
       if (lane == 0) {
-        if (huge_count && n > (uint32_t)kBlockBinCapacity) large_bins[bins - 1 - atomicAdd(huge_count, 1u)] = (uint32_t)bin;
-        else large_bins[atomicAdd(large_count, 1u)] = (uint32_t)bin;
+        const bool huge = huge_count && n > (uint32_t)kBlockBinCapacity;
+        large_bins[huge ? bins - 1 - atomicAdd(huge_count, 1u) : (long long)atomicAdd(large_count, 1u)] = (uint32_t)bin;
       }
       continue;
     }
@@ -287,7 +287,8 @@ __device__ __forceinline__ void block_sort(uint32_t* p, uint32_t n, uint32_t* s)
 // output d).
 __device__ __forceinline__ uint32_t merged(const uint32_t* src, uint32_t n, uint32_t width, uint32_t t) {
   const uint32_t run = uint32_t(t / (2ull * width) * (2ull * width));
-  const uint32_t a0 = run, a1 = min(uint32_t(n - run), width) + run, b1 = uint32_t(min(run + 2ull * width, (unsigned long long)n));
+  const uint32_t a0 = run, a1 = min(n - run, width) + run;
+  const uint32_t b1 = uint32_t(min(run + 2ull * width, (unsigned long long)n));
   const uint32_t la = a1 - a0, lb = b1 - a1, d = t - run;
   uint32_t lo = d > lb ? d - lb : 0, hi = d < la ? d : la;
   while (lo < hi) {
